@@ -435,3 +435,32 @@ def test_rotated_row_quantizer_both_kernels(cols):
     q, s = K.quant_row(w.to(DEV), L.QMODE_TRITON, 128)
     q_ref, s_ref = R.quant_token(R.hadamard(w, 128))
     _same(q, q_ref, "rotated row int8"); _same(s, s_ref.view(-1), "rotated row scale")
+
+
+@pytest.mark.parametrize("kb,n,values,decade", [
+    (1, 256, "random", 0), (2, 384, "random", 0), (3, 128, "random", 30), (5, 256, "random", -30), (6, 640, "random", 0),
+    (7, 256, "lowest", 0), (4, 256, "opposite", 0), (257, 128, "random", 0)])
+def test_fast_block_epilogue_shift(kb, n, values, decade):
+    """The tensor core adds 32 * 255^2 to every partial product so that its bits are a float: the extreme int8
+    operands (all products 128 * 128, all -128 * 127), numbers of K blocks around the group of four after which
+    the shift is taken out and around the 256 staged at a time, partial tiles, and factors far from one.
+    Bound: an fp32 operation on a value up to |sum| + two shifts rounds by 2^-24 of it; one per K block, one per
+    four for the correction, three at the end."""
+    g = torch.Generator().manual_seed(100 + kb)
+    M, Kd = 128, 128 * kb
+    aq, bq = _randq(g, 1, M, Kd), _randq(g, n, Kd)
+    if values == "lowest":
+        aq.fill_(-128), bq.fill_(-128)
+    elif values == "opposite":
+        aq.fill_(-128), bq.fill_(127)
+    a_s = (torch.rand(1, 1, kb, generator=g) + 0.5) * 10.0 ** decade
+    b_t = torch.rand(n // 128, kb, generator=g) + 0.5
+    P = torch.stack([R.int_mm(aq[0, :, k * 128:(k + 1) * 128], bq[:, k * 128:(k + 1) * 128]) for k in range(kb)]).double()
+    for b_s, kind in ((torch.rand(n, generator=g) + 0.5, L.BSCALE_CHANNEL), (b_t, L.BSCALE_TILE)):
+        f = a_s[0, 0].double().view(-1, 1, 1)
+        f = f * (b_s.double().view(1, 1, n) if kind == L.BSCALE_CHANNEL else b_s.double().t().repeat_interleave(128, 1).view(kb, 1, n))
+        ref = (P * f).sum(0)
+        bound = (1.25 * kb + 3) * 2.0 ** -24 * ((P * f).abs().sum(0) + 2 * 2080800 * f.max()) + 2.0 ** -23 * (P * f).abs().sum(0)
+        out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), b_kind=kind, flags=L.GEMM_OUT_F32)[0].cpu().double()
+        assert ((out - ref).abs() <= bound).all(), float(((out - ref).abs() / bound).max())
+    K.check_status(DEV)

@@ -1,20 +1,22 @@
 // INT8 GEMMs on the 5th-generation tensor cores: tcgen05.mma kind::i8 with int32 accumulators in
 // tensor memory, operands staged by TMA into a 128B-swizzled shared-memory ring.
 //
-// One persistent CTA per SM, 640 threads:
+// One persistent CTA per SM, 384 threads (fast block-scaled kind) or 640 (the others):
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      tensor-memory allocator + MMA issuer (one elected lane)
 //   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the signed per-K-block
 //               factors and the column scales the epilogue needs; idle in the other kinds
 //   warp 3      idle (completes the first warpgroup so register budgets can be rebalanced)
-//   warps 4-19  epilogue: warp%4 selects the 32 accumulator lanes (rows) a warp may read, the
-//               group of four warps selects 64 of the 256 columns of the 128x256 tile.  Sixteen
-//               warps (four per scheduler) because the per-K-block drain is bound by instruction
-//               latency, not by a pipe: more resident warps hide it.
+//   warps 4-    epilogue: warp%4 selects the 32 accumulator lanes (rows) a warp may read, the group of
+//               four warps a share of the 256 columns of the 128x256 tile.  Sixteen warps with 64 columns
+//               each where the per-K-block drain is bound by instruction latency (more resident warps hide
+//               it).  The fast block-scaled kind has one packed FMA per two elements left and wants long runs
+//               of tensor-memory loads instead: eight warps with 128 columns each and up to 208 registers, 32
+//               columns in flight per wait (8192^3: 16 warps 508 us, 8 warps 501, 8 warps and 32 columns 489).
 // Tensor memory holds two 128x256 int32 accumulators (all 512 columns).  In block-scaled mode the
 // MMA warp alternates between them every 128-wide K block while the epilogue drains the other one
-// into fp32 registers (acc += float(P) * scale; in the fast kind float(P) is formed by an integer add of
-// a magic number whose multiple is kept bounded by alternating signs and removed at the tile end); in
+// into fp32 registers (acc += float(P) * scale; in the fast kind a fifth MMA per K block shifts P into the
+// non-negative range, where its bits ARE a float, and the multiple of the shift is taken out again); in
 // row x column mode a buffer holds a whole tile and the epilogue of tile i overlaps the main loop of tile i+1.
 //
 // Every wait on an mbarrier is bounded (a poll count worth about two seconds); on expiry the CTA raises
@@ -49,10 +51,9 @@ template <bool TWO> struct Cfg {
   static constexpr uint32_t STAGE_TX = TWO ? 2u * (A_STAGE + BM * BK) : (uint32_t)(A_STAGE + BN * BK);
 };
 constexpr int MAX_STAGES = 6;
-constexpr int EPI_WARPS = 16;                 // four groups of four warps, 64 accumulator columns per group
-constexpr int EPI_COLS = BN / (EPI_WARPS / 4);
-constexpr int THREADS = 128 + 32 * EPI_WARPS;
-constexpr int FAC_MAX = 512;                  // K blocks whose factors are staged in shared memory at a time
+constexpr int MAX_EPI_WARPS = 16;             // groups of four warps share the 256 accumulator columns
+template <int KIND> constexpr int EPI_WARPS_OF = KIND == 2 /* K_BLOCK_FAST */ ? 8 : MAX_EPI_WARPS;
+constexpr int FAC_MAX = 256;                  // K blocks whose factors are staged in shared memory at a time (a multiple of 4)
 constexpr int TMEM_COLS = 512;
 constexpr int SMEM_DYN = 4 * (A_STAGE + BN * BK) + 1024;  // == 6 * (16 KB + 16 KB) + 1024
 
@@ -85,6 +86,8 @@ struct GemmParams {
 // Instruction descriptor: D=s32, A=B=s8, both K-major, M=128, N=256, dense, no saturation.
 constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                               ((uint32_t)(BM >> 4) << 24);
+// Same with both operands unsigned: the MMA that shifts a partial product (K_BLOCK_FAST).
+constexpr uint32_t IDESC_U8 = (2u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 // Same with M=256 for the CTA-pair instruction (128 rows per CTA).
 constexpr uint32_t IDESC_I8_PAIR = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                                    ((uint32_t)((2 * BM) >> 4) << 24);
@@ -103,20 +106,23 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int m_units, const GemmPa
   return tc;
 }
 
-struct __align__(8) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
+struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[2], tempty[2], done;
   uint64_t fready[2], ffree[2];  // fast block kind: factor buffers written (factor warp) / consumed (every epilogue thread)
   uint32_t tmem_base;
   int abort_flag;
-  float bscale[EPI_WARPS / 4][EPI_COLS];     // per-tile column scales of each epilogue group (CHANNEL)
-  float bstep[EPI_WARPS / 4][2][EPI_COLS];   // per-K-block column scales (GROUP), double buffered
-  // K_BLOCK_FAST, written by the factor warp one unit (tile, or 512-K-block chunk of a tile) ahead, two buffers:
-  float fac[2][EPI_WARPS / 4][FAC_MAX];      // signed per-K-block scalar factors
-  float fbscale[2][EPI_WARPS / 4][EPI_COLS]; // per-channel column scales (times post_scale)
-  float fbias[2][EPI_WARPS / 4][2];          // running sum of the signed factors of the tile (value, error term)
+  float bscale[BN];     // per-tile column scales (CHANNEL)
+  float bstep[2][BN];   // per-K-block column scales (GROUP), double buffered
+  // K_BLOCK_FAST, written by the factor warp one unit (tile, or FAC_MAX-K-block chunk of a tile) ahead, two
+  // buffers; each 128-column half (one epilogue group) has its factors:
+  float2 fac[2][2][FAC_MAX];                 // per K block: scaled factor, and the correction due at it (or 0)
+  float fbscale[2][BN];                      // per-channel column scales (times post_scale)
+  float fend[2][2][3];                       // tile end: what the corrections left over, and 2^-exponent as two factors
   // scatter mode of the fast block kind: four output rows x 128 bytes per epilogue warp, staged so that one
   // store instruction writes whole 128-byte row segments into the peer's memory
-  uint4 xpose[EPI_WARPS][4][8];
+  uint4 xpose[EPI_WARPS_OF<2>][4][8];
+  // K_BLOCK_FAST: 256 rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
+  __align__(256) uint8_t ones[BN * 32];
 };
 
 // Epilogue kinds.  Everything but K_ROWCOL drains the accumulator every 128-wide K block.
@@ -125,6 +131,13 @@ constexpr int K_BLOCK_GEN = 1;   // block-scaled, any scale layout, reference op
 constexpr int K_BLOCK_FAST = 2;  // block-scaled, one scalar factor per (tile, K block) and 64-column group
 constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x per-tile or per-channel B scale
 constexpr int K_BLOCK_COLFAC = 3;  // block-scaled, per-tile A scale x per-(column, K block) B scale (fused forward)
+// K_BLOCK_FAST: 32 products 255 * 255.  A partial product of 128 int8 pairs lies in [-128*128*127, 128*128*128],
+// so P + SHIFT lies in [32, 4177952]: never negative and below 2^23, where the bits of an int32, read as a
+// float, are the (denormal) number (P + SHIFT) * 2^-149 exactly.
+constexpr float SHIFT_F = 2080800.f;
+constexpr int FAC_EXP = 100;   // factors are scaled by a power of two that puts the tile's largest one near 2^100
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
+
 constexpr uint32_t MAGIC_I = 0x4B400000u;   // the bits of 1.5 * 2^23
 constexpr float MAGIC_F = 12582912.f;       // 1.5 * 2^23
 
@@ -162,7 +175,7 @@ __device__ __forceinline__ void st_global_256(void* ptr, const uint32_t* w) {
 // a warp writes a different row, so each store instruction touches 32 lines: 32-byte stores (whole
 // sectors, half as many instructions) are used when the output pointer allows them.
 // POST = false: the caller has already folded post_scale into the scales it passes.
-template <bool POST = true>
+template <int EPI_COLS, bool POST = true>
 __device__ __forceinline__ void store_cols(const GemmParams& p, const float* acc, const float* bscale_or_null,
                                            int64_t row, int col0, void* cbase) {
 #pragma unroll
@@ -203,10 +216,11 @@ __device__ __forceinline__ void store_cols(const GemmParams& p, const float* acc
 }
 
 template <int KIND, bool TWO>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND>, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const GemmParams p) {
   constexpr bool BLOCK = KIND != K_ROWCOL;
+  constexpr int EPI_WARPS = EPI_WARPS_OF<KIND>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
   constexpr int STAGES = Cfg<TWO>::STAGES, B_STAGE = Cfg<TWO>::B_STAGE;
   constexpr uint32_t STAGE_TX = Cfg<TWO>::STAGE_TX;
   extern __shared__ uint8_t smem_raw[];
@@ -223,6 +237,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #define I8L_UNIT (TWO ? (int)(blockIdx.x >> 1) : (int)blockIdx.x)
 #define I8L_N_UNITS (TWO ? (int)(gridDim.x >> 1) : (int)gridDim.x)
 
+  if constexpr (KIND == K_BLOCK_FAST) {
+    for (int i = threadIdx.x; i < (int)sizeof(ctl.ones) / 16; i += THREADS)
+      reinterpret_cast<uint4*>(ctl.ones)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&ctl.full[s]), 1);
@@ -324,6 +343,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     } else if (warp == 1 && leader) {
       // ------------------------------------------------------------------ MMA issuer
+      const uint64_t ones_desc = smem_desc_sw32(smem_u32(ctl.ones));
       int s = 0, ab = 0;
       uint32_t ph = 0, aph = 0;
       bool ok = true;
@@ -343,10 +363,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (lane == 0) {
             const uint64_t da = smem_desc(smem_a + s * A_STAGE), db = smem_desc(smem_b + s * B_STAGE);
             const uint32_t d = tmem_base + ab * BN;
+            if (KIND == K_BLOCK_FAST) tc_mma_i8(d, ones_desc, ones_desc, IDESC_U8, 0u);   // D = SHIFT, see the epilogue
 #pragma unroll
             for (int k4 = 0; k4 < BK / 32; ++k4) {
               if (TWO) tc_mma_i8_pair(d, da + 2 * k4, db + 2 * k4, IDESC_I8_PAIR, (k4 > 0 || !drain_start) ? 1u : 0u);
-              else tc_mma_i8(d, da + 2 * k4, db + 2 * k4, IDESC_I8, (k4 > 0 || !drain_start) ? 1u : 0u);
+              else tc_mma_i8(d, da + 2 * k4, db + 2 * k4, IDESC_I8, (KIND == K_BLOCK_FAST || k4 > 0 || !drain_start) ? 1u : 0u);
             }
             if (TWO) {  // both CTAs' producers and epilogues wait on their own copies of these barriers
               tc_commit_pair(smem_u32(&ctl.empty[s]));
@@ -374,17 +395,22 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_wait(smem_u32(&ctl.done), 0, &dummy);
     } else if (KIND == K_BLOCK_FAST && warp == 2) {
       // ------------------------------------------------------------------ factor warp (fast block kind)
-      // Prepares, one unit ahead of the epilogue, what the epilogue needs besides the accumulators: the
-      // signed factor of every K block and the column scales.  Block d contributes g_d * (MAGIC_F + s_d P_d)
-      // with g_d = s_d f_d (see the epilogue), so the accumulators carry MAGIC_F * sum(g) on top of sum(f P).
-      // Choosing s_d against the sign of the running sum keeps |sum(g)| <= max f whatever the scales are, which
-      // bounds the rounding error the bias can cause; the epilogue takes the sum out after the last K block.
+      // Prepares, one unit ahead of the epilogue, what the epilogue needs besides the accumulators: the factor
+      // of every K block, the corrections and the column scales.  K block d contributes F_d * (P_d + SHIFT) * 2^-149
+      // with F_d = f_d * 2^e, e common to the tile and chosen so that the largest |F_d| is near 2^FAC_EXP: nothing
+      // over- or underflows whatever the scales are.  SHIFT * F_d is taken out four K blocks at a time, after the
+      // second of them: the accumulators then stay within two K blocks' shift (4.2e6 f) of the true sum, an ulp of
+      // which is at most f/2.  What the rounded corrections leave over is summed in fp64 and goes out at the tile end.
       // Hand-over through two mbarrier pairs (buffer written / buffer consumed), waits bounded like all others.
       const bool chan = p.b_kind == I8L_BSCALE_CHANNEL;
-      float run = 0.f, low = 0.f;   // lanes 0-3: the running sum of column group `lane` as an unevaluated pair
+      constexpr double SHIFT_D = (double)SHIFT_F * 0x1p-149;
       uint32_t u = 0;
       for (int t = I8L_UNIT; t < total_tiles; t += I8L_N_UNITS) {
         const TileCoord tc = unit_tile(t);
+        const int64_t bcol0 = (int64_t)(p.b_batched ? tc.m_blk / p.mpb : 0) * p.N + tc.n_tile * BN;
+        const float* as_ptr = p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift);
+        float up0[2], up1[2];       // 2^e as two factors
+        double left[2] = {0., 0.};  // per lane, over the chunks of the tile
         for (int k0 = 0; k0 < KB; k0 += FAC_MAX, ++u) {
           const int dn = KB - k0 < FAC_MAX ? KB - k0 : FAC_MAX;
           const int buf = u & 1;
@@ -392,33 +418,53 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             t = total_tiles;   // gave up (or another warp did): leave both loops
             break;
           }
-          for (int g = 0; g < EPI_WARPS / 4; ++g) {
-            const int col0 = tc.n_tile * BN + g * EPI_COLS;
-            const bool active = col0 < p.N;
-            const int64_t bcol0 = (int64_t)(p.b_batched ? tc.m_blk / p.mpb : 0) * p.N + col0;
-            if (chan)   // post_scale rides on the column scale (on the factors otherwise)
-              for (int i = lane; i < EPI_COLS; i += 32)
-                ctl.fbscale[buf][g][i] = active ? __ldg(p.b_scale + bcol0 + i) * p.post_scale : 0.f;
-            const float* as_ptr = p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift);
-            const float* bs_ptr = p.b_scale + (bcol0 >> 7) * KB + k0;
-            for (int i = lane; i < dn; i += 32)
-              ctl.fac[buf][g][i] = __ldg(as_ptr + ((k0 + i) >> p.a_kshift)) * ((!chan && active) ? __ldg(bs_ptr + i) * p.post_scale : 1.f);
-          }
-          __syncwarp();
-          if (lane < EPI_WARPS / 4) {
-            if (k0 == 0) run = low = 0.f;
-            float* f = ctl.fac[buf][lane];
-            for (int i = 0; i < dn; ++i) {
-              float g = f[i];
-              g = run > 0.f ? -g : g;
-              const float sum = __fadd_rn(run, g);
-              const float bb = __fsub_rn(sum, run);   // two-sum: the rounding error of run + g, off the critical chain
-              low = __fadd_rn(low, __fadd_rn(__fsub_rn(run, __fsub_rn(sum, bb)), __fsub_rn(g, bb)));
-              run = sum;
-              f[i] = g;
+          if (chan)   // post_scale rides on the column scale (on the factors otherwise)
+            for (int i = lane; i < BN; i += 32)
+              ctl.fbscale[buf][i] = tc.n_tile * BN + i < p.N ? __ldg(p.b_scale + bcol0 + i) * p.post_scale : 0.f;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const bool with_b = !chan && tc.n_tile * BN + h * (BN / 2) < p.N;
+            const float* bs_ptr = p.b_scale + ((bcol0 >> 7) + h) * KB;
+            auto factor = [&](int d) {
+              return __ldg(as_ptr + (d >> p.a_kshift)) * (with_b ? __ldg(bs_ptr + d) * p.post_scale : 1.f);
+            };
+            float2* fac = ctl.fac[buf][h];
+            if (k0 == 0) {
+              float m = 0.f;
+              for (int i = lane; i < KB; i += 32) {
+                const float f = factor(i);
+                if (i < dn) fac[i].x = f;
+                m = fmaxf(m, fabsf(f));
+              }
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+              const int e = FAC_EXP + 127 - (int)(__float_as_uint(m) >> 23);
+              up0[h] = pow2f(e >> 1);
+              up1[h] = pow2f(e - (e >> 1));
+              if (lane < 2) ctl.fend[buf][h][1 + lane] = pow2f(lane ? (149 - e) - ((149 - e) >> 1) : (149 - e) >> 1);
+            } else {
+              for (int i = lane; i < dn; i += 32) fac[i].x = factor(k0 + i);
+              if (lane < 2) ctl.fend[buf][h][1 + lane] = ctl.fend[buf ^ 1][h][1 + lane];
             }
-            ctl.fbias[buf][lane][0] = run;
-            ctl.fbias[buf][lane][1] = low;
+            __syncwarp();
+            for (int i = lane; i < (dn + 3) / 4; i += 32) {   // one lane per four K blocks
+              float f4[4];
+              double sum = 0.;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                f4[j] = 4 * i + j < dn ? fac[4 * i + j].x * up0[h] * up1[h] : 0.f;
+                sum += (double)f4[j];
+              }
+              const float corr = 4 * i + 2 < dn ? -(float)(SHIFT_D * sum) : 0.f;
+              left[h] += SHIFT_D * sum + (double)corr;
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (4 * i + j < dn) fac[4 * i + j] = make_float2(f4[j], j == 2 ? corr : 0.f);
+            }
+            double all = left[h];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+            if (lane == 0) ctl.fend[buf][h][0] = (float)all;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&ctl.fready[buf]));   // release: the warp's writes above are visible to waiters
@@ -426,9 +472,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   } else {
-    // -------------------------------------------------------------------- epilogue (16 warps)
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
-    const int q = warp & 3, wg = (warp - 4) >> 2;  // lane quarter, 64-column group
+    // -------------------------------------------------------------------- epilogue
+    // 128 x 64 + 256 x 208 of the 384 x 168 registers of the launch; 128 x 64 + 512 x 104 of 640 x 96
+    if (KIND == K_BLOCK_FAST) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int q = warp & 3, wg = (warp - 4) >> 2;  // lane quarter, column group
     const int tix = q * 32 + lane;                 // row within the tile == thread index within the group
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     int ab = 0;
@@ -455,7 +503,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t taddr0 = tmem_base + lane_addr + wg * EPI_COLS, fac_base = smem_u32(&ctl.fac[0][wg][0]);
       asm volatile("" : "+r"(taddr0), "+r"(fac_base));
       const bool chan = p.b_kind == I8L_BSCALE_CHANNEL;
-      constexpr int CH = 8;
+      constexpr int CH = 32;
       uint32_t gstep = 0, unit = 0;
       // The loops below never exit early (one exit and nothing to carry but the accumulators compiles to the
       // leanest code): after a wait timeout a warp runs through the remaining tiles without waiting or storing.
@@ -473,8 +521,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           mbar_wait_or_flag(smem_u32(&ctl.fready[unit & 1]), (unit >> 1) & 1u, abort_flag, p.max_polls);   // written by the factor warp
           const uint32_t fac0 = fac_base + (unit & 1) * (uint32_t)sizeof(ctl.fac[0]);
           for (int d = 0; d < dn; ++d) {
-            float f;
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + 4 * d));
+            float f, corr;
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(f), "=f"(corr) : "r"(fac0 + 8 * d));
             // No early exit and no success flag: a loop with one exit and nothing to carry but the
             // accumulators compiles to the leanest code.  After a timeout the abort flag is set, the status
             // word reports it, and the remaining K blocks run on whatever tensor memory holds.
@@ -485,36 +533,30 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               mbar_arrive(tfull0 + TEMPTY_OFF + 8 * ab);   // every thread arrives for itself: no warp sync, no branch
             };
             if (active) {
-              // int32 -> fp32 without the conversion unit: |P| <= 128*127*127 < 2^22, so the integer MAGIC_I + P
-              // (or MAGIC_I - P), read as a float, IS the number 1.5*2^23 + P (or - P): one full-rate integer
-              // add per element instead of a half-rate conversion.  The factor carries the sign, so the product
-              // is f*P plus a multiple of MAGIC_F that the factor warp keeps small and the tile end removes.
+              // int32 -> fp32 without any conversion: an extra K step of the tensor core has added SHIFT to P, so
+              // the bits are the float (P + SHIFT) * 2^-149, which the FMA multiplies exactly.  One packed FMA per
+              // two elements is all that is left; the shift is taken out every fourth K block.
+              // The drain, not the MMA, bounds this kernel: a fifth MMA (+25 % tensor work) for half of the drain's
+              // instructions takes 8192^3 from 560 us (an integer add per element, sixteen warps) to 489 us (1.96 ->
+              // 2.24 POP/s), the error against fp64 from 2.1e-5 to 0.7e-5.
               const uint32_t taddr = taddr0 + ab * BN;
               const float2 f2 = make_float2(f, f);
-              if (f >= 0.f) {
+              if (corr != 0.f) {
+                const float2 c2 = make_float2(corr, corr);
 #pragma unroll
-                for (int c = 0; c < EPI_COLS / CH; ++c) {  // 8-column chunks: 16-column ones spill here
-                  uint32_t r[CH];
-                  tc_ld8(taddr + c * CH, r);
-                  tc_ld_wait();
-                  if (c == EPI_COLS / CH - 1) release();
+                for (int j = 0; j < EPI_COLS / 2; ++j) acc[j] = __fadd2_rn(acc[j], c2);
+              }
 #pragma unroll
-                  for (int j = 0; j < CH / 2; ++j)
-                    acc[c * (CH / 2) + j] = __ffma2_rn(make_float2(__uint_as_float(MAGIC_I + r[2 * j]), __uint_as_float(MAGIC_I + r[2 * j + 1])),
-                                                       f2, acc[c * (CH / 2) + j]);
-                }
-              } else {
+              for (int c = 0; c < EPI_COLS / CH; ++c) {
+                uint32_t r[CH];
+                tc_ld16(taddr + c * CH, r);   // two loads of 16: one of 32 makes the compiler spill (489 -> 513 us at 8192^3)
+                tc_ld16(taddr + c * CH + 16, r + 16);
+                tc_ld_wait();
+                if (c == EPI_COLS / CH - 1) release();
 #pragma unroll
-                for (int c = 0; c < EPI_COLS / CH; ++c) {
-                  uint32_t r[CH];
-                  tc_ld8(taddr + c * CH, r);
-                  tc_ld_wait();
-                  if (c == EPI_COLS / CH - 1) release();
-#pragma unroll
-                  for (int j = 0; j < CH / 2; ++j)
-                    acc[c * (CH / 2) + j] = __ffma2_rn(make_float2(__uint_as_float(MAGIC_I - r[2 * j]), __uint_as_float(MAGIC_I - r[2 * j + 1])),
-                                                       f2, acc[c * (CH / 2) + j]);
-                }
+                for (int j = 0; j < CH / 2; ++j)
+                  acc[c * (CH / 2) + j] = __ffma2_rn(make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), f2,
+                                                     acc[c * (CH / 2) + j]);
               }
             } else {
               release();
@@ -530,16 +572,13 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           int t2 = t;
           asm volatile("" : "+r"(t2));  // keeps the tile's coordinates out of the K-block loop's live registers
           const TileCoord tc = unit_tile(t2);
-          // take out MAGIC_F * sum(g): the leading part first (close to the accumulator, so the difference is
-          // nearly exact), then the small remainder
-          const float* fb = ctl.fbias[unit & 1][wg];
-          const float b_hi = __fmul_rn(-MAGIC_F, fb[0]);
-          const float b_lo = __fmaf_rn(-MAGIC_F, fb[0], -b_hi) + __fmul_rn(-MAGIC_F, fb[1]);
+          const float* fe = ctl.fend[unit & 1][wg];
+          const float left = fe[0], down0 = fe[1], down1 = fe[2];
           float out[EPI_COLS];
 #pragma unroll
           for (int j = 0; j < EPI_COLS / 2; ++j) {
-            out[2 * j] = __fadd_rn(__fadd_rn(acc[j].x, b_hi), b_lo);
-            out[2 * j + 1] = __fadd_rn(__fadd_rn(acc[j].y, b_hi), b_lo);
+            out[2 * j] = __fsub_rn(acc[j].x, left) * down0 * down1;
+            out[2 * j + 1] = __fsub_rn(acc[j].y, left) * down0 * down1;
           }
           int64_t row = (int64_t)tc.m_blk * BM + tix;
           void* cbase = p.c;
@@ -548,37 +587,40 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             cbase = p.c_slots[owner];
             row += (int64_t)(p.rs_rank - owner) * p.rs_rows;
           }
-          const float* bsc = chan ? ctl.fbscale[unit & 1][wg] : nullptr;
+          const float* bsc = chan ? ctl.fbscale[unit & 1] + wg * EPI_COLS : nullptr;
           const int col0 = tc.n_tile * BN + wg * EPI_COLS;
           if (p.rs_rows && !p.out_f32 && !p.bias) {
             // Peer stores.  A lane owns one row, so a plain store instruction would send 32 separate 32-byte
             // pieces over NVLink; here the warp passes four rows at a time through shared memory (16-byte
             // slots, XOR-swizzled so that writers and readers are conflict-free) and every store instruction
             // then covers four rows x 128 contiguous bytes.  Same values as store_cols.
-            uint32_t w[EPI_COLS / 2];
-#pragma unroll
-            for (int j = 0; j < EPI_COLS / 2; ++j) {
-              float a = out[2 * j], b = out[2 * j + 1];
-              if (bsc) { a *= bsc[2 * j]; b *= bsc[2 * j + 1]; }
-              w[j] = pack_bf16x2(a, b);
-            }
             uint4* xp = &ctl.xpose[warp - 4][0][0];
             const int wr = lane & 3, rr = lane >> 3, rc = lane & 7;
             __nv_bfloat16* obase = static_cast<__nv_bfloat16*>(cbase) + (row - lane) * p.N + col0 + rc * 8;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if ((lane >> 2) == j) {
+            for (int h = 0; h < EPI_COLS; h += 64) {
+              uint32_t w[32];
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                  xp[wr * 8 + (c ^ (wr << 1))] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+              for (int j = 0; j < 32; ++j) {
+                float a = out[h + 2 * j], b = out[h + 2 * j + 1];
+                if (bsc) { a *= bsc[h + 2 * j]; b *= bsc[h + 2 * j + 1]; }
+                w[j] = pack_bf16x2(a, b);
               }
-              __syncwarp();
-              const uint4 v = xp[rr * 8 + (rc ^ (rr << 1))];
-              *reinterpret_cast<uint4*>(obase + (int64_t)(4 * j + rr) * p.N) = v;
-              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                if ((lane >> 2) == j) {
+#pragma unroll
+                  for (int c = 0; c < 8; ++c)
+                    xp[wr * 8 + (c ^ (wr << 1))] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                }
+                __syncwarp();
+                const uint4 v = xp[rr * 8 + (rc ^ (rr << 1))];
+                *reinterpret_cast<uint4*>(obase + (int64_t)(4 * j + rr) * p.N + h) = v;
+                __syncwarp();
+              }
             }
           } else {
-            store_cols<false>(p, out, bsc, row, col0, cbase);
+            store_cols<EPI_COLS, false>(p, out, bsc, row, col0, cbase);
           }
         }
         mbar_arrive(smem_u32(&ctl.ffree[unit & 1]));   // this tile's factors and column scales are no longer needed
@@ -595,7 +637,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const bool chan = p.b_kind == I8L_BSCALE_CHANNEL && !p.dump;
       if (chan) {  // K-invariant column scales of this group -> shared memory
         named_sync(1 + wg, 128);
-        if (tix < EPI_COLS) ctl.bscale[wg][tix] = active ? __ldg(p.b_scale + bcol0 + tix) : 0.f;
+        if (tix < EPI_COLS) ctl.bscale[wg * EPI_COLS + tix] = active ? __ldg(p.b_scale + bcol0 + tix) : 0.f;
         named_sync(1 + wg, 128);
       }
 
@@ -642,7 +684,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             out[2 * j] = acc[j].x;
             out[2 * j + 1] = acc[j].y;
           }
-          store_cols(p, out, chan ? ctl.bscale[wg] : nullptr, row, col0, p.c);
+          store_cols<EPI_COLS>(p, out, chan ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
         }
       } else if constexpr (KIND == K_BLOCK_COLFAC) {
         constexpr bool COLFAC = true;
@@ -668,7 +710,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const float f = f_next;
           if (d + 1 < KB) f_next = factor(d + 1);
           if (COLFAC) {  // thread i < 64 publishes the factor of column i of this group for this K block
-            if (tix < EPI_COLS) ctl.bstep[wg][d & 1][tix] = f;
+            if (tix < EPI_COLS) ctl.bstep[d & 1][wg * EPI_COLS + tix] = f;
             named_sync(1 + wg, 128);
           }
           ok = ok && mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls);  // single-exit loop, see K_BLOCK_FAST
@@ -676,7 +718,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (ok && active) {
             const uint32_t taddr = tmem_base + lane_addr + ab * BN + wg * EPI_COLS;
             const float2 f2 = make_float2(f, f);
-            const float2* fcol = reinterpret_cast<const float2*>(ctl.bstep[wg][d & 1]);
+            const float2* fcol = reinterpret_cast<const float2*>(ctl.bstep[d & 1] + wg * EPI_COLS);
 #pragma unroll
             for (int c = 0; c < EPI_COLS / 16; ++c) {
               uint32_t r[16];
@@ -704,7 +746,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             out[2 * j] = acc[j].x;
             out[2 * j + 1] = acc[j].y;
           }
-          store_cols(p, out, (!COLFAC && chan) ? ctl.bscale[wg] : nullptr, row, col0, p.c);
+          store_cols<EPI_COLS>(p, out, (!COLFAC && chan) ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
         }
       } else {
         // ---- generic paths: reference operation order, per-column / per-step scales, dumps, row x column
@@ -721,7 +763,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                               : __ldg(p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift) + (d >> p.a_kshift));
             if (p.b_kind == I8L_BSCALE_TILE && active) sb = __ldg(p.b_scale + (bcol0 >> 7) * KB + d);
             if (p.b_kind == I8L_BSCALE_GROUP) {
-              if (tix < EPI_COLS) ctl.bstep[wg][d & 1][tix] = active ? __ldg(p.b_scale + (bcol0 + tix) * KB + d) : 0.f;
+              if (tix < EPI_COLS) ctl.bstep[d & 1][wg * EPI_COLS + tix] = active ? __ldg(p.b_scale + (bcol0 + tix) * KB + d) : 0.f;
               named_sync(1 + wg, 128);
             }
           }
@@ -746,8 +788,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 for (int j = 0; j < 16; j += 4)
                   *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
               } else {
-                const float* sbv = p.b_kind == I8L_BSCALE_CHANNEL ? ctl.bscale[wg]
-                                   : p.b_kind == I8L_BSCALE_GROUP ? ctl.bstep[wg][d & 1]
+                const float* sbv = p.b_kind == I8L_BSCALE_CHANNEL ? ctl.bscale + wg * EPI_COLS
+                                   : p.b_kind == I8L_BSCALE_GROUP ? ctl.bstep[d & 1] + wg * EPI_COLS
                                                                   : nullptr;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
@@ -771,7 +813,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               float v[16];
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                v[j] = __fmul_rn(__fmul_rn(__int2float_rn((int)r[j]), sar), ctl.bscale[wg][c * 16 + j]);
+                v[j] = __fmul_rn(__fmul_rn(__int2float_rn((int)r[j]), sar), ctl.bscale[wg * EPI_COLS + c * 16 + j]);
                 if (p.post_scale != 1.f || p.bias) {
                   // the reference stores the GEMM result in the output type before its 1/K pass: a bf16
                   // rounding for bf16 outputs, none for fp32 ones
@@ -798,7 +840,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (ab == 0) aph ^= 1u;
         }
         if constexpr (BLOCK) {
-          if (ok && active && !p.dump) store_cols(p, acc, nullptr, row, col0, p.c);
+          if (ok && active && !p.dump) store_cols<EPI_COLS>(p, acc, nullptr, row, col0, p.c);
         }
       }
     }
@@ -948,7 +990,7 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   auto kernel = gemm_i8_kernel<KIND, TWO>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  cfg.blockDim = dim3(THREADS, 1, 1);
+  cfg.blockDim = dim3(128 + 32 * EPI_WARPS_OF<KIND>, 1, 1);
   cfg.dynamicSmemBytes = SMEM_DYN;
   cfg.stream = st;
   if (TWO) {
@@ -1024,8 +1066,7 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   const bool column_factor = block && !p.exact && !p.dump && !scalar_factor && p.a_kind == I8L_ASCALE_TILE &&
                              p.b_kind != I8L_BSCALE_CHANNEL;
   if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, p, tiles, st);
-  // the fast kind encodes a sign in its factors: it needs them positive (scales are; post_scale must be too)
-  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && p.post_scale > 0.f) return launch_kind<K_BLOCK_FAST, false>(ma, mb, p, tiles, st);
+  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE) return launch_kind<K_BLOCK_FAST, false>(ma, mb, p, tiles, st);
   if (scalar_factor) return launch_kind<K_BLOCK_ROWFAC, false>(ma, mb, p, tiles, st);
   if (column_factor) return launch_kind<K_BLOCK_COLFAC, false>(ma, mb, p, tiles, st);
   return launch_kind<K_BLOCK_GEN, false>(ma, mb, p, tiles, st);

@@ -195,4 +195,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
   d |= (uint64_t)2 << 61;              // SWIZZLE_128B
   return d;
 }
+// Same with rows of 32 bytes and 32-byte swizzle (8-row groups 256 bytes apart).
+__device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t saddr) {
+  uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(256 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)6 << 61;              // SWIZZLE_32B
+  return d;
+}
 }  // namespace i8l
