@@ -464,3 +464,25 @@ def test_fast_block_epilogue_shift(kb, n, values, decade):
         out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), b_kind=kind, flags=L.GEMM_OUT_F32)[0].cpu().double()
         assert ((out - ref).abs() <= bound).all(), float(((out - ref).abs() / bound).max())
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("gran", [L.GRAN_TILE128, L.GRAN_GROUP128])
+def test_rotated_tile_quantizer_infinite_and_nan(gran):
+    """A rotated group with a NaN is all NaN: it leaves the maximum alone and quantizes to 0; one with an infinity
+    has scale factor 127/inf = 0 and quantizes to 0 with stored scale inf."""
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(1, 256, 384, generator=g).to(torch.bfloat16)
+    clean = x.clone()
+    x[0, 3, 5], x[0, 9, 140] = float("nan"), float("inf")
+    q, s, qt, st = K.quant_tile(x.to(DEV), gran, L.QMODE_TRITON, 128, transposed=True)
+    q0, s0, qt0, st0 = K.quant_tile(clean.to(DEV), gran, L.QMODE_TRITON, 128, transposed=True)
+    assert (q[0, 3, :128] == 0).all() and (q[0, 9, 128:256] == 0).all()
+    assert torch.equal(q[0, 128:], q0[0, 128:]) and torch.equal(qt[0, :, 128:], qt0[0, :, 128:])
+    assert (qt[0, 5, :128] == 0).all() and (qt[0, 140, :128] == 0).all()
+    if gran == L.GRAN_GROUP128:
+        assert torch.isinf(s[0, 9, 1]) and torch.isinf(st[0, 140, 0])
+        assert abs(float(s[0, 3, 0]) - 1e-4 / 127) < 1e-9    # no finite value: the floor of the maximum
+        keep = [r for r in range(128) if r not in (3, 9)]
+        assert torch.equal(q[0, keep], q0[0, keep]) and torch.equal(s[0, keep], s0[0, keep])
+    else:
+        assert torch.isinf(s[0, 0, 1]) and torch.isinf(st[0, 1, 0]) and torch.equal(s[0, 0, 2], s0[0, 0, 2])

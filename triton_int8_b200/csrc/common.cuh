@@ -19,6 +19,7 @@ int check_arch();
 // launched by this host thread may use (i8l_set_cta_limit, else the SM count).
 uint32_t gemm_wait_limit();
 int gemm_cta_budget();
+int sm_count();  // of the current device
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -111,6 +112,28 @@ __device__ __forceinline__ uint2 quant_piece(const uint4& u, float s) {
   for (int k = 0; k < 4; ++k)
     quant2<MODE>(make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u)), s2, q[2 * k], q[2 * k + 1]);
   return make_uint2(pack4(q[0], q[1], q[2], q[3]), pack4(q[4], q[5], q[6], q[7]));
+}
+
+// The same bytes for finite values whose |max| gave the scale: |v * s| < 127.5, so nothing saturates, and adding
+// 1.5 * 2^23 with the rounding wanted (down after the +0.5, to nearest even for the RNE mode) leaves the integer in
+// the low byte of the sum.  The saturating conversion runs on the slow conversion pipe, one value at a time.
+// It also turns NaN into 0, which this does not: infinite or NaN inputs take quant_piece.
+template <int MODE>
+__device__ __forceinline__ uint2 quant_piece_finite(const uint4& u, float s) {
+  const float2 s2 = make_float2(s, s), half2 = make_float2(0.5f, 0.5f), magic2 = make_float2(12582912.f, 12582912.f);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  uint32_t b[4];   // two bytes each
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 v = make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
+    float2 y;
+    if (MODE == I8L_QMODE_RNE)   // scalar products: a packed one is fused with the addition, which turns ties over
+      y = __fadd2_rn(make_float2(__fmul_rn(v.x, s), __fmul_rn(v.y, s)), magic2);
+    else
+      y = __fadd2_rd(__fadd2_rn(__fmul2_rn(v, s2), half2), magic2);
+    b[k] = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040);
+  }
+  return make_uint2(__byte_perm(b[0], b[1], 0x5410), __byte_perm(b[2], b[3], 0x5410));
 }
 
 __device__ __forceinline__ float bf16_bits_to_float(uint32_t b) { return __uint_as_float(b << 16); }

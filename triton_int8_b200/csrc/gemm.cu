@@ -4,8 +4,8 @@
 // One persistent CTA per SM, 384 threads (fast block-scaled kind) or 640 (the others):
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      tensor-memory allocator + MMA issuer (one elected lane)
-//   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the signed per-K-block
-//               factors and the column scales the epilogue needs; idle in the other kinds
+//   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the per-K-block
+//               factors, corrections and column scales the epilogue needs; idle in the other kinds
 //   warp 3      idle (completes the first warpgroup so register budgets can be rebalanced)
 //   warps 4-    epilogue: warp%4 selects the 32 accumulator lanes (rows) a warp may read, the group of
 //               four warps a share of the 256 columns of the 128x256 tile.  Sixteen warps with 64 columns
@@ -955,7 +955,7 @@ static int current_device() {
   return (dev < 0 || dev >= MAX_DEVICES) ? 0 : dev;
 }
 
-static int sm_count() {
+int sm_count() {
   static std::atomic<int> cached[MAX_DEVICES];
   const int dev = current_device();
   int n = cached[dev].load(std::memory_order_relaxed);

@@ -254,383 +254,152 @@ quant_tile256_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Natural operand with the 128-point rotation along the columns (its contraction axis).  Four lanes
-// share a row: lane j of the quad holds the 16-byte pieces 4c+j (c = 0..3) of the row's 128 values,
-// so each load instruction of a quad covers 64 contiguous bytes and only two of the seven butterfly
-// stages cross lanes (spans 8 and 16); spans 1-4 and 32-64 run in registers.
+// Rotated tiles: q = the tile rotated along its columns (the contraction axis of the natural operand), qt =
+// its transpose rotated along the rows (the contraction axis of the dW operands and of W^T), either or both
+// from ONE read, each with scales of its own.  One CTA of 128 threads per 128x128 tile; the tile is staged
+// in shared memory as bf16 and a thread owns a whole row, then a whole column, so that all seven butterfly
+// stages run in its registers as packed pairs: no shuffles, which together with 16-bit shared-memory reads
+// cost 4.2 load/store slots per element when four lanes shared a row and two a column (now 1.5).  Bound by
+// issue and latency at 12 warps per SM (150 registers; about 10 instructions per element and output) next to
+// HBM.  [32768, 8192]: both outputs 353 -> 300 us, q 194 -> 177, qt 284 -> 185; W^T of [28672, 8192] in its two
+// passes 404 -> 247.  A persistent form that copies the next tile meanwhile was slower (393 us with both outputs).
 // ------------------------------------------------------------------------------------------------
-template <int GRAN, int MODE>
-__global__ void __launch_bounds__(256, 4)
-quant_tile_hadcols_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
-                          int8_t* __restrict__ q, float* __restrict__ scale) {
-  __shared__ float s_red[8];
-  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, j4 = l & 3, rq = l >> 2;
-  const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
-  const int64_t boff = (int64_t)blockIdx.z * rows * cols;
-  float s_tile = 0.f, s_row[2];
-  uint4 packed[2][4];  // rotated values, rounded to bf16
-  float tmax = 0.f;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = 16 * w + 8 * it + rq;
-    const __nv_bfloat16* xr = x + boff + (r_base + r) * cols + c_base;
-    float2 pv[4][4];  // piece c, pair k = elements 2k, 2k+1 of the piece
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float v[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(xr + 8 * (4 * c + j4))), v);
-      // span 1: inside each pair
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pv[c][k] = make_float2(__fadd_rn(v[2 * k], v[2 * k + 1]), __fsub_rn(v[2 * k], v[2 * k + 1]));
-      // spans 2, 4: between the pairs of a piece, two butterflies per packed operation
-#pragma unroll
-      for (int h = 1; h < 4; h <<= 1)
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if ((k & h) == 0) {
-            const float2 a = pv[c][k], b = pv[c][k | h];
-            pv[c][k] = add2(a, b);
-            pv[c][k | h] = sub2(a, b);
-          }
-    }
-    // spans 8, 16: across the quad (element index = 32c + 8j + t): partner - own or own + partner
-#pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
-      const float sg = (j4 & m) ? -1.f : 1.f;
-      const float2 sg2 = make_float2(sg, sg);
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, pv[c][k].x, m), __shfl_xor_sync(0xffffffffu, pv[c][k].y, m));
-          pv[c][k] = __ffma2_rn(pv[c][k], sg2, o);   // exact products by +-1: own + partner, or partner - own
-        }
-    }
-    // spans 32, 64: across the four pieces of the lane
-#pragma unroll
-    for (int h = 1; h < 4; h <<= 1)
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if ((c & h) == 0)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float2 a = pv[c][k], b = pv[c | h][k];
-            pv[c][k] = add2(a, b);
-            pv[c | h][k] = sub2(a, b);
-          }
-    __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed[it][c]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        h2[k] = __floats2bfloat162_rn(pv[c][k].x, pv[c][k].y);
-        hm = __hmax2(hm, __habs2(h2[k]));
-      }
-    }
-    float m = fmaxf(__low2float(hm), __high2float(hm));
-    if (GRAN == I8L_GRAN_GROUP128) {
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-      float stored;
-      make_scale<MODE>(m, s_row[it], stored);
-      if (j4 == 0) scale[((int64_t)blockIdx.z * rows + r_base + r) * (cols / 128) + blockIdx.x] = stored;
-    }
-    tmax = fmaxf(tmax, m);
-  }
-  if (GRAN == I8L_GRAN_TILE128) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-    if (l == 0) s_red[w] = tmax;
-    __syncthreads();
-    tmax = s_red[0];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) tmax = fmaxf(tmax, s_red[k]);
-    float stored;
-    make_scale<MODE>(tmax, s_tile, stored);
-    if (tid == 0) scale[((int64_t)blockIdx.z * (rows / 128) + blockIdx.y) * (cols / 128) + blockIdx.x] = stored;
-  }
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = 16 * w + 8 * it + rq;
-    const float s = GRAN == I8L_GRAN_TILE128 ? s_tile : s_row[it];
-    int8_t* qr = q + boff + (r_base + r) * cols + c_base;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint2*>(qr + 8 * (4 * c + j4)) = quant_piece<MODE>(packed[it][c], s);
-  }
+constexpr int ROT_LD = 272;  // bytes per staged row: 256 + 16, conflict-free for 16-byte row reads and for column reads
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// ------------------------------------------------------------------------------------------------
-// Transposed operand with the rotation along ITS contraction axis, i.e. along the rows of x: the dW
-// operands dY^T and X^T of a rotated linear layer (contraction over the tokens).  One CTA per 128x128
-// tile: the tile is staged in shared memory as fp32, thread (c, h) then owns rows 64h..64h+63 of
-// column c, runs six butterfly stages in registers and the last one with its partner lane, rounds to
-// bf16, and writes 64 consecutive bytes of output row c.
-// ------------------------------------------------------------------------------------------------
-template <int GRAN, int MODE>
-__global__ void __launch_bounds__(256)
-quant_tile_hadrows_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
-                          int8_t* __restrict__ qt, float* __restrict__ scale_t, float* __restrict__ colmax) {
-  extern __shared__ float s_tile[];  // [128][132]: rows 16-byte aligned for vector stores
-  __shared__ float s_red[8];
-  constexpr int LD = 132;
-  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, cc = l & 15, half = l >> 4;
-  const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
-  const int64_t boff = (int64_t)blockIdx.z * rows * cols;
-  const __nv_bfloat16* xb = x + boff;
+// 128-point transform of p[k] = (x[k], x[k + 64]): spans 1..32 between the pairs, span 64 inside them, the
+// order of the CPU oracle.  Returns the results rounded to bf16, h[i] = (y[2i], y[2i+1]), and their |max|, NaN
+// if one of them is NaN.
+__device__ __forceinline__ float rot128(float2* p, uint32_t* h) {
 #pragma unroll
-  for (int it = 0; it < 2; ++it)
+  for (int span = 1; span < 64; span <<= 1)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 16 * w + 8 * it + 4 * half + i;
-      float v[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(xb + (r_base + r) * cols + c_base + 8 * cc)), v);
-      *reinterpret_cast<float4*>(s_tile + r * LD + 8 * cc) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4*>(s_tile + r * LD + 8 * cc + 4) = make_float4(v[4], v[5], v[6], v[7]);
-    }
-  __syncthreads();
-  const int c = tid >> 1, h = tid & 1;
-  float2 pv[32];  // pair k = rows 64h + 2k, 64h + 2k + 1 of column c
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {  // span 1 on the way in
-    const float a = s_tile[(64 * h + 2 * k) * LD + c], b = s_tile[(64 * h + 2 * k + 1) * LD + c];
-    pv[k] = make_float2(__fadd_rn(a, b), __fsub_rn(a, b));
-  }
-#pragma unroll
-  for (int span = 1; span < 32; span <<= 1) {  // spans 2..32 of the elements: two butterflies per packed operation
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
+    for (int k = 0; k < 64; ++k)
       if ((k & span) == 0) {
-        const float2 a = pv[k], b = pv[k | span];
-        pv[k] = add2(a, b);
-        pv[k | span] = sub2(a, b);
+        const float2 a = p[k], b = p[k | span];
+        p[k] = add2(a, b);
+        p[k | span] = sub2(a, b);
       }
-    }
-  }
-  // span 64: the partner lane holds the other half of the column; then round to bf16 as the
-  // reference's rotation does
-  uint32_t hv[32];
   __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
-  const float sg = h ? -1.f : 1.f;
-  const float2 sg2 = make_float2(sg, sg);
 #pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, pv[k].x, 1), __shfl_xor_sync(0xffffffffu, pv[k].y, 1));
-    const float2 r = __ffma2_rn(pv[k], sg2, o);  // own + partner, or partner - own
-    const __nv_bfloat162 b2 = __floats2bfloat162_rn(r.x, r.y);
-    hm = __hmax2(hm, __habs2(b2));
-    hv[k] = *reinterpret_cast<const uint32_t*>(&b2);
+  for (int i = 0; i < 32; ++i) {
+    const float2 a = p[2 * i], b = p[2 * i + 1];
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(__fadd_rn(a.x, a.y), __fadd_rn(b.x, b.y));
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(__fsub_rn(a.x, a.y), __fsub_rn(b.x, b.y));
+    hm = __hmax2_nan(hm, __hmax2_nan(__habs2(lo), __habs2(hi)));
+    h[i] = *reinterpret_cast<const uint32_t*>(&lo);
+    h[32 + i] = *reinterpret_cast<const uint32_t*>(&hi);
   }
-  float m = fmaxf(__low2float(hm), __high2float(hm));
-  float s, stored;
-  if (GRAN == I8L_GRAN_TILE128) {
+  const __nv_bfloat16 m = __hmax_nan(__low2bfloat16(hm), __high2bfloat16(hm));
+  return __bfloat162float(m);
+}
+
+// 128 rotated values -> 128 consecutive bytes (32-byte stores where the output pointer allows them).
+// FINITE: quant_piece_finite instead of the saturating conversions.
+template <int MODE, bool FINITE>
+__device__ __forceinline__ void quant_store128(const uint32_t* h, float s, int8_t* out, bool align32) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (l == 0) s_red[w] = m;
-    __syncthreads();
-    m = s_red[0];
+  for (int i = 0; i < 64; i += 16) {
+    uint32_t w[8];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) m = fmaxf(m, s_red[k]);
-    make_scale<MODE>(m, s, stored);
-    if (tid == 0) scale_t[((int64_t)blockIdx.z * (cols / 128) + blockIdx.x) * (rows / 128) + blockIdx.y] = stored;
-  } else if (GRAN == GRAN_COLMAX_PASS) {  // first pass of the whole-column scale: absmax of the rotated column
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    if (h == 0) atomicMax(reinterpret_cast<int*>(colmax + c_base + c), __float_as_int(m));
-    return;
-  } else if (GRAN == GRAN_COLFULL) {      // second pass: one scale per output row over all of its elements
-    make_scale<MODE>(colmax[c_base + c], s, stored);
-    if (h == 0 && blockIdx.y == 0) scale_t[c_base + c] = stored;
-  } else {  // one scale per output row (column of x) and 128 contraction elements
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    make_scale<MODE>(m, s, stored);
-    if (h == 0) scale_t[((int64_t)blockIdx.z * cols + c_base + c) * (rows / 128) + blockIdx.y] = stored;
-  }
-  int8_t* out = qt + boff + (c_base + c) * rows + r_base + 64 * h;
-#pragma unroll
-  for (int k = 0; k < 32; k += 8) {
-    const uint2 lo = quant_piece<MODE>(make_uint4(hv[k], hv[k + 1], hv[k + 2], hv[k + 3]), s);
-    const uint2 hi = quant_piece<MODE>(make_uint4(hv[k + 4], hv[k + 5], hv[k + 6], hv[k + 7]), s);
-    *reinterpret_cast<uint4*>(out + 2 * k) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+    for (int k = 0; k < 4; ++k) {
+      const uint4 u = make_uint4(h[i + 4 * k], h[i + 4 * k + 1], h[i + 4 * k + 2], h[i + 4 * k + 3]);
+      const uint2 o = FINITE ? quant_piece_finite<MODE>(u, s) : quant_piece<MODE>(u, s);
+      w[2 * k] = o.x;
+      w[2 * k + 1] = o.y;
+    }
+    if (align32) {
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                   ::"l"(out + 2 * i), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                   : "memory");
+    } else {
+      *reinterpret_cast<uint4*>(out + 2 * i) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(out + 2 * i + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
   }
 }
 
-// ------------------------------------------------------------------------------------------------
-// Both rotated operands of a 128x128 tile from ONE read of x: q (rotation along the columns, as
-// quant_tile_hadcols_kernel) and qt (the transpose, rotation along the rows, as quant_tile_hadrows_kernel),
-// each with its own per-tile scale.  Results are bit-identical to those two kernels.
-//   Phase A: hadcols thread mapping; every 16-byte piece is also parked in shared memory as raw bf16.
-//   Phase B: thread (c, h) owns column c and the 64 rows whose bit 1 equals h (rows 4m+2h, 4m+2h+1), so
-//   that the butterfly of span 2 is the one that crosses the lane pair and the two lanes read different
-//   shared-memory banks; spans run in the order 1, 2, 4, ... 64 like everywhere else.  The quantized byte
-//   pairs are exchanged once more so that each lane stores 64 contiguous bytes of output row c.
-// ------------------------------------------------------------------------------------------------
-template <int MODE>
-__global__ void __launch_bounds__(256, 3)
-quant_tile_had_dual_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
-                           int8_t* __restrict__ q, float* __restrict__ scale, int8_t* __restrict__ qt,
-                           float* __restrict__ scale_t) {
-  constexpr int LDB = 272;  // bytes per shared row: 256 + 16 (keeps 16-byte alignment, spreads the banks)
-  __shared__ __align__(16) uint8_t s_raw[128 * LDB];
-  __shared__ float s_red[8], s_red_t[8];
-  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, j4 = l & 3, rq = l >> 2;
+// GRAN: TILE128, GROUP128 (one scale per output row and 128 contraction elements), or for qt alone
+// GRAN_COLMAX_PASS / GRAN_COLFULL: the two passes of one scale per output row over all of its elements.
+template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
+__global__ void __launch_bounds__(128, 3)
+quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
+                      float* __restrict__ scale, int8_t* __restrict__ qt, float* __restrict__ scale_t,
+                      float* __restrict__ colmax) {
+  __shared__ __align__(16) uint8_t s_raw[128 * ROT_LD];
+  __shared__ float s_red[2][4];
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
-  // ---------------------------------------------------------------- phase A: rotation along the columns
-  float s_tile = 0.f;
-  uint4 packed[2][4];
-  float tmax = 0.f;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = 16 * w + 8 * it + rq;
-    const __nv_bfloat16* xr = x + boff + (r_base + r) * cols + c_base;
-    float2 pv[4][4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(xr + 8 * (4 * c + j4)));
-      *reinterpret_cast<uint4*>(s_raw + r * LDB + 16 * (4 * c + j4)) = u;
-      float v[8];
-      unpack8(u, v);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pv[c][k] = make_float2(__fadd_rn(v[2 * k], v[2 * k + 1]), __fsub_rn(v[2 * k], v[2 * k + 1]));
-#pragma unroll
-      for (int h = 1; h < 4; h <<= 1)
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if ((k & h) == 0) {
-            const float2 a = pv[c][k], b = pv[c][k | h];
-            pv[c][k] = add2(a, b);
-            pv[c][k | h] = sub2(a, b);
-          }
-    }
-#pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
-      const float sg = (j4 & m) ? -1.f : 1.f;
-      const float2 sg2 = make_float2(sg, sg);
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, pv[c][k].x, m), __shfl_xor_sync(0xffffffffu, pv[c][k].y, m));
-          pv[c][k] = __ffma2_rn(pv[c][k], sg2, o);
-        }
-    }
-#pragma unroll
-    for (int h = 1; h < 4; h <<= 1)
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if ((c & h) == 0)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float2 a = pv[c][k], b = pv[c | h][k];
-            pv[c][k] = add2(a, b);
-            pv[c | h][k] = sub2(a, b);
-          }
-    __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed[it][c]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        h2[k] = __floats2bfloat162_rn(pv[c][k].x, pv[c][k].y);
-        hm = __hmax2(hm, __habs2(h2[k]));
-      }
-    }
-    tmax = fmaxf(tmax, fmaxf(__low2float(hm), __high2float(hm)));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-  if (l == 0) s_red[w] = tmax;
-  __syncthreads();   // also: the raw tile is complete in shared memory
-  tmax = s_red[0];
-#pragma unroll
-  for (int k = 1; k < 8; ++k) tmax = fmaxf(tmax, s_red[k]);
   {
-    float stored;
-    make_scale<MODE>(tmax, s_tile, stored);
-    if (tid == 0) scale[((int64_t)blockIdx.z * (rows / 128) + blockIdx.y) * (cols / 128) + blockIdx.x] = stored;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
+    const __nv_bfloat16* src = x + boff + (r_base + (tid >> 4)) * cols + c_base + 8 * (tid & 15);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) cp_async16(dst + i * 8 * ROT_LD, src + (int64_t)i * 8 * cols);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   }
+  __syncthreads();
+  // Both orientations run through the same code, a row and then a column per thread (two unrolled copies of the
+  // transform measured the same).
+#pragma unroll 1
+  for (int ph = OUT_N ? 0 : 1; ph < (OUT_T ? 2 : 1); ++ph) {
+    float2 p[64];
+    if (ph == 0) {
 #pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = 16 * w + 8 * it + rq;
-    int8_t* qr = q + boff + (r_base + r) * cols + c_base;
+      for (int c = 0; c < 16; ++c) {
+        float v[8];
+        unpack8(*reinterpret_cast<const uint4*>(s_raw + tid * ROT_LD + 16 * c), v);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint2*>(qr + 8 * (4 * c + j4)) = quant_piece<MODE>(packed[it][c], s_tile);
-  }
-  // ---------------------------------------------------------------- phase B: rotation along the rows
-  const int c = tid >> 1, h = tid & 1;
-  float2 pv[32];   // pv[m] = rows 4m+2h, 4m+2h+1 of column c
+        for (int j = 0; j < 8; ++j) {
+          if (c < 8) p[8 * c + j].x = v[j];
+          else p[8 * (c - 8) + j].y = v[j];
+        }
+      }
+    } else {
+      const uint8_t* col = s_raw + 2 * tid;
 #pragma unroll
-  for (int m = 0; m < 32; ++m) {   // span 1 on the way in
-    const uint8_t* p0 = s_raw + (4 * m + 2 * h) * LDB + 2 * c;
-    const float a = bf16_bits_to_float(*reinterpret_cast<const uint16_t*>(p0));
-    const float b = bf16_bits_to_float(*reinterpret_cast<const uint16_t*>(p0 + LDB));
-    pv[m] = make_float2(__fadd_rn(a, b), __fsub_rn(a, b));
-  }
-  {   // span 2: the partner lane holds the rows with the other value of bit 1
-    const float sg = h ? -1.f : 1.f;
-    const float2 sg2 = make_float2(sg, sg);
-#pragma unroll
-    for (int m = 0; m < 32; ++m) {
-      const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, pv[m].x, 1), __shfl_xor_sync(0xffffffffu, pv[m].y, 1));
-      pv[m] = __ffma2_rn(pv[m], sg2, o);   // own + partner, or partner - own
-    }
-  }
-#pragma unroll
-  for (int span = 1; span < 32; span <<= 1) {   // spans 4..64 of the rows = 1..16 of m
-#pragma unroll
-    for (int m = 0; m < 32; ++m) {
-      if ((m & span) == 0) {
-        const float2 a = pv[m], b = pv[m | span];
-        pv[m] = add2(a, b);
-        pv[m | span] = sub2(a, b);
+      for (int k = 0; k < 64; ++k) {
+        p[k].x = bf16_bits_to_float(*reinterpret_cast<const uint16_t*>(col + k * ROT_LD));
+        p[k].y = bf16_bits_to_float(*reinterpret_cast<const uint16_t*>(col + (k + 64) * ROT_LD));
       }
     }
+    uint32_t h[64];
+    float m = rot128(p, h), s, stored;
+    const bool finite = m <= 3.3895314e38f;   // the largest bf16
+    if (!finite) {                            // the maximum leaves NaNs out
+      __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 64; i += 4) hm = absmax8(make_uint4(h[i], h[i + 1], h[i + 2], h[i + 3]), hm);
+      m = hmax_of(hm);
+    }
+    if (GRAN == GRAN_COLMAX_PASS) {  // |x| >= 0: the bit patterns order like integers, so an integer maximum is exact
+      atomicMax(reinterpret_cast<int*>(colmax + c_base + tid), __float_as_int(m));
+      return;
+    }
+    if (GRAN == I8L_GRAN_TILE128) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (l == 0) s_red[ph][w] = m;
+      __syncthreads();
+      m = fmaxf(fmaxf(s_red[ph][0], s_red[ph][1]), fmaxf(s_red[ph][2], s_red[ph][3]));
+    }
+    if (GRAN == GRAN_COLFULL) m = colmax[c_base + tid];
+    make_scale<MODE>(m, s, stored);
+    const int64_t o_base = ph == 0 ? r_base : c_base, k_base = ph == 0 ? c_base : r_base;  // output row, contraction axis
+    const int64_t o_n = ph == 0 ? rows : cols, k_n = ph == 0 ? cols : rows, kb = k_base / 128, nkb = k_n / 128;
+    float* sc = ph == 0 ? scale : scale_t;
+    if (GRAN == GRAN_COLFULL) { if (kb == 0) sc[o_base + tid] = stored; }
+    else if (GRAN == I8L_GRAN_GROUP128) sc[(blockIdx.z * o_n + o_base + tid) * nkb + kb] = stored;
+    else if (tid == 0) sc[(blockIdx.z * (o_n / 128) + o_base / 128) * nkb + kb] = stored;
+    int8_t* out = ph == 0 ? q : qt;
+    const bool align32 = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;
+    int8_t* row = out + boff + (o_base + tid) * k_n + k_base;
+    if (finite) quant_store128<MODE, true>(h, s, row, align32);
+    else quant_store128<MODE, false>(h, s, row, align32);
   }
-  uint32_t hv[32];
-  __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
-#pragma unroll
-  for (int m = 0; m < 32; ++m) {
-    const __nv_bfloat162 b2 = __floats2bfloat162_rn(pv[m].x, pv[m].y);
-    hm = __hmax2(hm, __habs2(b2));
-    hv[m] = *reinterpret_cast<const uint32_t*>(&b2);
-  }
-  float mt = fmaxf(__low2float(hm), __high2float(hm));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o));
-  if (l == 0) s_red_t[w] = mt;
-  __syncthreads();
-  mt = s_red_t[0];
-#pragma unroll
-  for (int k = 1; k < 8; ++k) mt = fmaxf(mt, s_red_t[k]);
-  float st, stored_t;
-  make_scale<MODE>(mt, st, stored_t);
-  if (tid == 0) scale_t[((int64_t)blockIdx.z * (cols / 128) + blockIdx.x) * (rows / 128) + blockIdx.y] = stored_t;
-  // quantize: byte pair m = (row 4m+2h, row 4m+2h+1) -> 16 bits; two pairs per 32-bit word
-  uint32_t pw[16];   // pw[i] = pair 2i | pair 2i+1 << 16
-  const float2 st2 = make_float2(st, st);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    int q0, q1, q2, q3;
-    quant2<MODE>(make_float2(__uint_as_float(hv[2 * i] << 16), __uint_as_float(hv[2 * i] & 0xffff0000u)), st2, q0, q1);
-    quant2<MODE>(make_float2(__uint_as_float(hv[2 * i + 1] << 16), __uint_as_float(hv[2 * i + 1] & 0xffff0000u)), st2, q2, q3);
-    pw[i] = pack4(q0, q1, q2, q3);
-  }
-  // lane h keeps the pairs of m in [16h, 16h+16) and receives the partner's pairs of the same m: output
-  // bytes 4m..4m+3 = (pair of lane 0, pair of lane 1)
-  uint32_t outw[16];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t send = h ? pw[i] : pw[8 + i];          // what the partner needs from this lane
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, send, 1);
-    const uint32_t mine = h ? pw[8 + i] : pw[i];          // pairs 2i', 2i'+1 of the m range this lane writes
-    const uint32_t lo = h ? got : mine, hi = h ? mine : got;   // lane 0's pairs go to bytes 0-1, lane 1's to bytes 2-3
-    outw[2 * i] = __byte_perm(lo, hi, 0x5410);            // m = 2i':   lo.pair0 | hi.pair0 << 16
-    outw[2 * i + 1] = __byte_perm(lo, hi, 0x7632);        // m = 2i'+1: lo.pair1 | hi.pair1 << 16
-  }
-  int8_t* out = qt + boff + (c_base + c) * rows + r_base + 64 * h;
-#pragma unroll
-  for (int i = 0; i < 16; i += 4)
-    *reinterpret_cast<uint4*>(out + 4 * i) = make_uint4(outw[i], outw[i + 1], outw[i + 2], outw[i + 3]);
 }
 
 // Column absmax of x [rows, cols] into colmax[cols] (pre-zeroed); |x| >= 0 so the float bit
@@ -845,22 +614,6 @@ quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8
 
 // ------------------------------------------------------------------------------------------------ host
 constexpr int MAX_DEVICES = 64;
-static int device_ordinal() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  return (dev < 0 || dev >= MAX_DEVICES) ? 0 : dev;
-}
-// Raises a kernel's dynamic shared-memory limit once per device (function attributes are per device;
-// the call is idempotent, so two threads racing here only repeat it).
-template <typename Kernel>
-static cudaError_t ensure_smem(Kernel kernel, std::atomic<bool>* done_per_device, size_t bytes) {
-  std::atomic<bool>& done = done_per_device[device_ordinal()];
-  if (done.load(std::memory_order_acquire)) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done.store(true, std::memory_order_release);
-  return e;
-}
-
 static int check_dims(int64_t batch, int64_t rows, int64_t cols) {
   if (batch <= 0 || rows <= 0 || cols <= 0 || rows % 128 || cols % 128)
     return fail(I8L_ERR_SHAPE, "batch=%lld rows=%lld cols=%lld: all must be positive and rows, cols multiples of 128",
@@ -882,21 +635,12 @@ template <int GRAN, int MODE>
 static int dispatch_tile(const void* x, int64_t batch, int64_t rows, int64_t cols, bool had, int8_t* q,
                          float* scale, int8_t* qt, float* scale_t, const float* colmax, cudaStream_t st) {
   const bool n = q != nullptr, t = qt != nullptr;
-  if (had && n && t && GRAN == I8L_GRAN_TILE128) {  // both rotated operands from one read of the tile
-    dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
-    quant_tile_had_dual_kernel<MODE><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, q, scale, qt, scale_t);
-  } else if (had) {  // the two orientations rotate along different axes: one launch each
-    if (n) {
-      dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
-      quant_tile_hadcols_kernel<GRAN, MODE><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, q, scale);
-    }
-    if (t) {
-      constexpr size_t smem = 128 * 132 * sizeof(float);
-      static std::atomic<bool> attr_done[MAX_DEVICES];
-      I8L_CUDA_OK(ensure_smem(quant_tile_hadrows_kernel<GRAN, MODE>, attr_done, smem));
-      dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
-      quant_tile_hadrows_kernel<GRAN, MODE><<<grid, 256, smem, st>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, qt, scale_t, nullptr);
-    }
+  if (had) {  // whatever is wanted of the two orientations, from one read of the tile
+    const dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
+    const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
+    if (n && t) quant_tile_rot_kernel<GRAN, MODE, true, true><<<grid, 128, 0, st>>>(xp, rows, cols, q, scale, qt, scale_t, nullptr);
+    else if (n) quant_tile_rot_kernel<GRAN, MODE, true, false><<<grid, 128, 0, st>>>(xp, rows, cols, q, scale, nullptr, nullptr, nullptr);
+    else quant_tile_rot_kernel<GRAN, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, qt, scale_t, nullptr);
   } else if (GRAN == I8L_GRAN_TILE128) {
     if (n && t) launch_tile<GRAN, MODE, false, true, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
     else if (n) launch_tile<GRAN, MODE, false, true, false>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
@@ -1021,14 +765,10 @@ extern "C" int i8l_quant_col_t(const void* x, int64_t rows, int64_t cols, int qm
 template <int MODE>
 static int launch_col_t_rot(const void* x, int64_t rows, int64_t cols, int8_t* qt, float* scale_t, float* colmax,
                             cudaStream_t st) {
-  constexpr size_t smem = 128 * 132 * sizeof(float);
-  static std::atomic<bool> attr_done_pass[MAX_DEVICES], attr_done_full[MAX_DEVICES];
-  I8L_CUDA_OK(ensure_smem(quant_tile_hadrows_kernel<GRAN_COLMAX_PASS, MODE>, attr_done_pass, smem));
-  I8L_CUDA_OK(ensure_smem(quant_tile_hadrows_kernel<GRAN_COLFULL, MODE>, attr_done_full, smem));
   const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-  dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), 1);
-  quant_tile_hadrows_kernel<GRAN_COLMAX_PASS, MODE><<<grid, 256, smem, st>>>(xp, rows, cols, nullptr, nullptr, colmax);
-  quant_tile_hadrows_kernel<GRAN_COLFULL, MODE><<<grid, 256, smem, st>>>(xp, rows, cols, qt, scale_t, colmax);
+  const dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), 1);
+  quant_tile_rot_kernel<GRAN_COLMAX_PASS, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, nullptr, nullptr, colmax);
+  quant_tile_rot_kernel<GRAN_COLFULL, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, qt, scale_t, colmax);
   I8L_CUDA_OK(cudaGetLastError());
   return I8L_OK;
 }
