@@ -486,3 +486,21 @@ def test_rotated_tile_quantizer_infinite_and_nan(gran):
         assert torch.equal(q[0, keep], q0[0, keep]) and torch.equal(s[0, keep], s0[0, keep])
     else:
         assert torch.isinf(s[0, 0, 1]) and torch.isinf(st[0, 1, 0]) and torch.equal(s[0, 0, 2], s0[0, 0, 2])
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 128), (9, 256), (3, 2048), (130, 2176), (6, 4096), (5, 4224), (3, 8320), (2, 16384), (2, 16512)])
+@pytest.mark.parametrize("had", [0, 128])
+def test_row_quantizer_row_lengths(rows, cols, had):
+    """Row lengths at which the number of threads or rows per CTA changes, and row counts that fill no CTA."""
+    g = torch.Generator().manual_seed(rows + cols)
+    w = torch.randn(rows, cols, generator=g).to(torch.bfloat16)
+    w[rows - 1, cols - 1] = -77.0
+    q, s = K.quant_row(w.to(DEV), L.QMODE_TRITON, had)
+    q_ref, s_ref = R.quant_token(R.hadamard(w, 128) if had else w)
+    _same(q, q_ref, "int8"); _same(s, s_ref.view(-1), "scale")
+    w[0, 5], w[0, 6] = float("nan"), 3.0     # without a rotation the NaN becomes 0 and leaves the maximum alone
+    if not had:
+        q, s = K.quant_row(w.to(DEV), L.QMODE_TRITON, had)
+        w[0, 5] = 0.0
+        q_ref, s_ref = R.quant_token(w)
+        _same(q, q_ref, "int8 with a NaN"); _same(s, s_ref.view(-1), "scale with a NaN")
