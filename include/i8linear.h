@@ -235,6 +235,40 @@ I8L_API int i8l_gemm_block_scatter(const int8_t* a_q, const int8_t* b_q, const f
 I8L_API int i8l_sum_slots(const void* slots, void* out, int world, int64_t rows, int64_t cols, void* stream);
 
 /*
+ * A whole product: quantize a [batch, M, K] with a_gran and b ([N, K], or [batch, N, K] if b_batched) with b_gran, both
+ * with qmode and hadamard, into `workspace`, then c = i8l_gemm_rowcol (a_gran = b_gran = I8L_GRAN_ROW) or
+ * i8l_gemm_block (a_gran TILE128, GROUP128 or TILE128X256; b_gran ROW, TILE128 or GROUP128) of them.  With a_qt
+ * (batch 1) the transposed operand of a is made as well, scaled with a_gran along M, for a later i8l_linear_backward.
+ * The workspace holds, each piece rounded up to 256 bytes: both int8 operands, both scale arrays and, with a_qt and
+ * per-row scales, K floats; 256-byte aligned.  Same results as the calls one by one: the pipelines of
+ * triton/block_channel_fwd32.py:216-240, triton/double-channle_fwd32.py:269-285 and their batched forms.
+ */
+I8L_API int i8l_quant_gemm(const void* a, const void* b, const void* bias, void* c, int8_t* a_qt, float* a_st,
+                   int64_t batch, int64_t M, int64_t N, int64_t K, int b_batched, int a_gran, int b_gran, int qmode,
+                   int hadamard, float post_scale, int flags, void* workspace, int64_t workspace_bytes, int32_t* status,
+                   void* stream);
+
+/*
+ * Backward pass of y = x w^T: dx [M, K] = dy w and dw [N, K] = dy^T x, either may be NULL.  x_qt, x_st: the transposed
+ * operand that i8l_quant_gemm made of x with the same gran, qmode and hadamard.  The workspace holds, each piece rounded up
+ * to 256 bytes: for dx the int8 dy and w^T, dy's scales and K floats; for dw the int8 dy^T and its scales;
+ * max(K, N) floats.  No counterpart in the reference, which has the two products only.
+ */
+I8L_API int i8l_linear_backward(const void* dy, const void* w, const int8_t* x_qt, const float* x_st, void* dx, void* dw,
+                   int64_t M, int64_t N, int64_t K, int gran, int qmode, int hadamard, float post_dx, float post_dw,
+                   int flags, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
+
+/*
+ * Non-blocking look at a status word (the `status` argument of the GEMMs) for hot loops.  i8l_status_open binds a
+ * device int32 and a pinned host int32 (NULL on failure, see i8l_last_error; the handle lives as long as the
+ * process).  i8l_status_poll returns I8L_ERR_TIMEOUT if the copy that an earlier poll started has completed and shows
+ * a set word, and otherwise starts the next copy on `stream`, unless the last one is still in flight or the stream is
+ * being captured.  Safe from several host threads.  No counterpart in the reference.
+ */
+I8L_API void* i8l_status_open(const int32_t* word, int32_t* host);
+I8L_API int i8l_status_poll(void* poller, void* stream);
+
+/*
  * The GEMMs are persistent kernels with one CTA per SM (about 210 KB of shared memory each), so a kernel
  * launched beside one on another stream finds no free SM until the GEMM ends.  This sets, for the calling
  * host thread, the number of CTAs the following GEMM launches may use (0 = all SMs, the default): a

@@ -54,3 +54,21 @@ def test_no_cpu_fallback(lib):
     p = ctypes.addressof(buf); p += (16 - p % 16) % 16
     rc = lib.i8l_quant_tile(p, 1, 128, 128, 0, 0, 0, p, p, None, None, None)
     assert rc in (-3, -4)   # no device / wrong architecture: an error, never a CPU result
+
+
+def test_product_calls_validate_before_any_launch(lib):
+    """i8l_quant_gemm and i8l_linear_backward check extents, the combination of groupings and the workspace first."""
+    buf = ctypes.create_string_buffer(1 << 16)
+    p = ctypes.addressof(buf); p += (256 - p % 256) % 256
+
+    def product(M=128, a_gran=0, b_gran=2, ws_bytes=1 << 15, a_qt=None, batch=1):
+        return lib.i8l_quant_gemm(p, p, None, p, a_qt, a_qt, batch, M, 128, 128, 0, a_gran, b_gran, 0, 0, 1.0, 0, p, ws_bytes,
+                                  None, None)
+    assert product(M=100) == -1 and product(M=0) == -1
+    assert product(a_gran=2, b_gran=0) == -6 and product(b_gran=5) == -6 and product(a_qt=p, batch=2) == -6
+    assert product(ws_bytes=1 << 15) == -6 and b"too small" in lib.i8l_last_error()
+
+    def backward(gran=0, ws_bytes=1 << 15, x_qt=p):
+        return lib.i8l_linear_backward(p, p, x_qt, p, p, p, 128, 128, 128, gran, 0, 0, 1.0, 1.0, 0, p, ws_bytes, None, None)
+    assert backward() == -6 and b"too small" in lib.i8l_last_error()
+    assert backward(gran=5, ws_bytes=1 << 20) == -6 and backward(x_qt=None, ws_bytes=1 << 20) == -6

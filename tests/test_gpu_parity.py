@@ -466,10 +466,11 @@ def test_fast_block_epilogue_shift(kb, n, values, decade):
     K.check_status(DEV)
 
 
-@pytest.mark.parametrize("gran", [L.GRAN_TILE128, L.GRAN_GROUP128])
-def test_rotated_tile_quantizer_infinite_and_nan(gran):
+@pytest.mark.parametrize("scaling", ["tile128", "row128"])
+def test_rotated_tile_quantizer_infinite_and_nan(scaling):
     """A rotated group with a NaN is all NaN: it leaves the maximum alone and quantizes to 0; one with an infinity
     has scale factor 127/inf = 0 and quantizes to 0 with stored scale inf."""
+    gran = L.GRAN_TILE128 if scaling == "tile128" else L.GRAN_GROUP128
     g = torch.Generator().manual_seed(3)
     x = torch.randn(1, 256, 384, generator=g).to(torch.bfloat16)
     clean = x.clone()

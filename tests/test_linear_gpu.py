@@ -135,3 +135,34 @@ def test_linear_double_channel_matches_oracle_composition(had):
     assert torch.equal(dw.cpu(), ref(dy.t().contiguous(), x.t().contiguous()))
     exact = dy.float() @ w.float()
     assert R.rel_fro(dx.cpu().float(), exact) < 5e-2
+
+
+@pytest.mark.parametrize("scaling,had", [("tile128", 0), ("tile128", 128), ("row128", 0), ("row128", 128),
+                                         ("double_channel", 0), ("double_channel", 128)])
+def test_one_call_products_equal_the_separate_steps(scaling, had):
+    """linear_forward / linear_backward run a whole product per library call; the quantizers and GEMMs called one by
+    one give the same bits, with and without the transposed operand, and with either gradient alone."""
+    from triton_int8_b200 import _lib as L, kernels as K
+    from triton_int8_b200.linear import grad_input, grad_weight, quantize_grad_output
+    M, Kd, N = 384, 256, 640
+    x, w, dy, b = [t.to(DEV) for t in _data(M, Kd, N, seed=11)]
+    cfg = Int8Config(scaling=scaling, round="rne" if scaling == "row128" else "half_up", hadamard=had)
+    y, saved = linear_forward(x, w, b, cfg)
+    y_only, none = linear_forward(x, w, b, cfg, want_xt=False)
+    assert none == (None, None) and torch.equal(y, y_only)
+    if cfg.whole_k:
+        xq, xs = K.quant_row(x[None], L.QMODE_ROWRCP, had)
+        wq, ws = K.quant_row(w, L.QMODE_ROWRCP, had)
+        ref = K.gemm_rowcol(xq, wq, xs, ws, b, cfg.post)[0]
+        qt, st = K.quant_col_t(x, L.QMODE_ROWRCP, had)
+        qt, st = qt[None], st[None]
+    else:
+        xq, xs, qt, st = K.quant_tile(x[None], cfg.gran, cfg.qmode, had, transposed=True)
+        wq, ws = K.quant_row(w, cfg.qmode, had)
+        ref = K.gemm_block(xq, wq, xs, ws, cfg.a_kind, L.BSCALE_CHANNEL, b, cfg.post)[0]
+    assert torch.equal(y, ref) and torch.equal(saved[0], qt) and torch.equal(saved[1], st)
+    dx, dw = linear_backward(dy, w, saved, cfg)
+    dy_op, dyt_op = quantize_grad_output(dy, cfg)
+    assert torch.equal(dx, grad_input(dy_op, w, cfg)) and torch.equal(dw, grad_weight(dyt_op, saved, cfg))
+    assert torch.equal(linear_backward(dy, w, None, cfg, need_dw=False)[0], dx)
+    assert torch.equal(linear_backward(dy, w, saved, cfg, need_dx=False)[1], dw)

@@ -11,7 +11,7 @@ import os
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("I8L_LIBRARY_PATH") or os.path.join(_PKG_DIR, "libi8linear.so")
 
-OK = 0
+OK, TIMEOUT = 0, -5
 ERR_NAMES = {-1: "SHAPE", -2: "ALIGN", -3: "ARCH", -4: "CUDA", -5: "TIMEOUT", -6: "ARG"}
 
 GRAN_TILE128, GRAN_GROUP128, GRAN_ROW, GRAN_TILE128X256 = 0, 1, 2, 5
@@ -36,6 +36,10 @@ SIGNATURES = {
     "i8l_gemm_dump_i32": [_P, _P, _I, _P, _I64, _I64, _I64, _I64, _I, _P, _P],
     "i8l_gemm_block_scatter": [_P, _P, _P, _P, _I, _F, _P, _I, _I, _I64, _I64, _I64, _P, _P],
     "i8l_sum_slots": [_P, _P, _I, _I64, _I64, _P],
+    "i8l_quant_gemm": [_P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I, _I, _I, _I, _I, _F, _I, _P, _I64, _P, _P],
+    "i8l_linear_backward": [_P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I, _I, _I, _F, _F, _I, _P, _I64, _P, _P],
+    "i8l_status_open": [_P, _P],
+    "i8l_status_poll": [_P, _P],
     "i8l_set_cta_limit": [_I],
     "i8l_test_set_wait_limit": [ctypes.c_uint32, _I],
     "i8l_version": [],
@@ -49,6 +53,7 @@ class I8LError(RuntimeError):
 
 
 _lib = None
+_fns: dict = {}   # bound entry points by name
 
 
 def load() -> ctypes.CDLL:
@@ -66,12 +71,16 @@ def load() -> ctypes.CDLL:
             fn.restype = _I
         lib.i8l_last_error.argtypes = []
         lib.i8l_last_error.restype = ctypes.c_char_p
+        lib.i8l_status_open.restype = _P
         _lib = lib
+        _fns.update((name, getattr(lib, name)) for name in SIGNATURES)
     return _lib
 
 
 def call(name: str, *args) -> None:
-    lib = load()
-    rc = getattr(lib, name)(*args)
+    fn = _fns.get(name)
+    if fn is None:
+        fn = getattr(load(), name)
+    rc = fn(*args)
     if rc != OK:
-        raise I8LError(rc, lib.i8l_last_error().decode())
+        raise I8LError(rc, _lib.i8l_last_error().decode())

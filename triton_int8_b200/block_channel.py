@@ -61,6 +61,15 @@ def triton_per_token_quant(x: torch.Tensor, round: str = "half_up", hadamard: in
     return q, s.view(-1, 1)
 
 
+def _flags(out_dtype, exact: bool, product_first: bool = False) -> int:
+    if out_dtype not in (torch.bfloat16, torch.float32):
+        raise TypeError("out_dtype must be bfloat16 or float32")
+    flags = (L.GEMM_EXACT_ORDER if exact else 0) | (L.GEMM_OUT_F32 if out_dtype == torch.float32 else 0)
+    if exact and product_first:   # the TileLang kernels' order: float(P) * (a_s * b_s)
+        flags |= L.GEMM_PRODUCT_FIRST
+    return flags
+
+
 def triton_gemm(A_int8, B_int8, A_scale, B_scale, out_dtype=torch.bfloat16, exact: bool = False,
                 bias=None, post_scale: float = 1.0, product_first: bool = False):
     """C[b] = sum_kb float(A_q[b,:,kb] . B_q[:,kb]^T) * A_scale * B_scale.
@@ -84,12 +93,8 @@ def triton_gemm(A_int8, B_int8, A_scale, B_scale, out_dtype=torch.bfloat16, exac
     else:
         N = B_int8.shape[1]
         b_kind = L.BSCALE_TILE if B_scale.shape[1] == N // 128 else L.BSCALE_GROUP
-    flags = (L.GEMM_EXACT_ORDER if exact else 0) | (L.GEMM_OUT_F32 if out_dtype == torch.float32 else 0)
-    if exact and product_first:   # the TileLang kernels' order: float(P) * (a_s * b_s)
-        flags |= L.GEMM_PRODUCT_FIRST
-    if out_dtype not in (torch.bfloat16, torch.float32):
-        raise TypeError("out_dtype must be bfloat16 or float32")
-    return K.gemm_block(A_int8, B_int8, A_scale, B_scale, a_kind, b_kind, bias, post_scale, flags)
+    return K.gemm_block(A_int8, B_int8, A_scale, B_scale, a_kind, b_kind, bias, post_scale,
+                        _flags(out_dtype, exact, product_first))
 
 
 def int8_gemm_pipeline(A_bf, B_bf, out_dtype=torch.bfloat16, **kw):
@@ -112,14 +117,14 @@ def fwd_32(a: torch.Tensor, b: torch.Tensor, *, scaling: str = "tile128", round:
         # scale per 128 x 256, both scale tensors rounded to bf16, a_s * b_s formed first in every K step
         if hadamard or round != "half_up":
             raise ValueError("tile128x256_bf16scale is defined without rotation and with round half up")
-        aq, a_s = triton_per_block256_quant(a)
-        bq, b_s = triton_per_token_quant_bf16scale(b)
-        return triton_gemm(aq, bq, a_s, b_s, out_dtype, exact=exact, bias=bias, product_first=True)
-    quant_a = triton_per_block_quant if scaling == "tile128" else triton_per_group_quant
-    aq, a_s = quant_a(a, round=round, hadamard=hadamard)
-    bq, b_s = triton_per_token_quant(b, round=round, hadamard=hadamard)
-    return triton_gemm(aq, bq, a_s, b_s, out_dtype, exact=exact, bias=bias,
-                       post_scale=1.0 / hadamard if hadamard else 1.0)
+        assert a.dim() == 3 and b.dim() == 2
+        return K.quant_gemm(a, b, L.GRAN_TILE128X256, L.GRAN_ROW, L.QMODE_TRITON_BF16S, 0, bias, 1.0,
+                            _flags(out_dtype, exact, True))[0]
+    assert a.dim() == 3
+    assert b.dim() == 2 and b.shape[1] % 128 == 0
+    gran = L.GRAN_TILE128 if scaling == "tile128" else L.GRAN_GROUP128
+    return K.quant_gemm(a, b, gran, L.GRAN_ROW, _QMODE[round], hadamard, bias, 1.0 / hadamard if hadamard else 1.0,
+                        _flags(out_dtype, exact))[0]
 
 
 def bwd_33(a: torch.Tensor, b: torch.Tensor, *, scaling: str = "tile128", round: str = "half_up",
@@ -127,8 +132,7 @@ def bwd_33(a: torch.Tensor, b: torch.Tensor, *, scaling: str = "tile128", round:
     """a bf16 [B, M, K], b bf16 [B, N, K] -> bf16 [B, M, N] = a @ b^T per batch, both operands
     scaled per 128x128 tile.  triton/block_channel_bwd33.py:175-177."""
     tilelang = scaling == "tilelang_tile128"   # tilelang/block_channel_bwd.py:197-223: tile scales, a_s * b_s first
-    quant = triton_per_block_quant if scaling in ("tile128", "tilelang_tile128") else triton_per_group_quant
-    aq, a_s = quant(a, round=round, hadamard=hadamard)
-    bq, b_s = quant(b, round=round, hadamard=hadamard)
-    return triton_gemm(aq, bq, a_s, b_s, out_dtype, exact=exact, post_scale=1.0 / hadamard if hadamard else 1.0,
-                       product_first=tilelang)
+    assert a.dim() == 3 and b.dim() == 3
+    gran = L.GRAN_TILE128 if scaling in ("tile128", "tilelang_tile128") else L.GRAN_GROUP128
+    return K.quant_gemm(a, b, gran, gran, _QMODE[round], hadamard, None, 1.0 / hadamard if hadamard else 1.0,
+                        _flags(out_dtype, exact, tilelang))[0]

@@ -12,7 +12,7 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libi8linear.so")
-SOURCES = ["quant.cu", "gemm.cu", "fused.cu"]
+SOURCES = ["quant.cu", "gemm.cu", "fused.cu", "compose.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "ptx.cuh"),
            os.path.join(os.path.dirname(PKG_DIR), "include", "i8linear.h")]
 NVCC_FLAGS = [

@@ -31,6 +31,8 @@
 
 #include <atomic>
 #include <cstring>
+#include <mutex>
+#include <new>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -1161,6 +1163,56 @@ extern "C" int i8l_sum_slots(const void* slots, void* out, int world, int64_t ro
   sum_slots_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(slots),
                                                                         static_cast<uint4*>(out), world, n16);
   I8L_CUDA_OK(cudaGetLastError());
+  return I8L_OK;
+}
+
+// One device's status word with its pinned host copy: see i8l_status_poll.
+struct StatusPoller {
+  const int32_t* word;
+  volatile int32_t* host;
+  cudaEvent_t event;
+  bool pending;
+  std::mutex lock;
+};
+
+extern "C" void* i8l_status_open(const int32_t* word, int32_t* host) {
+  if (!word || !host) { fail(I8L_ERR_ARG, "null pointer"); return nullptr; }
+  StatusPoller* s = new (std::nothrow) StatusPoller;
+  if (!s) { fail(I8L_ERR_CUDA, "out of host memory"); return nullptr; }
+  s->word = word;
+  s->host = host;
+  s->pending = false;
+  cudaError_t e = cudaEventCreateWithFlags(&s->event, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    fail(I8L_ERR_CUDA, "cudaEventCreateWithFlags failed: %s", cudaGetErrorString(e));
+    delete s;
+    return nullptr;
+  }
+  return s;
+}
+
+extern "C" int i8l_status_poll(void* poller, void* stream) {
+  if (!poller) return fail(I8L_ERR_ARG, "null pointer");
+  StatusPoller* s = static_cast<StatusPoller*>(poller);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  I8L_CUDA_OK(cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return I8L_OK;
+  const std::unique_lock<std::mutex> hold(s->lock, std::try_to_lock);
+  if (!hold.owns_lock()) return I8L_OK;   // another thread is polling this device
+  if (s->pending) {
+    const cudaError_t e = cudaEventQuery(s->event);
+    if (e == cudaErrorNotReady) {
+      (void)cudaGetLastError();   // not an error: leave no trace for the launches that check
+      return I8L_OK;
+    }
+    I8L_CUDA_OK(e);
+    s->pending = false;
+    if (*s->host) return fail(I8L_ERR_TIMEOUT, "a bounded device-side wait gave up");
+  }
+  I8L_CUDA_OK(cudaMemcpyAsync(const_cast<int32_t*>(s->host), s->word, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  I8L_CUDA_OK(cudaEventRecord(s->event, st));
+  s->pending = true;
   return I8L_OK;
 }
 

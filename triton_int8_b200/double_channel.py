@@ -54,9 +54,9 @@ def int8_gemm_pipeline(A_bf, B_bf, out_dtype=torch.bfloat16, hadamard="full", bi
     had = _had(hadamard)
     Kd = A_bf.shape[-1]
     post = 1.0 / Kd if had == L.HAD_FULL else (1.0 / 128 if had == L.HAD_128 else 1.0)
-    aq, a_s = triton_per_row_quant_3d(A_bf, hadamard=hadamard)
-    bq, b_s = K.quant_row(B_bf, L.QMODE_ROWRCP, had)
-    return triton_gemm(aq, bq, a_s, b_s, out_dtype, post_scale=post, bias=bias)
+    assert A_bf.dim() == 3
+    return K.quant_gemm(A_bf, B_bf, L.GRAN_ROW, L.GRAN_ROW, L.QMODE_ROWRCP, had, bias, post,
+                        L.GEMM_OUT_F32 if out_dtype == torch.float32 else 0)[0]
 
 
 def fwd_32(a: torch.Tensor, b: torch.Tensor, *, hadamard="full", bias=None):

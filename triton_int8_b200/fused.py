@@ -28,13 +28,9 @@ def fused_int8_gemm(A_bf: torch.Tensor, B_bf: torch.Tensor, out_dtype=torch.bflo
         # consumes them (same integers and scales as below, N/128 resp. M/128 times the quantization work)
         flags = (L.GEMM_EXACT_ORDER if exact else 0) | (L.GEMM_OUT_F32 if out_dtype == torch.float32 else 0)
         return K.fused_gemm(A_bf, B_bf, flags)
-    aq, a_s, _, _ = K.quant_tile(A_bf, L.GRAN_TILE128, L.QMODE_FUSED)
     flags = L.GEMM_DIVIDE | (L.GEMM_EXACT_ORDER if exact else 0) | (L.GEMM_OUT_F32 if out_dtype == torch.float32 else 0)
-    if B_bf.dim() == 2:
-        bq, b_s, _, _ = K.quant_tile(B_bf[None], L.GRAN_GROUP128, L.QMODE_FUSED)
-        return K.gemm_block(aq, bq[0], a_s, b_s[0], L.ASCALE_TILE, L.BSCALE_GROUP, flags=flags)
-    bq, b_s, _, _ = K.quant_tile(B_bf, L.GRAN_TILE128, L.QMODE_FUSED)
-    return K.gemm_block(aq, bq, a_s, b_s, L.ASCALE_TILE, L.BSCALE_TILE, flags=flags)
+    b_gran = L.GRAN_GROUP128 if B_bf.dim() == 2 else L.GRAN_TILE128
+    return K.quant_gemm(A_bf, B_bf, L.GRAN_TILE128, b_gran, L.QMODE_FUSED, flags=flags)[0]
 
 
 def fwd_32(a: torch.Tensor, b: torch.Tensor, *, single_kernel: bool = False):

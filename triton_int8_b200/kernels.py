@@ -7,6 +7,10 @@ import torch
 from . import _lib as L
 
 
+_current_device = torch._C._cuda_getDevice
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def _ptr(t):
     return None if t is None else t.data_ptr()
 
@@ -18,8 +22,12 @@ def _call(name: str, dev: torch.device, *args, tensors=()) -> None:
     for t in tensors:
         if t is not None and t.device != dev:
             raise ValueError(f"{name}: operands on different devices ({t.device} vs {dev})")
-    with torch.cuda.device(dev):
-        L.call(name, *args, torch.cuda.current_stream(dev).cuda_stream)
+    index = dev.index
+    if index == _current_device():   # the usual case, without the context manager (4 us of host time)
+        L.call(name, *args, _raw_stream(index))
+    else:
+        with torch.cuda.device(dev):
+            L.call(name, *args, _raw_stream(index))
 
 
 # ---------------------------------------------------------------------------------------- status word
@@ -35,7 +43,10 @@ class _StatusWord:
         self.dev = dev
         self.word = torch.zeros(1, dtype=torch.int32, device=dev)
         self.host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self.event = None
+        with torch.cuda.device(dev):
+            self.poller = L.load().i8l_status_open(self.word.data_ptr(), self.host.data_ptr())
+        if not self.poller:
+            raise L.I8LError(-4, "i8l_status_open failed")
 
 
 def _status_of(dev: torch.device) -> "_StatusWord":
@@ -48,7 +59,7 @@ def _status_of(dev: torch.device) -> "_StatusWord":
 
 def device_status(dev) -> torch.Tensor:
     """The int32 status word that GEMMs on `dev` report into (0 = no wait has ever given up)."""
-    return _status_of(torch.device(dev)).word
+    return _status_of(dev if isinstance(dev, torch.device) else torch.device(dev)).word
 
 
 def _raise_if_set(st: "_StatusWord", code: int) -> None:
@@ -62,24 +73,23 @@ def check_status(dev=None) -> None:
     """Synchronous check: raises I8LError (code TIMEOUT) if a GEMM on `dev` gave up a wait since the
     last check, and clears the word."""
     st = _status_of(torch.device(dev if dev is not None else ("cuda", torch.cuda.current_device())))
-    st.event = None
     _raise_if_set(st, int(st.word.item()))
 
 
 def poll_status(dev) -> None:
     """Non-blocking check for hot loops: raises if the copy started by an earlier poll has completed and
     shows a timeout; then starts the next copy.  Does nothing while the stream is being captured."""
-    st = _status_of(torch.device(dev))
-    if torch.cuda.is_current_stream_capturing():
-        return
-    if st.event is not None:
-        if not st.event.query():
-            return
-        st.event = None
-        _raise_if_set(st, int(st.host[0]))
-    st.host.copy_(st.word, non_blocking=True)
-    st.event = torch.cuda.Event()
-    st.event.record(torch.cuda.current_stream(st.dev))
+    st = _status_of(dev if isinstance(dev, torch.device) else torch.device(dev))
+    index = st.dev.index
+    if index == _current_device():
+        rc = L.load().i8l_status_poll(st.poller, _raw_stream(index))
+    else:
+        with torch.cuda.device(st.dev):
+            rc = L.load().i8l_status_poll(st.poller, _raw_stream(index))
+    if rc:
+        if rc == L.TIMEOUT:
+            _raise_if_set(st, rc)
+        raise L.I8LError(rc, L.load().i8l_last_error().decode())
 
 
 def _check_bf16(x: torch.Tensor, name: str) -> torch.Tensor:
@@ -185,6 +195,75 @@ def fused_gemm(a_bf, b_bf, flags=0, status=None):
     _call("i8l_fused_gemm", a_bf.device, a_bf.data_ptr(), b_bf.data_ptr(), out.data_ptr(), B, M, N, K, int(bb), flags,
           _ptr(status), tensors=(b_bf, status))
     return out
+
+
+def _pad(n: int) -> int:
+    return (n + 255) & -256
+
+
+def _scale_count(gran: int, batch: int, rows: int, cols: int) -> int:
+    if gran == L.GRAN_TILE128:
+        return batch * (rows // 128) * (cols // 128)
+    if gran == L.GRAN_TILE128X256:
+        return batch * (rows // 128) * (cols // 256)
+    return batch * rows * (cols // 128) if gran == L.GRAN_GROUP128 else batch * rows
+
+
+def quant_gemm(a, b, a_gran, b_gran, qmode, hadamard=0, bias=None, post_scale=1.0, flags=0, want_at=False):
+    """bf16 a [B, M, K] x bf16 b [N, K] or [B, N, K] -> ([B, M, N], at): both quantizations and the GEMM in one call
+    of the library, the int8 operands in one workspace.  want_at (B = 1): at = (int8 a^T [1, K, M], its scales along M)
+    for linear_backward, else (None, None)."""
+    a, b = _check_bf16(a, "a"), _check_bf16(b, "b")
+    B, M, K = a.shape
+    bb = b.dim() == 3
+    N = b.shape[-2]
+    if b.shape[-1] != K or (bb and b.shape[0] != B):
+        raise ValueError(f"operand shapes do not match: {tuple(a.shape)} x {tuple(b.shape)}")
+    dev = a.device
+    out = torch.empty((B, M, N), dtype=torch.float32 if flags & L.GEMM_OUT_F32 else torch.bfloat16, device=dev)
+    nb = B if bb else 1
+    size = (_pad(B * M * K) + _pad(nb * N * K) + _pad(4 * _scale_count(a_gran, B, M, K)) +
+            _pad(4 * _scale_count(b_gran, nb, N, K)) + (_pad(4 * K) if want_at else 0))
+    ws = torch.empty(size, dtype=torch.int8, device=dev)
+    qt = st = None
+    if want_at:
+        qt = torch.empty((B, K, M), dtype=torch.int8, device=dev)
+        shape = (B, K // 128, M // 128) if a_gran == L.GRAN_TILE128 else ((B, K) if a_gran == L.GRAN_ROW else (B, K, M // 128))
+        st = torch.empty(shape, dtype=torch.float32, device=dev)
+    status = device_status(dev)
+    _call("i8l_quant_gemm", dev, a.data_ptr(), b.data_ptr(), _ptr(bias), out.data_ptr(), _ptr(qt), _ptr(st), B, M, N, K,
+          int(bb), a_gran, b_gran, qmode, hadamard, float(post_scale), flags, ws.data_ptr(), size, status.data_ptr(),
+          tensors=(b, bias))
+    return out, (qt, st)
+
+
+def linear_backward(dy, w, xt, gran, qmode, hadamard=0, post_dx=1.0, post_dw=1.0, flags=0, need_dx=True, need_dw=True):
+    """dy bf16 [M, N], w bf16 [N, K], xt from quant_gemm(want_at=True) -> (dx [M, K] or None, dw [N, K] or None), all
+    quantizations and both GEMMs in one call of the library."""
+    dy, w = _check_bf16(dy, "dy"), _check_bf16(w, "w")
+    M, N = dy.shape
+    K = w.shape[1]
+    if w.shape[0] != N:
+        raise ValueError(f"operand shapes do not match: {tuple(dy.shape)} x {tuple(w.shape)}")
+    dev = dy.device
+    dx = torch.empty((M, K), dtype=torch.bfloat16, device=dev) if need_dx else None
+    dw = torch.empty((N, K), dtype=torch.bfloat16, device=dev) if need_dw else None
+    xqt, xst = xt if need_dw else (None, None)
+    if need_dw:
+        xqt, xst = xqt.contiguous(), xst.contiguous()
+        if xqt.dtype != torch.int8 or tuple(xqt.shape) != (1, K, M):
+            raise ValueError(f"saved operand {xqt.dtype} {tuple(xqt.shape)} does not match dy {tuple(dy.shape)}, w {tuple(w.shape)}")
+    size = _pad(4 * max(K, N))
+    if need_dx:
+        size += _pad(M * N) + _pad(4 * _scale_count(gran, 1, M, N)) + _pad(K * N) + _pad(4 * K)
+    if need_dw:
+        size += _pad(N * M) + _pad(4 * _scale_count(gran, 1, N, M))
+    ws = torch.empty(size, dtype=torch.int8, device=dev)
+    status = device_status(dev)
+    _call("i8l_linear_backward", dev, dy.data_ptr(), w.data_ptr(), _ptr(xqt), _ptr(xst), _ptr(dx), _ptr(dw), M, N, K, gran,
+          qmode, hadamard, float(post_dx), float(post_dw), flags, ws.data_ptr(), size, status.data_ptr(),
+          tensors=(w, xqt, xst))
+    return dx, dw
 
 
 def gemm_dump_i32(aq, bq, per_block=False, status=None):

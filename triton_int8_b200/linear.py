@@ -81,10 +81,8 @@ def linear_forward(x2: torch.Tensor, weight: torch.Tensor, bias, cfg: Int8Config
         return _dc_forward(x2, weight, bias, cfg, want_xt)
     # one call yields X (groups / rotation along K) and, for dW, X^T (along the tokens); with per-tile scales
     # both come from a single read of X, rotated or not
-    xq, xs, xqt, xst = K.quant_tile(x2[None], cfg.gran, cfg.qmode, cfg.hadamard, natural=True, transposed=want_xt)
-    wq, ws = K.quant_row(weight, cfg.qmode, cfg.hadamard)
-    y = K.gemm_block(xq, wq, xs, ws, cfg.a_kind, L.BSCALE_CHANNEL, bias, cfg.post, cfg.flags)[0]
-    return y, (xqt, xst)
+    y, saved = K.quant_gemm(x2[None], weight, cfg.gran, L.GRAN_ROW, cfg.qmode, cfg.hadamard, bias, cfg.post, cfg.flags, want_xt)
+    return y[0], saved
 
 
 def _dc_transposed(t2: torch.Tensor, cfg: Int8Config):
@@ -99,14 +97,13 @@ def _dc_transposed(t2: torch.Tensor, cfg: Int8Config):
 
 def _dc_forward(x2, weight, bias, cfg: Int8Config, want_xt: bool):
     """double_channel forward: per-token and per-output-channel scales over all of K."""
-    Kd = x2.shape[1]
-    xq, xs = K.quant_row(x2[None], L.QMODE_ROWRCP, cfg.hadamard)
-    wq, ws = K.quant_row(weight, L.QMODE_ROWRCP, cfg.hadamard)
-    y = K.gemm_rowcol(xq, wq, xs, ws, bias, cfg.post_for(Kd))[0]
-    saved = (None, None)
-    if want_xt:   # dW operand: X^T [K, M], one scale per input feature over all tokens
+    # dW operand: X^T [K, M], one scale per input feature over all tokens
+    one_call = cfg.hadamard in (0, 128)
+    y, saved = K.quant_gemm(x2[None], weight, L.GRAN_ROW, L.GRAN_ROW, L.QMODE_ROWRCP, cfg.hadamard, bias,
+                            cfg.post_for(x2.shape[1]), 0, want_xt and one_call)
+    if want_xt and not one_call:
         saved = _dc_transposed(x2, cfg)
-    return y, saved
+    return y[0], saved
 
 
 def quantize_grad_output(dy2: torch.Tensor, cfg: Int8Config = DEFAULT, need_dx: bool = True, need_dw: bool = True):
@@ -142,6 +139,10 @@ def grad_weight(dyt_op, saved_xt, cfg: Int8Config = DEFAULT) -> torch.Tensor:
 def linear_backward(dy2: torch.Tensor, weight: torch.Tensor, saved_xt, cfg: Int8Config = DEFAULT,
                     need_dx: bool = True, need_dw: bool = True):
     """dy2 bf16 [M, N] -> (dx bf16 [M, K] or None, dw bf16 [N, K] or None)."""
+    if cfg.hadamard in (0, 128):
+        gran, qmode = (L.GRAN_ROW, L.QMODE_ROWRCP) if cfg.whole_k else (cfg.gran, cfg.qmode)
+        return K.linear_backward(dy2, weight, saved_xt, gran, qmode, cfg.hadamard, cfg.post_for(dy2.shape[1]),
+                                 cfg.post_for(dy2.shape[0]), 0 if cfg.whole_k else cfg.flags, need_dx, need_dw)
     dy_op, dyt_op = quantize_grad_output(dy2, cfg, need_dx, need_dw)
     dx = grad_input(dy_op, weight, cfg) if need_dx else None
     dw = grad_weight(dyt_op, saved_xt, cfg) if need_dw else None
@@ -152,12 +153,12 @@ class Int8LinearFn(torch.autograd.Function):
     """y = x @ weight^T + bias with all three GEMMs in INT8."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, cfg: Int8Config):
+    def forward(ctx, x, weight, bias, cfg: Int8Config, grad_enabled: bool = True):
         x2 = x.reshape(-1, x.shape[-1])
         # Every GEMM reports a device-side wait that gave up into the device's status word; look at it
         # here without blocking (the copy was started by the previous call) and raise if it is set.
         K.poll_status(x.device)
-        need_w = weight.requires_grad
+        need_w = grad_enabled and weight.requires_grad   # without a backward pass X^T is not made
         y, saved_xt = linear_forward(x2, weight, bias, cfg, want_xt=need_w)
         ctx.cfg = cfg
         ctx.x_shape = x.shape
@@ -172,7 +173,7 @@ class Int8LinearFn(torch.autograd.Function):
         need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         dx, dw = linear_backward(dy2, weight, tuple(saved) if saved else None, ctx.cfg, need_dx, need_dw)
         db = dy2.sum(0).to(dy.dtype) if ctx.has_bias and ctx.needs_input_grad[2] else None
-        return (dx.view(ctx.x_shape) if dx is not None else None), dw, db, None
+        return (dx.view(ctx.x_shape) if dx is not None else None), dw, db, None, None
 
 
 class Int8Linear(nn.Module):
@@ -196,7 +197,7 @@ class Int8Linear(nn.Module):
         return m
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return Int8LinearFn.apply(x, self.weight, self.bias, self.config)
+        return Int8LinearFn.apply(x, self.weight, self.bias, self.config, torch.is_grad_enabled())
 
     def extra_repr(self) -> str:
         return f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}, {self.config}"
