@@ -505,3 +505,22 @@ def test_row_quantizer_row_lengths(rows, cols, had):
         w[0, 5] = 0.0
         q_ref, s_ref = R.quant_token(w)
         _same(q, q_ref, "int8 with a NaN"); _same(s, s_ref.view(-1), "scale with a NaN")
+
+
+@pytest.mark.parametrize("rows,cols", [(3100, 256), (1600, 512), (801, 1024), (401, 2048), (197, 4096), (99, 8192), (49, 16384),
+                                       (5, 128), (70, 256), (3, 16384), (2, 32768)])
+def test_whole_row_rotation_both_kernels(rows, cols):
+    """Rows of every power of two on both sides of the size from which a CTA takes whole rows of 128 groups, with a
+    last CTA that is not full; a NaN or an infinity spoils its own row only."""
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, cols, generator=g).to(torch.bfloat16)
+    x[rows - 1, cols - 1], x[1, :] = 60.0, 0
+    q, s = K.quant_row(x.to(DEV), L.QMODE_ROWRCP, -1)
+    q_ref, s_ref = R.quant_row(R.hadamard(x, cols)[None])
+    _same(q, q_ref[0], "int8"); _same(s, s_ref.view(-1), "scale")
+    if rows >= 40:
+        x[2, 7], x[30, 9] = float("nan"), float("inf")
+        q2, s2 = K.quant_row(x.to(DEV), L.QMODE_ROWRCP, -1)
+        keep = [r for r in range(rows) if r not in (2, 30)]
+        assert torch.equal(q2[keep], q[keep]) and torch.equal(s2[keep], s[keep])
+        assert (q2[2] == 0).all() and (q2[30] == 0).all() and torch.isinf(s2[30])

@@ -119,21 +119,20 @@ __device__ __forceinline__ uint2 quant_piece(const uint4& u, float s) {
 // the low byte of the sum.  The saturating conversion runs on the slow conversion pipe, one value at a time.
 // It also turns NaN into 0, which this does not: infinite or NaN inputs take quant_piece.
 template <int MODE>
-__device__ __forceinline__ uint2 quant_piece_finite(const uint4& u, float s) {
+__device__ __forceinline__ uint32_t quant_pair_finite(uint32_t w, float s) {   // two bf16 -> two bytes
   const float2 s2 = make_float2(s, s), half2 = make_float2(0.5f, 0.5f), magic2 = make_float2(12582912.f, 12582912.f);
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-  uint32_t b[4];   // two bytes each
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 v = make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
-    float2 y;
-    if (MODE == I8L_QMODE_RNE)   // scalar products: a packed one is fused with the addition, which turns ties over
-      y = __fadd2_rn(make_float2(__fmul_rn(v.x, s), __fmul_rn(v.y, s)), magic2);
-    else
-      y = __fadd2_rd(__fadd2_rn(__fmul2_rn(v, s2), half2), magic2);
-    b[k] = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040);
-  }
-  return make_uint2(__byte_perm(b[0], b[1], 0x5410), __byte_perm(b[2], b[3], 0x5410));
+  const float2 v = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  float2 y;
+  if (MODE == I8L_QMODE_RNE)   // scalar products: a packed one is fused with the addition, which turns ties over
+    y = __fadd2_rn(make_float2(__fmul_rn(v.x, s), __fmul_rn(v.y, s)), magic2);
+  else
+    y = __fadd2_rd(__fadd2_rn(__fmul2_rn(v, s2), half2), magic2);
+  return __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040);
+}
+template <int MODE>
+__device__ __forceinline__ uint2 quant_piece_finite(const uint4& u, float s) {
+  return make_uint2(__byte_perm(quant_pair_finite<MODE>(u.x, s), quant_pair_finite<MODE>(u.y, s), 0x5410),
+                    __byte_perm(quant_pair_finite<MODE>(u.z, s), quant_pair_finite<MODE>(u.w, s), 0x5410));
 }
 
 __device__ __forceinline__ float bf16_bits_to_float(uint32_t b) { return __uint_as_float(b << 16); }

@@ -3,6 +3,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -271,19 +272,39 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// 128-point transform of p[k] = (x[k], x[k + 64]): spans 1..32 between the pairs, span 64 inside them, the
-// order of the CPU oracle.  Returns the results rounded to bf16, h[i] = (y[2i], y[2i+1]), and their |max|, NaN
-// if one of them is NaN.
-__device__ __forceinline__ float rot128(float2* p, uint32_t* h) {
+// Transform of p[k] = (x[k], x[k + N]) over 2N points but for the last span: spans 1..N/2 between the pairs, in the
+// order of the CPU oracle; the caller adds and subtracts the halves of each pair (span N).
+template <int N>
+__device__ __forceinline__ void fwht_pairs(float2* p) {
 #pragma unroll
-  for (int span = 1; span < 64; span <<= 1)
+  for (int span = 1; span < N; span <<= 1)
 #pragma unroll
-    for (int k = 0; k < 64; ++k)
+    for (int k = 0; k < N; ++k)
       if ((k & span) == 0) {
         const float2 a = p[k], b = p[k | span];
         p[k] = add2(a, b);
         p[k | span] = sub2(a, b);
       }
+}
+
+// 128 staged bf16 values of a row -> p[k] = (x[k], x[k + 64]).
+__device__ __forceinline__ void load_row128(const uint8_t* row, float2* p) {
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    float v[8];
+    unpack8(*reinterpret_cast<const uint4*>(row + 16 * c), v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (c < 8) p[8 * c + j].x = v[j];
+      else p[8 * (c - 8) + j].y = v[j];
+    }
+  }
+}
+
+// 128-point transform of p[k] = (x[k], x[k + 64]).  Returns the results rounded to bf16, h[i] = (y[2i], y[2i+1]), and their |max|, NaN
+// if one of them is NaN.
+__device__ __forceinline__ float rot128(float2* p, uint32_t* h) {
+  fwht_pairs<64>(p);
   __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
@@ -356,16 +377,7 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
   for (int ph = OUT_N ? 0 : 1; ph < (OUT_T ? 2 : 1); ++ph) {
     float2 p[64];
     if (ph == 0) {
-#pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        float v[8];
-        unpack8(*reinterpret_cast<const uint4*>(s_raw + tid * ROT_LD + 16 * c), v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (c < 8) p[8 * c + j].x = v[j];
-          else p[8 * (c - 8) + j].y = v[j];
-        }
-      }
+      load_row128(s_raw + tid * ROT_LD, p);
     } else {
       const uint8_t* col = s_raw + 2 * tid;
 #pragma unroll
@@ -583,16 +595,7 @@ quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int grou
   bool finite = true;
   if (live) {
     float2 p[64];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      float v[8];
-      unpack8(*reinterpret_cast<const uint4*>(s_raw + tid * ROT_LD + 16 * c), v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (c < 8) p[8 * c + j].x = v[j];
-        else p[8 * (c - 8) + j].y = v[j];
-      }
-    }
+    load_row128(s_raw + tid * ROT_LD, p);
     m = rot128(p, h);
     finite = m <= BF16_LARGEST;
     if (!finite) m = max_without_nan(h);
@@ -609,8 +612,143 @@ quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int grou
   else quant_store128<MODE, false>(h, s, out, align32);
 }
 
-// Whole-row Hadamard (power-of-two cols <= 32768): the row lives in shared memory as fp32.
-// Spans 1..64 run in registers/shuffles exactly as above, spans >= 128 as shared-memory passes.
+// Whole-row rotation of rows of G groups of 128 (G = 2..128).  A CTA takes 128/G whole rows.  Spans 1..64 run in
+// the registers of the thread that owns the group; one exchange through shared memory then gives thread i the
+// elements i, i + 128, ... of every row, where the remaining spans run in registers too.  Bytes of four neighbouring
+// positions are gathered by two shuffles per word, so that every store fills whole sectors.  Bound by issue and
+// latency (20 instructions per element, 12 warps per SM).  Against one CTA per row with a shared-memory pass per
+// span: [8192, 4096] 92 -> 45 us, [8192, 8192] 187 -> 80, [8192, 1024] 37 -> 21, [2048, 16384] 116 -> 46.
+template <int MODE, bool FINITE>
+__device__ __forceinline__ uint32_t quant_word(uint32_t h0, uint32_t h1, float s0, float s1) {
+  if (FINITE) return __byte_perm(quant_pair_finite<MODE>(h0, s0), quant_pair_finite<MODE>(h1, s1), 0x5410);
+  int q[4];
+  quant2<MODE>(make_float2(__uint_as_float(h0 << 16), __uint_as_float(h0 & 0xffff0000u)), make_float2(s0, s0), q[0], q[1]);
+  quant2<MODE>(make_float2(__uint_as_float(h1 << 16), __uint_as_float(h1 & 0xffff0000u)), make_float2(s1, s1), q[2], q[3]);
+  return pack4(q[0], q[1], q[2], q[3]);
+}
+
+constexpr int FULL_LD = 132;   // floats per staged group: 16-byte aligned, conflict-free both ways
+constexpr size_t FULL_SMEM = 128 * FULL_LD * sizeof(float);
+
+template <int MODE, int G>
+__global__ void __launch_bounds__(128, 3)
+quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8_t* __restrict__ q, float* __restrict__ scale) {
+  constexpr int R = 128 / G;   // rows per CTA
+  extern __shared__ __align__(16) float s_f[];   // [128][FULL_LD]; the bf16 input lies in it first
+  __shared__ __nv_bfloat16 s_red[R][4];
+  __shared__ float s_scale[R];
+  uint8_t* s_raw = reinterpret_cast<uint8_t*>(s_f);
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  const int64_t row0 = (int64_t)blockIdx.x * R;
+  const int n_rows = (int)(rows - row0 < R ? rows - row0 : R), n = n_rows * G;
+  {
+    const __nv_bfloat16* src = x + row0 * G * 128 + 8 * tid;   // whole rows are contiguous
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (i * 8 + (tid >> 4) < n) cp_async16(dst + i * 8 * ROT_LD, src + i * 1024);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  }
+  __syncthreads();
+  {
+    float2 p[64];
+    if (tid < n) {
+      load_row128(s_raw + tid * ROT_LD, p);
+    } else {   // rows past the end
+#pragma unroll
+      for (int k = 0; k < 64; ++k) p[k] = make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    fwht_pairs<64>(p);
+    float* out = s_f + tid * FULL_LD;
+#pragma unroll
+    for (int k = 0; k < 64; k += 4) {
+      *reinterpret_cast<float4*>(out + k) = make_float4(__fadd_rn(p[k].x, p[k].y), __fadd_rn(p[k + 1].x, p[k + 1].y),
+                                                        __fadd_rn(p[k + 2].x, p[k + 2].y), __fadd_rn(p[k + 3].x, p[k + 3].y));
+      *reinterpret_cast<float4*>(out + 64 + k) = make_float4(__fsub_rn(p[k].x, p[k].y), __fsub_rn(p[k + 1].x, p[k + 1].y),
+                                                             __fsub_rn(p[k + 2].x, p[k + 2].y), __fsub_rn(p[k + 3].x, p[k + 3].y));
+    }
+    __syncthreads();
+  }
+  // h[e / 2] = elements tid of groups e, e + 1 (e counts the groups of all rows), rounded to bf16
+  uint32_t h[64];
+  __nv_bfloat16 m[R];
+  bool finite = true;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float2 p[G / 2];
+#pragma unroll
+    for (int g = 0; g < G / 2; ++g) {
+      p[g].x = s_f[(r * G + g) * FULL_LD + tid];
+      p[g].y = s_f[(r * G + g + G / 2) * FULL_LD + tid];
+    }
+    fwht_pairs<G / 2>(p);
+    __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
+    if constexpr (G == 2) {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(__fadd_rn(p[0].x, p[0].y), __fsub_rn(p[0].x, p[0].y));
+      hm = __hmax2_nan(hm, __habs2(v));
+      h[r] = *reinterpret_cast<const uint32_t*>(&v);
+    } else {
+#pragma unroll
+      for (int g = 0; g < G / 2; g += 2) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(__fadd_rn(p[g].x, p[g].y), __fadd_rn(p[g + 1].x, p[g + 1].y));
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(__fsub_rn(p[g].x, p[g].y), __fsub_rn(p[g + 1].x, p[g + 1].y));
+        hm = __hmax2_nan(hm, __hmax2_nan(__habs2(lo), __habs2(hi)));
+        h[(r * G + g) / 2] = *reinterpret_cast<const uint32_t*>(&lo);
+        h[(r * G + g) / 2 + G / 4] = *reinterpret_cast<const uint32_t*>(&hi);
+      }
+    }
+    m[r] = __hmax_nan(__low2bfloat16(hm), __high2bfloat16(hm));
+    finite = finite && __bfloat162float(m[r]) <= BF16_LARGEST;
+  }
+  if (!finite) {   // the maximum leaves NaNs out
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < G / 2; ++i) hm = __hmax2(hm, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&h[r * G / 2 + i])));
+      m[r] = __hmax(__low2bfloat16(hm), __high2bfloat16(hm));
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r += 2) {   // two rows per shuffle
+    __nv_bfloat162 v = __halves2bfloat162(m[r], m[r + 1 < R ? r + 1 : r]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = __hmax2(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (l == 0) {
+      s_red[r][w] = __low2bfloat16(v);
+      if (r + 1 < R) s_red[r + 1][w] = __high2bfloat16(v);
+    }
+  }
+  __syncthreads();
+  if (tid < R) {
+    float s, stored;
+    const float mm = fmaxf(fmaxf(__bfloat162float(s_red[tid][0]), __bfloat162float(s_red[tid][1])),
+                           fmaxf(__bfloat162float(s_red[tid][2]), __bfloat162float(s_red[tid][3])));
+    make_scale<MODE>(mm, s, stored);
+    s_scale[tid] = s;
+    if (tid < n_rows) scale[row0 + tid] = stored;
+  }
+  __syncthreads();
+  int8_t* out = q + row0 * G * 128 + (tid & 3) * 128 + 4 * (tid >> 2);
+  auto write = [&](auto finite_c) {
+    constexpr bool FINITE = decltype(finite_c)::value;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {   // groups 4k..4k+3: one byte each of position tid -> four positions of group 4k + lane % 4
+      const uint32_t a = quant_word<MODE, FINITE>(h[2 * k], h[2 * k + 1], s_scale[4 * k / G], s_scale[(4 * k + 2) / G]);
+      const uint32_t b = __shfl_xor_sync(0xffffffffu, a, 1);
+      const uint32_t c = __byte_perm(a, b, (l & 1) ? 0x3715 : 0x6240);
+      const uint32_t d = __shfl_xor_sync(0xffffffffu, c, 2);
+      if (4 * k + (tid & 3) < n)
+        *reinterpret_cast<uint32_t*>(out + 4 * k * 128) = __byte_perm(c, d, (l & 2) ? 0x3276 : 0x5410);
+    }
+  };
+  if (__all_sync(0xffffffffu, finite)) write(std::true_type{});   // one branch per warp: the shuffles need all lanes
+  else write(std::false_type{});
+}
+
+// Whole-row Hadamard, one CTA per row (few rows, or rows of 32768 elements): the row lives in shared memory as fp32.
+// Spans 1..64 run in registers/shuffles, spans >= 128 as shared-memory passes.
 template <int MODE>
 __global__ void __launch_bounds__(256)
 quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __restrict__ q,
@@ -671,6 +809,54 @@ quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8
 
 // ------------------------------------------------------------------------------------------------ host
 constexpr int MAX_DEVICES = 64;
+static int device_ordinal() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return (dev < 0 || dev >= MAX_DEVICES) ? 0 : dev;
+}
+// Raises a kernel's dynamic shared-memory limit once per device (function attributes are per device;
+// the call is idempotent, so two threads racing here only repeat it).
+template <typename Kernel>
+static cudaError_t ensure_smem(Kernel kernel, std::atomic<bool>* done_per_device, size_t bytes) {
+  std::atomic<bool>& done = done_per_device[device_ordinal()];
+  if (done.load(std::memory_order_acquire)) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.store(true, std::memory_order_release);
+  return e;
+}
+
+template <int MODE, int G>
+static int launch_rotfull(const __nv_bfloat16* x, int64_t rows, int8_t* q, float* scale, cudaStream_t st) {
+  static std::atomic<bool> attr_done[MAX_DEVICES];
+  I8L_CUDA_OK(ensure_smem(quant_row_rotfull_kernel<MODE, G>, attr_done, FULL_SMEM));
+  constexpr int R = 128 / G;
+  quant_row_rotfull_kernel<MODE, G><<<(unsigned)((rows + R - 1) / R), 128, FULL_SMEM, st>>>(x, rows, q, scale);
+  I8L_CUDA_OK(cudaGetLastError());
+  return I8L_OK;
+}
+template <int MODE>
+static int launch_hadfull(const __nv_bfloat16* x, int64_t rows, int64_t cols, int8_t* q, float* scale, cudaStream_t st) {
+  // Few rows do not fill the chip with 128 groups per CTA, and a group per thread is the longer chain: below 3/4 M
+  // elements one CTA per row is faster ([512, 256] 7 against 10 us, [1000, 512] 9.4 / 10.2, [1000, 1024] 10.6 / 10.2,
+  // [512, 4096] 14.3 / 11.8), and it takes rows of 32768, more groups than a CTA of the other has threads.
+  if (rows * cols >= 3ll << 18) switch (cols / 128) {
+    case 2: return launch_rotfull<MODE, 2>(x, rows, q, scale, st);
+    case 4: return launch_rotfull<MODE, 4>(x, rows, q, scale, st);
+    case 8: return launch_rotfull<MODE, 8>(x, rows, q, scale, st);
+    case 16: return launch_rotfull<MODE, 16>(x, rows, q, scale, st);
+    case 32: return launch_rotfull<MODE, 32>(x, rows, q, scale, st);
+    case 64: return launch_rotfull<MODE, 64>(x, rows, q, scale, st);
+    case 128: return launch_rotfull<MODE, 128>(x, rows, q, scale, st);
+    default: break;
+  }
+  static std::atomic<bool> attr_done[MAX_DEVICES];
+  const size_t smem = (size_t)cols * sizeof(float);
+  I8L_CUDA_OK(ensure_smem(quant_row_hadfull_kernel<MODE>, attr_done, 32768 * sizeof(float)));
+  quant_row_hadfull_kernel<MODE><<<(unsigned)rows, 256, smem, st>>>(x, cols, q, scale);
+  I8L_CUDA_OK(cudaGetLastError());
+  return I8L_OK;
+}
+
 static int check_dims(int64_t batch, int64_t rows, int64_t cols) {
   if (batch <= 0 || rows <= 0 || cols <= 0 || rows % 128 || cols % 128)
     return fail(I8L_ERR_SHAPE, "batch=%lld rows=%lld cols=%lld: all must be positive and rows, cols multiples of 128",
@@ -762,20 +948,15 @@ extern "C" int i8l_quant_row(const void* x, int64_t rows, int64_t cols, int qmod
   if (hadamard == I8L_HAD_FULL) {
     if ((cols & (cols - 1)) || cols > 32768)
       return fail(I8L_ERR_SHAPE, "full Hadamard needs cols a power of two <= 32768, got %lld", (long long)cols);
-    const size_t smem = (size_t)cols * sizeof(float);
-#define I8L_HF_CASE(Mo)                                                                                        \
-  if (qmode == Mo) {                                                                                           \
-    I8L_CUDA_OK(cudaFuncSetAttribute(quant_row_hadfull_kernel<Mo>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     (int)smem));                                                              \
-    quant_row_hadfull_kernel<Mo><<<(unsigned)rows, 256, smem, st>>>(xp, cols, q, scale);                       \
-    I8L_CUDA_OK(cudaGetLastError());                                                                           \
-    return I8L_OK;                                                                                             \
-  }
-    I8L_HF_CASE(I8L_QMODE_TRITON)
-    I8L_HF_CASE(I8L_QMODE_RNE)
-    I8L_HF_CASE(I8L_QMODE_ROWRCP)
-#undef I8L_HF_CASE
-    return fail(I8L_ERR_ARG, "i8l_quant_row: unsupported qmode=%d", qmode);
+    if (cols > 128) {
+      if (qmode == I8L_QMODE_TRITON) return launch_hadfull<I8L_QMODE_TRITON>(xp, rows, cols, q, scale, st);
+      if (qmode == I8L_QMODE_RNE) return launch_hadfull<I8L_QMODE_RNE>(xp, rows, cols, q, scale, st);
+      if (qmode == I8L_QMODE_ROWRCP) return launch_hadfull<I8L_QMODE_ROWRCP>(xp, rows, cols, q, scale, st);
+      return fail(I8L_ERR_ARG, "i8l_quant_row: unsupported qmode=%d", qmode);
+    }
+    if (qmode != I8L_QMODE_TRITON && qmode != I8L_QMODE_RNE && qmode != I8L_QMODE_ROWRCP)
+      return fail(I8L_ERR_ARG, "i8l_quant_row: unsupported qmode=%d", qmode);
+    hadamard = I8L_HAD_128;   // a row of 128 is one group
   }
   if (hadamard != I8L_HAD_NONE && hadamard != I8L_HAD_128) return fail(I8L_ERR_ARG, "bad hadamard=%d", hadamard);
   // Rows of up to 16384 elements stay on chip; longer ones are swept twice.  Threads per row: the fewest that hold
