@@ -524,3 +524,42 @@ def test_whole_row_rotation_both_kernels(rows, cols):
         keep = [r for r in range(rows) if r not in (2, 30)]
         assert torch.equal(q2[keep], q[keep]) and torch.equal(s2[keep], s[keep])
         assert (q2[2] == 0).all() and (q2[30] == 0).all() and torch.isinf(s2[30])
+
+
+@pytest.mark.parametrize("kb,n,values,decade", [(1, 256, "random", 0), (2, 384, "random", 0), (5, 128, "random", 30), (6, 640, "random", -25),
+                                                (3, 256, "lowest", 0), (4, 256, "opposite", 0)])
+@pytest.mark.parametrize("b_kind", ["channel", "tile", "group", "column"])
+def test_row_and_column_factor_epilogues(kb, n, values, decade, b_kind):
+    """Per-(row, K block) A scales with every kind of B scale, and per-tile A scales with per-(column, K block) ones
+    ("column", as products and, for moderate sizes, as divisors).  The shifted partial product is brought back exactly, so
+    each K block costs three fp32 roundings (product of the scales, of the factors, the sum) and the end three more."""
+    g = torch.Generator().manual_seed(200 + kb)
+    M, Kd = 256, 128 * kb
+    aq, bq = _randq(g, 1, M, Kd), _randq(g, n, Kd)
+    if values == "lowest":
+        aq.fill_(-128), bq.fill_(-128)
+    elif values == "opposite":
+        aq.fill_(-128), bq.fill_(127)
+    P = torch.stack([R.int_mm(aq[0, :, k * 128:(k + 1) * 128], bq[:, k * 128:(k + 1) * 128]) for k in range(kb)]).double()
+    if b_kind == "column":
+        a_s = (torch.rand(1, M // 128, kb, generator=g) + 0.5) * 10.0 ** decade
+        fa = a_s[0].double().t().repeat_interleave(128, 1)[:, :, None]
+    else:
+        a_s = (torch.rand(1, M, kb, generator=g) + 0.5) * 10.0 ** decade
+        fa = a_s[0].double().t()[:, :, None]
+    if b_kind == "channel":
+        b_s, kind = torch.rand(n, generator=g) + 0.5, L.BSCALE_CHANNEL
+        fb = b_s.double().view(1, 1, n)
+    elif b_kind == "tile":
+        b_s, kind = torch.rand(n // 128, kb, generator=g) + 0.5, L.BSCALE_TILE
+        fb = b_s.double().t().repeat_interleave(128, 1)[:, None, :]
+    else:
+        b_s, kind = torch.rand(n, kb, generator=g) + 0.5, L.BSCALE_GROUP
+        fb = b_s.double().t()[:, None, :]
+    a_kind = L.ASCALE_TILE if b_kind == "column" else L.ASCALE_GROUP
+    modes = [(0, fa * fb)] + ([(L.GEMM_DIVIDE, 1.0 / (fa * fb))] if b_kind == "column" and decade == 0 else [])
+    for flag, f in modes:
+        ref, mag = (P * f).sum(0), (P * f).abs().sum(0)
+        out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), a_kind, kind, flags=L.GEMM_OUT_F32 | flag)[0].cpu().double()
+        assert ((out - ref).abs() <= (3 * kb + 3) * 2.0 ** -24 * mag).all(), float(((out - ref).abs() / mag.clamp_min(1e-300)).max())
+    K.check_status(DEV)

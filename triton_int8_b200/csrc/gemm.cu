@@ -54,7 +54,9 @@ template <bool TWO> struct Cfg {
 };
 constexpr int MAX_STAGES = 6;
 constexpr int MAX_EPI_WARPS = 16;             // groups of four warps share the 256 accumulator columns
-template <int KIND> constexpr int EPI_WARPS_OF = KIND == 2 /* K_BLOCK_FAST */ ? 8 : MAX_EPI_WARPS;
+// the kinds whose partial products are shifted by an extra MMA (K_BLOCK_FAST and the row and column factor kinds)
+template <int KIND> constexpr bool SHIFTED_OF = KIND >= 2;
+template <int KIND> constexpr int EPI_WARPS_OF = SHIFTED_OF<KIND> ? 8 : MAX_EPI_WARPS;
 constexpr int FAC_MAX = 256;                  // K blocks whose factors are staged in shared memory at a time (a multiple of 4)
 constexpr int TMEM_COLS = 512;
 constexpr int SMEM_DYN = 4 * (A_STAGE + BN * BK) + 1024;  // == 6 * (16 KB + 16 KB) + 1024
@@ -123,7 +125,7 @@ struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fa
   // scatter mode of the fast block kind: four output rows x 128 bytes per epilogue warp, staged so that one
   // store instruction writes whole 128-byte row segments into the peer's memory
   uint4 xpose[EPI_WARPS_OF<2>][4][8];
-  // K_BLOCK_FAST: 256 rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
+  // shifted kinds: 256 rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
   __align__(256) uint8_t ones[BN * 32];
 };
 
@@ -131,35 +133,21 @@ struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fa
 constexpr int K_ROWCOL = 0;      // one drain per tile, (float(acc)*a_s[m])*b_s[n]
 constexpr int K_BLOCK_GEN = 1;   // block-scaled, any scale layout, reference operation order, dumps
 constexpr int K_BLOCK_FAST = 2;  // block-scaled, one scalar factor per (tile, K block) and 64-column group
-constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x per-tile or per-channel B scale
 constexpr int K_BLOCK_COLFAC = 3;  // block-scaled, per-tile A scale x per-(column, K block) B scale (fused forward)
-// K_BLOCK_FAST: 32 products 255 * 255.  A partial product of 128 int8 pairs lies in [-128*128*127, 128*128*128],
+constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x per-tile or per-channel B scale
+constexpr int K_BLOCK_OUTER = 5;   // block-scaled, per-(row, K block) A scale x per-(column, K block) B scale
+// Shifted kinds: 32 products 255 * 255.  A partial product of 128 int8 pairs lies in [-128*128*127, 128*128*128],
 // so P + SHIFT lies in [32, 4177952]: never negative and below 2^23, where the bits of an int32, read as a
 // float, are the (denormal) number (P + SHIFT) * 2^-149 exactly.
 constexpr float SHIFT_F = 2080800.f;
 constexpr int FAC_EXP = 100;   // factors are scaled by a power of two that puts the tile's largest one near 2^100
 __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
 
-constexpr uint32_t MAGIC_I = 0x4B400000u;   // the bits of 1.5 * 2^23
-constexpr float MAGIC_F = 12582912.f;       // 1.5 * 2^23
-
-// Sixteen int32 partial products (|P| < 2^22) -> fp32, exactly.  The conversion instruction runs at half
-// rate on one pipe; MAGIC_I + P read as a float is 1.5*2^23 + P, and subtracting 1.5*2^23 (a packed add on
-// the other pipe) gives the same float(P).  Alternating the two forms between chunks balances the pipes
-// (measured 6 % faster than either alone).
-__device__ __forceinline__ void to_float16(bool via_add, const uint32_t* r, float* v) {
-  if (via_add) {
-    const float2 nm = make_float2(-MAGIC_F, -MAGIC_F);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float2 t = __fadd2_rn(make_float2(__uint_as_float(MAGIC_I + r[2 * j]), __uint_as_float(MAGIC_I + r[2 * j + 1])), nm);
-      v[2 * j] = t.x;
-      v[2 * j + 1] = t.y;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = __int2float_rn((int)r[j]);
-  }
+// Two shifted partial products as they come from tensor memory -> P * 2^-23, exactly, by one packed FMA.
+constexpr float FROM_SHIFTED = 8388608.f;   // 2^23, multiplied in at the tile end: factors of any size stay finite
+__device__ __forceinline__ float2 from_shifted(uint32_t r0, uint32_t r1) {
+  const float up = 0x1p126f, off = -SHIFT_F * 0x1p-23f;
+  return __ffma2_rn(make_float2(__uint_as_float(r0), __uint_as_float(r1)), make_float2(up, up), make_float2(off, off));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
@@ -221,7 +209,7 @@ template <int KIND, bool TWO>
 __global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND>, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const GemmParams p) {
-  constexpr bool BLOCK = KIND != K_ROWCOL;
+  constexpr bool BLOCK = KIND != K_ROWCOL, SHIFTED = SHIFTED_OF<KIND>;
   constexpr int EPI_WARPS = EPI_WARPS_OF<KIND>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
   constexpr int STAGES = Cfg<TWO>::STAGES, B_STAGE = Cfg<TWO>::B_STAGE;
   constexpr uint32_t STAGE_TX = Cfg<TWO>::STAGE_TX;
@@ -239,7 +227,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #define I8L_UNIT (TWO ? (int)(blockIdx.x >> 1) : (int)blockIdx.x)
 #define I8L_N_UNITS (TWO ? (int)(gridDim.x >> 1) : (int)gridDim.x)
 
-  if constexpr (KIND == K_BLOCK_FAST) {
+  if constexpr (SHIFTED) {
     for (int i = threadIdx.x; i < (int)sizeof(ctl.ones) / 16; i += THREADS)
       reinterpret_cast<uint4*>(ctl.ones)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -251,9 +239,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&ctl.tfull[b]), 1);
-      // arrivals that free an accumulator buffer: one per epilogue warp (of both CTAs of a pair); the fast
-      // block kernel lets every epilogue thread arrive for itself (no warp sync, no branch in its loop)
-      mbar_init(smem_u32(&ctl.tempty[b]), KIND == K_BLOCK_FAST ? EPI_WARPS * 32 : (TWO ? 2 : 1) * EPI_WARPS);
+      // arrivals that free an accumulator buffer: one per epilogue warp (of both CTAs of a pair); the shifted
+      // kinds let every epilogue thread arrive for itself (no warp sync, no branch in their loop)
+      mbar_init(smem_u32(&ctl.tempty[b]), SHIFTED ? EPI_WARPS * 32 : (TWO ? 2 : 1) * EPI_WARPS);
     }
     mbar_init(smem_u32(&ctl.done), 1);
     for (int b = 0; b < 2; ++b) {
@@ -365,11 +353,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (lane == 0) {
             const uint64_t da = smem_desc(smem_a + s * A_STAGE), db = smem_desc(smem_b + s * B_STAGE);
             const uint32_t d = tmem_base + ab * BN;
-            if (KIND == K_BLOCK_FAST) tc_mma_i8(d, ones_desc, ones_desc, IDESC_U8, 0u);   // D = SHIFT, see the epilogue
+            if (SHIFTED) tc_mma_i8(d, ones_desc, ones_desc, IDESC_U8, 0u);   // D = SHIFT, see the epilogue
 #pragma unroll
             for (int k4 = 0; k4 < BK / 32; ++k4) {
               if (TWO) tc_mma_i8_pair(d, da + 2 * k4, db + 2 * k4, IDESC_I8_PAIR, (k4 > 0 || !drain_start) ? 1u : 0u);
-              else tc_mma_i8(d, da + 2 * k4, db + 2 * k4, IDESC_I8, (KIND == K_BLOCK_FAST || k4 > 0 || !drain_start) ? 1u : 0u);
+              else tc_mma_i8(d, da + 2 * k4, db + 2 * k4, IDESC_I8, (SHIFTED || k4 > 0 || !drain_start) ? 1u : 0u);
             }
             if (TWO) {  // both CTAs' producers and epilogues wait on their own copies of these barriers
               tc_commit_pair(smem_u32(&ctl.empty[s]));
@@ -428,7 +416,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const bool with_b = !chan && tc.n_tile * BN + h * (BN / 2) < p.N;
             const float* bs_ptr = p.b_scale + ((bcol0 >> 7) + h) * KB;
             auto factor = [&](int d) {
-              return __ldg(as_ptr + (d >> p.a_kshift)) * (with_b ? __ldg(bs_ptr + d) * p.post_scale : 1.f);
+              const float a = __ldg(as_ptr + (d >> p.a_kshift));
+              if (!with_b) return a;
+              if (p.divide) return __frcp_rn(a * __ldg(bs_ptr + d)) * p.post_scale;
+              return a * (__ldg(bs_ptr + d) * p.post_scale);
             };
             float2* fac = ctl.fac[buf][h];
             if (k0 == 0) {
@@ -476,7 +467,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else {
     // -------------------------------------------------------------------- epilogue
     // 128 x 64 + 256 x 208 of the 384 x 168 registers of the launch; 128 x 64 + 512 x 104 of 640 x 96
-    if (KIND == K_BLOCK_FAST) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    if (SHIFTED) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     const int q = warp & 3, wg = (warp - 4) >> 2;  // lane quarter, column group
     const int tix = q * 32 + lane;                 // row within the tile == thread index within the group
@@ -643,112 +634,81 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         named_sync(1 + wg, 128);
       }
 
-      if constexpr (KIND == K_BLOCK_ROWFAC) {
-        // one factor a_s * b_s per (row or tile, K block) and column group, fetched by each thread
-        const float* as_ptr = p.a_scale + (p.a_kind == I8L_ASCALE_TILE ? (int64_t)tc.m_blk : row) * KB;
-        const float* bs_ptr = p.b_scale + (bcol0 >> 7) * KB;
-        float2 acc[EPI_COLS / 2];
-#pragma unroll
-        for (int j = 0; j < EPI_COLS / 2; ++j) acc[j] = make_float2(0.f, 0.f);
-        float f_next = __ldg(as_ptr) * ((!chan && active) ? __ldg(bs_ptr) : 1.f);
-        for (int d = 0; d < KB; ++d) {
-          const float f = f_next;
-          if (d + 1 < KB) f_next = __ldg(as_ptr + d + 1) * ((!chan && active) ? __ldg(bs_ptr + d + 1) : 1.f);
-          ok = ok && mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls);  // single-exit loop, see K_BLOCK_FAST
-          tc_fence_after();
-          if (ok && active) {
-            const uint32_t taddr = tmem_base + lane_addr + ab * BN + wg * EPI_COLS;
-            const float2 f2 = make_float2(f, f);
-#pragma unroll
-            for (int c = 0; c < EPI_COLS / 16; ++c) {
-              uint32_t r[16];
-              tc_ld16(taddr + c * 16, r);
-              tc_ld_wait();
-              if (c == EPI_COLS / 16 - 1) release_accumulator();
-              // one conversion and half a packed FMA per accumulator element; each pass is a run of
-              // independent instructions
-              float v[16];
-              to_float16((c & 1) != 0, r, v);   // c is an unrolled loop index: the choice folds at compile time
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                acc[c * 8 + j] = __ffma2_rn(make_float2(v[2 * j], v[2 * j + 1]), f2, acc[c * 8 + j]);
-            }
-          } else {
-            release_accumulator();
-          }
-          ab ^= 1;
-          if (ab == 0) aph ^= 1u;
-        }
-        if (ok && active) {
-          float out[EPI_COLS];
-#pragma unroll
-          for (int j = 0; j < EPI_COLS / 2; ++j) {
-            out[2 * j] = acc[j].x;
-            out[2 * j + 1] = acc[j].y;
-          }
-          store_cols<EPI_COLS>(p, out, chan ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
-        }
-      } else if constexpr (KIND == K_BLOCK_COLFAC) {
-        constexpr bool COLFAC = true;
-        // factor of a K block: a_s * b_s, or its reciprocal when the scales are multipliers (fused
-        // variants: acc += P / (s_a * s_b); the reciprocal replaces the reference's division, 1 ulp)
-        const float* as_ptr = p.a_scale + (p.a_kind == I8L_ASCALE_TILE ? (int64_t)tc.m_blk : row) * KB;
-        const int64_t bcol = bcol0 + (tix & (EPI_COLS - 1));  // COLFAC: the column whose factor this thread publishes
-        const float* bs_ptr = COLFAC ? p.b_scale + (p.b_kind == I8L_BSCALE_GROUP ? bcol : bcol >> 7) * KB
-                                     : p.b_scale + (bcol0 >> 7) * KB;
-        const bool use_b = COLFAC ? active : (!chan && active);
-        const bool recip = COLFAC && p.divide;
-        auto factor = [&](int d) {
+      if constexpr (SHIFTED) {
+        // Before, with sixteen warps converting on two pipes, and now, 8192^3: row x channel 787 -> 662 us, column
+        // 1051 -> 862; row x column took the generic path: 4020 -> 896.
+        // A factor per row, per column or both for every K block.  Two packed FMAs per two elements (the first
+        // brings P back from its shift), a packed product more for row x column factors.  Row factors live in the
+        // thread that owns the row; column factors (a_s * b_s or its reciprocal when the scales are multipliers, the
+        // fused forward: acc += P / (s_a * s_b)) are published through shared memory, one column per thread.
+        constexpr bool ROWF = KIND != K_BLOCK_COLFAC, COLF = KIND != K_BLOCK_ROWFAC;
+        constexpr int CH = 32;
+        static_assert(EPI_COLS == 128, "a thread of the group publishes one column");
+        const float* as_ptr = p.a_scale + (ROWF ? row : (int64_t)tc.m_blk) * KB;
+        const float* bc_ptr = p.b_scale + (p.b_kind == I8L_BSCALE_GROUP ? bcol0 + tix : (bcol0 + tix) >> 7) * KB;   // COLF
+        const float* bt_ptr = p.b_scale + (bcol0 >> 7) * KB;                                                       // ROWFAC, per tile
+        auto row_factor = [&](int d) {
           float f = __ldg(as_ptr + d);
-          if (use_b) f *= __ldg(bs_ptr + d);
-          if (COLFAC) f = recip ? __frcp_rn(f) : f;
+          if (!COLF && !chan && active) f *= __ldg(bt_ptr + d);
           return f;
+        };
+        auto col_factor = [&](int d) {
+          float f = active ? __ldg(bc_ptr + d) : 1.f;
+          if (ROWF) return f;
+          f *= __ldg(as_ptr + d);
+          return p.divide ? __frcp_rn(f) : f;
         };
         float2 acc[EPI_COLS / 2];
 #pragma unroll
         for (int j = 0; j < EPI_COLS / 2; ++j) acc[j] = make_float2(0.f, 0.f);
-        float f_next = factor(0);
-        for (int d = 0; d < KB; ++d) {
-          const float f = f_next;
-          if (d + 1 < KB) f_next = factor(d + 1);
-          if (COLFAC) {  // thread i < 64 publishes the factor of column i of this group for this K block
-            if (tix < EPI_COLS) ctl.bstep[d & 1][wg * EPI_COLS + tix] = f;
+        float fr_next = ROWF ? row_factor(0) : 0.f, fc_next = COLF ? col_factor(0) : 0.f;
+        for (int d = 0; d < KB; ++d) {   // single exit, see K_BLOCK_FAST
+          const float2 fr = make_float2(fr_next, fr_next);
+          if (COLF) {
+            ctl.bstep[d & 1][wg * EPI_COLS + tix] = fc_next;
             named_sync(1 + wg, 128);
           }
-          ok = ok && mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls);  // single-exit loop, see K_BLOCK_FAST
+          if (d + 1 < KB) {
+            if (ROWF) fr_next = row_factor(d + 1);
+            if (COLF) fc_next = col_factor(d + 1);
+          }
+          mbar_spin_or_flag(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls);
           tc_fence_after();
-          if (ok && active) {
+          auto release = [&]() {
+            tc_fence_before();
+            mbar_arrive(smem_u32(&ctl.tempty[ab]));
+          };
+          if (active) {
             const uint32_t taddr = tmem_base + lane_addr + ab * BN + wg * EPI_COLS;
-            const float2 f2 = make_float2(f, f);
             const float2* fcol = reinterpret_cast<const float2*>(ctl.bstep[d & 1] + wg * EPI_COLS);
 #pragma unroll
-            for (int c = 0; c < EPI_COLS / 16; ++c) {
-              uint32_t r[16];
-              tc_ld16(taddr + c * 16, r);
+            for (int c = 0; c < EPI_COLS / CH; ++c) {
+              uint32_t r[CH];
+              tc_ld16(taddr + c * CH, r);
+              tc_ld16(taddr + c * CH + 16, r + 16);
               tc_ld_wait();
-              if (c == EPI_COLS / 16 - 1) release_accumulator();
-              // one conversion and half a packed FMA per accumulator element; each pass is a run of
-              // independent instructions
-              float v[16];
-              to_float16((c & 1) != 0, r, v);   // c is an unrolled loop index: the choice folds at compile time
+              if (c == EPI_COLS / CH - 1) release();
 #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                acc[c * 8 + j] = __ffma2_rn(make_float2(v[2 * j], v[2 * j + 1]), COLFAC ? fcol[c * 8 + j] : f2, acc[c * 8 + j]);
+              for (int j = 0; j < CH / 2; ++j) {
+                float2 f = fr;
+                if (COLF) f = ROWF ? __fmul2_rn(fcol[c * (CH / 2) + j], fr) : fcol[c * (CH / 2) + j];
+                acc[c * (CH / 2) + j] = __ffma2_rn(from_shifted(r[2 * j], r[2 * j + 1]), f, acc[c * (CH / 2) + j]);
+              }
             }
           } else {
-            release_accumulator();
+            release();
           }
           ab ^= 1;
           if (ab == 0) aph ^= 1u;
         }
-        if (ok && active) {
+        if (active && __all_sync(0xffffffffu, !*abort_flag)) {
           float out[EPI_COLS];
 #pragma unroll
           for (int j = 0; j < EPI_COLS / 2; ++j) {
-            out[2 * j] = acc[j].x;
-            out[2 * j + 1] = acc[j].y;
+            out[2 * j] = acc[j].x * FROM_SHIFTED;
+            out[2 * j + 1] = acc[j].y * FROM_SHIFTED;
           }
-          store_cols<EPI_COLS>(p, out, (!COLFAC && chan) ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
+          store_cols<EPI_COLS>(p, out, !COLF && chan ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
         }
       } else {
         // ---- generic paths: reference operation order, per-column / per-step scales, dumps, row x column
@@ -1064,12 +1024,17 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
     p.raster = two ? blocks / 2 : blocks;
   }
   const int64_t tiles = (int64_t)(two ? p.m_blocks / 2 : p.m_blocks) * p.n_tiles;
-  const bool scalar_factor = block && !p.exact && !p.dump && !p.divide && p.b_kind != I8L_BSCALE_GROUP;
+  // one factor per (row, K block) and 128 columns; as divisors only with per-tile A scales (fused backward)
+  const bool scalar_factor = block && !p.exact && !p.dump && p.b_kind != I8L_BSCALE_GROUP &&
+                             (!p.divide || p.a_kind == I8L_ASCALE_TILE);
   const bool column_factor = block && !p.exact && !p.dump && !scalar_factor && p.a_kind == I8L_ASCALE_TILE &&
                              p.b_kind != I8L_BSCALE_CHANNEL;
+  const bool outer_factor = block && !p.exact && !p.dump && !p.divide && p.a_kind == I8L_ASCALE_GROUP &&
+                            p.b_kind == I8L_BSCALE_GROUP;
   if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, p, tiles, st);
   if (scalar_factor && p.a_kind == I8L_ASCALE_TILE) return launch_kind<K_BLOCK_FAST, false>(ma, mb, p, tiles, st);
   if (scalar_factor) return launch_kind<K_BLOCK_ROWFAC, false>(ma, mb, p, tiles, st);
+  if (outer_factor) return launch_kind<K_BLOCK_OUTER, false>(ma, mb, p, tiles, st);
   if (column_factor) return launch_kind<K_BLOCK_COLFAC, false>(ma, mb, p, tiles, st);
   return launch_kind<K_BLOCK_GEN, false>(ma, mb, p, tiles, st);
 }
