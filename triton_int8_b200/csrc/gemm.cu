@@ -112,16 +112,17 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int m_units, const GemmPa
 
 struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[2], tempty[2], done;
-  uint64_t fready[2], ffree[2];  // fast block kind: factor buffers written (factor warp) / consumed (every epilogue thread)
+  // fast block kind: factors written (factor warp), what the tile end needs written, all consumed (every epilogue thread)
+  uint64_t fready[2], eready[2], ffree[2];
   uint32_t tmem_base;
   int abort_flag;
   float bscale[BN];     // per-tile column scales (CHANNEL)
   float bstep[2][BN];   // per-K-block column scales (GROUP), double buffered
   // K_BLOCK_FAST, written by the factor warp one unit (tile, or FAC_MAX-K-block chunk of a tile) ahead, two
-  // buffers; each 128-column half (one epilogue group) has its factors:
-  float2 fac[2][2][FAC_MAX];                 // per K block: scaled factor, and the correction due at it (or 0)
-  float fbscale[2][BN];                      // per-channel column scales (times post_scale)
-  float fend[2][2][3];                       // tile end: what the corrections left over, and 2^-exponent as two factors
+  // buffers; each 128-column half (one epilogue group) has its factors (both share the first with per-channel B scales):
+  float2 fac[2][2][FAC_MAX];   // per K block: scaled factor, and the correction due at it (or 0)
+  float fbscale[2][BN];        // what the sums are multiplied by at the end: per-channel column scale times post_scale, or 1
+  float2 fend[2][2];           // in front of that: times .x plus .y (undoes the scaling of the factors, takes out what is left of the shift)
   // scatter mode of the fast block kind: four output rows x 128 bytes per epilogue warp, staged so that one
   // store instruction writes whole 128-byte row segments into the peer's memory
   uint4 xpose[EPI_WARPS_OF<2>][4][8];
@@ -135,6 +136,7 @@ constexpr int K_BLOCK_GEN = 1;   // block-scaled, any scale layout, reference op
 constexpr int K_BLOCK_FAST = 2;  // block-scaled, one scalar factor per (tile, K block) and 64-column group
 constexpr int K_BLOCK_COLFAC = 3;  // block-scaled, per-tile A scale x per-(column, K block) B scale (fused forward)
 constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x per-tile or per-channel B scale
+constexpr int K_BLOCK_TILEDIV = 6; // block-scaled, per-tile scales on both sides as divisors (fused backward)
 constexpr int K_BLOCK_OUTER = 5;   // block-scaled, per-(row, K block) A scale x per-(column, K block) B scale
 // Shifted kinds: 32 products 255 * 255.  A partial product of 128 int8 pairs lies in [-128*128*127, 128*128*128],
 // so P + SHIFT lies in [32, 4177952]: never negative and below 2^23, where the bits of an int32, read as a
@@ -233,6 +235,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_a);
+    prefetch_tensormap(&map_b);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&ctl.full[s]), 1);
       mbar_init(smem_u32(&ctl.empty[s]), 1);
@@ -246,6 +250,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     mbar_init(smem_u32(&ctl.done), 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&ctl.fready[b]), 1);
+      mbar_init(smem_u32(&ctl.eready[b]), 1);
       mbar_init(smem_u32(&ctl.ffree[b]), EPI_WARPS * 32);
     }
     ctl.abort_flag = 0;
@@ -391,7 +396,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // over- or underflows whatever the scales are.  SHIFT * F_d is taken out four K blocks at a time, after the
       // second of them: the accumulators then stay within two K blocks' shift (4.2e6 f) of the true sum, an ulp of
       // which is at most f/2.  What the rounded corrections leave over is summed in fp64 and goes out at the tile end.
-      // Hand-over through two mbarrier pairs (buffer written / buffer consumed), waits bounded like all others.
+      // Hand-over through mbarrier pairs (factors written, tile-end values written / buffer consumed), waits bounded like
+      // all others.  The factors go out first: a kernel of one tile per CTA waits for them (3.2 us after its start when
+      // everything was handed over at once).
       const bool chan = p.b_kind == I8L_BSCALE_CHANNEL;
       constexpr double SHIFT_D = (double)SHIFT_F * 0x1p-149;
       uint32_t u = 0;
@@ -399,8 +406,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const TileCoord tc = unit_tile(t);
         const int64_t bcol0 = (int64_t)(p.b_batched ? tc.m_blk / p.mpb : 0) * p.N + tc.n_tile * BN;
         const float* as_ptr = p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift);
-        float up0[2], up1[2];       // 2^e as two factors
-        double left[2] = {0., 0.};  // per lane, over the chunks of the tile
+        const int halves = chan ? 1 : 2;   // with per-channel B scales a factor is the A scale alone
+        float up0[2], up1[2], down0[2], down1[2];   // 2^e and 2^(149 - e), as two factors each
+        double left[2] = {0., 0.};                  // per lane, over the chunks of the tile
         for (int k0 = 0; k0 < KB; k0 += FAC_MAX, ++u) {
           const int dn = KB - k0 < FAC_MAX ? KB - k0 : FAC_MAX;
           const int buf = u & 1;
@@ -408,38 +416,44 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             t = total_tiles;   // gave up (or another warp did): leave both loops
             break;
           }
-          if (chan)   // post_scale rides on the column scale (on the factors otherwise)
-            for (int i = lane; i < BN; i += 32)
-              ctl.fbscale[buf][i] = tc.n_tile * BN + i < p.N ? __ldg(p.b_scale + bcol0 + i) * p.post_scale : 0.f;
+          auto factor = [&](int h, int d) {
+            const float a = __ldg(as_ptr + (d >> p.a_kshift));
+            if (chan || tc.n_tile * BN + h * (BN / 2) >= p.N) return a;   // no second half: a number that does no harm
+            return a * (__ldg(p.b_scale + ((bcol0 >> 7) + h) * KB + d) * p.post_scale);
+          };
+          if (k0 == 0) {
+            float m[2] = {0.f, 0.f};
+            for (int i = lane; i < KB; i += 32)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const bool with_b = !chan && tc.n_tile * BN + h * (BN / 2) < p.N;
-            const float* bs_ptr = p.b_scale + ((bcol0 >> 7) + h) * KB;
-            auto factor = [&](int d) {
-              const float a = __ldg(as_ptr + (d >> p.a_kshift));
-              if (!with_b) return a;
-              if (p.divide) return __frcp_rn(a * __ldg(bs_ptr + d)) * p.post_scale;
-              return a * (__ldg(bs_ptr + d) * p.post_scale);
-            };
-            float2* fac = ctl.fac[buf][h];
-            if (k0 == 0) {
-              float m = 0.f;
-              for (int i = lane; i < KB; i += 32) {
-                const float f = factor(i);
-                if (i < dn) fac[i].x = f;
-                m = fmaxf(m, fabsf(f));
+              for (int h = 0; h < 2; ++h) {
+                if (h < halves) {
+                  const float f = factor(h, i);
+                  if (i < dn) ctl.fac[buf][h][i].x = f;
+                  m[h] = fmaxf(m[h], fabsf(f));
+                }
               }
 #pragma unroll
-              for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-              const int e = FAC_EXP + 127 - (int)(__float_as_uint(m) >> 23);
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) m[h] = fmaxf(m[h], __shfl_xor_sync(0xffffffffu, m[h], o));
+              const int e = FAC_EXP + 127 - (int)(__float_as_uint(m[h]) >> 23), back = 149 - e;
               up0[h] = pow2f(e >> 1);
               up1[h] = pow2f(e - (e >> 1));
-              if (lane < 2) ctl.fend[buf][h][1 + lane] = pow2f(lane ? (149 - e) - ((149 - e) >> 1) : (149 - e) >> 1);
-            } else {
-              for (int i = lane; i < dn; i += 32) fac[i].x = factor(k0 + i);
-              if (lane < 2) ctl.fend[buf][h][1 + lane] = ctl.fend[buf ^ 1][h][1 + lane];
+              // the sums are far below 1, so the first factor may take all of it, up to the largest power there is
+              down0[h] = pow2f(back < 127 ? back : 127);
+              down1[h] = pow2f(back < 127 ? 0 : back - 127);
             }
-            __syncwarp();
+          } else {
+            for (int i = lane; i < dn; i += 32)
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                if (h < halves) ctl.fac[buf][h][i].x = factor(h, k0 + i);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (h >= halves) continue;
+            float2* fac = ctl.fac[buf][h];
             for (int i = lane; i < (dn + 3) / 4; i += 32) {   // one lane per four K blocks
               float f4[4];
               double sum = 0.;
@@ -454,13 +468,25 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               for (int j = 0; j < 4; ++j)
                 if (4 * i + j < dn) fac[4 * i + j] = make_float2(f4[j], j == 2 ? corr : 0.f);
             }
-            double all = left[h];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-            if (lane == 0) ctl.fend[buf][h][0] = (float)all;
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&ctl.fready[buf]));   // release: the warp's writes above are visible to waiters
+          if (lane == 0) mbar_arrive(smem_u32(&ctl.fready[buf]));   // the K blocks may start; the rest is due at the tile end
+          if (k0 + dn == KB) {
+            for (int i = lane; i < BN; i += 32) {
+              const float d = (chan || i < BN / 2) ? down1[0] : down1[1];
+              ctl.fbscale[buf][i] = chan && tc.n_tile * BN + i < p.N ? __ldg(p.b_scale + bcol0 + i) * p.post_scale * d : d;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              double all = left[chan ? 0 : h];
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+              const float d = down0[chan ? 0 : h];
+              if (lane == 0) ctl.fend[buf][h] = make_float2(d, -(float)all * d);
+            }
+            __syncwarp();
+          }
+          if (lane == 0) mbar_arrive(smem_u32(&ctl.eready[buf]));   // every chunk, so that one count gives all parities
         }
       }
     }
@@ -493,9 +519,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // Values derived from the thread index pass through an empty asm statement: the compiler then
       // keeps them in registers instead of recomputing them from the special register at every use
       // inside the K-block loop (which cost about 35 ALU instructions per warp and K block).
-      uint32_t taddr0 = tmem_base + lane_addr + wg * EPI_COLS, fac_base = smem_u32(&ctl.fac[0][wg][0]);
+      uint32_t taddr0 = tmem_base + lane_addr + wg * EPI_COLS, fac_base = smem_u32(&ctl.fac[0][p.b_kind == I8L_BSCALE_CHANNEL ? 0 : wg][0]);
       asm volatile("" : "+r"(taddr0), "+r"(fac_base));
-      const bool chan = p.b_kind == I8L_BSCALE_CHANNEL;
       constexpr int CH = 32;
       uint32_t gstep = 0, unit = 0;
       // The loops below never exit early (one exit and nothing to carry but the accumulators compiles to the
@@ -561,18 +586,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         // after a timeout the accumulators are not a product: nothing is stored (decided per warp: the store
         // path below synchronises the warp)
+        mbar_wait_or_flag(smem_u32(&ctl.eready[unit & 1]), (unit >> 1) & 1u, abort_flag, p.max_polls);
         if (active && __all_sync(0xffffffffu, !*abort_flag)) {
           int t2 = t;
           asm volatile("" : "+r"(t2));  // keeps the tile's coordinates out of the K-block loop's live registers
           const TileCoord tc = unit_tile(t2);
-          const float* fe = ctl.fend[unit & 1][wg];
-          const float left = fe[0], down0 = fe[1], down1 = fe[2];
-          float out[EPI_COLS];
-#pragma unroll
-          for (int j = 0; j < EPI_COLS / 2; ++j) {
-            out[2 * j] = __fsub_rn(acc[j].x, left) * down0 * down1;
-            out[2 * j + 1] = __fsub_rn(acc[j].y, left) * down0 * down1;
-          }
           int64_t row = (int64_t)tc.m_blk * BM + tix;
           void* cbase = p.c;
           if (p.rs_rows) {  // scatter mode: this 128-row block belongs to rank `owner`; write into our slot of its buffer
@@ -580,7 +598,16 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             cbase = p.c_slots[owner];
             row += (int64_t)(p.rs_rank - owner) * p.rs_rows;
           }
-          const float* bsc = chan ? ctl.fbscale[unit & 1] + wg * EPI_COLS : nullptr;
+          const float2 fe = ctl.fend[unit & 1][wg];
+          const float2 fe_mul = make_float2(fe.x, fe.x), fe_add = make_float2(fe.y, fe.y);
+          const float4* bsc4 = reinterpret_cast<const float4*>(ctl.fbscale[unit & 1] + wg * EPI_COLS);
+          float2 out[EPI_COLS / 2];
+#pragma unroll
+          for (int j = 0; j < EPI_COLS / 4; ++j) {
+            const float4 bs = bsc4[j];
+            out[2 * j] = __fmul2_rn(__ffma2_rn(acc[2 * j], fe_mul, fe_add), make_float2(bs.x, bs.y));
+            out[2 * j + 1] = __fmul2_rn(__ffma2_rn(acc[2 * j + 1], fe_mul, fe_add), make_float2(bs.z, bs.w));
+          }
           const int col0 = tc.n_tile * BN + wg * EPI_COLS;
           if (p.rs_rows && !p.out_f32 && !p.bias) {
             // Peer stores.  A lane owns one row, so a plain store instruction would send 32 separate 32-byte
@@ -594,11 +621,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int h = 0; h < EPI_COLS; h += 64) {
               uint32_t w[32];
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                float a = out[h + 2 * j], b = out[h + 2 * j + 1];
-                if (bsc) { a *= bsc[h + 2 * j]; b *= bsc[h + 2 * j + 1]; }
-                w[j] = pack_bf16x2(a, b);
-              }
+              for (int j = 0; j < 32; ++j) w[j] = pack_bf16x2(out[h / 2 + j].x, out[h / 2 + j].y);
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 if ((lane >> 2) == j) {
@@ -613,7 +636,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               }
             }
           } else {
-            store_cols<EPI_COLS, false>(p, out, bsc, row, col0, cbase);
+            store_cols<EPI_COLS, false>(p, reinterpret_cast<const float*>(out), nullptr, row, col0, cbase);
           }
         }
         mbar_arrive(smem_u32(&ctl.ffree[unit & 1]));   // this tile's factors and column scales are no longer needed
@@ -641,16 +664,16 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // brings P back from its shift), a packed product more for row x column factors.  Row factors live in the
         // thread that owns the row; column factors (a_s * b_s or its reciprocal when the scales are multipliers, the
         // fused forward: acc += P / (s_a * s_b)) are published through shared memory, one column per thread.
-        constexpr bool ROWF = KIND != K_BLOCK_COLFAC, COLF = KIND != K_BLOCK_ROWFAC;
+        constexpr bool ROWF = KIND != K_BLOCK_COLFAC, COLF = KIND == K_BLOCK_COLFAC || KIND == K_BLOCK_OUTER;
         constexpr int CH = 32;
         static_assert(EPI_COLS == 128, "a thread of the group publishes one column");
-        const float* as_ptr = p.a_scale + (ROWF ? row : (int64_t)tc.m_blk) * KB;
+        const float* as_ptr = p.a_scale + (ROWF && KIND != K_BLOCK_TILEDIV ? row : (int64_t)tc.m_blk) * KB;
         const float* bc_ptr = p.b_scale + (p.b_kind == I8L_BSCALE_GROUP ? bcol0 + tix : (bcol0 + tix) >> 7) * KB;   // COLF
         const float* bt_ptr = p.b_scale + (bcol0 >> 7) * KB;                                                       // ROWFAC, per tile
         auto row_factor = [&](int d) {
           float f = __ldg(as_ptr + d);
           if (!COLF && !chan && active) f *= __ldg(bt_ptr + d);
-          return f;
+          return KIND == K_BLOCK_TILEDIV ? __frcp_rn(f) : f;
         };
         auto col_factor = [&](int d) {
           float f = active ? __ldg(bc_ptr + d) : 1.f;
@@ -1024,7 +1047,9 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
     p.raster = two ? blocks / 2 : blocks;
   }
   const int64_t tiles = (int64_t)(two ? p.m_blocks / 2 : p.m_blocks) * p.n_tiles;
-  // one factor per (row, K block) and 128 columns; as divisors only with per-tile A scales (fused backward)
+  // One factor per (row or tile, K block) and 128 columns.  Divisors (fused backward, per-tile A scales only) take the
+  // exact conversion of the row kind: the fast kind's running shift rounds to about 7e-6, the fused variants are held
+  // to 1e-6.
   const bool scalar_factor = block && !p.exact && !p.dump && p.b_kind != I8L_BSCALE_GROUP &&
                              (!p.divide || p.a_kind == I8L_ASCALE_TILE);
   const bool column_factor = block && !p.exact && !p.dump && !scalar_factor && p.a_kind == I8L_ASCALE_TILE &&
@@ -1032,7 +1057,8 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   const bool outer_factor = block && !p.exact && !p.dump && !p.divide && p.a_kind == I8L_ASCALE_GROUP &&
                             p.b_kind == I8L_BSCALE_GROUP;
   if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, p, tiles, st);
-  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE) return launch_kind<K_BLOCK_FAST, false>(ma, mb, p, tiles, st);
+  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && !p.divide) return launch_kind<K_BLOCK_FAST, false>(ma, mb, p, tiles, st);
+  if (scalar_factor && p.divide) return launch_kind<K_BLOCK_TILEDIV, false>(ma, mb, p, tiles, st);
   if (scalar_factor) return launch_kind<K_BLOCK_ROWFAC, false>(ma, mb, p, tiles, st);
   if (outer_factor) return launch_kind<K_BLOCK_OUTER, false>(ma, mb, p, tiles, st);
   if (column_factor) return launch_kind<K_BLOCK_COLFAC, false>(ma, mb, p, tiles, st);
