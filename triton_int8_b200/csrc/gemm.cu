@@ -3,7 +3,7 @@
 //
 // One persistent CTA per SM, 384 threads (fast block-scaled kind) or 640 (the others):
 //   warp 0      TMA producer (one elected lane)
-//   warp 1      tensor-memory allocator + MMA issuer (one elected lane)
+//   warp 1      tensor-memory allocator + MMA issuer (one elected lane, see elect_one)
 //   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the per-K-block
 //               factors, corrections and column scales the epilogue needs; idle in the other kinds
 //   warp 3      idle (completes the first warpgroup so register budgets can be rebalanced)
@@ -339,6 +339,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1 && leader) {
       // ------------------------------------------------------------------ MMA issuer
       const uint64_t ones_desc = smem_desc_sw32(smem_u32(ctl.ones));
+      const bool elected = elect_one();
       int s = 0, ab = 0;
       uint32_t ph = 0, aph = 0;
       bool ok = true;
@@ -355,7 +356,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.tempty[ab]), aph ^ 1u, abort_flag, p.max_polls))) break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          if (elected) {
             const uint64_t da = smem_desc(smem_a + s * A_STAGE), db = smem_desc(smem_b + s * B_STAGE);
             const uint32_t d = tmem_base + ab * BN;
             if (SHIFTED) tc_mma_i8(d, ones_desc, ones_desc, IDESC_U8, 0u);   // D = SHIFT, see the epilogue
@@ -381,7 +382,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
       // all MMAs issued by this thread must have retired before tensor memory is freed
-      if (lane == 0) {
+      if (elected) {
         if (TWO) tc_commit_pair_local(smem_u32(&ctl.done));
         else tc_commit(smem_u32(&ctl.done));
       }
