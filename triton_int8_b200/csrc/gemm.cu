@@ -346,20 +346,24 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       for (int t = I8L_UNIT; t < total_tiles && ok; t += I8L_N_UNITS) {
         for (int kb = 0; kb < KB; ++kb) {
           const bool drain_start = BLOCK || kb == 0, drain_end = BLOCK || kb == KB - 1;
-          // block-scaled kinds wait for the accumulator buffer last (the epilogue's release is what holds
-          // the next MMA up); the whole-K kinds measured 0.7 % faster the other way round
+          // the generic block kind waits for the accumulator buffer last; the whole-K kinds measured 0.7 % faster the
+          // other way round, the shifted kinds 1 % (8192^3 458 -> 454 us) with their first MMA in between
           if (!BLOCK && drain_start) {
             if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.tempty[ab]), aph ^ 1u, abort_flag, p.max_polls))) break;
           }
+          if (SHIFTED) {   // D = SHIFT (see the epilogue) needs the buffer only: it goes out ahead of the operands' wait
+            if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.tempty[ab]), aph ^ 1u, abort_flag, p.max_polls))) break;
+            tc_fence_after();
+            if (elected) tc_mma_i8(tmem_base + ab * BN, ones_desc, ones_desc, IDESC_U8, 0u);
+          }
           if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.full[s]), ph, abort_flag, p.max_polls))) break;
-          if (BLOCK) {
+          if (BLOCK && !SHIFTED) {
             if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.tempty[ab]), aph ^ 1u, abort_flag, p.max_polls))) break;
           }
           tc_fence_after();
           if (elected) {
             const uint64_t da = smem_desc(smem_a + s * A_STAGE), db = smem_desc(smem_b + s * B_STAGE);
             const uint32_t d = tmem_base + ab * BN;
-            if (SHIFTED) tc_mma_i8(d, ones_desc, ones_desc, IDESC_U8, 0u);   // D = SHIFT, see the epilogue
 #pragma unroll
             for (int k4 = 0; k4 < BK / 32; ++k4) {
               if (TWO) tc_mma_i8_pair(d, da + 2 * k4, db + 2 * k4, IDESC_I8_PAIR, (k4 > 0 || !drain_start) ? 1u : 0u);
