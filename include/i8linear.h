@@ -140,11 +140,16 @@ I8L_API int i8l_quant_col_t_static(const void* x, int64_t rows, int64_t cols, in
 
 #define I8L_GEMM_EXACT_ORDER 1 /* per K step evaluate (float(P)*a_s)*b_s then add, unfused: bit-equal to the
                                   reference's fp32 result.  Without it the K-invariant factor is applied once
-                                  at the end, multiply-adds are fused and, for per-tile A scales with per-tile or
-                                  per-channel B scales, the int32 partials enter the fp32 sum through a bounded
-                                  bias that is removed at the end of the tile (same int32 partials; fp32 result
-                                  within 1e-4 relative of the exact sum at K = 32768, typically 1e-6; scale
-                                  products times 1.3e7 must stay finite in fp32). */
+                                  at the end and multiply-adds are fused.  For per-tile A scales with per-tile or
+                                  per-channel B scales the int32 partials enter the fp32 sum shifted by a constant that
+                                  is taken out again.  Its rounding is absolute: with f the largest factor of the tile
+                                  (A scale, times B scale if that is per tile), each K block adds at most f/4, distinct
+                                  factors as good as randomly (rms 0.5 f at K = 8192, 1 f at 32768; at most 4 f seen).  That is
+                                  1e-5 of a typical result; a row whose products are zero comes out within it, not at
+                                  0, and one that is zero where the tile has a scale R times the others has R times
+                                  the error.  Factors that repeat are exact: an all-zero tile gives 0.  The other
+                                  scale layouts (GROUP, DIVIDE) take P itself, scaled by 2^-23 until the end of the tile:
+                                  scale products below 2^-103 lose bits, which no quantizer here produces. */
 #define I8L_GEMM_DIVIDE 2      /* scales are multipliers s: acc += float(P) / (a_s*b_s)  (fused variants); together with
                                   EXACT_ORDER a true division per element, otherwise a multiplication by the rounded
                                   reciprocal of a_s*b_s (differs from the division by at most 1 ulp per K block) */

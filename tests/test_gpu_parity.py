@@ -563,3 +563,65 @@ def test_row_and_column_factor_epilogues(kb, n, values, decade, b_kind):
         out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), a_kind, kind, flags=L.GEMM_OUT_F32 | flag)[0].cpu().double()
         assert ((out - ref).abs() <= (3 * kb + 3) * 2.0 ** -24 * mag).all(), float(((out - ref).abs() / mag.clamp_min(1e-300)).max())
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("kb,n,share", [(1, 256, 1.0), (3, 128, 1.0), (8, 384, 1.0), (64, 256, 1.0), (258, 128, 1.0), (64, 384, 0.5),
+                                        (256, 256, 0.25)])
+@pytest.mark.parametrize("kind", ["channel", "tile"])
+def test_fast_block_epilogue_repeated_factors(kb, n, share, kind):
+    """A factor that repeats (an all-zero 128-row block, whose scales sit on the quantizers' floor; clipped data) must not
+    let the roundings of the shift add up along K.  Where all factors are equal nothing is rounded but the sum itself:
+    zero rows give exactly zero and small constant partial products their exact sum, times c and the column scale (three
+    roundings).  Where `share` of them are, the other K blocks round like distinct ones: three roundings in four K blocks, each
+    within a quarter of the factor and uniform (standard deviation f / 7), so five standard deviations of their sum
+    for the rows whose products are zero."""
+    g = torch.Generator().manual_seed(300 + kb)
+    M, Kd = 128, 128 * kb
+    aq, bq = torch.zeros(1, M, Kd, dtype=torch.int8), torch.zeros(n, Kd, dtype=torch.int8)
+    aq[0, 40:, ::128] = 1                    # rows 40-: partial product 1 or -3 in every K block
+    bq[:, ::128] = 1
+    bq[1::2, ::128] = -3
+    a_s = torch.rand(1, 1, kb, generator=g) + 0.5
+    same = int(share * kb)
+    a_s[0, 0, :same] = a_s[0, 0, 0]
+    if kind == "channel":
+        b_s, b_kind = torch.rand(n, generator=g) + 0.5, L.BSCALE_CHANNEL
+        fb = b_s.double().view(1, n)
+    else:
+        b_s, b_kind = (torch.rand(n // 128, 1, generator=g) + 0.5).expand(-1, kb).contiguous(), L.BSCALE_TILE
+        fb = b_s[:, 0].double().repeat_interleave(128).view(1, n)
+    P = torch.zeros(M, n, dtype=torch.double)
+    P[40:] = bq[:, 0].double()
+    ref = P * a_s.double().sum() * fb
+    out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), b_kind=b_kind, flags=L.GEMM_OUT_F32)[0].cpu().double()
+    err = (out - ref).abs()
+    if share == 1.0:
+        assert (out[:40] == 0).all(), float(out[:40].abs().max())
+        assert (err <= 4 * 2.0 ** -24 * ref.abs()).all()
+    else:
+        unit = float(a_s.max()) * fb
+        assert (err <= 5 / 7 * (0.75 * (kb - same)) ** 0.5 * unit).all(), float((err / unit).max())
+    K.check_status(DEV)
+
+
+def test_fast_block_epilogue_zero_rows_and_a_dominant_block():
+    """The rounding of the shift is an absolute error, a fraction of the tile's largest factor: rows of zeros beside
+    other rows come out within it (five standard deviations, see above), and a row that is zero in the one K block whose
+    scale is 1e4 times the others is off by no more than the roundings around that block (four times a quarter of its
+    factor)."""
+    g = torch.Generator().manual_seed(400)
+    kb, n = 64, 256
+    aq, bq = _randq(g, 1, 256, 128 * kb), _randq(g, n, 128 * kb)
+    aq[0, 5], aq[0, 77] = 0, 0
+    a_s, b_s = torch.rand(1, 2, kb, generator=g) + 0.5, torch.rand(n, generator=g) + 0.5
+    a_s[0, 1, 30] = 1e4
+    aq[0, 200:, 30 * 128:31 * 128] = 0
+    out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), flags=L.GEMM_OUT_F32)[0].cpu().double()
+    unit = b_s.double().view(1, n)
+    bound = 5 / 7 * (0.75 * kb) ** 0.5 * float(a_s[0, 0].max())
+    assert (out[[5, 77]].abs() <= bound * unit).all(), float((out[[5, 77]].abs() / unit).max())
+    P = torch.stack([R.int_mm(aq[0, 128:, k * 128:(k + 1) * 128], bq[:, k * 128:(k + 1) * 128]) for k in range(kb)]).double()
+    ref = (P * a_s[0, 1].double().view(-1, 1, 1)).sum(0) * unit
+    err = (out[128:] - ref).abs() / unit
+    assert (err[72:] <= 1e4 + bound).all(), float(err[72:].max())
+    K.check_status(DEV)

@@ -143,6 +143,7 @@ constexpr int K_BLOCK_OUTER = 5;   // block-scaled, per-(row, K block) A scale x
 // float, are the (denormal) number (P + SHIFT) * 2^-149 exactly.
 constexpr float SHIFT_F = 2080800.f;
 constexpr int FAC_EXP = 100;   // factors are scaled by a power of two that puts the tile's largest one near 2^100
+constexpr int REPEATED = 4;    // a factor that this many of 32 K blocks share is divided out of the tile (see the factor warp)
 __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
 
 // Two shifted partial products as they come from tensor memory -> P * 2^-23, exactly, by one packed FMA.
@@ -401,6 +402,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // over- or underflows whatever the scales are.  SHIFT * F_d is taken out four K blocks at a time, after the
       // second of them: the accumulators then stay within two K blocks' shift (4.2e6 f) of the true sum, an ulp of
       // which is at most f/2.  What the rounded corrections leave over is summed in fp64 and goes out at the tile end.
+      // These roundings are as good as random while the factors differ.  Equal ones round the same way every time and
+      // the error grows with K: an all-zero 128-row block, whose scales all sit on the quantizers' floor, came out at up
+      // to 8 f (K = 32768).  So a factor that repeats is divided out of the whole tile and multiplied back at its end:
+      // it becomes a power of two, SHIFT times it a float, and its K blocks add nothing but P.
       // Hand-over through mbarrier pairs (factors written, tile-end values written / buffer consumed), waits bounded like
       // all others.  The factors go out first: a kernel of one tile per CTA waits for them (3.2 us after its start when
       // everything was handed over at once).
@@ -412,7 +417,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int64_t bcol0 = (int64_t)(p.b_batched ? tc.m_blk / p.mpb : 0) * p.N + tc.n_tile * BN;
         const float* as_ptr = p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift);
         const int halves = chan ? 1 : 2;   // with per-channel B scales a factor is the A scale alone
-        float up0[2], up1[2], down0[2], down1[2];   // 2^e and 2^(149 - e), as two factors each
+        int e[2];                                   // factors are scaled by 2^e, the sums by 2^(149 - e)
+        float unit[2];                              // the factor that is divided out, or 1
         double left[2] = {0., 0.};                  // per lane, over the chunks of the tile
         for (int k0 = 0; k0 < KB; k0 += FAC_MAX, ++u) {
           const int dn = KB - k0 < FAC_MAX ? KB - k0 : FAC_MAX;
@@ -428,25 +434,35 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           };
           if (k0 == 0) {
             float m[2] = {0.f, 0.f};
+            // one factor per lane, spread over K (lanes past K: a pattern of their own), to see which one repeats
+            const int pick = lane + 32 * ((lane * (KB >> 5)) >> 5);
+            uint32_t seen[2] = {0x7fc00000u | lane, 0x7fc00000u | lane};
             for (int i = lane; i < KB; i += 32)
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 if (h < halves) {
                   const float f = factor(h, i);
                   if (i < dn) ctl.fac[buf][h][i].x = f;
+                  if (i == pick) seen[h] = __float_as_uint(f);
                   m[h] = fmaxf(m[h], fabsf(f));
                 }
               }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
+              unit[h] = 1.f;
+              if (h >= halves) continue;
 #pragma unroll
               for (int o = 16; o > 0; o >>= 1) m[h] = fmaxf(m[h], __shfl_xor_sync(0xffffffffu, m[h], o));
-              const int e = FAC_EXP + 127 - (int)(__float_as_uint(m[h]) >> 23), back = 149 - e;
-              up0[h] = pow2f(e >> 1);
-              up1[h] = pow2f(e - (e >> 1));
-              // the sums are far below 1, so the first factor may take all of it, up to the largest power there is
-              down0[h] = pow2f(back < 127 ? back : 127);
-              down1[h] = pow2f(back < 127 ? 0 : back - 127);
+              const uint32_t peers = __match_any_sync(0xffffffffu, seen[h]);
+              const uint32_t most = __reduce_max_sync(0xffffffffu, lane < KB ? (uint32_t)__popc(peers) << 5 | lane : 0u);
+              const float c = __uint_as_float(__shfl_sync(0xffffffffu, seen[h], most & 31));
+              // normal, and no factor overflows when divided by it
+              const int ec = (int)(__float_as_uint(c) >> 23 & 0xffu), em = (int)(__float_as_uint(m[h]) >> 23);
+              if ((int)(most >> 5) >= (KB < REPEATED ? KB : REPEATED) && ec > 0 && ec < 255 && em - ec < 64) {
+                unit[h] = c;
+                m[h] = __fdiv_rn(m[h], fabsf(c));
+              }
+              e[h] = FAC_EXP + 127 - (int)(__float_as_uint(m[h]) >> 23);
             }
           } else {
             for (int i = lane; i < dn; i += 32)
@@ -459,12 +475,19 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           for (int h = 0; h < 2; ++h) {
             if (h >= halves) continue;
             float2* fac = ctl.fac[buf][h];
+            const float up0 = pow2f(e[h] >> 1), up1 = pow2f(e[h] - (e[h] >> 1));   // 2^e may be too large for one float
             for (int i = lane; i < (dn + 3) / 4; i += 32) {   // one lane per four K blocks
               float f4[4];
               double sum = 0.;
 #pragma unroll
+              for (int j = 0; j < 4; ++j) f4[j] = 4 * i + j < dn ? fac[4 * i + j].x : 0.f;
+              if (unit[h] != 1.f) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) f4[j] = __fdiv_rn(f4[j], unit[h]);
+              }
+#pragma unroll
               for (int j = 0; j < 4; ++j) {
-                f4[j] = 4 * i + j < dn ? fac[4 * i + j].x * up0[h] * up1[h] : 0.f;
+                f4[j] = f4[j] * up0 * up1;
                 sum += (double)f4[j];
               }
               const float corr = 4 * i + 2 < dn ? -(float)(SHIFT_D * sum) : 0.f;
@@ -477,8 +500,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&ctl.fready[buf]));   // the K blocks may start; the rest is due at the tile end
           if (k0 + dn == KB) {
+            // 2^(149 - e) as two factors: the sums are far below 1, so the first may take all of it, up to the largest
+            // power there is; the rest goes with the column scale
             for (int i = lane; i < BN; i += 32) {
-              const float d = (chan || i < BN / 2) ? down1[0] : down1[1];
+              const int h = (chan || i < BN / 2) ? 0 : 1, back = 149 - (h ? e[1] : e[0]);
+              const float d = pow2f(back < 127 ? 0 : back - 127) * (h ? unit[1] : unit[0]);
               ctl.fbscale[buf][i] = chan && tc.n_tile * BN + i < p.N ? __ldg(p.b_scale + bcol0 + i) * p.post_scale * d : d;
             }
 #pragma unroll
@@ -486,7 +512,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               double all = left[chan ? 0 : h];
 #pragma unroll
               for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-              const float d = down0[chan ? 0 : h];
+              const int back = 149 - e[chan ? 0 : h];
+              const float d = pow2f(back < 127 ? back : 127);
               if (lane == 0) ctl.fend[buf][h] = make_float2(d, -(float)all * d);
             }
             __syncwarp();

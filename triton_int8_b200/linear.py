@@ -30,7 +30,9 @@ class Int8Config:
     a power of two <= 32768); round: 'half_up' (reference) or 'rne'; hadamard: 0 or 128 (rotate both
     operands of every GEMM in 128-wide groups along that GEMM's contraction axis: K for Y, N for dX,
     the tokens for dW; each product is rescaled by 1/128);
-    exact: reproduce the reference's fp32 operation order bit for bit (slower)."""
+    exact: reproduce the reference's fp32 operation order bit for bit (slower).  Without it the products of 'tile128'
+    carry an absolute error of about half of a tile's largest scale times the other operand's (1e-5 of a typical
+    result; all-zero 128-row blocks give exactly 0), see I8L_GEMM_EXACT_ORDER in include/i8linear.h."""
     scaling: str = "tile128"
     round: str = "half_up"
     hadamard: int = 0
