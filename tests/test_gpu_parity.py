@@ -625,3 +625,43 @@ def test_fast_block_epilogue_zero_rows_and_a_dominant_block():
     err = (out[128:] - ref).abs() / unit
     assert (err[72:] <= 1e4 + bound).all(), float(err[72:].max())
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("kb", [1, 3, 4])
+@pytest.mark.parametrize("kind", ["row_channel", "row_tile", "outer", "column", "column_div", "tile_div", "outer_exact", "column_exact"])
+def test_row_and_column_factors_over_many_tiles_of_one_cta(kind, kb):
+    """Two CTAs for all tiles, so that each runs many in a row, with odd and even numbers of K blocks: the column factors
+    are published through two buffers that alternate over the K blocks of all tiles.  Bound as in
+    test_row_and_column_factor_epilogues; the reference's operation order is met bit for bit."""
+    g = torch.Generator().manual_seed(500 + kb)
+    M, n, Kd = 512, 1152, 128 * kb
+    aq, bq = _randq(g, 1, M, Kd), _randq(g, n, Kd)
+    rnd = lambda *shape: torch.rand(*shape, generator=g) + 0.5
+    a_tile, a_row = rnd(1, M // 128, kb), rnd(1, M, kb)
+    flags, exact = (L.GEMM_DIVIDE if "div" in kind else 0), "exact" in kind
+    a_s, a_kind = (a_row, L.ASCALE_GROUP) if kind.startswith(("row", "outer")) else (a_tile, L.ASCALE_TILE)
+    if kind == "row_channel":
+        b_s, b_kind = rnd(n), L.BSCALE_CHANNEL
+        fb = b_s.view(1, 1, n)
+    elif kind in ("row_tile", "tile_div"):
+        b_s, b_kind = rnd(n // 128, kb), L.BSCALE_TILE
+        fb = b_s.t().repeat_interleave(128, 1)[:, None, :]
+    else:
+        b_s, b_kind = rnd(n, kb), L.BSCALE_GROUP
+        fb = b_s.t()[:, None, :]
+    fa = (a_s[0].t() if a_kind == L.ASCALE_GROUP else a_s[0].t().repeat_interleave(128, 1))[:, :, None]
+    P = torch.stack([R.int_mm(aq[0, :, k * 128:(k + 1) * 128], bq[:, k * 128:(k + 1) * 128]) for k in range(kb)])
+    with K.cta_limit(2):
+        out = K.gemm_block(aq.to(DEV), bq.to(DEV), a_s.to(DEV), b_s.to(DEV), a_kind, b_kind,
+                           flags=L.GEMM_OUT_F32 | flags | (L.GEMM_EXACT_ORDER if exact else 0))[0].cpu()
+    if exact:
+        acc = torch.zeros(M, n)
+        for k in range(kb):
+            acc = acc + (P[k].float() * fa[k]) * fb[k]
+        assert torch.equal(out, acc)
+    else:
+        f = 1.0 / (fa.double() * fb.double()) if flags else fa.double() * fb.double()
+        mag = (P.double() * f).abs().sum(0)
+        err = (out.double() - (P.double() * f).sum(0)).abs()
+        assert (err <= (3 * kb + 3) * 2.0 ** -24 * mag).all(), float((err / mag.clamp_min(1e-300)).max())
+    K.check_status(DEV)
