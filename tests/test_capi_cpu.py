@@ -72,3 +72,21 @@ def test_product_calls_validate_before_any_launch(lib):
         return lib.i8l_linear_backward(p, p, x_qt, p, p, p, 128, 128, 128, gran, 0, 0, 1.0, 1.0, 0, p, ws_bytes, None, None)
     assert backward() == -6 and b"too small" in lib.i8l_last_error()
     assert backward(gran=5, ws_bytes=1 << 20) == -6 and backward(x_qt=None, ws_bytes=1 << 20) == -6
+
+
+@pytest.mark.parametrize("batch,M,N", [(65535, 128, 128), (70000, 128, 128), (131071, 128, 256), ((1 << 24) - 1, 128, 128)])
+def test_product_call_takes_the_batches_of_its_steps(lib, batch, M, N):
+    """Per-row scales have no limit on the batch of their own: the quantizer and the GEMM take batch * M below 2^31.  The
+    128x128-tile quantizer takes 65535.  No device here: what passes the checks ends in an architecture or CUDA error."""
+    buf = ctypes.create_string_buffer(1 << 12)
+    p = ctypes.addressof(buf); p += (256 - p % 256) % 256
+
+    def product(gran, b_batched=0, batch=batch, M=M, N=N, K=128):
+        return lib.i8l_quant_gemm(p, p, None, p, None, None, batch, M, N, K, b_batched, gran, 2, 3 if gran == 2 else 0, 0, 1.0, 0,
+                                  p, 1 << 50, None, None)
+    fits = batch * max(M, N) < 1 << 31
+    for b_batched in (0, 1):
+        assert product(2, b_batched) in ((-3, -4) if fits else (-1,)), lib.i8l_last_error()
+    assert product(0) in ((-3, -4) if batch <= 65535 else (-1,))
+    # extents whose products would not fit 64 bits are refused before they are multiplied
+    assert product(2, batch=1 << 30, M=1 << 30, K=1 << 30) == -1 and product(2, batch=1 << 62) == -1

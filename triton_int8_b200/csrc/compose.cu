@@ -49,10 +49,12 @@ int quant_col_t(const void* x, int64_t rows, int64_t cols, int qmode, int had, i
   if (had == I8L_HAD_NONE) return i8l_quant_col_t(x, rows, cols, qmode, qt, st, scratch, stream);
   return fail(I8L_ERR_ARG, "a transposed operand is rotated in 128-wide groups or not at all");
 }
-// Before sizes are multiplied: the entry points below check the rest.
+// Before sizes are multiplied (batch * rows * K must fit 64 bits): the entry points below check the rest, with the limits
+// of their own grids.  batch * M and batch * N fit 31 bits wherever a GEMM accepts them.
 int check_extents(int64_t batch, int64_t M, int64_t N, int64_t K) {
-  if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || M % 128 || N % 128 || K % 128 || batch > 65535 || M >= (1ll << 31) ||
-      N >= (1ll << 31) || K >= (1ll << 31))
+  constexpr int64_t LIM = 1ll << 31;
+  if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || M % 128 || N % 128 || K % 128 || batch >= LIM || M >= LIM || N >= LIM ||
+      K >= LIM || batch * M >= LIM || batch * N >= LIM)
     return fail(I8L_ERR_SHAPE, "batch=%lld M=%lld N=%lld K=%lld: all positive, M, N, K multiples of 128", (long long)batch,
                 (long long)M, (long long)N, (long long)K);
   return I8L_OK;
