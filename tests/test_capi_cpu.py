@@ -90,3 +90,34 @@ def test_product_call_takes_the_batches_of_its_steps(lib, batch, M, N):
     assert product(0) in ((-3, -4) if batch <= 65535 else (-1,))
     # extents whose products would not fit 64 bits are refused before they are multiplied
     assert product(2, batch=1 << 30, M=1 << 30, K=1 << 30) == -1 and product(2, batch=1 << 62) == -1
+
+
+def test_wrappers_check_what_their_pointers_describe():
+    """A bias is read as N consecutive bf16 values and saved scales in the layout of the grouping: what is shorter, of another
+    type or of another grouping is refused, a strided bias is made contiguous."""
+    from triton_int8_b200 import _lib as L, kernels as K
+    b = torch.arange(256, dtype=torch.float32)
+    assert K._check_bias(None, 128) is None
+    with pytest.raises(TypeError):
+        K._check_bias(b, 256)
+    with pytest.raises(ValueError):
+        K._check_bias(b.to(torch.bfloat16)[:100], 128)
+    strided = b.to(torch.bfloat16)[::2]
+    got = K._check_bias(strided, 128)
+    assert got.is_contiguous() and torch.equal(got, strided)
+
+    M, Kd = 256, 384
+    q = torch.zeros(1, Kd, M, dtype=torch.int8)
+    scales = {L.GRAN_TILE128: torch.zeros(1, Kd // 128, M // 128), L.GRAN_GROUP128: torch.zeros(1, Kd, M // 128),
+              L.GRAN_ROW: torch.zeros(1, Kd)}
+    for gran in scales:
+        for made_with, st in scales.items():
+            if made_with == gran:
+                assert K._check_saved(q, st, M, Kd, gran)[1] is st
+            else:
+                with pytest.raises(ValueError):
+                    K._check_saved(q, st, M, Kd, gran)
+        with pytest.raises(ValueError):
+            K._check_saved(q, scales[gran].double(), M, Kd, gran)
+        with pytest.raises(ValueError):
+            K._check_saved(q[:, :, :128], scales[gran], M, Kd, gran)

@@ -166,3 +166,24 @@ def test_one_call_products_equal_the_separate_steps(scaling, had):
     assert torch.equal(dx, grad_input(dy_op, w, cfg)) and torch.equal(dw, grad_weight(dyt_op, saved, cfg))
     assert torch.equal(linear_backward(dy, w, None, cfg, need_dw=False)[0], dx)
     assert torch.equal(linear_backward(dy, w, saved, cfg, need_dx=False)[1], dw)
+
+
+def test_strided_bias_equals_contiguous_and_wrong_ones_are_refused():
+    """The same bias as every other element of a longer tensor gives the same bits; a short or fp32 bias and scales saved under
+    another grouping raise before any launch."""
+    M, Kd, N = 128, 256, 384
+    x, w, dy, _ = [t.to(DEV) for t in _data(M, Kd, N, seed=12)]
+    wide = torch.randn(2 * N, device=DEV).to(torch.bfloat16)
+    for scaling in ("tile128", "row128", "double_channel"):
+        cfg = Int8Config(scaling=scaling)
+        y, saved = linear_forward(x, w, wide[::2], cfg)
+        assert torch.equal(y, linear_forward(x, w, wide[::2].contiguous(), cfg)[0])
+        with pytest.raises(ValueError):
+            linear_forward(x, w, wide[:N - 1], cfg)
+        with pytest.raises(TypeError):
+            linear_forward(x, w, wide[:N].float(), cfg)
+        for other in ("tile128", "row128", "double_channel"):
+            if other != scaling:
+                with pytest.raises(ValueError):
+                    linear_backward(dy, w, saved, Int8Config(scaling=other))
+        linear_backward(dy, w, saved, cfg)

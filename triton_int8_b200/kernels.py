@@ -100,6 +100,27 @@ def _check_bf16(x: torch.Tensor, name: str) -> torch.Tensor:
     return x.contiguous()
 
 
+def _check_bias(bias, N: int):
+    """The kernels read N consecutive bf16 values."""
+    if bias is None:
+        return None
+    if bias.dtype != torch.bfloat16:
+        raise TypeError(f"bias must be bfloat16, got {bias.dtype}")
+    if bias.numel() < N:
+        raise ValueError(f"bias has {bias.numel()} elements, {N} are needed")
+    return bias.contiguous()
+
+
+def _check_saved(xqt, xst, M: int, K: int, gran: int):
+    """The operand that linear_backward takes over from quant_gemm: its scales must be those of the same grouping."""
+    shape = {L.GRAN_TILE128: (1, K // 128, M // 128), L.GRAN_GROUP128: (1, K, M // 128)}.get(gran, (1, K))
+    if xqt.dtype != torch.int8 or tuple(xqt.shape) != (1, K, M):
+        raise ValueError(f"saved operand {xqt.dtype} {tuple(xqt.shape)}, expected int8 {(1, K, M)}")
+    if xst.dtype != torch.float32 or tuple(xst.shape) != shape:
+        raise ValueError(f"saved scales {xst.dtype} {tuple(xst.shape)}, expected float32 {shape} for this grouping")
+    return xqt.contiguous(), xst.contiguous()
+
+
 def quant_tile(x: torch.Tensor, gran: int = L.GRAN_TILE128, qmode: int = L.QMODE_TRITON, hadamard: int = 0,
                natural: bool = True, transposed: bool = False):
     """x bf16 [B, R, C] -> (q, scale, qt, scale_t); entries not requested are None."""
@@ -160,6 +181,7 @@ def gemm_block(aq, bq, a_s, b_s, a_kind=L.ASCALE_TILE, b_kind=L.BSCALE_CHANNEL, 
     """Block-scaled GEMM; returns bf16 (fp32 with GEMM_OUT_F32) [B, M, N]."""
     aq, bq = aq.contiguous(), bq.contiguous()
     B, M, N, K, bb = _gemm_dims(aq, bq)
+    bias = _check_bias(bias, N)
     out = torch.empty((B, M, N), dtype=torch.float32 if flags & L.GEMM_OUT_F32 else torch.bfloat16, device=aq.device)
     a_s, b_s = a_s.contiguous(), b_s.contiguous()
     status = device_status(aq.device) if status is None else status
@@ -172,6 +194,7 @@ def gemm_block(aq, bq, a_s, b_s, a_kind=L.ASCALE_TILE, b_kind=L.BSCALE_CHANNEL, 
 def gemm_rowcol(aq, bq, a_s, b_s, bias=None, post_scale=1.0, flags=0, status=None):
     aq, bq = aq.contiguous(), bq.contiguous()
     B, M, N, K, bb = _gemm_dims(aq, bq)
+    bias = _check_bias(bias, N)
     out = torch.empty((B, M, N), dtype=torch.float32 if flags & L.GEMM_OUT_F32 else torch.bfloat16, device=aq.device)
     a_s, b_s = a_s.contiguous(), b_s.contiguous()
     status = device_status(aq.device) if status is None else status
@@ -219,6 +242,7 @@ def quant_gemm(a, b, a_gran, b_gran, qmode, hadamard=0, bias=None, post_scale=1.
     N = b.shape[-2]
     if b.shape[-1] != K or (bb and b.shape[0] != B):
         raise ValueError(f"operand shapes do not match: {tuple(a.shape)} x {tuple(b.shape)}")
+    bias = _check_bias(bias, N)
     dev = a.device
     out = torch.empty((B, M, N), dtype=torch.float32 if flags & L.GEMM_OUT_F32 else torch.bfloat16, device=dev)
     nb = B if bb else 1
@@ -248,11 +272,7 @@ def linear_backward(dy, w, xt, gran, qmode, hadamard=0, post_dx=1.0, post_dw=1.0
     dev = dy.device
     dx = torch.empty((M, K), dtype=torch.bfloat16, device=dev) if need_dx else None
     dw = torch.empty((N, K), dtype=torch.bfloat16, device=dev) if need_dw else None
-    xqt, xst = xt if need_dw else (None, None)
-    if need_dw:
-        xqt, xst = xqt.contiguous(), xst.contiguous()
-        if xqt.dtype != torch.int8 or tuple(xqt.shape) != (1, K, M):
-            raise ValueError(f"saved operand {xqt.dtype} {tuple(xqt.shape)} does not match dy {tuple(dy.shape)}, w {tuple(w.shape)}")
+    xqt, xst = _check_saved(*xt, M, K, gran) if need_dw else (None, None)
     size = _pad(4 * max(K, N))
     if need_dx:
         size += _pad(M * N) + _pad(4 * _scale_count(gran, 1, M, N)) + _pad(K * N) + _pad(4 * K)
