@@ -91,3 +91,48 @@ def test_status_word_of_the_wrappers_reports_and_clears():
     K.check_status(DEV)                    # cleared by the raise
     K.gemm_block(a, b, a_tile, b_ch)
     K.check_status(DEV)
+
+
+def _set_word():
+    word = K.device_status(torch.device("cuda", torch.cuda.current_device()))
+    word.fill_(TIMEOUT)
+    torch.cuda.synchronize()
+    return word
+
+
+def test_poll_reports_a_set_word_once():
+    """poll_status: nothing, then (its copy has completed and shows the word) one error, then nothing again."""
+    dev = torch.device("cuda", torch.cuda.current_device())
+    K.poll_status(dev)
+    torch.cuda.synchronize()
+    word = _set_word()
+    K.poll_status(dev)              # takes the copy from before, which is clean, and starts one of the set word
+    torch.cuda.synchronize()
+    with pytest.raises(L.I8LError) as e:
+        K.poll_status(dev)
+    assert e.value.code == TIMEOUT
+    assert word.item() == 0
+    for _ in range(3):
+        K.poll_status(dev)
+        torch.cuda.synchronize()
+    K.check_status(dev)
+
+
+def test_check_status_voids_the_copy_of_an_earlier_poll():
+    """A poll's copy may land after check_status has reported and cleared the word (another stream): here the late value is
+    written by hand.  It must not be reported again."""
+    dev = torch.device("cuda", torch.cuda.current_device())
+    K.poll_status(dev)
+    torch.cuda.synchronize()
+    _set_word()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        K.poll_status(dev)
+    with pytest.raises(L.I8LError):
+        K.check_status(dev)
+    torch.cuda.synchronize()
+    K._status_of(dev).host.fill_(TIMEOUT)
+    for _ in range(2):
+        K.poll_status(dev)
+        torch.cuda.synchronize()
+    K.check_status(dev)

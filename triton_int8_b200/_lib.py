@@ -40,6 +40,7 @@ SIGNATURES = {
     "i8l_linear_backward": [_P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I, _I, _I, _F, _F, _I, _P, _I64, _P, _P],
     "i8l_status_open": [_P, _P],
     "i8l_status_poll": [_P, _P],
+    "i8l_status_reset": [_P],
     "i8l_set_cta_limit": [_I],
     "i8l_test_set_wait_limit": [ctypes.c_uint32, _I],
     "i8l_version": [],

@@ -1242,6 +1242,16 @@ extern "C" int i8l_status_poll(void* poller, void* stream) {
   return I8L_OK;
 }
 
+extern "C" int i8l_status_reset(void* poller) {
+  if (!poller) return fail(I8L_ERR_ARG, "null pointer");
+  StatusPoller* s = static_cast<StatusPoller*>(poller);
+  const std::lock_guard<std::mutex> hold(s->lock);
+  if (s->pending) I8L_CUDA_OK(cudaEventSynchronize(s->event));
+  s->pending = false;
+  *s->host = 0;
+  return I8L_OK;
+}
+
 extern "C" int i8l_set_cta_limit(int max_ctas) {
   if (max_ctas < 0) return fail(I8L_ERR_ARG, "i8l_set_cta_limit: max_ctas must be >= 0");
   g_cta_limit = max_ctas;

@@ -65,7 +65,9 @@ def device_status(dev) -> torch.Tensor:
 def _raise_if_set(st: "_StatusWord", code: int) -> None:
     if code:
         st.word.zero_()
-        st.host.zero_()
+        # a copy started from now on, on whatever stream, must see the cleared word, and one started before is void
+        torch.cuda.current_stream(st.dev).synchronize()
+        L.call("i8l_status_reset", st.poller)
         raise L.I8LError(code, f"a GEMM on {st.dev} gave up a bounded device-side wait; its output is incomplete")
 
 
