@@ -256,8 +256,9 @@ I8L_API int i8l_quant_gemm(const void* a, const void* b, const void* bias, void*
 /*
  * Backward pass of y = x w^T: dx [M, K] = dy w and dw [N, K] = dy^T x, either may be NULL.  x_qt, x_st: the transposed
  * operand that i8l_quant_gemm made of x with the same gran, qmode and hadamard.  The workspace holds, each piece rounded up
- * to 256 bytes: for dx the int8 dy and w^T, dy's scales and K floats; for dw the int8 dy^T and its scales;
- * max(K, N) floats.  No counterpart in the reference, which has the two products only.
+ * to 256 bytes: for dx the int8 dy, dy's scales, K floats and, unless dw is given, the int8 w^T; for dw the int8 dy^T and
+ * its scales; max(K, N) floats.  With both gradients the int8 w^T lies in dw until dx is done.  No counterpart in the
+ * reference, which has the two products only.
  */
 I8L_API int i8l_linear_backward(const void* dy, const void* w, const int8_t* x_qt, const float* x_st, void* dx, void* dw,
                    int64_t M, int64_t N, int64_t K, int gran, int qmode, int hadamard, float post_dx, float post_dw,

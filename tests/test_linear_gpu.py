@@ -187,3 +187,23 @@ def test_strided_bias_equals_contiguous_and_wrong_ones_are_refused():
                 with pytest.raises(ValueError):
                     linear_backward(dy, w, saved, Int8Config(scaling=other))
         linear_backward(dy, w, saved, cfg)
+
+
+@pytest.mark.parametrize("scaling", ["tile128", "double_channel"])
+def test_backward_peak_memory(scaling):
+    """A backward pass holds both int8 forms of dY, their scales and the two gradients, no int8 W^T beside them: the peak of
+    separate calls, which free W^T ahead of dW."""
+    M, Kd, N = 2048, 4096, 4096
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, w, dy = [(torch.randn(*s, generator=g, device=DEV) * f).to(torch.bfloat16)
+                for s, f in (((M, Kd), 1.0), ((N, Kd), 0.02), ((M, N), 1e-3))]
+    cfg = Int8Config(scaling=scaling)
+    _, saved = linear_forward(x, w, None, cfg)
+    linear_backward(dy, w, saved, cfg)
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    linear_backward(dy, w, saved, cfg)
+    peak = torch.cuda.max_memory_allocated() - base
+    scales = 4 * (2 * M * N // 128 ** 2 if scaling == "tile128" else M + N)
+    assert peak <= 2 * M * N + 2 * M * Kd + 2 * N * Kd + scales + 8 * max(Kd, N) + (2 << 20)   # blocks are rounded up to 512 bytes or 2 MiB

@@ -277,7 +277,8 @@ def linear_backward(dy, w, xt, gran, qmode, hadamard=0, post_dx=1.0, post_dw=1.0
     xqt, xst = _check_saved(*xt, M, K, gran) if need_dw else (None, None)
     size = _pad(4 * max(K, N))
     if need_dx:
-        size += _pad(M * N) + _pad(4 * _scale_count(gran, 1, M, N)) + _pad(K * N) + _pad(4 * K)
+        size += _pad(M * N) + _pad(4 * _scale_count(gran, 1, M, N)) + _pad(4 * K)
+        size += 0 if need_dw else _pad(K * N)   # with both gradients the int8 w^T lies in dw until dx is done
     if need_dw:
         size += _pad(N * M) + _pad(4 * _scale_count(gran, 1, N, M))
     ws = torch.empty(size, dtype=torch.int8, device=dev)
