@@ -673,6 +673,7 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
   // h[e / 2] = elements tid of groups e, e + 1 (e counts the groups of all rows), rounded to bf16
   uint32_t h[64];
   __nv_bfloat16 m[R];
+  __nv_bfloat162 any = __floats2bfloat162_rn(0.f, 0.f);
   bool finite = true;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -685,9 +686,12 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
     fwht_pairs<G / 2>(p);
     __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
     if constexpr (G == 2) {
-      const __nv_bfloat162 v = __floats2bfloat162_rn(__fadd_rn(p[0].x, p[0].y), __fsub_rn(p[0].x, p[0].y));
-      hm = __hmax2_nan(hm, __habs2(v));
+      // 64 maxima: taken without NaNs at once, the NaNs seen by a second one (replacing them all below spills 144 bytes)
+      const __nv_bfloat162 v = __floats2bfloat162_rn(__fadd_rn(p[0].x, p[0].y), __fsub_rn(p[0].x, p[0].y)), a = __habs2(v);
+      hm = __hmax2(hm, a);
+      any = __hmax2_nan(any, a);
       h[r] = *reinterpret_cast<const uint32_t*>(&v);
+      m[r] = __hmax(__low2bfloat16(hm), __high2bfloat16(hm));
     } else {
 #pragma unroll
       for (int g = 0; g < G / 2; g += 2) {
@@ -697,11 +701,13 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
         h[(r * G + g) / 2] = *reinterpret_cast<const uint32_t*>(&lo);
         h[(r * G + g) / 2 + G / 4] = *reinterpret_cast<const uint32_t*>(&hi);
       }
+      m[r] = __hmax_nan(__low2bfloat16(hm), __high2bfloat16(hm));
+      finite = finite && __bfloat162float(m[r]) <= BF16_LARGEST;
     }
-    m[r] = __hmax_nan(__low2bfloat16(hm), __high2bfloat16(hm));
-    finite = finite && __bfloat162float(m[r]) <= BF16_LARGEST;
   }
-  if (!finite) {   // the maximum leaves NaNs out
+  if constexpr (G == 2) {
+    finite = __bfloat162float(__hmax_nan(__low2bfloat16(any), __high2bfloat16(any))) <= BF16_LARGEST;
+  } else if (!finite) {   // the maximum leaves NaNs out
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
