@@ -33,7 +33,8 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // ---------------------------------------------------------------- scale / rounding arithmetic
 // All operations are spelled with explicit round-to-nearest intrinsics so that the compiler can
 // neither contract x*s+0.5 into an FMA nor replace a division by a reciprocal: the int8 values
-// and the stored scales must equal the reference's bit for bit.
+// and the stored scales must equal the reference's bit for bit.  The exception are packed products
+// (__fmul2_rn), which may be fused with a packed addition behind them: see quant2.
 
 template <int MODE>
 __device__ __forceinline__ void make_scale(float amax, float& s, float& stored) {
@@ -86,7 +87,10 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 
-// Two values at once: the multiply and the +0.5 stay separate roundings, as in quant1.
+// Two values at once.  The packed product may be fused with the +0.5 (one rounding instead of two).  That changes a byte only
+// where the product lies just below -0.5 and its rounding moves it there, and for a scale that belongs to the bf16
+// maximum of the group no bf16 value does (tests/test_half_up_products_cpu.py goes through all of them, in each mode).
+// Nearest-even ties do part, so that mode keeps its product away from any addition.
 template <int MODE>
 __device__ __forceinline__ void quant2(float2 v, float2 s2, int& q0, int& q1) {
   float2 y = __fmul2_rn(v, s2);
@@ -123,7 +127,7 @@ __device__ __forceinline__ uint32_t quant_pair_finite(uint32_t w, float s) {   /
   const float2 s2 = make_float2(s, s), half2 = make_float2(0.5f, 0.5f), magic2 = make_float2(12582912.f, 12582912.f);
   const float2 v = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
   float2 y;
-  if (MODE == I8L_QMODE_RNE)   // scalar products: a packed one is fused with the addition, which turns ties over
+  if (MODE == I8L_QMODE_RNE)   // scalar products: a packed one is fused with the addition, which turns ties over (see quant2)
     y = __fadd2_rn(make_float2(__fmul_rn(v.x, s), __fmul_rn(v.y, s)), magic2);
   else
     y = __fadd2_rd(__fadd2_rn(__fmul2_rn(v, s2), half2), magic2);
