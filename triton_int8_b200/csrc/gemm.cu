@@ -703,8 +703,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         constexpr int CH = 32;
         static_assert(EPI_COLS == 128, "a thread of the group publishes one column");
         const float* as_ptr = p.a_scale + (ROWF && KIND != K_BLOCK_TILEDIV ? row : (int64_t)tc.m_blk) * KB;
-        const float* bc_ptr = p.b_scale + (p.b_kind == I8L_BSCALE_GROUP ? bcol0 + tix : (bcol0 + tix) >> 7) * KB;   // COLF
-        const float* bt_ptr = p.b_scale + (bcol0 >> 7) * KB;                                                       // ROWFAC, per tile
+        const float* bc_ptr = p.b_scale + (bcol0 + tix) * KB;      // COLF: one scale per column and K block
+        const float* bt_ptr = p.b_scale + (bcol0 >> 7) * KB;       // per-tile B scales
         auto row_factor = [&](int d) {
           float f = __ldg(as_ptr + d);
           if (!COLF && !chan && active) f *= __ldg(bt_ptr + d);
@@ -1087,8 +1087,7 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   // to 1e-6.
   const bool scalar_factor = block && !p.exact && !p.dump && p.b_kind != I8L_BSCALE_GROUP &&
                              (!p.divide || p.a_kind == I8L_ASCALE_TILE);
-  const bool column_factor = block && !p.exact && !p.dump && !scalar_factor && p.a_kind == I8L_ASCALE_TILE &&
-                             p.b_kind != I8L_BSCALE_CHANNEL;
+  const bool column_factor = block && !p.exact && !p.dump && p.a_kind == I8L_ASCALE_TILE && p.b_kind == I8L_BSCALE_GROUP;
   const bool outer_factor = block && !p.exact && !p.dump && !p.divide && p.a_kind == I8L_ASCALE_GROUP &&
                             p.b_kind == I8L_BSCALE_GROUP;
   if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, p, tiles, st);

@@ -1,5 +1,5 @@
-// bf16 -> int8 absmax quantizers (HBM-bound): 128x128-tile kernel with optional transposed
-// output and fused 128-point Hadamard rotation, whole-row kernel, column-absmax kernel.
+// bf16 -> int8 absmax quantizers: 128x128-tile kernels (plain, rotated, either or both orientations), 128x256 tiles,
+// row kernels (rows on chip, rotated in 128-groups or whole, long rows in two sweeps), column-absmax kernel.
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -53,7 +53,7 @@ __device__ __forceinline__ __nv_bfloat162 absmax8(const uint4& u, __nv_bfloat162
 constexpr float BF16_LARGEST = 3.3895314e38f;
 __device__ __forceinline__ float hmax_of(__nv_bfloat162 m) { return fmaxf(__low2float(m), __high2float(m)); }
 
-template <int GRAN, int MODE, bool HAD, bool OUT_N, bool OUT_T>
+template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
 __global__ void __launch_bounds__(256, 4)
 quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
                   int8_t* __restrict__ q, float* __restrict__ scale, int8_t* __restrict__ qt,
@@ -68,8 +68,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
   const __nv_bfloat16* xb = x + boff;
 
-  // The tile stays in registers as packed bf16 (32 registers per thread, 4 CTAs per SM); with the
-  // Hadamard rotation the rotated values, already rounded to bf16, replace the raw ones.
+  // The tile stays in registers as packed bf16 (32 registers per thread, 4 CTAs per SM).
   uint4 raw[2][4];
 #pragma unroll
   for (int it = 0; it < 2; ++it)
@@ -77,14 +76,6 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
     for (int i = 0; i < 4; ++i) {
       const int r = 16 * w + 8 * it + 4 * half + i;
       raw[it][i] = __ldg(reinterpret_cast<const uint4*>(xb + (r_base + r) * cols + c_base + 8 * cc));
-      if (HAD) {
-        float v[8];
-        unpack8(raw[it][i], v);
-        fwht128_lanes16(v, l);
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw[it][i]);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) h[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-      }
     }
 
   // ---- scales
@@ -872,11 +863,11 @@ static int check_dims(int64_t batch, int64_t rows, int64_t cols) {
   return I8L_OK;
 }
 
-template <int GRAN, int MODE, bool HAD, bool OUT_N, bool OUT_T>
+template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
 static void launch_tile(const void* x, int64_t batch, int64_t rows, int64_t cols, int8_t* q, float* scale,
                         int8_t* qt, float* scale_t, const float* colmax, cudaStream_t st) {
   dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
-  quant_tile_kernel<GRAN, MODE, HAD, OUT_N, OUT_T><<<grid, 256, 0, st>>>(
+  quant_tile_kernel<GRAN, MODE, OUT_N, OUT_T><<<grid, 256, 0, st>>>(
       static_cast<const __nv_bfloat16*>(x), rows, cols, q, scale, qt, scale_t, colmax);
 }
 
@@ -891,12 +882,12 @@ static int dispatch_tile(const void* x, int64_t batch, int64_t rows, int64_t col
     else if (n) quant_tile_rot_kernel<GRAN, MODE, true, false><<<grid, 128, 0, st>>>(xp, rows, cols, q, scale, nullptr, nullptr, nullptr);
     else quant_tile_rot_kernel<GRAN, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, qt, scale_t, nullptr);
   } else if (GRAN == I8L_GRAN_TILE128) {
-    if (n && t) launch_tile<GRAN, MODE, false, true, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
-    else if (n) launch_tile<GRAN, MODE, false, true, false>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
-    else launch_tile<GRAN, MODE, false, false, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
+    if (n && t) launch_tile<GRAN, MODE, true, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
+    else if (n) launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
+    else launch_tile<GRAN, MODE, false, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
   } else {  // grouped scales differ between the two orientations: one launch each
-    if (n) launch_tile<GRAN, MODE, false, true, false>(x, batch, rows, cols, q, scale, nullptr, nullptr, colmax, st);
-    if (t) launch_tile<GRAN, MODE, false, false, true>(x, batch, rows, cols, nullptr, nullptr, qt, scale_t, colmax, st);
+    if (n) launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, nullptr, nullptr, colmax, st);
+    if (t) launch_tile<GRAN, MODE, false, true>(x, batch, rows, cols, nullptr, nullptr, qt, scale_t, colmax, st);
   }
   I8L_CUDA_OK(cudaGetLastError());
   return I8L_OK;
@@ -1005,7 +996,7 @@ extern "C" int i8l_quant_col_t(const void* x, int64_t rows, int64_t cols, int qm
   I8L_CUDA_OK(cudaGetLastError());
 #define I8L_COL_CASE(Mo)                                                                                     \
   if (qmode == Mo) {                                                                                         \
-    launch_tile<GRAN_COLFULL, Mo, false, false, true>(x, 1, rows, cols, nullptr, nullptr, qt, scale_t,       \
+    launch_tile<GRAN_COLFULL, Mo, false, true>(x, 1, rows, cols, nullptr, nullptr, qt, scale_t,       \
                                                       colmax_scratch, st);                                   \
     I8L_CUDA_OK(cudaGetLastError());                                                                         \
     return I8L_OK;                                                                                           \
