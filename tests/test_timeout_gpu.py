@@ -136,3 +136,36 @@ def test_check_status_voids_the_copy_of_an_earlier_poll():
         K.poll_status(dev)
         torch.cuda.synchronize()
     K.check_status(dev)
+
+
+@pytest.mark.parametrize("a_kind,b_kind,flags", [("group", "channel", 0), ("group", "tile", 0), ("tile", "group", 0),
+                                                 ("tile", "group", "divide"), ("group", "group", 0), ("tile", "tile", "divide")])
+@pytest.mark.parametrize("M,N,Kd", [(256, 384, 384), (2048, 4096, 640)])   # one tile per CTA; a second one behind the withheld load
+def test_row_and_column_factor_kinds_give_up_and_recover(a_kind, b_kind, flags, M, N, Kd):
+    """The kinds with a factor per row, per column or both have a loop without an early exit, a named barrier per K block and a
+    shifting MMA ahead of the operands: they return, report TIMEOUT, and the next call is exact."""
+    lib = L.load()
+    a, b = _operands(M, N, Kd)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kb = Kd // 128
+    a_s, ak = ((torch.ones(1, M, kb, device=DEV), L.ASCALE_GROUP) if a_kind == "group"
+               else (torch.ones(1, M // 128, kb, device=DEV), L.ASCALE_TILE))
+    b_s, bk = {"channel": (torch.ones(N, device=DEV), L.BSCALE_CHANNEL), "tile": (torch.ones(N // 128, kb, device=DEV), L.BSCALE_TILE),
+               "group": (torch.ones(N, kb, device=DEV), L.BSCALE_GROUP)}[b_kind]
+    fl = L.GEMM_OUT_F32 | (L.GEMM_DIVIDE if flags else 0)
+
+    def launch():
+        return K.gemm_block(a, b, a_s, b_s, ak, bk, flags=fl, status=status)
+
+    assert lib.i8l_test_set_wait_limit(256, 1) == 0
+    try:
+        launch()
+        torch.cuda.synchronize()
+    finally:
+        assert lib.i8l_test_set_wait_limit(0, 0) == 0
+    assert status.item() == TIMEOUT
+    status.zero_()
+    out = launch()
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    assert torch.equal(out[0].cpu(), _exact_i32(a, b).float())   # unit scales, sums below 2^24
