@@ -169,3 +169,12 @@ def test_row_and_column_factor_kinds_give_up_and_recover(a_kind, b_kind, flags, 
     torch.cuda.synchronize()
     assert status.item() == 0
     assert torch.equal(out[0].cpu(), _exact_i32(a, b).float())   # unit scales, sums below 2^24
+
+
+def test_check_status_without_an_argument_is_the_current_device():
+    K.check_status()
+    word = _set_word()
+    with pytest.raises(L.I8LError):
+        K.check_status()
+    assert word.item() == 0
+    K.check_status()

@@ -74,7 +74,7 @@ def _raise_if_set(st: "_StatusWord", code: int) -> None:
 def check_status(dev=None) -> None:
     """Synchronous check: raises I8LError (code TIMEOUT) if a GEMM on `dev` gave up a wait since the
     last check, and clears the word."""
-    st = _status_of(torch.device(dev if dev is not None else ("cuda", torch.cuda.current_device())))
+    st = _status_of(torch.device(dev if dev is not None else "cuda"))   # without an index: the current device
     _raise_if_set(st, int(st.word.item()))
 
 
