@@ -350,8 +350,8 @@ def test_rotated_operand_pair_from_one_read(mode):
 
 @pytest.mark.parametrize("spread", ["smooth", "wild"])
 def test_fast_block_epilogue_accuracy_deep_k(spread):
-    """The fast block-scaled epilogue turns the int32 partials into floats by an integer add of a magic
-    number and lets the accumulators carry a bounded multiple of that number, removed at the tile end.
+    """The fast block-scaled epilogue takes the int32 partials as floats shifted by a constant, whose multiple the
+    accumulators carry for four K blocks at a time.
     At K = 32768 (256 K blocks), with per-tile scales that are smooth or jump by three decades from one
     K block to the next, the fp32 result must stay within 1e-4 (relative Frobenius) of the float64 value of
     sum_kb P_kb * a_s * b_s, like the reference-order mode."""
@@ -409,7 +409,7 @@ def test_single_kernel_fused_matches_reference_kernels(golden_dir):
 
 
 def test_fast_block_epilogue_more_than_512_k_blocks():
-    """K = 73728 = 576 K blocks: the factors of a tile are handed over in two chunks (512 + 64); int32
+    """K = 73728 = 576 K blocks: the factors of a tile are handed over in three chunks (256 + 256 + 64); int32
     partials via the dump entry, fp32 result against float64."""
     M, N, Kd = 128, 256, 128 * 576
     g = torch.Generator().manual_seed(43)

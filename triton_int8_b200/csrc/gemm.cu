@@ -1,7 +1,7 @@
 // INT8 GEMMs on the 5th-generation tensor cores: tcgen05.mma kind::i8 with int32 accumulators in
 // tensor memory, operands staged by TMA into a 128B-swizzled shared-memory ring.
 //
-// One persistent CTA per SM, 384 threads (fast block-scaled kind) or 640 (the others):
+// One persistent CTA per SM, 384 threads (the five shifted block-scaled kinds) or 640 (row x column, generic):
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      tensor-memory allocator + MMA issuer (one elected lane, see elect_one)
 //   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the per-K-block
@@ -10,13 +10,13 @@
 //   warps 4-    epilogue: warp%4 selects the 32 accumulator lanes (rows) a warp may read, the group of
 //               four warps a share of the 256 columns of the 128x256 tile.  Sixteen warps with 64 columns
 //               each where the per-K-block drain is bound by instruction latency (more resident warps hide
-//               it).  The fast block-scaled kind has one packed FMA per two elements left and wants long runs
+//               it).  The shifted kinds have one or two packed FMAs per two elements left and want long runs
 //               of tensor-memory loads instead: eight warps with 128 columns each and up to 208 registers, 32
-//               columns in flight per wait (8192^3: 16 warps 508 us, 8 warps 501, 8 warps and 32 columns 489).
+//               columns in flight per wait (fast kind, 8192^3: 16 warps 508 us, 8 warps 501, 8 warps and 32 columns 489).
 // Tensor memory holds two 128x256 int32 accumulators (all 512 columns).  In block-scaled mode the
 // MMA warp alternates between them every 128-wide K block while the epilogue drains the other one
-// into fp32 registers (acc += float(P) * scale; in the fast kind a fifth MMA per K block shifts P into the
-// non-negative range, where its bits ARE a float, and the multiple of the shift is taken out again); in
+// into fp32 registers (acc += float(P) * scale; in the shifted kinds a fifth MMA per K block moves P into the
+// non-negative range, where its bits ARE a float, and the shift is taken out again); in
 // row x column mode a buffer holds a whole tile and the epilogue of tile i overlaps the main loop of tile i+1.
 //
 // Every wait on an mbarrier is bounded (a poll count worth about two seconds); on expiry the CTA raises
@@ -90,7 +90,7 @@ struct GemmParams {
 // Instruction descriptor: D=s32, A=B=s8, both K-major, M=128, N=256, dense, no saturation.
 constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                               ((uint32_t)(BM >> 4) << 24);
-// Same with both operands unsigned: the MMA that shifts a partial product (K_BLOCK_FAST).
+// Same with both operands unsigned: the MMA that shifts a partial product (the shifted kinds).
 constexpr uint32_t IDESC_U8 = (2u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 // Same with M=256 for the CTA-pair instruction (128 rows per CTA).
 constexpr uint32_t IDESC_I8_PAIR = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
@@ -133,7 +133,7 @@ struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fa
 // Epilogue kinds.  Everything but K_ROWCOL drains the accumulator every 128-wide K block.
 constexpr int K_ROWCOL = 0;      // one drain per tile, (float(acc)*a_s[m])*b_s[n]
 constexpr int K_BLOCK_GEN = 1;   // block-scaled, any scale layout, reference operation order, dumps
-constexpr int K_BLOCK_FAST = 2;  // block-scaled, one scalar factor per (tile, K block) and 64-column group
+constexpr int K_BLOCK_FAST = 2;  // block-scaled, one scalar factor per (tile, K block) and 128-column half
 constexpr int K_BLOCK_COLFAC = 3;  // block-scaled, per-tile A scale x per-(column, K block) B scale (fused forward)
 constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x per-tile or per-channel B scale
 constexpr int K_BLOCK_TILEDIV = 6; // block-scaled, per-tile scales on both sides as divisors (fused backward)
@@ -586,9 +586,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               // int32 -> fp32 without any conversion: an extra K step of the tensor core has added SHIFT to P, so
               // the bits are the float (P + SHIFT) * 2^-149, which the FMA multiplies exactly.  One packed FMA per
               // two elements is all that is left; the shift is taken out every fourth K block.
-              // The drain, not the MMA, bounds this kernel: a fifth MMA (+25 % tensor work) for half of the drain's
-              // instructions takes 8192^3 from 560 us (an integer add per element, sixteen warps) to 489 us (1.96 ->
-              // 2.24 POP/s), the error against fp64 from 2.1e-5 to 0.7e-5.
+              // A fifth MMA (+25 % tensor work) for half of the drain's instructions took 8192^3 from 560 us (an integer
+              // add per element, sixteen warps; the drain was the bound) to 489 us, the error against fp64 from 2.1e-5 to
+              // 0.7e-5.  With the MMAs issued by an elected lane the tensor pipe is the bound: 640 of 813 cycles per K block,
+              // 426-455 us.
               const uint32_t taddr = taddr0 + ab * BN;
               const float2 f2 = make_float2(f, f);
               if (corr != 0.f) {
@@ -690,8 +691,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
 
       if constexpr (SHIFTED) {
-        // Before, with sixteen warps converting on two pipes, and now, 8192^3: row x channel 787 -> 662 us, column
-        // 1051 -> 862; row x column took the generic path: 4020 -> 896.
+        // Before, with sixteen warps converting on two pipes, and now, 8192^3: row x channel 787 -> 607-620 us, column
+        // 1051 -> 843-940 (box to box); row x column took the generic path: 4020 -> 871-920.
         // A factor per row, per column or both for every K block.  Two packed FMAs per two elements (the first
         // brings P back from its shift), a packed product more for row x column factors.  Row factors live in the
         // thread that owns the row; column factors (a_s * b_s or its reciprocal when the scales are multipliers, the
