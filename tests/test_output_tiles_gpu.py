@@ -1,0 +1,56 @@
+"""bf16 outputs of every GEMM kind leave through shared memory and TMA stores, fp32 outputs straight from registers: for
+the same operands the bf16 result is the fp32 result rounded once, bit for bit, at tiles that the output ends in, and
+nothing around the output is written."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if torch.cuda.is_available():
+    from triton_int8_b200 import _lib as L
+    from triton_int8_b200 import kernels as K
+
+DEV = "cuda"
+GUARD = 1024   # bf16 elements kept around the output
+# kind: a_scale_kind, b_scale_kind, flags (None: row x column)
+KINDS = {"rowcol": None, "fast": (0, 0, 0), "fast_tile": (0, 1, 0), "row_channel": (1, 0, 0), "row_tile": (1, 1, 0),
+         "column": (0, 2, 2), "outer": (1, 2, 0), "tile_divisors": (0, 1, 2), "exact": (0, 0, 1)}
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+@pytest.mark.parametrize("B,M,N,Kd,bias", [
+    (1, 128, 128, 128, False),      # one tile, its second half outside the output
+    (1, 256, 384, 256, True),       # CTA pair; the last tile is half outside
+    (3, 384, 640, 384, True),       # batches, an odd number of row blocks
+    (1, 4992, 1664, 640, False),    # 39 x 7 tiles: a second and a third tile per CTA
+    (1, 10240, 1152, 256, False),   # 40 x 5 pair tiles, 80 x 5 single ones
+])
+def test_bf16_output_is_the_fp32_output_rounded(kind, B, M, N, Kd, bias):
+    g = torch.Generator().manual_seed(M + N)
+    a = torch.randint(-127, 128, (B, M, Kd), generator=g, dtype=torch.int8).to(DEV)
+    b = torch.randint(-127, 128, (N, Kd), generator=g, dtype=torch.int8).to(DEV)
+    a_s = (torch.rand(B * M * (Kd // 128), generator=g) * 0.1 + 0.01).to(DEV)
+    b_s = (torch.rand(N * (Kd // 128), generator=g) * 0.1 + 0.01).to(DEV)
+    bv = (torch.randn(N, generator=g) * 30).to(torch.bfloat16).to(DEV) if bias and kind != "rowcol" else None
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def call(out, flags):
+        stream = torch.cuda.current_stream().cuda_stream
+        if KINDS[kind] is None:
+            L.call("i8l_gemm_rowcol", a.data_ptr(), b.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), 0, None, 1.0, out,
+                   B, M, N, Kd, flags, status.data_ptr(), stream)
+        else:
+            ak, bk, fl = KINDS[kind]
+            L.call("i8l_gemm_block", a.data_ptr(), b.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), ak, bk, 0,
+                   None if bv is None else bv.data_ptr(), 0.25, out, B, M, N, Kd, fl | flags, status.data_ptr(), stream)
+
+    f32 = torch.empty(B * M, N, device=DEV)
+    call(f32.data_ptr(), L.GEMM_OUT_F32)
+    for shift in (0, 8):   # 32-byte aligned, 16-byte aligned
+        buf = torch.full((2 * GUARD + B * M * N,), 7.0, dtype=torch.bfloat16, device=DEV)
+        call(buf[GUARD + shift:].data_ptr(), 0)
+        torch.cuda.synchronize()
+        got = buf[GUARD + shift:GUARD + shift + B * M * N].view(B * M, N)
+        assert torch.equal(got, f32.to(torch.bfloat16))
+        assert (buf[:GUARD + shift] == 7).all() and (buf[GUARD + shift + B * M * N:] == 7).all()
+    assert status.item() == 0

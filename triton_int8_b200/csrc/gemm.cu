@@ -40,26 +40,25 @@
 namespace i8l {
 
 constexpr int BM = 128, BN = 256, BK = 128;
-#ifndef I8L_STAGES
-#define I8L_STAGES 4
-#endif
 constexpr int A_STAGE = BM * BK;  // bytes
-// One CTA per tile: 128x256 tile, 4 stages of 16 KB (A) + 32 KB (B).
+// One CTA per tile: 128x256 tile, 3 stages of 16 KB (A) + 32 KB (B).
 // CTA pair per tile (cta_group::2): 256x256 tile, each CTA stages its own 128 rows of A and 128 of the
-// 256 rows of B (16 KB + 16 KB), 6 stages: half the B traffic through each SM's shared memory.
+// 256 rows of B (16 KB + 16 KB), 5 stages: half the B traffic through each SM's shared memory.
+// One stage less than fits leaves the 64 KB that a bf16 output tile is staged in (store_tile).
 template <bool TWO> struct Cfg {
-  static constexpr int STAGES = TWO ? 6 : I8L_STAGES;
+  static constexpr int STAGES = TWO ? 5 : 3;
   static constexpr int B_STAGE = TWO ? BM * BK : BN * BK;
   static constexpr uint32_t STAGE_TX = TWO ? 2u * (A_STAGE + BM * BK) : (uint32_t)(A_STAGE + BN * BK);
 };
-constexpr int MAX_STAGES = 6;
+constexpr int MAX_STAGES = 5;
 constexpr int MAX_EPI_WARPS = 16;             // groups of four warps share the 256 accumulator columns
 // the kinds whose partial products are shifted by an extra MMA (K_BLOCK_FAST and the row and column factor kinds)
 template <int KIND> constexpr bool SHIFTED_OF = KIND >= 2;
 template <int KIND> constexpr int EPI_WARPS_OF = SHIFTED_OF<KIND> ? 8 : MAX_EPI_WARPS;
-constexpr int FAC_MAX = 256;                  // K blocks whose factors are staged in shared memory at a time (a multiple of 4)
+constexpr int FAC_MAX = 192;                  // K blocks whose factors are staged in shared memory at a time (a multiple of 4)
 constexpr int TMEM_COLS = 512;
-constexpr int SMEM_DYN = 4 * (A_STAGE + BN * BK) + 1024;  // == 6 * (16 KB + 16 KB) + 1024
+constexpr int OUT_STAGE = BM * BN * 2;        // the bf16 output tile
+template <bool TWO> constexpr int SMEM_DYN = Cfg<TWO>::STAGES * (A_STAGE + Cfg<TWO>::B_STAGE) + OUT_STAGE + 1024;
 
 struct GemmParams {
   const float* a_scale;
@@ -110,26 +109,6 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int m_units, const GemmPa
   return tc;
 }
 
-struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
-  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[2], tempty[2], done;
-  // fast block kind: factors written (factor warp), what the tile end needs written, all consumed (every epilogue thread)
-  uint64_t fready[2], eready[2], ffree[2];
-  uint32_t tmem_base;
-  int abort_flag;
-  float bscale[BN];     // per-tile column scales (CHANNEL)
-  float bstep[2][BN];   // per-K-block column scales or factors (GROUP), double buffered
-  // K_BLOCK_FAST, written by the factor warp one unit (tile, or FAC_MAX-K-block chunk of a tile) ahead, two
-  // buffers; each 128-column half (one epilogue group) has its factors (both share the first with per-channel B scales):
-  float2 fac[2][2][FAC_MAX];   // per K block: scaled factor, and the correction due at it (or 0)
-  float fbscale[2][BN];        // what the sums are multiplied by at the end: per-channel column scale times post_scale, or 1
-  float2 fend[2][2];           // in front of that: times .x plus .y (undoes the scaling of the factors, takes out what is left of the shift)
-  // scatter mode of the fast block kind: four output rows x 128 bytes per epilogue warp, staged so that one
-  // store instruction writes whole 128-byte row segments into the peer's memory
-  uint4 xpose[EPI_WARPS_OF<2>][4][8];
-  // shifted kinds: 256 rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
-  __align__(256) uint8_t ones[BN * 32];
-};
-
 // Epilogue kinds.  Everything but K_ROWCOL drains the accumulator every 128-wide K block.
 constexpr int K_ROWCOL = 0;      // one drain per tile, (float(acc)*a_s[m])*b_s[n]
 constexpr int K_BLOCK_GEN = 1;   // block-scaled, any scale layout, reference operation order, dumps
@@ -138,6 +117,30 @@ constexpr int K_BLOCK_COLFAC = 3;  // block-scaled, per-tile A scale x per-(colu
 constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x per-tile or per-channel B scale
 constexpr int K_BLOCK_TILEDIV = 6; // block-scaled, per-tile scales on both sides as divisors (fused backward)
 constexpr int K_BLOCK_OUTER = 5;   // block-scaled, per-(row, K block) A scale x per-(column, K block) B scale
+
+template <int KIND> struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[2], tempty[2], done;
+  // fast block kind: factors written (factor warp), what the tile end needs written, all consumed (every epilogue thread)
+  uint64_t fready[2], eready[2], ffree[2];
+  uint32_t tmem_base;
+  int abort_flag;
+  union {
+    struct {
+      float bscale[BN];     // per-tile column scales (CHANNEL)
+      float bstep[KIND == K_ROWCOL ? 1 : 2][KIND == K_ROWCOL ? 1 : BN];   // per-K-block column scales or factors (GROUP), double buffered
+    };
+    // K_BLOCK_FAST, written by the factor warp one unit (tile, or FAC_MAX-K-block chunk of a tile) ahead, two
+    // buffers; each 128-column half (one epilogue group) has its factors (both share the first with per-channel B scales):
+    struct {
+      float2 fac[KIND == K_BLOCK_FAST ? 2 : 1][2][KIND == K_BLOCK_FAST ? FAC_MAX : 1];   // per K block: scaled factor, and the correction due at it (or 0)
+      float fbscale[KIND == K_BLOCK_FAST ? 2 : 1][KIND == K_BLOCK_FAST ? BN : 1];        // what the sums are multiplied by at the end: per-channel column scale times post_scale, or 1
+      float2 fend[2][2];           // in front of that: times .x plus .y (undoes the scaling of the factors, takes out what is left of the shift)
+    };
+  };
+  // shifted kinds: 256 rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
+  __align__(256) uint8_t ones[SHIFTED_OF<KIND> ? BN * 32 : 1];
+};
+
 // Shifted kinds: 32 products 255 * 255.  A partial product of 128 int8 pairs lies in [-128*128*127, 128*128*128],
 // so P + SHIFT lies in [32, 4177952]: never negative and below 2^23, where the bits of an int32, read as a
 // float, are the (denormal) number (P + SHIFT) * 2^-149 exactly.
@@ -164,13 +167,62 @@ __device__ __forceinline__ void st_global_256(void* ptr, const uint32_t* w) {
                : "memory");
 }
 
-// Final rescale, bias, cast and store of one thread's EPI_COLS consecutive columns.  Every lane of
-// a warp writes a different row, so each store instruction touches 32 lines: 32-byte stores (whole
-// sectors, half as many instructions) are used when the output pointer allows them.
+// Bias of 16 consecutive columns.
+__device__ __forceinline__ void add_bias16(const __nv_bfloat16* bias, float* v) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __fadd_rn(v[j], __bfloat162float(bias[j]));
+}
+// 16 fp32 results of one row, straight to memory (32-byte stores where the output pointer allows them).
+__device__ __forceinline__ void store16_f32(const GemmParams& p, const float* v, void* cbase, int64_t row, int col) {
+  float* o = static_cast<float*>(cbase) + row * p.N + col;
+  if (p.c_align32) {
+    st_global_256(o, reinterpret_cast<const uint32_t*>(v));
+    st_global_256(o + 8, reinterpret_cast<const uint32_t*>(v + 8));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  }
+}
+
+// bf16 results leave through shared memory: a lane owns one row of the tile, so a plain store instruction touches 32
+// lines (about 45 cycles of the load/store unit each, 1.6 us a tile that nothing overlaps).  Each warp writes its 32 rows in
+// pieces of 64 columns (32 x 128 bytes, 128-byte swizzle: conflict-free) and one lane hands them to the TMA, which
+// stores whole rows while the warp goes on with the next tile.  Against stores from registers: fast block kind 4096^3
+// 71.4 -> 67.6 us, 8192^3 442 -> 434; row x channel 4096^3 100 -> 96.8; whole-K 384x11008x4096 20.5 -> 16.4, 4096^3
+// 49.3 -> 48.0 (the tile end overlaps the next main loop there, but the last one).  The stage of operands given up for
+// the staging memory costs nothing (4096^3 70.9 -> 70.4 us with 3 stages and stores from registers).
+__device__ __forceinline__ void stage_wait(int lane) {   // the warp's previous pieces have left shared memory
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ void stage16(uint32_t piece, int lane, int chunk, const float* v) {   // chunk: 16-byte unit, 0..7
+  uint32_t w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+  const uint32_t row = piece + lane * 128;
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                 ::"r"(row + (((chunk + k) ^ (lane & 7)) << 4)), "r"(w[4 * k]), "r"(w[4 * k + 1]), "r"(w[4 * k + 2]), "r"(w[4 * k + 3])
+                 : "memory");
+}
+template <int PIECES>
+__device__ __forceinline__ void stage_send(const CUtensorMap* map_c, uint32_t stage, int lane, int col, int row) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+#pragma unroll
+    for (int h = 0; h < PIECES; ++h) tma_store_2d(map_c, stage + h * 4096, col + 64 * h, row);
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+
+// Final rescale, bias, cast and store of one thread's EPI_COLS consecutive columns.
 // POST = false: the caller has already folded post_scale into the scales it passes.
 template <int EPI_COLS, bool POST = true>
-__device__ __forceinline__ void store_cols(const GemmParams& p, const float* acc, const float* bscale_or_null,
-                                           int64_t row, int col0, void* cbase) {
+__device__ __forceinline__ void store_cols(const GemmParams& p, const CUtensorMap* map_c, uint32_t stage, int lane, const float* acc,
+                                           const float* bscale_or_null, int64_t row, int col0, void* cbase) {
+  if (!p.out_f32) stage_wait(lane);
 #pragma unroll
   for (int j0 = 0; j0 < EPI_COLS; j0 += 16) {
     float v[16];
@@ -180,44 +232,23 @@ __device__ __forceinline__ void store_cols(const GemmParams& p, const float* acc
       if (bscale_or_null) v[j] *= bscale_or_null[j0 + j];
       if (POST && p.post_scale != 1.f) v[j] = __fmul_rn(v[j], p.post_scale);
     }
-    if (p.bias) {  // a uniform branch: no predicated-off loads and adds when there is no bias
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = __fadd_rn(v[j], __bfloat162float(p.bias[col0 + j0 + j]));
-    }
-    if (p.out_f32) {
-      float* o = static_cast<float*>(cbase) + row * p.N + col0 + j0;
-      if (p.c_align32) {
-        st_global_256(o, reinterpret_cast<const uint32_t*>(v));
-        st_global_256(o + 8, reinterpret_cast<const uint32_t*>(v + 8));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-      }
-    } else {
-      __nv_bfloat16* o = static_cast<__nv_bfloat16*>(cbase) + row * p.N + col0 + j0;
-      uint32_t w[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-      if (p.c_align32) {
-        st_global_256(o, w);
-      } else {
-        *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(o + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-      }
-    }
+    if (p.bias) add_bias16(p.bias + col0 + j0, v);   // a uniform branch: no predicated-off loads and adds when there is no bias
+    if (p.out_f32) store16_f32(p, v, cbase, row, col0 + j0);
+    else stage16(stage + j0 / 64 * 4096, lane, j0 % 64 / 8, v);
   }
+  if (!p.out_f32) stage_send<EPI_COLS / 64>(map_c, stage, lane, col0, (int)row - lane);
 }
 
 template <int KIND, bool TWO>
 __global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND>, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const GemmParams p) {
+               const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   constexpr bool BLOCK = KIND != K_ROWCOL, SHIFTED = SHIFTED_OF<KIND>;
   constexpr int EPI_WARPS = EPI_WARPS_OF<KIND>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
   constexpr int STAGES = Cfg<TWO>::STAGES, B_STAGE = Cfg<TWO>::B_STAGE;
   constexpr uint32_t STAGE_TX = Cfg<TWO>::STAGE_TX;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ SharedCtl ctl;
+  __shared__ SharedCtl<KIND> ctl;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a = smem_base, smem_b = smem_base + STAGES * A_STAGE;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -238,6 +269,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (threadIdx.x == 0) {
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
+    prefetch_tensormap(&map_c);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&ctl.full[s]), 1);
       mbar_init(smem_u32(&ctl.empty[s]), 1);
@@ -530,6 +562,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int q = warp & 3, wg = (warp - 4) >> 2;  // lane quarter, column group
     const int tix = q * 32 + lane;                 // row within the tile == thread index within the group
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    // this warp's 32 rows x EPI_COLS bf16 of the output tile; from the special register at each use, not kept live
+    auto out_stage = [&]() {
+      uint32_t tid;
+      asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+      return ((smem_u32(smem_raw) + 1023u) & ~1023u) + STAGES * (A_STAGE + B_STAGE) + ((tid >> 5) - 4) * (OUT_STAGE / EPI_WARPS);
+    };
     int ab = 0;
     uint32_t aph = 0;
     bool ok = true;
@@ -647,7 +685,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // pieces over NVLink; here the warp passes four rows at a time through shared memory (16-byte
             // slots, XOR-swizzled so that writers and readers are conflict-free) and every store instruction
             // then covers four rows x 128 contiguous bytes.  Same values as store_cols.
-            uint4* xp = &ctl.xpose[warp - 4][0][0];
+            uint4* xp = reinterpret_cast<uint4*>(smem_raw + (out_stage() - smem_u32(smem_raw)));
             const int wr = lane & 3, rr = lane >> 3, rc = lane & 7;
             __nv_bfloat16* obase = static_cast<__nv_bfloat16*>(cbase) + (row - lane) * p.N + col0 + rc * 8;
 #pragma unroll
@@ -669,7 +707,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               }
             }
           } else {
-            store_cols<EPI_COLS, false>(p, reinterpret_cast<const float*>(out), nullptr, row, col0, cbase);
+            store_cols<EPI_COLS, false>(p, &map_c, out_stage(), lane, reinterpret_cast<const float*>(out), nullptr, row, col0, cbase);
           }
         }
         mbar_arrive(smem_u32(&ctl.ffree[unit & 1]));   // this tile's factors and column scales are no longer needed
@@ -771,7 +809,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             out[2 * j] = acc[j].x * FROM_SHIFTED;
             out[2 * j + 1] = acc[j].y * FROM_SHIFTED;
           }
-          store_cols<EPI_COLS>(p, out, !COLF && chan ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
+          store_cols<EPI_COLS>(p, &map_c, out_stage(), lane, out, !COLF && chan ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
         }
       } else {
         // ---- generic paths: reference operation order, per-column / per-step scales, dumps, row x column
@@ -792,7 +830,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               named_sync(1 + wg, 128);
             }
           }
-          ok = ok && mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls);
+          float sar = 0.f;
+          if (!BLOCK && !p.dump) {
+            sar = __ldg(p.a_scale + row);
+            if (!p.out_f32) stage_wait(lane);
+          }
+          ok = ok && __all_sync(0xffffffffu, mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls));   // per warp: what follows synchronises it
           tc_fence_after();
           const bool live = ok && active;
           const uint32_t taddr = tmem_base + lane_addr + ab * BN + wg * EPI_COLS;
@@ -834,44 +877,46 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
             } else {
               // row x column epilogue straight from the accumulator chunk
-              const float sar = __ldg(p.a_scale + row);
+              const float4* bs4 = reinterpret_cast<const float4*>(ctl.bscale + wg * EPI_COLS + c * 16);
+              const float2 sar2 = make_float2(sar, sar);
               float v[16];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                v[j] = __fmul_rn(__fmul_rn(__int2float_rn((int)r[j]), sar), ctl.bscale[wg * EPI_COLS + c * 16 + j]);
-                if (p.post_scale != 1.f || p.bias) {
+              for (int j = 0; j < 4; ++j) {
+                const float4 bs = bs4[j];
+                const float2 lo = __fmul2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[4 * j]), __int2float_rn((int)r[4 * j + 1])), sar2), make_float2(bs.x, bs.y));
+                const float2 hi = __fmul2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[4 * j + 2]), __int2float_rn((int)r[4 * j + 3])), sar2), make_float2(bs.z, bs.w));
+                v[4 * j] = lo.x;
+                v[4 * j + 1] = lo.y;
+                v[4 * j + 2] = hi.x;
+                v[4 * j + 3] = hi.y;
+              }
+              if (p.post_scale != 1.f || p.bias) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
                   // the reference stores the GEMM result in the output type before its 1/K pass: a bf16
                   // rounding for bf16 outputs, none for fp32 ones
                   if (!p.out_f32) v[j] = round_to_bf16(v[j]);
                   v[j] = __fmul_rn(v[j], p.post_scale);
-                  if (p.bias) v[j] = __fadd_rn(v[j], __bfloat162float(p.bias[col0 + c * 16 + j]));
                 }
+                if (p.bias) add_bias16(p.bias + col0 + c * 16, v);
               }
-              if (p.out_f32) {
-                float* o = static_cast<float*>(p.c) + row * p.N + col0 + c * 16;
-#pragma unroll
-                for (int j = 0; j < 16; j += 4)
-                  *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-              } else {
-                __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.c) + row * p.N + col0 + c * 16;
-#pragma unroll
-                for (int j = 0; j < 16; j += 8)
-                  *reinterpret_cast<uint4*>(o + j) = make_uint4(pack_bf16x2(v[j], v[j + 1]), pack_bf16x2(v[j + 2], v[j + 3]),
-                                                                pack_bf16x2(v[j + 4], v[j + 5]), pack_bf16x2(v[j + 6], v[j + 7]));
-              }
+              if (p.out_f32) store16_f32(p, v, p.c, row, col0 + c * 16);
+              else stage16(out_stage(), lane, 2 * c, v);
             }
           }
+          if (!BLOCK && live && !p.dump && !p.out_f32) stage_send<EPI_COLS / 64>(&map_c, out_stage(), lane, col0, (int)row - lane);
           ab ^= 1;
           if (ab == 0) aph ^= 1u;
         }
         if constexpr (BLOCK) {
-          if (ok && active && !p.dump) store_cols<EPI_COLS>(p, acc, nullptr, row, col0, p.c);
+          if (ok && active && !p.dump) store_cols<EPI_COLS>(p, &map_c, out_stage(), lane, acc, nullptr, row, col0, p.c);
           if (p.b_kind == I8L_BSCALE_GROUP) named_sync(1 + wg, 128);   // bstep is free for the next tile (see the column factors above)
         }
       }
     }
   }
 
+  if (warp >= 4 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory outlives the copies out of it
 #undef I8L_UNIT
 #undef I8L_N_UNITS
   tc_fence_before();
@@ -927,32 +972,35 @@ static EncodeTiledFn get_encode() {
 // on (pointer, rows, K, box rows); a training loop calls with the same few operands step after step, so
 // the last maps of each host thread are kept (no lock: the cache is thread local) and the driver's
 // encode call leaves the launch path.
+// bf16_out: an output [rows, K] in boxes of box_rows x 64 elements instead (128 bytes as well).
 struct MapKey {
   const void* ptr;
   int64_t rows, K;
   int box_rows;
+  bool bf16_out;
 };
-static int make_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t K, int box_rows) {
+static int make_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t K, int box_rows, bool bf16_out = false) {
   constexpr int SLOTS = 16;
   thread_local MapKey keys[SLOTS] = {};
   thread_local CUtensorMap maps[SLOTS];
   thread_local int next_slot = 0;
   for (int i = 0; i < SLOTS; ++i)
-    if (keys[i].ptr == ptr && keys[i].rows == rows && keys[i].K == K && keys[i].box_rows == box_rows) {
+    if (keys[i].ptr == ptr && keys[i].rows == rows && keys[i].K == K && keys[i].box_rows == box_rows &&
+        keys[i].bf16_out == bf16_out) {
       *map = maps[i];
       return I8L_OK;
     }
   EncodeTiledFn enc = get_encode();
   if (!enc) return fail(I8L_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t gstr[1] = {(cuuint64_t)K};
-  cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+  cuuint64_t gstr[1] = {(cuuint64_t)K * (bf16_out ? 2 : 1)};
+  cuuint32_t box[2] = {(cuuint32_t)(bf16_out ? 64 : BK), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstr, box, estr,
+  CUresult r = enc(map, bf16_out ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstr, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(I8L_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-  keys[next_slot] = MapKey{ptr, rows, K, box_rows};
+  keys[next_slot] = MapKey{ptr, rows, K, box_rows, bf16_out};
   maps[next_slot] = *map;
   next_slot = (next_slot + 1) % SLOTS;
   return I8L_OK;
@@ -1009,7 +1057,7 @@ int gemm_cta_budget() {
 }
 
 template <int KIND, bool TWO>
-static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int64_t tiles, cudaStream_t st) {
+static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p, int64_t tiles, cudaStream_t st) {
   // per-device set-up, done by whichever thread comes first (idempotent, so a race only repeats it)
   static std::atomic<int> max_units[MAX_DEVICES];   // 0 = not set up yet
   const int dev = current_device();
@@ -1017,7 +1065,7 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.blockDim = dim3(128 + 32 * EPI_WARPS_OF<KIND>, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_DYN;
+  cfg.dynamicSmemBytes = SMEM_DYN<TWO>;
   cfg.stream = st;
   if (TWO) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1029,7 +1077,7 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   }
   int units = max_units[dev].load(std::memory_order_acquire);
   if (!units) {
-    I8L_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYN));
+    I8L_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYN<TWO>));
     units = sm_count();
     if (TWO) {  // how many CTA pairs can be co-resident (GPCs with an odd SM count leave one SM unpaired)
       cfg.gridDim = dim3(2 * sm_count(), 1, 1);
@@ -1045,7 +1093,7 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   }
   const int grid_units = (int)(tiles < units ? tiles : units);
   cfg.gridDim = dim3(TWO ? 2 * grid_units : grid_units, 1, 1);
-  I8L_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, ma, mb, p));
+  I8L_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, ma, mb, mc, p));
   return I8L_OK;
 }
 
@@ -1064,9 +1112,12 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   // whole-K accumulation (half the B traffic per SM: +2.5 % sustained at the power cap); the per-K-block
   // hand-off of the block-scaled kinds is slower across two CTAs (990 vs 1510 TOP/s), so those stay 1-CTA.
   const bool two = !block && (M % 256 == 0);
-  CUtensorMap ma, mb;
+  CUtensorMap ma, mb, mc;
   if (int e = make_map(&ma, a_q, batch * M, K, BM)) return e;
   if (int e = make_map(&mb, b_q, p.b_batched ? batch * N : N, K, two ? BM : BN)) return e;
+  mc = ma;   // read by nobody when the output is not bf16, or leaves for the owners of its rows
+  if (!p.out_f32 && !p.dump && !p.rs_rows)
+    if (int e = make_map(&mc, p.c, batch * M, N, 32, true)) return e;
   p.m_blocks = (int)(batch * M / 128);
   p.mpb = (int)(M / 128);
   p.n_tiles = (int)((N + BN - 1) / BN);
@@ -1096,13 +1147,13 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   const bool column_factor = block && !p.exact && !p.dump && p.a_kind == I8L_ASCALE_TILE && p.b_kind == I8L_BSCALE_GROUP;
   const bool outer_factor = block && !p.exact && !p.dump && !p.divide && p.a_kind == I8L_ASCALE_GROUP &&
                             p.b_kind == I8L_BSCALE_GROUP;
-  if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, p, tiles, st);
-  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && !p.divide) return launch_kind<K_BLOCK_FAST, false>(ma, mb, p, tiles, st);
-  if (scalar_factor && p.divide) return launch_kind<K_BLOCK_TILEDIV, false>(ma, mb, p, tiles, st);
-  if (scalar_factor) return launch_kind<K_BLOCK_ROWFAC, false>(ma, mb, p, tiles, st);
-  if (outer_factor) return launch_kind<K_BLOCK_OUTER, false>(ma, mb, p, tiles, st);
-  if (column_factor) return launch_kind<K_BLOCK_COLFAC, false>(ma, mb, p, tiles, st);
-  return launch_kind<K_BLOCK_GEN, false>(ma, mb, p, tiles, st);
+  if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, mc, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, mc, p, tiles, st);
+  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && !p.divide) return launch_kind<K_BLOCK_FAST, false>(ma, mb, mc, p, tiles, st);
+  if (scalar_factor && p.divide) return launch_kind<K_BLOCK_TILEDIV, false>(ma, mb, mc, p, tiles, st);
+  if (scalar_factor) return launch_kind<K_BLOCK_ROWFAC, false>(ma, mb, mc, p, tiles, st);
+  if (outer_factor) return launch_kind<K_BLOCK_OUTER, false>(ma, mb, mc, p, tiles, st);
+  if (column_factor) return launch_kind<K_BLOCK_COLFAC, false>(ma, mb, mc, p, tiles, st);
+  return launch_kind<K_BLOCK_GEN, false>(ma, mb, mc, p, tiles, st);
 }
 
 }  // namespace i8l
