@@ -1,0 +1,82 @@
+"""The kernels of one composed call overlap on the device (programmatic serialization).  Many calls in a row, each on
+other inputs and all in the same recycled memory, equal the separate steps, which are launched one after the other, bit
+for bit; so does a replayed graph."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if torch.cuda.is_available():
+    from triton_int8_b200 import linear as LN
+    from triton_int8_b200.linear import Int8Config
+
+DEV = "cuda"
+SHAPES = [(128, 128, 128), (128, 2048, 384), (1920, 640, 1408), (3968, 1152, 2176)]
+
+
+def _separate(x, w, dy, bias, cfg):
+    """Every kernel through its own entry point."""
+    from triton_int8_b200 import _lib as L
+    from triton_int8_b200 import kernels as K
+    if cfg.whole_k:
+        xq, xs = K.quant_row(x[None], L.QMODE_ROWRCP, cfg.hadamard)
+        wq, ws = K.quant_row(w, L.QMODE_ROWRCP, cfg.hadamard)
+        xt = LN._dc_transposed(x, cfg)
+        y = K.gemm_rowcol(xq, wq, xs, ws, bias, cfg.post_for(x.shape[1]))[0]
+    else:
+        xq, xs, xqt, xst = K.quant_tile(x[None], cfg.gran, cfg.qmode, cfg.hadamard, natural=True, transposed=True)
+        wq, ws = K.quant_row(w, cfg.qmode, cfg.hadamard)
+        xt = (xqt, xst)
+        y = K.gemm_block(xq, wq, xs, ws, cfg.a_kind, L.BSCALE_CHANNEL, bias, cfg.post, cfg.flags)[0]
+    dy_op, dyt_op = LN.quantize_grad_output(dy, cfg)
+    return y, LN.grad_input(dy_op, w, cfg), LN.grad_weight(dyt_op, xt, cfg)
+
+
+def _composed(x, w, dy, bias, cfg):
+    y, saved = LN.linear_forward(x, w, bias, cfg)
+    dx, dw = LN.linear_backward(dy, w, saved, cfg)
+    return y, dx, dw
+
+
+def _inputs(shape, n):
+    M, N, K = shape
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)
+    return [(r(M, K), r(N, K), r(M, N), r(N)) for _ in range(n)]
+
+
+@pytest.mark.parametrize("scaling,rnd,had", [("tile128", "half_up", 0), ("tile128", "half_up", 128), ("row128", "rne", 0),
+                                             ("row128", "rne", 128), ("double_channel", "half_up", 0),
+                                             ("double_channel", "half_up", 128)])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_calls_in_a_row_equal_separate_steps(shape, scaling, rnd, had):
+    cfg = Int8Config(scaling=scaling, round=rnd, hadamard=had)
+    ins = _inputs(shape, 4)
+    refs = []
+    for i in ins:
+        refs.append([t.clone() for t in _separate(*i, cfg)])
+        torch.cuda.synchronize()
+    outs = [_composed(*ins[k % 4], cfg) for k in range(12)]   # nothing waits in between
+    torch.cuda.synchronize()
+    for k, out in enumerate(outs):
+        for name, got, ref in zip(("y", "dx", "dw"), out, refs[k % 4]):
+            assert torch.equal(got, ref), f"call {k}: {name}"
+
+
+def test_chain_in_a_graph_equals_separate_steps():
+    cfg = Int8Config(hadamard=128)
+    ins = _inputs((1920, 640, 1408), 3)
+    static = [t.clone() for t in ins[0]]
+    _composed(*static, cfg)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = _composed(*static, cfg)
+    for i in ins:
+        ref = _separate(*i, cfg)
+        for s, t in zip(static, i):
+            s.copy_(t)
+        g.replay()
+        torch.cuda.synchronize()
+        for got, want in zip(out, ref):
+            assert torch.equal(got, want)

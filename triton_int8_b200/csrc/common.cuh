@@ -21,6 +21,10 @@ uint32_t gemm_wait_limit();
 int gemm_cta_budget();
 int sm_count();  // of the current device
 
+// i8l_quant_col_t (rot = false) or i8l_quant_col_t_rot; zeroed: colmax is zero already, no memset goes in front.
+int quant_col_t(const char* name, const void* x, int64_t rows, int64_t cols, int qmode, bool rot, int8_t* qt, float* scale_t,
+                float* colmax, bool zeroed, cudaStream_t st);
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 #define I8L_CUDA_OK(expr)                                                                  \
@@ -29,6 +33,48 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
     if (_e != cudaSuccess)                                                                 \
       return i8l::fail(I8L_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(_e));      \
   } while (0)
+
+// ---------------------------------------------------------------- chains of launches
+// The kernels of one composed call (compose.cu) follow one another on a stream.  The first is launched as usual and so
+// starts when all earlier work of the stream is done; the others are launched with programmatic serialization and start
+// as soon as every block of their predecessor has started and there is room: launch latency, prologues and the tails
+// of small grids overlap (2-3 us a launch).  Every kernel triggers its successor first thing.  What it may do ahead of
+// chain_wait(), which returns when the predecessor has completed and its writes are visible:
+//   quantizers  everything: they read the caller's inputs and write memory that no kernel of the chain reads or writes
+//               before them.  They wait at their end, so that "predecessor completed" covers the whole chain;
+//   passes that need a predecessor's result (scales from a column maximum) and GEMMs: nothing but their set-up.
+// Outside a chain both are no-ops.
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// This host thread's chain: 0 none, 1 its first kernel is not launched yet, 2 the stream's last operation is one of its kernels.
+extern thread_local int launch_chain;
+struct LaunchChain {
+  LaunchChain() { launch_chain = 1; }
+  ~LaunchChain() { launch_chain = 0; }
+  static void broken() { if (launch_chain) launch_chain = 1; }   // an operation that is not a kernel went into the stream
+};
+// Adds the attribute to a launch of the chain; attrs has room for one more.
+inline void chain_attribute(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs) {
+  if (launch_chain == 2) {
+    attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    ++cfg.numAttrs;
+  }
+  if (launch_chain == 1) launch_chain = 2;
+}
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attrs[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  chain_attribute(cfg, attrs);
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // ---------------------------------------------------------------- scale / rounding arithmetic
 // All operations are spelled with explicit round-to-nearest intrinsics so that the compiler can

@@ -44,10 +44,11 @@ int quant(const void* x, int64_t batch, int64_t rows, int64_t cols, int gran, in
   return i8l_quant_tile(x, batch, rows, cols, gran, qmode, had, q, s, nullptr, nullptr, stream);
 }
 int quant_col_t(const void* x, int64_t rows, int64_t cols, int qmode, int had, int8_t* qt, float* st, float* scratch,
-                void* stream) {
-  if (had == I8L_HAD_128) return i8l_quant_col_t_rot(x, rows, cols, qmode, qt, st, scratch, stream);
-  if (had == I8L_HAD_NONE) return i8l_quant_col_t(x, rows, cols, qmode, qt, st, scratch, stream);
-  return fail(I8L_ERR_ARG, "a transposed operand is rotated in 128-wide groups or not at all");
+                bool zeroed, void* stream) {
+  if (had != I8L_HAD_128 && had != I8L_HAD_NONE)
+    return fail(I8L_ERR_ARG, "a transposed operand is rotated in 128-wide groups or not at all");
+  return i8l::quant_col_t("quant_col_t", x, rows, cols, qmode, had == I8L_HAD_128, qt, st, scratch, zeroed,
+                          static_cast<cudaStream_t>(stream));
 }
 // Before sizes are multiplied (batch * rows * K must fit 64 bits): the entry points below check the rest, with the limits
 // of their own grids.  batch * M and batch * N fit 31 bits wherever a GEMM accepts them.
@@ -78,6 +79,7 @@ extern "C" int i8l_quant_gemm(const void* a, const void* b, const void* bias, vo
   float* bs = ws.take<float>(scale_count(b_gran, b_n, N, K));
   float* colmax = a_qt && a_gran == I8L_GRAN_ROW ? ws.take<float>(K) : nullptr;
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_quant_gemm: workspace of %lld bytes is too small", (long long)workspace_bytes);
+  const LaunchChain chain;
   if (a_qt && a_gran != I8L_GRAN_ROW) {   // both orientations of A from one call
     if (int e = i8l_quant_tile(a, batch, M, K, a_gran, qmode, hadamard, aq, as, a_qt, a_st, stream)) return e;
   } else {
@@ -86,7 +88,7 @@ extern "C" int i8l_quant_gemm(const void* a, const void* b, const void* bias, vo
   if (int e = quant(b, b_n, N, K, b_gran, qmode, hadamard, bq, bs, stream)) return e;
   if (a_gran == I8L_GRAN_ROW) {
     if (int e = i8l_gemm_rowcol(aq, bq, as, bs, b_batched, bias, post_scale, c, batch, M, N, K, flags, status, stream)) return e;
-    return a_qt ? quant_col_t(a, M, K, qmode, hadamard, a_qt, a_st, colmax, stream) : I8L_OK;
+    return a_qt ? quant_col_t(a, M, K, qmode, hadamard, a_qt, a_st, colmax, false, stream) : I8L_OK;
   }
   return i8l_gemm_block(aq, bq, as, bs, a_kind_of(a_gran), b_kind_of(b_gran), b_batched, bias, post_scale, c, batch, M, N, K,
                         flags, status, stream);
@@ -117,16 +119,24 @@ extern "C" int i8l_linear_backward(const void* dy, const void* w, const int8_t* 
   }
   float* colmax = ws.take<float>(K > N ? K : N);
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_linear_backward: workspace of %lld bytes is too small", (long long)workspace_bytes);
+  // The column maxima of W start from zeros that go in first, where no other pass needs the scratch: a memset between
+  // the kernels would break the chain.
+  const bool zeroed = dx && !whole_k;
+  if (zeroed) {
+    if (int e = check_arch()) return e;
+    I8L_CUDA_OK(cudaMemsetAsync(colmax, 0, (size_t)K * sizeof(float), static_cast<cudaStream_t>(stream)));
+  }
+  const LaunchChain chain;
   if (whole_k) {
     if (dx)
       if (int e = i8l_quant_row(dy, M, N, qmode, hadamard, dyq, dys, stream)) return e;
     if (dw)
-      if (int e = quant_col_t(dy, M, N, qmode, hadamard, dyqt, dyst, colmax, stream)) return e;
+      if (int e = quant_col_t(dy, M, N, qmode, hadamard, dyqt, dyst, colmax, false, stream)) return e;
   } else if (dx || dw) {
     if (int e = i8l_quant_tile(dy, 1, M, N, gran, qmode, hadamard, dyq, dys, dyqt, dyst, stream)) return e;
   }
   if (dx) {   // dX = dY W, contraction over N
-    if (int e = quant_col_t(w, N, K, qmode, hadamard, wqt, wst, colmax, stream)) return e;
+    if (int e = quant_col_t(w, N, K, qmode, hadamard, wqt, wst, colmax, zeroed, stream)) return e;
     const int e = whole_k ? i8l_gemm_rowcol(dyq, wqt, dys, wst, 0, nullptr, post_dx, dx, 1, M, K, N, flags, status, stream)
                           : i8l_gemm_block(dyq, wqt, dys, wst, a_kind_of(gran), I8L_BSCALE_CHANNEL, 0, nullptr, post_dx, dx, 1, M,
                                            K, N, flags, status, stream);

@@ -10,6 +10,7 @@
 namespace i8l {
 
 static thread_local char g_err[512] = "";
+thread_local int launch_chain = 0;
 
 int fail(int code, const char* fmt, ...) {
   va_list ap;
@@ -67,6 +68,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
   const __nv_bfloat16* xb = x + boff;
+  chain_trigger();
 
   // The tile stays in registers as packed bf16 (32 registers per thread, 4 CTAs per SM).
   uint4 raw[2][4];
@@ -145,7 +147,8 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
 #pragma unroll
         for (int k = 1; k < 8; ++k) m = fmaxf(m, s_colred[k * 128 + tid]);
       } else {
-        m = colmax[c_base + tid];
+        chain_wait();
+        m = __ldcg(colmax + c_base + tid);
       }
       float s, stored;
       make_scale<MODE>(m, s, stored);
@@ -208,6 +211,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
       *reinterpret_cast<uint32_t*>(qtb + (c_base + c) * rows + r_base + 4 * l) = word;
     }
   }
+  chain_wait();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -223,6 +227,7 @@ quant_tile256_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t 
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 256;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
+  chain_trigger();
   uint4 raw[16];
   __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
@@ -244,6 +249,7 @@ quant_tile256_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t 
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     *reinterpret_cast<uint2*>(q + boff + (r_base + 16 * w + i) * cols + c_base + 8 * l) = quant_piece<MODE>(raw[i], s);
+  chain_wait();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -354,6 +360,7 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
+  chain_trigger();
   {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
     const __nv_bfloat16* src = x + boff + (r_base + (tid >> 4)) * cols + c_base + 8 * (tid & 15);
@@ -383,7 +390,7 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
     if (!finite) m = max_without_nan(h);
     if (GRAN == GRAN_COLMAX_PASS) {  // |x| >= 0: the bit patterns order like integers, so an integer maximum is exact
       atomicMax(reinterpret_cast<int*>(colmax + c_base + tid), __float_as_int(m));
-      return;
+      break;
     }
     if (GRAN == I8L_GRAN_TILE128) {
 #pragma unroll
@@ -392,7 +399,10 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
       __syncthreads();
       m = fmaxf(fmaxf(s_red[ph][0], s_red[ph][1]), fmaxf(s_red[ph][2], s_red[ph][3]));
     }
-    if (GRAN == GRAN_COLFULL) m = colmax[c_base + tid];
+    if (GRAN == GRAN_COLFULL) {
+      chain_wait();
+      m = __ldcg(colmax + c_base + tid);
+    }
     make_scale<MODE>(m, s, stored);
     const int64_t o_base = ph == 0 ? r_base : c_base, k_base = ph == 0 ? c_base : r_base;  // output row, contraction axis
     const int64_t o_n = ph == 0 ? rows : cols, k_n = ph == 0 ? cols : rows, kb = k_base / 128, nkb = k_n / 128;
@@ -406,6 +416,7 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
     if (finite) quant_store128<MODE, true>(h, s, row, align32);
     else quant_store128<MODE, false>(h, s, row, align32);
   }
+  chain_wait();
 }
 
 // Column absmax of x [rows, cols] into colmax[cols] (pre-zeroed); |x| >= 0 so the float bit
@@ -415,6 +426,7 @@ col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
   __shared__ float s_colred[8 * 128];
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, cc = l & 15, half = l >> 4;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
+  chain_trigger();
   float m[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) m[j] = 0.f;
@@ -441,6 +453,7 @@ col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
     for (int k = 1; k < 8; ++k) mm = fmaxf(mm, s_colred[k * 128 + tid]);
     atomicMax(reinterpret_cast<int*>(colmax + c_base + tid), __float_as_int(mm));
   }
+  chain_wait();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -456,6 +469,7 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __re
   const int64_t row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int nchunks = (int)(cols / 8);
+  chain_trigger();
 
   float m = 0.f;
   for (int base = 0; base < nchunks; base += 256) {
@@ -506,6 +520,7 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __re
       qr[ch] = o;
     }
   }
+  chain_wait();
 }
 
 // Rows of at most 16384 elements: T threads per row (256/T rows per CTA) keep the row in registers, up to
@@ -522,6 +537,7 @@ quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64
   const bool live = row < rows;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int nchunks = live ? (int)(cols / 8) : 0;
+  chain_trigger();
   uint4 cache[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) cache[i] = i * T + t < nchunks ? __ldg(xr + i * T + t) : make_uint4(0, 0, 0, 0);
@@ -557,6 +573,7 @@ quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     if (i * T + t < nchunks) qr[i * T + t] = finite ? quant_piece_finite<MODE>(cache[i], s) : quant_piece<MODE>(cache[i], s);
+  chain_wait();
 }
 
 // The same with the 128-point rotation.  A CTA takes as many whole rows as fit into 128 groups of 128 elements,
@@ -572,6 +589,7 @@ quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int grou
   const int tid = threadIdx.x, my_row = tid / groups;
   const int64_t row0 = (int64_t)blockIdx.x * rows_per_cta;
   const int n_rows = (int)(rows - row0 < rows_per_cta ? rows - row0 : rows_per_cta), n = n_rows * groups;
+  chain_trigger();
   const __nv_bfloat16* src = x + row0 * groups * 128 + 8 * tid;   // whole rows are contiguous
   const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
 #pragma unroll
@@ -601,6 +619,7 @@ quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int grou
   const bool align32 = (reinterpret_cast<uintptr_t>(q) & 31u) == 0;
   if (finite) quant_store128<MODE, true>(h, s, out, align32);
   else quant_store128<MODE, false>(h, s, out, align32);
+  chain_wait();   // the first group of a block is always live
 }
 
 // Whole-row rotation of rows of G groups of 128 (G = 2..128).  A CTA takes 128/G whole rows.  Spans 1..64 run in
@@ -632,6 +651,7 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t row0 = (int64_t)blockIdx.x * R;
   const int n_rows = (int)(rows - row0 < R ? rows - row0 : R), n = n_rows * G;
+  chain_trigger();
   {
     const __nv_bfloat16* src = x + row0 * G * 128 + 8 * tid;   // whole rows are contiguous
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
@@ -742,6 +762,7 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
   };
   if (__all_sync(0xffffffffu, finite)) write(std::true_type{});   // one branch per warp: the shuffles need all lanes
   else write(std::false_type{});
+  chain_wait();
 }
 
 // Whole-row Hadamard, one CTA per row (few rows, or rows of 32768 elements): the row lives in shared memory as fp32.
@@ -756,6 +777,7 @@ quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8
   const int64_t row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int n = (int)cols, nchunks = n / 8;
+  chain_trigger();
 
   for (int base = 0; base < nchunks; base += 256) {
     const int ch = base + tid;
@@ -802,6 +824,7 @@ quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8
     const float4 f = *reinterpret_cast<const float4*>(s_row + 4 * i);
     qr[i] = pack4(quant1<MODE>(f.x, s), quant1<MODE>(f.y, s), quant1<MODE>(f.z, s), quant1<MODE>(f.w, s));
   }
+  chain_wait();
 }
 
 // ------------------------------------------------------------------------------------------------ host
@@ -827,8 +850,7 @@ static int launch_rotfull(const __nv_bfloat16* x, int64_t rows, int8_t* q, float
   static std::atomic<bool> attr_done[MAX_DEVICES];
   I8L_CUDA_OK(ensure_smem(quant_row_rotfull_kernel<MODE, G>, attr_done, FULL_SMEM));
   constexpr int R = 128 / G;
-  quant_row_rotfull_kernel<MODE, G><<<(unsigned)((rows + R - 1) / R), 128, FULL_SMEM, st>>>(x, rows, q, scale);
-  I8L_CUDA_OK(cudaGetLastError());
+  I8L_CUDA_OK(launch(quant_row_rotfull_kernel<MODE, G>, dim3((unsigned)((rows + R - 1) / R)), 128, FULL_SMEM, st, x, rows, q, scale));
   return I8L_OK;
 }
 template <int MODE>
@@ -849,8 +871,7 @@ static int launch_hadfull(const __nv_bfloat16* x, int64_t rows, int64_t cols, in
   static std::atomic<bool> attr_done[MAX_DEVICES];
   const size_t smem = (size_t)cols * sizeof(float);
   I8L_CUDA_OK(ensure_smem(quant_row_hadfull_kernel<MODE>, attr_done, 32768 * sizeof(float)));
-  quant_row_hadfull_kernel<MODE><<<(unsigned)rows, 256, smem, st>>>(x, cols, q, scale);
-  I8L_CUDA_OK(cudaGetLastError());
+  I8L_CUDA_OK(launch(quant_row_hadfull_kernel<MODE>, dim3((unsigned)rows), 256, smem, st, x, cols, q, scale));
   return I8L_OK;
 }
 
@@ -864,11 +885,11 @@ static int check_dims(int64_t batch, int64_t rows, int64_t cols) {
 }
 
 template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
-static void launch_tile(const void* x, int64_t batch, int64_t rows, int64_t cols, int8_t* q, float* scale,
+static cudaError_t launch_tile(const void* x, int64_t batch, int64_t rows, int64_t cols, int8_t* q, float* scale,
                         int8_t* qt, float* scale_t, const float* colmax, cudaStream_t st) {
   dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
-  quant_tile_kernel<GRAN, MODE, OUT_N, OUT_T><<<grid, 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(x), rows, cols, q, scale, qt, scale_t, colmax);
+  return launch(quant_tile_kernel<GRAN, MODE, OUT_N, OUT_T>, grid, 256, 0, st, static_cast<const __nv_bfloat16*>(x), rows, cols, q,
+                scale, qt, scale_t, colmax);
 }
 
 template <int GRAN, int MODE>
@@ -878,18 +899,17 @@ static int dispatch_tile(const void* x, int64_t batch, int64_t rows, int64_t col
   if (had) {  // whatever is wanted of the two orientations, from one read of the tile
     const dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-    if (n && t) quant_tile_rot_kernel<GRAN, MODE, true, true><<<grid, 128, 0, st>>>(xp, rows, cols, q, scale, qt, scale_t, nullptr);
-    else if (n) quant_tile_rot_kernel<GRAN, MODE, true, false><<<grid, 128, 0, st>>>(xp, rows, cols, q, scale, nullptr, nullptr, nullptr);
-    else quant_tile_rot_kernel<GRAN, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, qt, scale_t, nullptr);
+    if (n && t) I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, true, true>, grid, 128, 0, st, xp, rows, cols, q, scale, qt, scale_t, nullptr));
+    else if (n) I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, true, false>, grid, 128, 0, st, xp, rows, cols, q, scale, nullptr, nullptr, nullptr));
+    else I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr, qt, scale_t, nullptr));
   } else if (GRAN == I8L_GRAN_TILE128) {
-    if (n && t) launch_tile<GRAN, MODE, true, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
-    else if (n) launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
-    else launch_tile<GRAN, MODE, false, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st);
+    if (n && t) I8L_CUDA_OK((launch_tile<GRAN, MODE, true, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st)));
+    else if (n) I8L_CUDA_OK((launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st)));
+    else I8L_CUDA_OK((launch_tile<GRAN, MODE, false, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st)));
   } else {  // grouped scales differ between the two orientations: one launch each
-    if (n) launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, nullptr, nullptr, colmax, st);
-    if (t) launch_tile<GRAN, MODE, false, true>(x, batch, rows, cols, nullptr, nullptr, qt, scale_t, colmax, st);
+    if (n) I8L_CUDA_OK((launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, nullptr, nullptr, colmax, st)));
+    if (t) I8L_CUDA_OK((launch_tile<GRAN, MODE, false, true>(x, batch, rows, cols, nullptr, nullptr, qt, scale_t, colmax, st)));
   }
-  I8L_CUDA_OK(cudaGetLastError());
   return I8L_OK;
 }
 
@@ -914,10 +934,9 @@ extern "C" int i8l_quant_tile(const void* x, int64_t batch, int64_t rows, int64_
     if (cols % 256 || had || qt || !q) return fail(I8L_ERR_ARG, "i8l_quant_tile: 128x256 groups need cols %% 256 == 0, no rotation, q only");
     const dim3 grid((unsigned)(cols / 256), (unsigned)(rows / 128), (unsigned)batch);
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-    if (qmode == I8L_QMODE_TRITON) quant_tile256_kernel<I8L_QMODE_TRITON><<<grid, 256, 0, st>>>(xp, rows, cols, q, scale);
-    else if (qmode == I8L_QMODE_TRITON_BF16S) quant_tile256_kernel<I8L_QMODE_TRITON_BF16S><<<grid, 256, 0, st>>>(xp, rows, cols, q, scale);
+    if (qmode == I8L_QMODE_TRITON) I8L_CUDA_OK(launch(quant_tile256_kernel<I8L_QMODE_TRITON>, grid, 256, 0, st, xp, rows, cols, q, scale));
+    else if (qmode == I8L_QMODE_TRITON_BF16S) I8L_CUDA_OK(launch(quant_tile256_kernel<I8L_QMODE_TRITON_BF16S>, grid, 256, 0, st, xp, rows, cols, q, scale));
     else return fail(I8L_ERR_ARG, "i8l_quant_tile: 128x256 groups support qmode TRITON and TRITON_BF16S");
-    I8L_CUDA_OK(cudaGetLastError());
     return I8L_OK;
   }
 #define I8L_TILE_CASE(G, Mo) \
@@ -960,19 +979,19 @@ extern "C" int i8l_quant_row(const void* x, int64_t rows, int64_t cols, int qmod
   // it in eight pieces each.
   const int groups = (int)(cols / 128), rpc = 128 / groups;
 #define I8L_ROW_T(Mo, T) \
-  quant_row_cached_kernel<Mo, T><<<(unsigned)((rows + 256 / T - 1) / (256 / T)), 256, 0, st>>>(xp, rows, cols, q, scale)
-#define I8L_ROW_CASE(Mo)                                                                                  \
-  if (qmode == Mo) {                                                                                      \
-    if (hadamard && rpc)                                                                                  \
-      quant_row_rot_kernel<Mo><<<(unsigned)((rows + rpc - 1) / rpc), 128, 0, st>>>(xp, rows, groups, rpc, q, scale); \
-    else if (hadamard) quant_row_kernel<Mo, true><<<(unsigned)rows, 256, 0, st>>>(xp, cols, q, scale);    \
-    else if (cols <= 2048) I8L_ROW_T(Mo, 32);                                                             \
-    else if (cols <= 4096) I8L_ROW_T(Mo, 64);                                                             \
-    else if (cols <= 8192) I8L_ROW_T(Mo, 128);                                                            \
-    else if (cols <= 16384) I8L_ROW_T(Mo, 256);                                                           \
-    else quant_row_kernel<Mo, false><<<(unsigned)rows, 256, 0, st>>>(xp, cols, q, scale);                 \
-    I8L_CUDA_OK(cudaGetLastError());                                                                      \
-    return I8L_OK;                                                                                        \
+  launch(quant_row_cached_kernel<Mo, T>, dim3((unsigned)((rows + 256 / T - 1) / (256 / T))), 256, 0, st, xp, rows, cols, q, scale)
+#define I8L_ROW_CASE(Mo)                                                                                      \
+  if (qmode == Mo) {                                                                                          \
+    I8L_CUDA_OK(                                                                                              \
+        hadamard && rpc ? launch(quant_row_rot_kernel<Mo>, dim3((unsigned)((rows + rpc - 1) / rpc)), 128, 0, st, xp, rows, groups, \
+                                 rpc, q, scale)                                                               \
+        : hadamard      ? launch(quant_row_kernel<Mo, true>, dim3((unsigned)rows), 256, 0, st, xp, cols, q, scale) \
+        : cols <= 2048  ? I8L_ROW_T(Mo, 32)                                                                   \
+        : cols <= 4096  ? I8L_ROW_T(Mo, 64)                                                                   \
+        : cols <= 8192  ? I8L_ROW_T(Mo, 128)                                                                  \
+        : cols <= 16384 ? I8L_ROW_T(Mo, 256)                                                                  \
+                        : launch(quant_row_kernel<Mo, false>, dim3((unsigned)rows), 256, 0, st, xp, cols, q, scale)); \
+    return I8L_OK;                                                                                            \
   }
   I8L_ROW_CASE(I8L_QMODE_TRITON)
   I8L_ROW_CASE(I8L_QMODE_RNE)
@@ -983,54 +1002,50 @@ extern "C" int i8l_quant_row(const void* x, int64_t rows, int64_t cols, int qmod
   return fail(I8L_ERR_ARG, "i8l_quant_row: unsupported qmode=%d", qmode);
 }
 
-extern "C" int i8l_quant_col_t(const void* x, int64_t rows, int64_t cols, int qmode, int8_t* qt, float* scale_t,
-                               float* colmax_scratch, void* stream) {
-  if (int e = check_dims(1, rows, cols)) return e;
-  if (!x || !qt || !scale_t || !colmax_scratch) return fail(I8L_ERR_ARG, "null pointer");
-  if (!aligned16(x) || !aligned16(qt)) return fail(I8L_ERR_ALIGN, "x, qt must be 16-byte aligned");
-  if (int e = check_arch()) return e;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  I8L_CUDA_OK(cudaMemsetAsync(colmax_scratch, 0, (size_t)cols * sizeof(float), st));
-  dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), 1);
-  col_absmax_kernel<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, colmax_scratch);
-  I8L_CUDA_OK(cudaGetLastError());
-#define I8L_COL_CASE(Mo)                                                                                     \
-  if (qmode == Mo) {                                                                                         \
-    launch_tile<GRAN_COLFULL, Mo, false, true>(x, 1, rows, cols, nullptr, nullptr, qt, scale_t,       \
-                                                      colmax_scratch, st);                                   \
-    I8L_CUDA_OK(cudaGetLastError());                                                                         \
-    return I8L_OK;                                                                                           \
-  }
-  I8L_COL_CASE(I8L_QMODE_TRITON)
-  I8L_COL_CASE(I8L_QMODE_RNE)
-  I8L_COL_CASE(I8L_QMODE_ROWRCP)
-#undef I8L_COL_CASE
-  return fail(I8L_ERR_ARG, "i8l_quant_col_t: unsupported qmode=%d", qmode);
-}
-
+// Both passes of one scale per column; colmax is zero.
 template <int MODE>
-static int launch_col_t_rot(const void* x, int64_t rows, int64_t cols, int8_t* qt, float* scale_t, float* colmax,
-                            cudaStream_t st) {
+static int launch_col_t(const void* x, int64_t rows, int64_t cols, bool rot, int8_t* qt, float* scale_t, float* colmax,
+                        cudaStream_t st) {
   const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
   const dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), 1);
-  quant_tile_rot_kernel<GRAN_COLMAX_PASS, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, nullptr, nullptr, colmax);
-  quant_tile_rot_kernel<GRAN_COLFULL, MODE, false, true><<<grid, 128, 0, st>>>(xp, rows, cols, nullptr, nullptr, qt, scale_t, colmax);
-  I8L_CUDA_OK(cudaGetLastError());
+  if (rot) {
+    I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN_COLMAX_PASS, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr,
+                       nullptr, nullptr, colmax));
+    I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN_COLFULL, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr, qt,
+                       scale_t, colmax));
+  } else {
+    I8L_CUDA_OK(launch(col_absmax_kernel, grid, 256, 0, st, xp, rows, cols, colmax));
+    I8L_CUDA_OK((launch_tile<GRAN_COLFULL, MODE, false, true>(x, 1, rows, cols, nullptr, nullptr, qt, scale_t, colmax, st)));
+  }
   return I8L_OK;
+}
+
+namespace i8l {
+int quant_col_t(const char* name, const void* x, int64_t rows, int64_t cols, int qmode, bool rot, int8_t* qt, float* scale_t,
+                float* colmax, bool zeroed, cudaStream_t st) {
+  if (int e = check_dims(1, rows, cols)) return e;
+  if (!x || !qt || !scale_t || !colmax) return fail(I8L_ERR_ARG, "null pointer");
+  if (!aligned16(x) || !aligned16(qt)) return fail(I8L_ERR_ALIGN, "x, qt must be 16-byte aligned");
+  if (int e = check_arch()) return e;
+  if (!zeroed) {
+    I8L_CUDA_OK(cudaMemsetAsync(colmax, 0, (size_t)cols * sizeof(float), st));
+    LaunchChain::broken();
+  }
+  if (qmode == I8L_QMODE_TRITON) return launch_col_t<I8L_QMODE_TRITON>(x, rows, cols, rot, qt, scale_t, colmax, st);
+  if (qmode == I8L_QMODE_RNE) return launch_col_t<I8L_QMODE_RNE>(x, rows, cols, rot, qt, scale_t, colmax, st);
+  if (qmode == I8L_QMODE_ROWRCP) return launch_col_t<I8L_QMODE_ROWRCP>(x, rows, cols, rot, qt, scale_t, colmax, st);
+  return fail(I8L_ERR_ARG, "%s: unsupported qmode=%d", name, qmode);
+}
+}  // namespace i8l
+
+extern "C" int i8l_quant_col_t(const void* x, int64_t rows, int64_t cols, int qmode, int8_t* qt, float* scale_t,
+                               float* colmax_scratch, void* stream) {
+  return quant_col_t("i8l_quant_col_t", x, rows, cols, qmode, false, qt, scale_t, colmax_scratch, false, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int i8l_quant_col_t_rot(const void* x, int64_t rows, int64_t cols, int qmode, int8_t* qt, float* scale_t,
                                    float* colmax_scratch, void* stream) {
-  if (int e = check_dims(1, rows, cols)) return e;
-  if (!x || !qt || !scale_t || !colmax_scratch) return fail(I8L_ERR_ARG, "null pointer");
-  if (!aligned16(x) || !aligned16(qt)) return fail(I8L_ERR_ALIGN, "x, qt must be 16-byte aligned");
-  if (int e = check_arch()) return e;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  I8L_CUDA_OK(cudaMemsetAsync(colmax_scratch, 0, (size_t)cols * sizeof(float), st));
-  if (qmode == I8L_QMODE_TRITON) return launch_col_t_rot<I8L_QMODE_TRITON>(x, rows, cols, qt, scale_t, colmax_scratch, st);
-  if (qmode == I8L_QMODE_RNE) return launch_col_t_rot<I8L_QMODE_RNE>(x, rows, cols, qt, scale_t, colmax_scratch, st);
-  if (qmode == I8L_QMODE_ROWRCP) return launch_col_t_rot<I8L_QMODE_ROWRCP>(x, rows, cols, qt, scale_t, colmax_scratch, st);
-  return fail(I8L_ERR_ARG, "i8l_quant_col_t_rot: unsupported qmode=%d", qmode);
+  return quant_col_t("i8l_quant_col_t_rot", x, rows, cols, qmode, true, qt, scale_t, colmax_scratch, false, static_cast<cudaStream_t>(stream));
 }
 
 // ------------------------------------------------------------------------------------------------
