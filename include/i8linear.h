@@ -268,8 +268,8 @@ I8L_API int i8l_linear_backward(const void* dy, const void* w, const int8_t* x_q
  * Non-blocking look at a status word (the `status` argument of the GEMMs) for hot loops.  i8l_status_open binds a
  * device int32 and a pinned host int32 (NULL on failure, see i8l_last_error; the handle lives as long as the
  * process).  i8l_status_poll returns I8L_ERR_TIMEOUT if the copy that an earlier poll started has completed and shows
- * a set word, and otherwise starts the next copy on `stream`, unless the last one is still in flight or the stream is
- * being captured.  i8l_status_reset, called after the word has been cleared, waits for a copy in flight and discards it.
+ * a set word, and otherwise starts the next copy, on a stream of its own, unless the last one is still in flight or
+ * `stream` is being captured: the word is sampled at some time after the call, and must have been initialised before it.  i8l_status_reset, called after the word has been cleared, waits for a copy in flight and discards it.
  * Safe from several host threads.  No counterpart in the reference.
  */
 I8L_API void* i8l_status_open(const int32_t* word, int32_t* host);

@@ -21,7 +21,9 @@ uint32_t gemm_wait_limit();
 int gemm_cta_budget();
 int sm_count();  // of the current device
 
-// i8l_quant_col_t (rot = false) or i8l_quant_col_t_rot; zeroed: colmax is zero already, no memset goes in front.
+// Clears n floats; in a chain the next kernel waits for it before anything else.
+int clear(float* ptr, int64_t n, cudaStream_t st);
+// i8l_quant_col_t (rot = false) or i8l_quant_col_t_rot; zeroed: colmax is zero already.
 int quant_col_t(const char* name, const void* x, int64_t rows, int64_t cols, int qmode, bool rot, int8_t* qt, float* scale_t,
                 float* colmax, bool zeroed, cudaStream_t st);
 
@@ -35,34 +37,57 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
   } while (0)
 
 // ---------------------------------------------------------------- chains of launches
-// The kernels of one composed call (compose.cu) follow one another on a stream.  The first is launched as usual and so
-// starts when all earlier work of the stream is done; the others are launched with programmatic serialization and start
-// as soon as every block of their predecessor has started and there is room: launch latency, prologues and the tails
-// of small grids overlap (2-3 us a launch).  Every kernel triggers its successor first thing.  What it may do ahead of
-// chain_wait(), which returns when the predecessor has completed and its writes are visible:
-//   quantizers  everything: they read the caller's inputs and write memory that no kernel of the chain reads or writes
-//               before them.  They wait at their end, so that "predecessor completed" covers the whole chain;
-//   passes that need a predecessor's result (scales from a column maximum) and GEMMs: nothing but their set-up.
-// Outside a chain both are no-ops.
+// The kernels of one composed call (compose.cu) follow one another on a stream and are launched with programmatic
+// serialization: each starts as soon as every block of its predecessor has triggered it (or ended) and there is room, so
+// that launch latency, prologues and the tails of small grids overlap (2-3 us a launch).  chain_wait() returns when the
+// predecessor has completed and its writes are visible.
+//   The first kernel of a chain waits before anything else and triggers its successor then: when the successor starts,
+//   whatever was in the stream before the chain is done.  (The predecessor is any kernel of the caller's.)
+//   Quantizers behind it read the caller's inputs and write memory that no kernel of the chain reads or writes before them.
+//   They trigger first thing and wait at their end, so that "predecessor completed" covers the whole chain.
+//   Passes that need a predecessor's result (scales from a column maximum) and GEMMs wait behind their set-up, and a GEMM
+//   triggers only another GEMM, the rest starts when its blocks have ended; a kernel
+//   that clears memory for a later pass and the one behind it wait like a first one.
+// Outside a chain both instructions do nothing.
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_start(int first) {
+  if (first) chain_wait();
+  chain_trigger();
+}
 
-// This host thread's chain: 0 none, 1 its first kernel is not launched yet, 2 the stream's last operation is one of its kernels.
-extern thread_local int launch_chain;
-struct LaunchChain {
-  LaunchChain() { launch_chain = 1; }
-  ~LaunchChain() { launch_chain = 0; }
-  static void broken() { if (launch_chain) launch_chain = 1; }   // an operation that is not a kernel went into the stream
+// This host thread's chain.
+struct ChainState {
+  bool active, attribute;   // a chain is being launched; its next kernel may start ahead of its predecessor's end
+  int wait;                 // it waits before anything else
+  int gemm_next;            // it is a GEMM and another one follows
 };
+extern thread_local ChainState chain_state;
+struct LaunchChain {
+  explicit LaunchChain(cudaStream_t st) {
+    // while a stream is captured, the first kernel depends on whatever precedes it in full: the graph's edges into it
+    // may come from other things than one kernel
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool plain = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    chain_state = ChainState{true, !plain, 1, 0};
+  }
+  ~LaunchChain() { chain_state = ChainState{}; }
+};
+// The argument `first` of the kernel launched next.
+inline int chain_first() {
+  const int w = chain_state.wait;
+  chain_state.wait = 0;
+  return w;
+}
 // Adds the attribute to a launch of the chain; attrs has room for one more.
 inline void chain_attribute(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs) {
-  if (launch_chain == 2) {
+  if (chain_state.attribute) {
     attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     ++cfg.numAttrs;
   }
-  if (launch_chain == 1) launch_chain = 2;
+  chain_state.attribute = chain_state.active;
 }
 template <typename... P, typename... A>
 cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {

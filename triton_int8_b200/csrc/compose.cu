@@ -79,7 +79,7 @@ extern "C" int i8l_quant_gemm(const void* a, const void* b, const void* bias, vo
   float* bs = ws.take<float>(scale_count(b_gran, b_n, N, K));
   float* colmax = a_qt && a_gran == I8L_GRAN_ROW ? ws.take<float>(K) : nullptr;
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_quant_gemm: workspace of %lld bytes is too small", (long long)workspace_bytes);
-  const LaunchChain chain;
+  const LaunchChain chain(static_cast<cudaStream_t>(stream));
   if (a_qt && a_gran != I8L_GRAN_ROW) {   // both orientations of A from one call
     if (int e = i8l_quant_tile(a, batch, M, K, a_gran, qmode, hadamard, aq, as, a_qt, a_st, stream)) return e;
   } else {
@@ -119,14 +119,14 @@ extern "C" int i8l_linear_backward(const void* dy, const void* w, const int8_t* 
   }
   float* colmax = ws.take<float>(K > N ? K : N);
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_linear_backward: workspace of %lld bytes is too small", (long long)workspace_bytes);
-  // The column maxima of W start from zeros that go in first, where no other pass needs the scratch: a memset between
-  // the kernels would break the chain.
+  const LaunchChain chain(static_cast<cudaStream_t>(stream));
+  // The column maxima of W start from zeros; cleared up front, where no other pass needs the scratch, the first maximum
+  // pass does not have to wait for it.
   const bool zeroed = dx && !whole_k;
   if (zeroed) {
     if (int e = check_arch()) return e;
-    I8L_CUDA_OK(cudaMemsetAsync(colmax, 0, (size_t)K * sizeof(float), static_cast<cudaStream_t>(stream)));
+    if (int e = clear(colmax, K, static_cast<cudaStream_t>(stream))) return e;
   }
-  const LaunchChain chain;
   if (whole_k) {
     if (dx)
       if (int e = i8l_quant_row(dy, M, N, qmode, hadamard, dyq, dys, stream)) return e;
@@ -137,6 +137,7 @@ extern "C" int i8l_linear_backward(const void* dy, const void* w, const int8_t* 
   }
   if (dx) {   // dX = dY W, contraction over N
     if (int e = quant_col_t(w, N, K, qmode, hadamard, wqt, wst, colmax, zeroed, stream)) return e;
+    chain_state.gemm_next = dw != nullptr;
     const int e = whole_k ? i8l_gemm_rowcol(dyq, wqt, dys, wst, 0, nullptr, post_dx, dx, 1, M, K, N, flags, status, stream)
                           : i8l_gemm_block(dyq, wqt, dys, wst, a_kind_of(gran), I8L_BSCALE_CHANNEL, 0, nullptr, post_dx, dx, 1, M,
                                            K, N, flags, status, stream);

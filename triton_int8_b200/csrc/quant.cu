@@ -10,7 +10,7 @@
 namespace i8l {
 
 static thread_local char g_err[512] = "";
-thread_local int launch_chain = 0;
+thread_local ChainState chain_state;
 
 int fail(int code, const char* fmt, ...) {
   va_list ap;
@@ -58,7 +58,7 @@ template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
 __global__ void __launch_bounds__(256, 4)
 quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
                   int8_t* __restrict__ q, float* __restrict__ scale, int8_t* __restrict__ qt,
-                  float* __restrict__ scale_t, const float* __restrict__ colmax) {
+                  float* __restrict__ scale_t, const float* __restrict__ colmax, int first) {
   __shared__ float s_red[8];
   __shared__ float s_colred[(GRAN == I8L_GRAN_GROUP128 && OUT_T) ? 8 * 128 : 1];
   __shared__ float s_cols[(GRAN != I8L_GRAN_TILE128 && OUT_T) ? 128 : 1];
@@ -68,7 +68,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
   const __nv_bfloat16* xb = x + boff;
-  chain_trigger();
+  chain_start(first);
 
   // The tile stays in registers as packed bf16 (32 registers per thread, 4 CTAs per SM).
   uint4 raw[2][4];
@@ -222,12 +222,12 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
 template <int MODE>
 __global__ void __launch_bounds__(256, 3)
 quant_tile256_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
-                     float* __restrict__ scale) {
+                     float* __restrict__ scale, int first) {
   __shared__ float s_red[8];
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 256;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
-  chain_trigger();
+  chain_start(first);
   uint4 raw[16];
   __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
@@ -354,13 +354,13 @@ template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
 __global__ void __launch_bounds__(128, 3)
 quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
                       float* __restrict__ scale, int8_t* __restrict__ qt, float* __restrict__ scale_t,
-                      float* __restrict__ colmax) {
+                      float* __restrict__ colmax, int first) {
   __shared__ __align__(16) uint8_t s_raw[128 * ROT_LD];
   __shared__ float s_red[2][4];
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
   const int64_t boff = (int64_t)blockIdx.z * rows * cols;
-  chain_trigger();
+  chain_start(first);
   {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
     const __nv_bfloat16* src = x + boff + (r_base + (tid >> 4)) * cols + c_base + 8 * (tid & 15);
@@ -422,11 +422,11 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
 // Column absmax of x [rows, cols] into colmax[cols] (pre-zeroed); |x| >= 0 so the float bit
 // patterns order like integers and atomicMax on int is exact.
 __global__ void __launch_bounds__(256)
-col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, float* __restrict__ colmax) {
+col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, float* __restrict__ colmax, int first) {
   __shared__ float s_colred[8 * 128];
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, cc = l & 15, half = l >> 4;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
-  chain_trigger();
+  chain_start(first);
   float m[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) m[j] = 0.f;
@@ -463,13 +463,13 @@ col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
 template <int MODE, bool HAD128>
 __global__ void __launch_bounds__(256)
 quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __restrict__ q,
-                 float* __restrict__ scale) {
+                 float* __restrict__ scale, int first) {
   __shared__ float s_red[8];
   const int tid = threadIdx.x, l = tid & 31;
   const int64_t row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int nchunks = (int)(cols / 8);
-  chain_trigger();
+  chain_start(first);
 
   float m = 0.f;
   for (int base = 0; base < nchunks; base += 256) {
@@ -530,14 +530,14 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __re
 template <int MODE, int T>
 __global__ void __launch_bounds__(256)
 quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
-                        float* __restrict__ scale) {
+                        float* __restrict__ scale, int first) {
   __shared__ float s_red[8];
   const int tid = threadIdx.x, l = tid & 31, t = tid & (T - 1);
   const int64_t row = (int64_t)blockIdx.x * (256 / T) + tid / T;
   const bool live = row < rows;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int nchunks = live ? (int)(cols / 8) : 0;
-  chain_trigger();
+  chain_start(first);
   uint4 cache[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) cache[i] = i * T + t < nchunks ? __ldg(xr + i * T + t) : make_uint4(0, 0, 0, 0);
@@ -583,13 +583,13 @@ quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64
 template <int MODE>
 __global__ void __launch_bounds__(128, 3)
 quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int groups, int rows_per_cta, int8_t* __restrict__ q,
-                     float* __restrict__ scale) {
+                     float* __restrict__ scale, int first) {
   __shared__ __align__(16) uint8_t s_raw[128 * ROT_LD];
   __shared__ int s_max[128];
   const int tid = threadIdx.x, my_row = tid / groups;
   const int64_t row0 = (int64_t)blockIdx.x * rows_per_cta;
   const int n_rows = (int)(rows - row0 < rows_per_cta ? rows - row0 : rows_per_cta), n = n_rows * groups;
-  chain_trigger();
+  chain_start(first);
   const __nv_bfloat16* src = x + row0 * groups * 128 + 8 * tid;   // whole rows are contiguous
   const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
 #pragma unroll
@@ -642,7 +642,8 @@ constexpr size_t FULL_SMEM = 128 * FULL_LD * sizeof(float);
 
 template <int MODE, int G>
 __global__ void __launch_bounds__(128, 3)
-quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8_t* __restrict__ q, float* __restrict__ scale) {
+quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8_t* __restrict__ q, float* __restrict__ scale,
+                         int first) {
   constexpr int R = 128 / G;   // rows per CTA
   extern __shared__ __align__(16) float s_f[];   // [128][FULL_LD]; the bf16 input lies in it first
   __shared__ __nv_bfloat16 s_red[R][4];
@@ -651,7 +652,7 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t row0 = (int64_t)blockIdx.x * R;
   const int n_rows = (int)(rows - row0 < R ? rows - row0 : R), n = n_rows * G;
-  chain_trigger();
+  chain_start(first);
   {
     const __nv_bfloat16* src = x + row0 * G * 128 + 8 * tid;   // whole rows are contiguous
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw) + (tid >> 4) * ROT_LD + 16 * (tid & 15);
@@ -770,14 +771,14 @@ quant_row_rotfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int8
 template <int MODE>
 __global__ void __launch_bounds__(256)
 quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __restrict__ q,
-                         float* __restrict__ scale) {
+                         float* __restrict__ scale, int first) {
   extern __shared__ float s_row[];
   __shared__ float s_red[8];
   const int tid = threadIdx.x, l = tid & 31;
   const int64_t row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int n = (int)cols, nchunks = n / 8;
-  chain_trigger();
+  chain_start(first);
 
   for (int base = 0; base < nchunks; base += 256) {
     const int ch = base + tid;
@@ -850,7 +851,7 @@ static int launch_rotfull(const __nv_bfloat16* x, int64_t rows, int8_t* q, float
   static std::atomic<bool> attr_done[MAX_DEVICES];
   I8L_CUDA_OK(ensure_smem(quant_row_rotfull_kernel<MODE, G>, attr_done, FULL_SMEM));
   constexpr int R = 128 / G;
-  I8L_CUDA_OK(launch(quant_row_rotfull_kernel<MODE, G>, dim3((unsigned)((rows + R - 1) / R)), 128, FULL_SMEM, st, x, rows, q, scale));
+  I8L_CUDA_OK(launch(quant_row_rotfull_kernel<MODE, G>, dim3((unsigned)((rows + R - 1) / R)), 128, FULL_SMEM, st, x, rows, q, scale, chain_first()));
   return I8L_OK;
 }
 template <int MODE>
@@ -871,7 +872,7 @@ static int launch_hadfull(const __nv_bfloat16* x, int64_t rows, int64_t cols, in
   static std::atomic<bool> attr_done[MAX_DEVICES];
   const size_t smem = (size_t)cols * sizeof(float);
   I8L_CUDA_OK(ensure_smem(quant_row_hadfull_kernel<MODE>, attr_done, 32768 * sizeof(float)));
-  I8L_CUDA_OK(launch(quant_row_hadfull_kernel<MODE>, dim3((unsigned)rows), 256, smem, st, x, cols, q, scale));
+  I8L_CUDA_OK(launch(quant_row_hadfull_kernel<MODE>, dim3((unsigned)rows), 256, smem, st, x, cols, q, scale, chain_first()));
   return I8L_OK;
 }
 
@@ -889,7 +890,7 @@ static cudaError_t launch_tile(const void* x, int64_t batch, int64_t rows, int64
                         int8_t* qt, float* scale_t, const float* colmax, cudaStream_t st) {
   dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
   return launch(quant_tile_kernel<GRAN, MODE, OUT_N, OUT_T>, grid, 256, 0, st, static_cast<const __nv_bfloat16*>(x), rows, cols, q,
-                scale, qt, scale_t, colmax);
+                scale, qt, scale_t, colmax, chain_first());
 }
 
 template <int GRAN, int MODE>
@@ -899,9 +900,9 @@ static int dispatch_tile(const void* x, int64_t batch, int64_t rows, int64_t col
   if (had) {  // whatever is wanted of the two orientations, from one read of the tile
     const dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), (unsigned)batch);
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-    if (n && t) I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, true, true>, grid, 128, 0, st, xp, rows, cols, q, scale, qt, scale_t, nullptr));
-    else if (n) I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, true, false>, grid, 128, 0, st, xp, rows, cols, q, scale, nullptr, nullptr, nullptr));
-    else I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr, qt, scale_t, nullptr));
+    if (n && t) I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, true, true>, grid, 128, 0, st, xp, rows, cols, q, scale, qt, scale_t, nullptr, chain_first()));
+    else if (n) I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, true, false>, grid, 128, 0, st, xp, rows, cols, q, scale, nullptr, nullptr, nullptr, chain_first()));
+    else I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr, qt, scale_t, nullptr, chain_first()));
   } else if (GRAN == I8L_GRAN_TILE128) {
     if (n && t) I8L_CUDA_OK((launch_tile<GRAN, MODE, true, true>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st)));
     else if (n) I8L_CUDA_OK((launch_tile<GRAN, MODE, true, false>(x, batch, rows, cols, q, scale, qt, scale_t, colmax, st)));
@@ -934,8 +935,8 @@ extern "C" int i8l_quant_tile(const void* x, int64_t batch, int64_t rows, int64_
     if (cols % 256 || had || qt || !q) return fail(I8L_ERR_ARG, "i8l_quant_tile: 128x256 groups need cols %% 256 == 0, no rotation, q only");
     const dim3 grid((unsigned)(cols / 256), (unsigned)(rows / 128), (unsigned)batch);
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-    if (qmode == I8L_QMODE_TRITON) I8L_CUDA_OK(launch(quant_tile256_kernel<I8L_QMODE_TRITON>, grid, 256, 0, st, xp, rows, cols, q, scale));
-    else if (qmode == I8L_QMODE_TRITON_BF16S) I8L_CUDA_OK(launch(quant_tile256_kernel<I8L_QMODE_TRITON_BF16S>, grid, 256, 0, st, xp, rows, cols, q, scale));
+    if (qmode == I8L_QMODE_TRITON) I8L_CUDA_OK(launch(quant_tile256_kernel<I8L_QMODE_TRITON>, grid, 256, 0, st, xp, rows, cols, q, scale, chain_first()));
+    else if (qmode == I8L_QMODE_TRITON_BF16S) I8L_CUDA_OK(launch(quant_tile256_kernel<I8L_QMODE_TRITON_BF16S>, grid, 256, 0, st, xp, rows, cols, q, scale, chain_first()));
     else return fail(I8L_ERR_ARG, "i8l_quant_tile: 128x256 groups support qmode TRITON and TRITON_BF16S");
     return I8L_OK;
   }
@@ -979,18 +980,18 @@ extern "C" int i8l_quant_row(const void* x, int64_t rows, int64_t cols, int qmod
   // it in eight pieces each.
   const int groups = (int)(cols / 128), rpc = 128 / groups;
 #define I8L_ROW_T(Mo, T) \
-  launch(quant_row_cached_kernel<Mo, T>, dim3((unsigned)((rows + 256 / T - 1) / (256 / T))), 256, 0, st, xp, rows, cols, q, scale)
+  launch(quant_row_cached_kernel<Mo, T>, dim3((unsigned)((rows + 256 / T - 1) / (256 / T))), 256, 0, st, xp, rows, cols, q, scale, chain_first())
 #define I8L_ROW_CASE(Mo)                                                                                      \
   if (qmode == Mo) {                                                                                          \
     I8L_CUDA_OK(                                                                                              \
         hadamard && rpc ? launch(quant_row_rot_kernel<Mo>, dim3((unsigned)((rows + rpc - 1) / rpc)), 128, 0, st, xp, rows, groups, \
-                                 rpc, q, scale)                                                               \
-        : hadamard      ? launch(quant_row_kernel<Mo, true>, dim3((unsigned)rows), 256, 0, st, xp, cols, q, scale) \
+                                 rpc, q, scale, chain_first())                                                \
+        : hadamard      ? launch(quant_row_kernel<Mo, true>, dim3((unsigned)rows), 256, 0, st, xp, cols, q, scale, chain_first()) \
         : cols <= 2048  ? I8L_ROW_T(Mo, 32)                                                                   \
         : cols <= 4096  ? I8L_ROW_T(Mo, 64)                                                                   \
         : cols <= 8192  ? I8L_ROW_T(Mo, 128)                                                                  \
         : cols <= 16384 ? I8L_ROW_T(Mo, 256)                                                                  \
-                        : launch(quant_row_kernel<Mo, false>, dim3((unsigned)rows), 256, 0, st, xp, cols, q, scale)); \
+                        : launch(quant_row_kernel<Mo, false>, dim3((unsigned)rows), 256, 0, st, xp, cols, q, scale, chain_first())); \
     return I8L_OK;                                                                                            \
   }
   I8L_ROW_CASE(I8L_QMODE_TRITON)
@@ -1002,6 +1003,12 @@ extern "C" int i8l_quant_row(const void* x, int64_t rows, int64_t cols, int qmod
   return fail(I8L_ERR_ARG, "i8l_quant_row: unsupported qmode=%d", qmode);
 }
 
+__global__ void __launch_bounds__(1024) clear_kernel(float* __restrict__ ptr, int64_t n) {
+  chain_start(1);   // a kernel ahead of it may still read what it clears
+  const int64_t i = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+  if (i < n) ptr[i] = 0.f;
+}
+
 // Both passes of one scale per column; colmax is zero.
 template <int MODE>
 static int launch_col_t(const void* x, int64_t rows, int64_t cols, bool rot, int8_t* qt, float* scale_t, float* colmax,
@@ -1010,27 +1017,30 @@ static int launch_col_t(const void* x, int64_t rows, int64_t cols, bool rot, int
   const dim3 grid((unsigned)(cols / 128), (unsigned)(rows / 128), 1);
   if (rot) {
     I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN_COLMAX_PASS, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr,
-                       nullptr, nullptr, colmax));
+                       nullptr, nullptr, colmax, chain_first()));
     I8L_CUDA_OK(launch(quant_tile_rot_kernel<GRAN_COLFULL, MODE, false, true>, grid, 128, 0, st, xp, rows, cols, nullptr, nullptr, qt,
-                       scale_t, colmax));
+                       scale_t, colmax, chain_first()));
   } else {
-    I8L_CUDA_OK(launch(col_absmax_kernel, grid, 256, 0, st, xp, rows, cols, colmax));
+    I8L_CUDA_OK(launch(col_absmax_kernel, grid, 256, 0, st, xp, rows, cols, colmax, chain_first()));
     I8L_CUDA_OK((launch_tile<GRAN_COLFULL, MODE, false, true>(x, 1, rows, cols, nullptr, nullptr, qt, scale_t, colmax, st)));
   }
   return I8L_OK;
 }
 
 namespace i8l {
+int clear(float* ptr, int64_t n, cudaStream_t st) {   // a kernel and not a memset, which would break the chain
+  I8L_CUDA_OK(launch(clear_kernel, dim3((unsigned)((n + 1023) / 1024)), 1024, 0, st, ptr, n));
+  chain_state.wait = 1;
+  return I8L_OK;
+}
 int quant_col_t(const char* name, const void* x, int64_t rows, int64_t cols, int qmode, bool rot, int8_t* qt, float* scale_t,
                 float* colmax, bool zeroed, cudaStream_t st) {
   if (int e = check_dims(1, rows, cols)) return e;
   if (!x || !qt || !scale_t || !colmax) return fail(I8L_ERR_ARG, "null pointer");
   if (!aligned16(x) || !aligned16(qt)) return fail(I8L_ERR_ALIGN, "x, qt must be 16-byte aligned");
   if (int e = check_arch()) return e;
-  if (!zeroed) {
-    I8L_CUDA_OK(cudaMemsetAsync(colmax, 0, (size_t)cols * sizeof(float), st));
-    LaunchChain::broken();
-  }
+  if (!zeroed)
+    if (int e = clear(colmax, cols, st)) return e;
   if (qmode == I8L_QMODE_TRITON) return launch_col_t<I8L_QMODE_TRITON>(x, rows, cols, rot, qt, scale_t, colmax, st);
   if (qmode == I8L_QMODE_RNE) return launch_col_t<I8L_QMODE_RNE>(x, rows, cols, rot, qt, scale_t, colmax, st);
   if (qmode == I8L_QMODE_ROWRCP) return launch_col_t<I8L_QMODE_ROWRCP>(x, rows, cols, rot, qt, scale_t, colmax, st);

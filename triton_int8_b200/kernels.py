@@ -43,6 +43,8 @@ class _StatusWord:
         self.dev = dev
         self.word = torch.zeros(1, dtype=torch.int32, device=dev)
         self.host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        if not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(dev).synchronize()   # polls copy the word on a stream of their own
         with torch.cuda.device(dev):
             self.poller = L.load().i8l_status_open(self.word.data_ptr(), self.host.data_ptr())
         if not self.poller:
