@@ -277,6 +277,14 @@ I8L_API int i8l_status_poll(void* poller, void* stream);
 I8L_API int i8l_status_reset(void* poller);
 
 /*
+ * The same without any copy: i8l_status_mirror binds a second pinned host int32, zero, to the poller's status word, and a
+ * GEMM that reports into that word writes there as well.  i8l_status_peek reads it: I8L_ERR_TIMEOUT or 0 (also without a
+ * mirror).  i8l_status_reset clears it.  No counterpart in the reference.
+ */
+I8L_API int i8l_status_mirror(void* poller, int32_t* pinned);
+I8L_API int i8l_status_peek(void* poller);
+
+/*
  * The GEMMs are persistent kernels with one CTA per SM (about 210 KB of shared memory each), so a kernel
  * launched beside one on another stream finds no free SM until the GEMM ends.  This sets, for the calling
  * host thread, the number of CTAs the following GEMM launches may use (0 = all SMs, the default): a

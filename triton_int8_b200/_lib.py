@@ -41,6 +41,8 @@ SIGNATURES = {
     "i8l_status_open": [_P, _P],
     "i8l_status_poll": [_P, _P],
     "i8l_status_reset": [_P],
+    "i8l_status_mirror": [_P, _P],
+    "i8l_status_peek": [_P],
     "i8l_set_cta_limit": [_I],
     "i8l_test_set_wait_limit": [ctypes.c_uint32, _I],
     "i8l_version": [],
@@ -76,6 +78,11 @@ def load() -> ctypes.CDLL:
         _lib = lib
         _fns.update((name, getattr(lib, name)) for name in SIGNATURES)
     return _lib
+
+
+def address(name: str) -> int:
+    """Address of an entry point, for native callers."""
+    return ctypes.cast(getattr(load(), name), _P).value
 
 
 def call(name: str, *args) -> None:

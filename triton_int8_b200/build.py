@@ -1,4 +1,5 @@
-"""Build libi8linear.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Build the native parts in-tree: libi8linear.so (CUDA, with nvcc for sm_100a, which cross-compiles without a GPU) and
+_host.so (the host path of the composed calls, a torch extension module, with g++).
 
     python -m triton_int8_b200.build [--force]
 """
@@ -12,9 +13,11 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libi8linear.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 SOURCES = ["quant.cu", "gemm.cu", "fused.cu", "compose.cu"]
-HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "ptx.cuh"),
-           os.path.join(os.path.dirname(PKG_DIR), "include", "i8linear.h")]
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
+ABI_HEADER = os.path.join(os.path.dirname(PKG_DIR), "include", "i8linear.h")
+HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "ptx.cuh"), ABI_HEADER]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--shared", "-cudart", "static",
@@ -28,26 +31,51 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or add it to PATH")
 
 
-def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _stale(target: str, deps) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, s) for s in SOURCES] + HEADERS
+    t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def needs_build() -> bool:
+    return _stale(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS)
+
+
+def needs_host_build() -> bool:
+    return _stale(HOST_PATH, [HOST_SOURCE, ABI_HEADER])
+
+
+def _host_command() -> list:
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), cuda,
+               sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in include),
+            "-o", HOST_PATH, HOST_SOURCE, f"-L{os.path.join(root, 'lib')}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
+            "-lc10_cuda"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB_PATH
-    cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB_PATH] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-        print(" ".join(cmd))
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+    jobs = []
+    if force or needs_build():
+        cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB_PATH] + [os.path.join(CSRC, s) for s in SOURCES]
+        if verbose:
+            cmd.insert(1, "-Xptxas=-v")
+        jobs.append(cmd)
+    if force or needs_host_build():
+        jobs.append(_host_command())
+    running = [(cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)) for cmd in jobs]
+    for cmd, proc in running:
+        out = proc.communicate()[0]
+        if verbose:
+            print(" ".join(cmd) + "\n" + out)
+        if proc.returncode != 0:
+            raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n{out}")
     return LIB_PATH
 
 

@@ -20,6 +20,7 @@ int check_arch();
 uint32_t gemm_wait_limit();
 int gemm_cta_budget();
 int sm_count();  // of the current device
+int32_t* mirror_of(const int32_t* status_word);   // see i8l_status_mirror; null without one
 
 // Clears n floats; in a chain the next kernel waits for it before anything else.
 int clear(float* ptr, int64_t n, cudaStream_t st);

@@ -50,6 +50,7 @@ constexpr float MAGIC_F = 12582912.f;
 struct Params {
   void* c;
   int32_t* status;
+  int32_t* mirror;   // pinned host memory that follows the status word, or null
   int64_t K;
   int m_blocks, mpb, n_tiles, N, KB;
   int b_batched, per_row_b, exact, out_f32;
@@ -345,7 +346,10 @@ fused_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && ctl.abort_flag && p.status) atomicExch(p.status, I8L_ERR_TIMEOUT);
+  if (threadIdx.x == 0 && ctl.abort_flag && p.status) {
+    atomicExch(p.status, I8L_ERR_TIMEOUT);
+    if (p.mirror) *static_cast<volatile int32_t*>(p.mirror) = I8L_ERR_TIMEOUT;
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -374,6 +378,7 @@ extern "C" int i8l_fused_gemm(const void* a_bf, const void* b_bf, void* c, int64
   if (int e = make_tile_map_bf16(&map_b, b_bf, b_batched ? batch * N : N, K)) return e;
   p.c = c;
   p.status = status;
+  p.mirror = status ? mirror_of(status) : nullptr;
   p.K = K;
   p.m_blocks = (int)(batch * M / 128);
   p.mpb = (int)(M / 128);

@@ -66,6 +66,7 @@ struct GemmParams {
   const __nv_bfloat16* bias;
   void* c;
   int32_t* status;
+  int32_t* mirror;   // pinned host memory that follows the status word (i8l_status_mirror), or null
   int m_blocks;  // batch*M/128
   int mpb;       // M/128 (m-blocks per batch)
   int n_tiles;   // ceil(N/256)
@@ -942,7 +943,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (TWO) cluster_sync_all();  // no remote arrival or tensor-memory write of the pair is still pending
-  if (threadIdx.x == 0 && ctl.abort_flag && p.status) atomicExch(p.status, I8L_ERR_TIMEOUT);
+  if (threadIdx.x == 0 && ctl.abort_flag && p.status) {
+    atomicExch(p.status, I8L_ERR_TIMEOUT);
+    if (p.mirror) *static_cast<volatile int32_t*>(p.mirror) = I8L_ERR_TIMEOUT;
+  }
   if (warp == 1) {
     tc_fence_after();
     if (TWO) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -1076,6 +1080,22 @@ int gemm_cta_budget() {
   return (g_cta_limit > 0 && g_cta_limit < sms) ? g_cta_limit : sms;
 }
 
+// Status words with a mirror: a few per process, written when a poller is set up and read by every launch.
+struct Mirror {
+  std::atomic<const int32_t*> word{nullptr};
+  int32_t* device_ptr = nullptr;
+};
+static Mirror g_mirrors[MAX_DEVICES];
+static std::mutex g_mirror_lock;
+int32_t* mirror_of(const int32_t* word) {
+  for (const Mirror& m : g_mirrors) {
+    const int32_t* w = m.word.load(std::memory_order_acquire);
+    if (!w) return nullptr;
+    if (w == word) return m.device_ptr;
+  }
+  return nullptr;
+}
+
 template <int KIND, bool TWO>
 static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p, int64_t tiles, cudaStream_t st) {
   // per-device set-up, done by whichever thread comes first (idempotent, so a race only repeats it)
@@ -1149,6 +1169,7 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   p.N = (int)N;
   p.KB = (int)(K / 128);
   {
+    p.mirror = p.status ? mirror_of(p.status) : nullptr;
     p.max_polls = gemm_wait_limit();
     p.withhold = g_test_withhold.load(std::memory_order_relaxed);
   }
@@ -1276,6 +1297,7 @@ extern "C" int i8l_sum_slots(const void* slots, void* out, int world, int64_t ro
 struct StatusPoller {
   const int32_t* word;
   volatile int32_t* host;
+  volatile int32_t* mirror;   // or null
   cudaStream_t side;
   cudaEvent_t event;
   bool pending;
@@ -1288,6 +1310,7 @@ extern "C" void* i8l_status_open(const int32_t* word, int32_t* host) {
   if (!s) { fail(I8L_ERR_CUDA, "out of host memory"); return nullptr; }
   s->word = word;
   s->host = host;
+  s->mirror = nullptr;
   s->pending = false;
   cudaError_t e = cudaEventCreateWithFlags(&s->event, cudaEventDisableTiming);
   s->side = nullptr;
@@ -1334,6 +1357,31 @@ extern "C" int i8l_status_reset(void* poller) {
   if (s->pending) I8L_CUDA_OK(cudaEventSynchronize(s->event));
   s->pending = false;
   *s->host = 0;
+  if (s->mirror) *s->mirror = 0;
+  return I8L_OK;
+}
+
+extern "C" int i8l_status_mirror(void* poller, int32_t* pinned) {
+  if (!poller || !pinned) return fail(I8L_ERR_ARG, "null pointer");
+  StatusPoller* s = static_cast<StatusPoller*>(poller);
+  void* dev = nullptr;
+  I8L_CUDA_OK(cudaHostGetDevicePointer(&dev, pinned, 0));
+  const std::lock_guard<std::mutex> hold(g_mirror_lock);
+  for (Mirror& m : g_mirrors) {
+    const int32_t* w = m.word.load(std::memory_order_relaxed);
+    if (w == s->word) return fail(I8L_ERR_ARG, "the status word has a mirror");
+    if (w) continue;
+    m.device_ptr = static_cast<int32_t*>(dev);
+    s->mirror = pinned;
+    m.word.store(s->word, std::memory_order_release);
+    return I8L_OK;
+  }
+  return fail(I8L_ERR_ARG, "too many mirrored status words");
+}
+
+extern "C" int i8l_status_peek(void* poller) {
+  const StatusPoller* s = static_cast<const StatusPoller*>(poller);
+  if (s && s->mirror && *s->mirror) return fail(I8L_ERR_TIMEOUT, "a bounded device-side wait gave up");
   return I8L_OK;
 }
 

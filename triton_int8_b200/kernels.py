@@ -47,8 +47,10 @@ class _StatusWord:
             torch.cuda.current_stream(dev).synchronize()   # polls copy the word on a stream of their own
         with torch.cuda.device(dev):
             self.poller = L.load().i8l_status_open(self.word.data_ptr(), self.host.data_ptr())
-        if not self.poller:
-            raise L.I8LError(-4, "i8l_status_open failed")
+            if not self.poller:
+                raise L.I8LError(-4, "i8l_status_open failed")
+            self.mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
+            L.call("i8l_status_mirror", self.poller, self.mirror.data_ptr())
 
 
 def _status_of(dev: torch.device) -> "_StatusWord":
@@ -94,6 +96,46 @@ def poll_status(dev) -> None:
         if rc == L.TIMEOUT:
             _raise_if_set(st, rc)
         raise L.I8LError(rc, L.load().i8l_last_error().decode())
+
+
+# ---------------------------------------------------------------------------------------- native host path
+# _host.so (csrc/host.cpp) runs the composed calls on plain tensors without the interpreter in between and returns None for
+# anything else, which the Python code below then takes.
+_host = None
+
+
+def _on_error(name: str, code: int, index: int) -> None:
+    dev = torch.device("cuda", index)
+    if name == "i8l_status_peek":
+        _raise_if_set(_status_of(dev), code)
+    raise L.I8LError(code, L.load().i8l_last_error().decode())
+
+
+def _open_status(index: int):
+    st = _status_of(torch.device("cuda", index))
+    return st.word.data_ptr(), st.poller
+
+
+def _backward_in_python(dy, w, xqt, xst, gran, qmode, hadamard, flags, whole_k, need_dx, need_dw):
+    post = [1.0 / hadamard if hadamard else 1.0] * 2
+    return linear_backward(dy, w, (xqt, xst), L.GRAN_ROW if whole_k else gran, L.QMODE_ROWRCP if whole_k else qmode, hadamard,
+                           *post, 0 if whole_k else flags, bool(need_dx), bool(need_dw))
+
+
+def host():
+    """The native module, bound to the loaded library."""
+    global _host
+    if _host is None:
+        L.load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise ImportError(f"triton_int8_b200/_host.so is missing or does not fit this torch: build it with "
+                              f"`python -m triton_int8_b200.build` ({e})") from e
+        mod.setup(L.address("i8l_quant_gemm"), L.address("i8l_linear_backward"), L.address("i8l_status_peek"), _on_error,
+                  _open_status, _backward_in_python)
+        _host = mod
+    return _host
 
 
 def _check_bf16(x: torch.Tensor, name: str) -> torch.Tensor:
@@ -240,6 +282,9 @@ def quant_gemm(a, b, a_gran, b_gran, qmode, hadamard=0, bias=None, post_scale=1.
     """bf16 a [B, M, K] x bf16 b [N, K] or [B, N, K] -> ([B, M, N], at): both quantizations and the GEMM in one call
     of the library, the int8 operands in one workspace.  want_at (B = 1): at = (int8 a^T [1, K, M], its scales along M)
     for linear_backward, else (None, None)."""
+    done = host().quant_gemm(a, b, a_gran, b_gran, qmode, hadamard, bias, post_scale, flags, want_at)
+    if done is not None:
+        return done
     a, b = _check_bf16(a, "a"), _check_bf16(b, "b")
     B, M, K = a.shape
     bb = b.dim() == 3

@@ -13,6 +13,7 @@ by a column-scaled transposing kernel, so no bf16 transpose is ever materialised
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import cached_property
 
 import torch
 from torch import nn
@@ -65,6 +66,11 @@ class Int8Config:
     @property
     def whole_k(self) -> bool:
         return self.scaling == "double_channel"
+
+    @cached_property
+    def native(self) -> tuple:
+        """The arguments that stand for this configuration in the native host path."""
+        return self.gran, self.qmode, self.hadamard, self.flags, self.whole_k
 
     def post_for(self, contraction: int) -> float:
         """Rescale that undoes the rotation of both operands: 1/128, or 1/length for a whole-axis rotation."""
@@ -199,6 +205,10 @@ class Int8Linear(nn.Module):
         return m
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if not torch.compiler.is_compiling():   # plain tensors: the same calls and autograd node without the interpreter
+            y = K.host().linear(x, self.weight, self.bias, *self.config.native)
+            if y is not None:
+                return y
         return Int8LinearFn.apply(x, self.weight, self.bias, self.config, torch.is_grad_enabled())
 
     def extra_repr(self) -> str:
