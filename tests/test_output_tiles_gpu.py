@@ -24,6 +24,7 @@ KINDS = {"rowcol": None, "fast": (0, 0, 0), "fast_tile": (0, 1, 0), "row_channel
     (3, 384, 640, 384, True),       # batches, an odd number of row blocks
     (1, 4992, 1664, 640, False),    # 39 x 7 tiles: a second and a third tile per CTA
     (1, 10240, 1152, 256, False),   # 40 x 5 pair tiles, 80 x 5 single ones
+    (1, 12544, 384, 384, True),     # narrow tiles, 98 x 3: a second one on most CTAs
 ])
 def test_bf16_output_is_the_fp32_output_rounded(kind, B, M, N, Kd, bias):
     g = torch.Generator().manual_seed(M + N)
@@ -54,3 +55,27 @@ def test_bf16_output_is_the_fp32_output_rounded(kind, B, M, N, Kd, bias):
         assert torch.equal(got, f32.to(torch.bfloat16))
         assert (buf[:GUARD + shift] == 7).all() and (buf[GUARD + shift + B * M * N:] == 7).all()
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("kind", [k for k in KINDS if k not in ("rowcol", "exact")] + ["rowcol"])
+@pytest.mark.parametrize("B,M,N,Kd", [(1, 128, 128, 128), (2, 128, 384, 1152), (1, 256, 256, 24960)])   # 195 K blocks: a second chunk of factors
+def test_narrow_tiles_equal_wide_ones(kind, B, M, N, Kd):
+    """Few tiles are 128 columns wide; on a single CTA (cta_limit) the same product takes wide ones.  Same bits."""
+    g = torch.Generator().manual_seed(N + Kd)
+    a = torch.randint(-127, 128, (B, M, Kd), generator=g, dtype=torch.int8).to(DEV)
+    b = torch.randint(-127, 128, (N, Kd), generator=g, dtype=torch.int8).to(DEV)
+    kb = Kd // 128
+    if kind == "rowcol":
+        a_s, b_s = torch.rand(B, M, generator=g).to(DEV), torch.rand(N, generator=g).to(DEV)
+        call = lambda: K.gemm_rowcol(a, b, a_s, b_s)
+    else:
+        ak, bk, fl = KINDS[kind]
+        a_s = (torch.rand(B, M // 128 if ak == 0 else M, kb, generator=g) * 0.1 + 0.01).to(DEV)
+        b_s = (torch.rand({0: (N,), 1: (N // 128, kb), 2: (N, kb)}[bk], generator=g) * 0.1 + 0.01).to(DEV)
+        call = lambda: K.gemm_block(a, b, a_s, b_s, ak, bk, None, 0.25, fl)
+    narrow = call()
+    with K.cta_limit(1):
+        wide = call()
+    torch.cuda.synchronize()
+    assert torch.equal(narrow, wide)
+    K.check_status(DEV)

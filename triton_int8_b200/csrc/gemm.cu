@@ -1,7 +1,7 @@
 // INT8 GEMMs on the 5th-generation tensor cores: tcgen05.mma kind::i8 with int32 accumulators in
 // tensor memory, operands staged by TMA into a 128B-swizzled shared-memory ring.
 //
-// One persistent CTA per SM, 384 threads (the five shifted block-scaled kinds) or 640 (row x column, generic):
+// One persistent CTA per SM, 384 threads (the five shifted block-scaled kinds, narrow tiles) or 640 (row x column, generic):
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      tensor-memory allocator + MMA issuer (one elected lane, see elect_one)
 //   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the per-K-block
@@ -13,7 +13,7 @@
 //               it).  The shifted kinds have one or two packed FMAs per two elements left and want long runs
 //               of tensor-memory loads instead: eight warps with 128 columns each and up to 208 registers, 32
 //               columns in flight per wait (fast kind, 8192^3: 16 warps 508 us, 8 warps 501, 8 warps and 32 columns 489).
-// Tensor memory holds two 128x256 int32 accumulators (all 512 columns).  In block-scaled mode the
+// Tensor memory holds two 128x256 int32 accumulators (all 512 columns), or four of the narrow tiles' 128x128.  In block-scaled mode the
 // MMA warp alternates between them every 128-wide K block while the epilogue drains the other one
 // into fp32 registers (acc += float(P) * scale; in the shifted kinds a fifth MMA per K block moves P into the
 // non-negative range, where its bits ARE a float, and the shift is taken out again); in
@@ -39,26 +39,27 @@
 
 namespace i8l {
 
-constexpr int BM = 128, BN = 256, BK = 128;
+constexpr int BM = 128, BK = 128;
+constexpr int WIDE = 256, NARROW = 128;   // columns of a tile (BN below), see narrow_tiles
 constexpr int A_STAGE = BM * BK;  // bytes
-// One CTA per tile: 128x256 tile, 3 stages of 16 KB (A) + 32 KB (B).
+// One CTA per tile: 128x256 tile, 3 stages of 16 KB (A) + 32 KB (B), or 128x128, 5 stages of 16 + 16 KB.
 // CTA pair per tile (cta_group::2): 256x256 tile, each CTA stages its own 128 rows of A and 128 of the
 // 256 rows of B (16 KB + 16 KB), 5 stages: half the B traffic through each SM's shared memory.
 // One stage less than fits leaves the 64 KB that a bf16 output tile is staged in (store_tile).
-template <bool TWO> struct Cfg {
-  static constexpr int STAGES = TWO ? 5 : 3;
+template <bool TWO, int BN> struct Cfg {
+  static constexpr int STAGES = TWO || BN == NARROW ? 5 : 3;
   static constexpr int B_STAGE = TWO ? BM * BK : BN * BK;
   static constexpr uint32_t STAGE_TX = TWO ? 2u * (A_STAGE + BM * BK) : (uint32_t)(A_STAGE + BN * BK);
+  static constexpr int OUT_STAGE = BM * BN * 2;   // the bf16 output tile
+  static constexpr int SMEM_DYN = STAGES * (A_STAGE + B_STAGE) + OUT_STAGE + 1024;
 };
 constexpr int MAX_STAGES = 5;
 constexpr int MAX_EPI_WARPS = 16;             // groups of four warps share the 256 accumulator columns
 // the kinds whose partial products are shifted by an extra MMA (K_BLOCK_FAST and the row and column factor kinds)
 template <int KIND> constexpr bool SHIFTED_OF = KIND >= 2;
-template <int KIND> constexpr int EPI_WARPS_OF = SHIFTED_OF<KIND> ? 8 : MAX_EPI_WARPS;
+template <int KIND, int BN> constexpr int EPI_WARPS_OF = SHIFTED_OF<KIND> || BN == NARROW ? 8 : MAX_EPI_WARPS;
 constexpr int FAC_MAX = 192;                  // K blocks whose factors are staged in shared memory at a time (a multiple of 4)
 constexpr int TMEM_COLS = 512;
-constexpr int OUT_STAGE = BM * BN * 2;        // the bf16 output tile
-template <bool TWO> constexpr int SMEM_DYN = Cfg<TWO>::STAGES * (A_STAGE + Cfg<TWO>::B_STAGE) + OUT_STAGE + 1024;
 
 struct GemmParams {
   const float* a_scale;
@@ -88,14 +89,11 @@ struct GemmParams {
   int withhold;        // test hook: the producer leaves out the last operand load of its first tile
 };
 
-// Instruction descriptor: D=s32, A=B=s8, both K-major, M=128, N=256, dense, no saturation.
-constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                              ((uint32_t)(BM >> 4) << 24);
-// Same with both operands unsigned: the MMA that shifts a partial product (the shifted kinds).
-constexpr uint32_t IDESC_U8 = (2u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-// Same with M=256 for the CTA-pair instruction (128 rows per CTA).
-constexpr uint32_t IDESC_I8_PAIR = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                   ((uint32_t)((2 * BM) >> 4) << 24);
+// Instruction descriptor: D=s32, A and B s8 or (the MMA that shifts a partial product) u8, both K-major, dense, no
+// saturation.  m: 128, or 256 for the CTA-pair instruction (128 rows per CTA).
+__host__ __device__ constexpr uint32_t idesc(bool s8, int m, int n) {
+  return (2u << 4) | (s8 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
 
 struct TileCoord {
   int m_blk, n_tile;
@@ -120,8 +118,8 @@ constexpr int K_BLOCK_ROWFAC = 4;  // block-scaled, per-(row, K block) A scale x
 constexpr int K_BLOCK_TILEDIV = 6; // block-scaled, per-tile scales on both sides as divisors (fused backward)
 constexpr int K_BLOCK_OUTER = 5;   // block-scaled, per-(row, K block) A scale x per-(column, K block) B scale
 
-template <int KIND> struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
-  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[2], tempty[2], done;
+template <int KIND, int BN> struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[TMEM_COLS / BN], tempty[TMEM_COLS / BN], done;
   // fast block kind: factors written (factor warp), what the tile end needs written, all consumed (every epilogue thread)
   uint64_t fready[2], eready[2], ffree[2];
   uint32_t tmem_base;
@@ -249,16 +247,17 @@ __device__ __forceinline__ float ld_scale(const float* ptr) {
   return v;
 }
 
-template <int KIND, bool TWO>
-__global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND>, 1)
+template <int KIND, bool TWO, int BN>
+__global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND, BN>, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   constexpr bool BLOCK = KIND != K_ROWCOL, SHIFTED = SHIFTED_OF<KIND>;
-  constexpr int EPI_WARPS = EPI_WARPS_OF<KIND>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
-  constexpr int STAGES = Cfg<TWO>::STAGES, B_STAGE = Cfg<TWO>::B_STAGE;
-  constexpr uint32_t STAGE_TX = Cfg<TWO>::STAGE_TX;
+  constexpr int EPI_WARPS = EPI_WARPS_OF<KIND, BN>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
+  constexpr int STAGES = Cfg<TWO, BN>::STAGES, B_STAGE = Cfg<TWO, BN>::B_STAGE, OUT_STAGE = Cfg<TWO, BN>::OUT_STAGE;
+  constexpr uint32_t STAGE_TX = Cfg<TWO, BN>::STAGE_TX;
+  constexpr int BUFS = TMEM_COLS / BN;   // accumulators
   extern __shared__ uint8_t smem_raw[];
-  __shared__ SharedCtl<KIND> ctl;
+  __shared__ SharedCtl<KIND, BN> ctl;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a = smem_base, smem_b = smem_base + STAGES * A_STAGE;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -284,7 +283,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(smem_u32(&ctl.full[s]), 1);
       mbar_init(smem_u32(&ctl.empty[s]), 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < BUFS; ++b) {
       mbar_init(smem_u32(&ctl.tfull[b]), 1);
       // arrivals that free an accumulator buffer: one per epilogue warp (of both CTAs of a pair); the shifted
       // kinds let every epilogue thread arrive for itself (no warp sync, no branch in their loop)
@@ -401,7 +400,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (SHIFTED) {   // D = SHIFT (see the epilogue) needs the buffer only: it goes out ahead of the operands' wait
             if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.tempty[ab]), aph ^ 1u, abort_flag, p.max_polls))) break;
             tc_fence_after();
-            if (elected) tc_mma_i8(tmem_base + ab * BN, ones_desc, ones_desc, IDESC_U8, 0u);
+            if (elected) tc_mma_i8(tmem_base + ab * BN, ones_desc, ones_desc, idesc(false, BM, BN), 0u);
           }
           if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.full[s]), ph, abort_flag, p.max_polls))) break;
           if (BLOCK && !SHIFTED) {
@@ -413,8 +412,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint32_t d = tmem_base + ab * BN;
 #pragma unroll
             for (int k4 = 0; k4 < BK / 32; ++k4) {
-              if (TWO) tc_mma_i8_pair(d, da + 2 * k4, db + 2 * k4, IDESC_I8_PAIR, (k4 > 0 || !drain_start) ? 1u : 0u);
-              else tc_mma_i8(d, da + 2 * k4, db + 2 * k4, IDESC_I8, (SHIFTED || k4 > 0 || !drain_start) ? 1u : 0u);
+              if (TWO) tc_mma_i8_pair(d, da + 2 * k4, db + 2 * k4, idesc(true, 2 * BM, BN), (k4 > 0 || !drain_start) ? 1u : 0u);
+              else tc_mma_i8(d, da + 2 * k4, db + 2 * k4, idesc(true, BM, BN), (SHIFTED || k4 > 0 || !drain_start) ? 1u : 0u);
             }
             if (TWO) {  // both CTAs' producers and epilogues wait on their own copies of these barriers
               tc_commit_pair(smem_u32(&ctl.empty[s]));
@@ -425,9 +424,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
           }
           __syncwarp();
-          if (drain_end) {
-            ab ^= 1;
-            if (ab == 0) aph ^= 1u;
+          if (drain_end && ++ab == BUFS) {
+            ab = 0;
+            aph ^= 1u;
           }
           if (++s == STAGES) { s = 0; ph ^= 1u; }
         }
@@ -462,7 +461,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const TileCoord tc = unit_tile(t);
         const int64_t bcol0 = (int64_t)(p.b_batched ? tc.m_blk / p.mpb : 0) * p.N + tc.n_tile * BN;
         const float* as_ptr = p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift);
-        const int halves = chan ? 1 : 2;   // with per-channel B scales a factor is the A scale alone
+        const int halves = chan || BN == NARROW ? 1 : 2;   // with per-channel B scales a factor is the A scale alone
         int e[2];                                   // factors are scaled by 2^e, the sums by 2^(149 - e)
         float unit[2];                              // the factor that is divided out, or 1
         double left[2] = {0., 0.};                  // per lane, over the chunks of the tile
@@ -475,7 +474,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
           auto factor = [&](int h, int d) {
             const float a = ld_scale(as_ptr + (d >> p.a_kshift));
-            if (chan || tc.n_tile * BN + h * (BN / 2) >= p.N) return a;   // no second half: a number that does no harm
+            if (chan || tc.n_tile * BN + h * 128 >= p.N) return a;   // no second half: a number that does no harm
             return a * (ld_scale(p.b_scale + ((bcol0 >> 7) + h) * KB + d) * p.post_scale);
           };
           if (k0 == 0) {
@@ -549,16 +548,16 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // 2^(149 - e) as two factors: the sums are far below 1, so the first may take all of it, up to the largest
             // power there is; the rest goes with the column scale
             for (int i = lane; i < BN; i += 32) {
-              const int h = (chan || i < BN / 2) ? 0 : 1, back = 149 - (h ? e[1] : e[0]);
+              const int h = (chan || i < 128) ? 0 : 1, back = 149 - (h ? e[1] : e[0]);
               const float d = pow2f(back < 127 ? 0 : back - 127) * (h ? unit[1] : unit[0]);
               ctl.fbscale[buf][i] = chan && tc.n_tile * BN + i < p.N ? ld_scale(p.b_scale + bcol0 + i) * p.post_scale * d : d;
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              double all = left[chan ? 0 : h];
+              double all = left[h < halves ? h : 0];
 #pragma unroll
               for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-              const int back = 149 - e[chan ? 0 : h];
+              const int back = 149 - e[h < halves ? h : 0];
               const float d = pow2f(back < 127 ? back : 127);
               if (lane == 0) ctl.fend[buf][h] = make_float2(d, -(float)all * d);
             }
@@ -571,7 +570,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else {
     // -------------------------------------------------------------------- epilogue
     // 128 x 64 + 256 x 208 of the 384 x 168 registers of the launch; 128 x 64 + 512 x 104 of 640 x 96
-    if (SHIFTED) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    if (EPI_WARPS == 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     const int q = warp & 3, wg = (warp - 4) >> 2;  // lane quarter, column group
     const int tix = q * 32 + lane;                 // row within the tile == thread index within the group
@@ -599,11 +598,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // data and a few scalars live: the factors of the tile are staged in shared memory first, and
       // what the final store needs is recomputed from the tile index afterwards.
       const uint32_t tfull0 = smem_u32(&ctl.tfull[0]);
-      constexpr uint32_t TEMPTY_OFF = 2 * sizeof(uint64_t);   // tempty[] follows tfull[2] in SharedCtl: one base register serves both
+      constexpr uint32_t TEMPTY_OFF = BUFS * sizeof(uint64_t);   // tempty[] follows tfull[] in SharedCtl: one base register serves both
       // Values derived from the thread index pass through an empty asm statement: the compiler then
       // keeps them in registers instead of recomputing them from the special register at every use
       // inside the K-block loop (which cost about 35 ALU instructions per warp and K block).
-      uint32_t taddr0 = tmem_base + lane_addr + wg * EPI_COLS, fac_base = smem_u32(&ctl.fac[0][p.b_kind == I8L_BSCALE_CHANNEL ? 0 : wg][0]);
+      uint32_t taddr0 = tmem_base + lane_addr + wg * EPI_COLS, fac_base = smem_u32(&ctl.fac[0][p.b_kind == I8L_BSCALE_CHANNEL || BN == NARROW ? 0 : wg][0]);
       asm volatile("" : "+r"(taddr0), "+r"(fac_base));
       constexpr int CH = 32;
       uint32_t gstep = 0, unit = 0;
@@ -665,8 +664,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               release();
             }
             ++gstep;  // buffer and phase from one running count of K blocks
-            ab = gstep & 1;
-            aph = (gstep >> 1) & 1u;
+            ab = gstep % BUFS;
+            aph = gstep / BUFS & 1u;
           }
         }
         // after a timeout the accumulators are not a product: nothing is stored (decided per warp: the store
@@ -751,9 +750,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // fused forward: acc += P / (s_a * s_b)) are published through shared memory, one column per thread.
         constexpr bool ROWF = KIND != K_BLOCK_COLFAC, COLF = KIND == K_BLOCK_COLFAC || KIND == K_BLOCK_OUTER;
         constexpr int CH = 32;
-        static_assert(EPI_COLS == 128, "a thread of the group publishes one column");
+        static_assert(EPI_COLS <= 128, "a thread of the group publishes one column");
         const float* as_ptr = p.a_scale + (ROWF && KIND != K_BLOCK_TILEDIV ? row : (int64_t)tc.m_blk) * KB;
-        const float* bc_ptr = p.b_scale + (bcol0 + tix) * KB;      // COLF: one scale per column and K block
+        const bool publish = tix < EPI_COLS && active;
+        const float* bc_ptr = p.b_scale + (bcol0 + (publish ? tix : 0)) * KB;   // COLF: one scale per column and K block
         const float* bt_ptr = p.b_scale + (bcol0 >> 7) * KB;       // per-tile B scales
         // The scales of the next K block are loaded a whole block ahead and multiplied when it starts: multiplied at once
         // they held every warp up for the load (400 of 1200 cycles per K block with per-tile B scales, 900 of 1775 in the
@@ -761,7 +761,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         float a_next, b_next = 1.f;
         auto load_scales = [&](int d) {
           a_next = ld_scale(as_ptr + d);
-          if (COLF) b_next = active ? ld_scale(bc_ptr + d) : 1.f;
+          if (COLF) b_next = publish ? ld_scale(bc_ptr + d) : 1.f;
           else if (!chan && active) b_next = ld_scale(bt_ptr + d);
         };
         asm volatile("" : "+l"(bc_ptr));   // kept in registers: recomputed in every K block otherwise (column kind 877 -> 851 us)
@@ -780,7 +780,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (KIND == K_BLOCK_TILEDIV || (KIND == K_BLOCK_COLFAC && p.divide)) f = __frcp_rn(f);
           const float2 fr = make_float2(f, f);
           if (COLF) {
-            ctl.bstep[d & 1][wg * EPI_COLS + tix] = ROWF ? b_next : f;
+            if (EPI_COLS == 128 || tix < EPI_COLS) ctl.bstep[d & 1][wg * EPI_COLS + tix] = ROWF ? b_next : f;
             named_sync(1 + wg, 128);
           }
           if (d + 1 < KB) load_scales(d + 1);
@@ -820,8 +820,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           } else {
             release();
           }
-          ab ^= 1;
-          if (ab == 0) aph ^= 1u;
+          if (++ab == BUFS) {
+            ab = 0;
+            aph ^= 1u;
+          }
         }
         if (active && __all_sync(0xffffffffu, !*abort_flag)) {
           float out[EPI_COLS];
@@ -926,8 +928,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
           }
           if (!BLOCK && live && !p.dump && !p.out_f32) stage_send<EPI_COLS / 64>(&map_c, out_stage(), lane, col0, (int)row - lane);
-          ab ^= 1;
-          if (ab == 0) aph ^= 1u;
+          if (++ab == BUFS) {
+            ab = 0;
+            aph ^= 1u;
+          }
         }
         if constexpr (BLOCK) {
           if (ok && active && !p.dump) store_cols<EPI_COLS>(p, &map_c, out_stage(), lane, acc, nullptr, row, col0, p.c);
@@ -1096,16 +1100,17 @@ int32_t* mirror_of(const int32_t* word) {
   return nullptr;
 }
 
-template <int KIND, bool TWO>
+template <int KIND, bool TWO, int BN>
 static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p, int64_t tiles, cudaStream_t st) {
   // per-device set-up, done by whichever thread comes first (idempotent, so a race only repeats it)
   static std::atomic<int> max_units[MAX_DEVICES];   // 0 = not set up yet
   const int dev = current_device();
-  auto kernel = gemm_i8_kernel<KIND, TWO>;
+  auto kernel = gemm_i8_kernel<KIND, TWO, BN>;
+  constexpr int SMEM_DYN = Cfg<TWO, BN>::SMEM_DYN;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  cfg.blockDim = dim3(128 + 32 * EPI_WARPS_OF<KIND>, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_DYN<TWO>;
+  cfg.blockDim = dim3(128 + 32 * EPI_WARPS_OF<KIND, BN>, 1, 1);
+  cfg.dynamicSmemBytes = SMEM_DYN;
   cfg.stream = st;
   if (TWO) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1117,7 +1122,7 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   }
   int units = max_units[dev].load(std::memory_order_acquire);
   if (!units) {
-    I8L_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYN<TWO>));
+    I8L_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYN));
     units = sm_count();
     if (TWO) {  // how many CTA pairs can be co-resident (GPCs with an odd SM count leave one SM unpaired)
       cfg.gridDim = dim3(2 * sm_count(), 1, 1);
@@ -1138,13 +1143,24 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   return I8L_OK;
 }
 
+// Tiles of 128 columns (a CTA each) or of 256?  A grid that fills no SM twice finishes with its slowest CTA, and a narrow tile takes
+// 0.62 of a wide one's time (0.67 with row x column factors; 0.8 in the whole-K kind, whose wide tiles run two tensor pipes
+// on one): half the columns to drain and store, four accumulators instead of two to hide the hand-off in, but as many MMAs of
+// nearly the same duration.  So narrow ones pay where they need fewer than 1 / 0.62 times as many waves.  Kernel time, wide
+// and narrow: 128x1024x1024 fast kind 9.3 / 7.3 us, row x channel 10.1 / 6.9; 1024x1024x4096 19.1 / 13.7, 24.9 / 15.5, whole-K
+// 15.9 / 13.2; 12544x384x2048 (2 waves and 2) 22.2 / 16.1; 6400x1024x4096 (2 and 3) 36.3 / 34.4, row x column factors 69.6 /
+// 70.7, whole-K 26.9 / 32.0; 2048^3 (1 and 2) 14.3 / 16.0; 4096^3 (4 and 7) 67.8 / 72.2.
+static bool narrow_tiles(int64_t wide, int64_t narrow, int sms, int percent) {
+  return (narrow + sms - 1) / sms * percent < (wide + sms - 1) / sms * 100;
+}
+
 static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmParams p, int64_t batch, int64_t M,
                        int64_t N, int64_t K, cudaStream_t st) {
   if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || M % 128 || N % 128 || K % 128)
     return fail(I8L_ERR_SHAPE, "batch=%lld M=%lld N=%lld K=%lld: all positive, M, N, K multiples of 128",
                 (long long)batch, (long long)M, (long long)N, (long long)K);
   if (batch * M >= (1ll << 31) || batch * N >= (1ll << 31) || K >= (1ll << 31) ||
-      (batch * M / 128) * ((N + BN - 1) / BN) >= (1ll << 31))
+      (batch * M / 128) * (N / 128) >= (1ll << 31))
     return fail(I8L_ERR_SHAPE, "problem too large for 32-bit tile coordinates");
   if (!a_q || !b_q || !p.c) return fail(I8L_ERR_ARG, "null pointer");
   if (!aligned16(a_q) || !aligned16(b_q) || !aligned16(p.c)) return fail(I8L_ERR_ALIGN, "a_q, b_q, c must be 16-byte aligned");
@@ -1152,7 +1168,12 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   // CTA pairs (cta_group::2) need two 128-row blocks of the same batch per tile.  They pay off for the
   // whole-K accumulation (half the B traffic per SM: +2.5 % sustained at the power cap); the per-K-block
   // hand-off of the block-scaled kinds is slower across two CTAs (990 vs 1510 TOP/s), so those stay 1-CTA.
-  const bool two = !block && (M % 256 == 0);
+  const bool exact_path = block && (p.exact || p.dump);   // the generic kind has wide tiles only
+  const int64_t m_blocks = batch * M / 128, wide_tiles = (N + WIDE - 1) / WIDE;
+  const int percent = !block ? 80 : (p.a_kind == I8L_ASCALE_GROUP && p.b_kind == I8L_BSCALE_GROUP ? 67 : 62);
+  const bool narrow = !exact_path && narrow_tiles(m_blocks * wide_tiles, m_blocks * (N / NARROW), gemm_cta_budget(), percent);
+  const bool two = !block && !narrow && (M % 256 == 0);
+  const int BN = narrow ? NARROW : WIDE;
   (void)chain_first();   // GEMMs always wait
   p.early = chain_state.gemm_next;
   chain_state.gemm_next = 0;
@@ -1162,9 +1183,9 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   mc = ma;   // read by nobody when the output is not bf16, or leaves for the owners of its rows
   if (!p.out_f32 && !p.dump && !p.rs_rows)
     if (int e = make_map(&mc, p.c, batch * M, N, 32, true)) return e;
-  p.m_blocks = (int)(batch * M / 128);
+  p.m_blocks = (int)m_blocks;
   p.mpb = (int)(M / 128);
-  p.n_tiles = (int)((N + BN - 1) / BN);
+  p.n_tiles = (int)(narrow ? N / NARROW : wide_tiles);
   p.M = (int)M;
   p.N = (int)N;
   p.KB = (int)(K / 128);
@@ -1187,18 +1208,19 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   // One factor per (row or tile, K block) and 128 columns.  Divisors (fused backward, per-tile A scales only) take the
   // exact conversion of the row kind: the fast kind's running shift rounds to about 7e-6, the fused variants are held
   // to 1e-6.
-  const bool scalar_factor = block && !p.exact && !p.dump && p.b_kind != I8L_BSCALE_GROUP &&
-                             (!p.divide || p.a_kind == I8L_ASCALE_TILE);
-  const bool column_factor = block && !p.exact && !p.dump && p.a_kind == I8L_ASCALE_TILE && p.b_kind == I8L_BSCALE_GROUP;
-  const bool outer_factor = block && !p.exact && !p.dump && !p.divide && p.a_kind == I8L_ASCALE_GROUP &&
-                            p.b_kind == I8L_BSCALE_GROUP;
-  if (!block) return two ? launch_kind<K_ROWCOL, true>(ma, mb, mc, p, tiles, st) : launch_kind<K_ROWCOL, false>(ma, mb, mc, p, tiles, st);
-  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && !p.divide) return launch_kind<K_BLOCK_FAST, false>(ma, mb, mc, p, tiles, st);
-  if (scalar_factor && p.divide) return launch_kind<K_BLOCK_TILEDIV, false>(ma, mb, mc, p, tiles, st);
-  if (scalar_factor) return launch_kind<K_BLOCK_ROWFAC, false>(ma, mb, mc, p, tiles, st);
-  if (outer_factor) return launch_kind<K_BLOCK_OUTER, false>(ma, mb, mc, p, tiles, st);
-  if (column_factor) return launch_kind<K_BLOCK_COLFAC, false>(ma, mb, mc, p, tiles, st);
-  return launch_kind<K_BLOCK_GEN, false>(ma, mb, mc, p, tiles, st);
+  const bool scalar_factor = block && !exact_path && p.b_kind != I8L_BSCALE_GROUP && (!p.divide || p.a_kind == I8L_ASCALE_TILE);
+  const bool column_factor = block && !exact_path && p.a_kind == I8L_ASCALE_TILE && p.b_kind == I8L_BSCALE_GROUP;
+  const bool outer_factor = block && !exact_path && !p.divide && p.a_kind == I8L_ASCALE_GROUP && p.b_kind == I8L_BSCALE_GROUP;
+#define I8L_KIND(K) \
+  (narrow ? launch_kind<K, false, NARROW>(ma, mb, mc, p, tiles, st) : launch_kind<K, false, WIDE>(ma, mb, mc, p, tiles, st))
+  if (!block) return two ? launch_kind<K_ROWCOL, true, WIDE>(ma, mb, mc, p, tiles, st) : I8L_KIND(K_ROWCOL);
+  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && !p.divide) return I8L_KIND(K_BLOCK_FAST);
+  if (scalar_factor && p.divide) return I8L_KIND(K_BLOCK_TILEDIV);
+  if (scalar_factor) return I8L_KIND(K_BLOCK_ROWFAC);
+  if (outer_factor) return I8L_KIND(K_BLOCK_OUTER);
+  if (column_factor) return I8L_KIND(K_BLOCK_COLFAC);
+#undef I8L_KIND
+  return launch_kind<K_BLOCK_GEN, false, WIDE>(ma, mb, mc, p, tiles, st);
 }
 
 }  // namespace i8l
