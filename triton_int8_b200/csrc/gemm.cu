@@ -1,18 +1,19 @@
 // INT8 GEMMs on the 5th-generation tensor cores: tcgen05.mma kind::i8 with int32 accumulators in
 // tensor memory, operands staged by TMA into a 128B-swizzled shared-memory ring.
 //
-// One persistent CTA per SM, 384 threads (the five shifted block-scaled kinds, narrow tiles) or 640 (row x column, generic):
+// One persistent CTA per SM, 384 threads, or 640 in the generic kind:
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      tensor-memory allocator + MMA issuer (one elected lane, see elect_one)
 //   warp 2      factor warp (fast block-scaled kind): prepares, one tile ahead, the per-K-block
 //               factors, corrections and column scales the epilogue needs; idle in the other kinds
 //   warp 3      idle (completes the first warpgroup so register budgets can be rebalanced)
 //   warps 4-    epilogue: warp%4 selects the 32 accumulator lanes (rows) a warp may read, the group of
-//               four warps a share of the 256 columns of the 128x256 tile.  Sixteen warps with 64 columns
-//               each where the per-K-block drain is bound by instruction latency (more resident warps hide
-//               it).  The shifted kinds have one or two packed FMAs per two elements left and want long runs
-//               of tensor-memory loads instead: eight warps with 128 columns each and up to 208 registers, 32
+//               four warps a share of the columns of the 128x256 tile.  Sixteen warps with 64 columns
+//               each in the generic kind, whose per-K-block drain is bound by instruction latency (more resident
+//               warps hide it).  The shifted kinds have one or two packed FMAs per two elements left and want long
+//               runs of tensor-memory loads instead: eight warps with 128 columns each and up to 208 registers, 32
 //               columns in flight per wait (fast kind, 8192^3: 16 warps 508 us, 8 warps 501, 8 warps and 32 columns 489).
+//               Eight warps in the row x column kind as well, which take their whole share into registers at once.
 // Tensor memory holds two 128x256 int32 accumulators (all 512 columns), or four of the narrow tiles' 128x128.  In block-scaled mode the
 // MMA warp alternates between them every 128-wide K block while the epilogue drains the other one
 // into fp32 registers (acc += float(P) * scale; in the shifted kinds a fifth MMA per K block moves P into the
@@ -30,9 +31,11 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -54,12 +57,27 @@ template <bool TWO, int BN> struct Cfg {
   static constexpr int SMEM_DYN = STAGES * (A_STAGE + B_STAGE) + OUT_STAGE + 1024;
 };
 constexpr int MAX_STAGES = 5;
-constexpr int MAX_EPI_WARPS = 16;             // groups of four warps share the 256 accumulator columns
 // the kinds whose partial products are shifted by an extra MMA (K_BLOCK_FAST and the row and column factor kinds)
 template <int KIND> constexpr bool SHIFTED_OF = KIND >= 2;
-template <int KIND, int BN> constexpr int EPI_WARPS_OF = SHIFTED_OF<KIND> || BN == NARROW ? 8 : MAX_EPI_WARPS;
+template <int KIND> constexpr int EPI_WARPS_OF = KIND == 1 ? 16 : 8;   // 1: K_BLOCK_GEN
 constexpr int FAC_MAX = 192;                  // K blocks whose factors are staged in shared memory at a time (a multiple of 4)
 constexpr int TMEM_COLS = 512;
+
+// Division of 0 <= n < 2^31 by a number known at launch: n * mul >> shift with mul = ceil(2^shift / d) and shift = 31 + ceil(log2 d),
+// so that mul fits 32 bits and the rounding of mul stays below one part in 2^31.  Dividing costs an epilogue warp about
+// 500 cycles for the coordinates of a tile, which it needs at its start and at its end, this about 100.
+struct FastDiv {
+  uint32_t mul, shift;
+  int d;
+  __device__ __forceinline__ int div(int n) const { return (int)((uint64_t)(uint32_t)n * mul >> shift); }
+  void set(int divisor) {
+    int log = 0;
+    while ((1ll << log) < divisor) ++log;
+    d = divisor;
+    shift = 31 + log;
+    mul = (uint32_t)(((1ull << shift) + divisor - 1) / divisor);
+  }
+};
 
 struct GemmParams {
   const float* a_scale;
@@ -76,7 +94,8 @@ struct GemmParams {
   int exact, divide, out_f32, dump;  // dump: 0 none, 1 whole-K int32, 2 per-K-block int32
   int a_kshift;       // an A tile scale serves 2^a_kshift consecutive K blocks (1 for 128x256 groups)
   int product_first;  // exact order only: float(P) * (a_s*b_s) instead of (float(P)*a_s)*b_s
-  int raster;
+  int raster;     // M-units per group of the tile order
+  FastDiv per_group, full_group, last_group, per_batch;   // tiles of a group, M-units of a group (all but the last; the last), mpb
   int c_align32;  // the output pointer is 32-byte aligned: 256-bit stores
   // scatter mode (rs_rows > 0): rows [o*rs_rows, (o+1)*rs_rows) of the product go to c_slots[o], a
   // [world, rs_rows, N] bf16 buffer of rank o (peer memory), at slot rs_rank
@@ -99,13 +118,11 @@ struct TileCoord {
   int m_blk, n_tile;
 };
 __device__ __forceinline__ TileCoord tile_coord(int t, int m_units, const GemmParams& p) {
-  const int per_group = p.raster * p.n_tiles;
-  const int g = t / per_group, local = t - g * per_group;
-  const int first = g * p.raster;
-  const int gsize = min(p.raster, m_units - first);
+  const int g = p.per_group.div(t), local = t - g * p.per_group.d, first = g * p.raster;
+  const FastDiv& size = first + p.raster <= m_units ? p.full_group : p.last_group;
   TileCoord tc;
-  tc.m_blk = first + local % gsize;
-  tc.n_tile = local / gsize;
+  tc.n_tile = size.div(local);
+  tc.m_blk = first + local - tc.n_tile * size.d;
   return tc;
 }
 
@@ -119,14 +136,17 @@ constexpr int K_BLOCK_TILEDIV = 6; // block-scaled, per-tile scales on both side
 constexpr int K_BLOCK_OUTER = 5;   // block-scaled, per-(row, K block) A scale x per-(column, K block) B scale
 
 template <int KIND, int BN> struct __align__(256) SharedCtl {   // tempty must directly follow tfull (the fast epilogue addresses both from one base)
+  // shifted kinds: BN rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
+  __align__(256) uint8_t ones[SHIFTED_OF<KIND> ? BN * 32 : 1];
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[TMEM_COLS / BN], tempty[TMEM_COLS / BN], done;
   // fast block kind: factors written (factor warp), what the tile end needs written, all consumed (every epilogue thread)
   uint64_t fready[2], eready[2], ffree[2];
   uint32_t tmem_base;
   int abort_flag;
-  union {
+  union __align__(16) {   // scales are read four at a time
     struct {
       float bscale[BN];     // per-tile column scales (CHANNEL)
+      __nv_bfloat16 bias[BN];
       float bstep[KIND == K_ROWCOL ? 1 : 2][KIND == K_ROWCOL ? 1 : BN];   // per-K-block column scales or factors (GROUP), double buffered
     };
     // K_BLOCK_FAST, written by the factor warp one unit (tile, or FAC_MAX-K-block chunk of a tile) ahead, two
@@ -134,11 +154,10 @@ template <int KIND, int BN> struct __align__(256) SharedCtl {   // tempty must d
     struct {
       float2 fac[KIND == K_BLOCK_FAST ? 2 : 1][2][KIND == K_BLOCK_FAST ? FAC_MAX : 1];   // per K block: scaled factor, and the correction due at it (or 0)
       float fbscale[KIND == K_BLOCK_FAST ? 2 : 1][KIND == K_BLOCK_FAST ? BN : 1];        // what the sums are multiplied by at the end: per-channel column scale times post_scale, or 1
+      __nv_bfloat16 fbias[KIND == K_BLOCK_FAST ? 2 : 1][KIND == K_BLOCK_FAST ? BN : 1];
       float2 fend[2][2];           // in front of that: times .x plus .y (undoes the scaling of the factors, takes out what is left of the shift)
     };
   };
-  // shifted kinds: 256 rows x 32 bytes of 0xFF, both operands of the shifting MMA (32-byte swizzle atoms)
-  __align__(256) uint8_t ones[SHIFTED_OF<KIND> ? BN * 32 : 1];
 };
 
 // Shifted kinds: 32 products 255 * 255.  A partial product of 128 int8 pairs lies in [-128*128*127, 128*128*128],
@@ -167,11 +186,6 @@ __device__ __forceinline__ void st_global_256(void* ptr, const uint32_t* w) {
                : "memory");
 }
 
-// Bias of 16 consecutive columns.
-__device__ __forceinline__ void add_bias16(const __nv_bfloat16* bias, float* v) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __fadd_rn(v[j], __bfloat162float(bias[j]));
-}
 // 16 fp32 results of one row, straight to memory (32-byte stores where the output pointer allows them).
 __device__ __forceinline__ void store16_f32(const GemmParams& p, const float* v, void* cbase, int64_t row, int col) {
   float* o = static_cast<float*>(cbase) + row * p.N + col;
@@ -217,26 +231,50 @@ __device__ __forceinline__ void stage_send(const CUtensorMap* map_c, uint32_t st
   }
 }
 
-// Final rescale, bias, cast and store of one thread's EPI_COLS consecutive columns.
-// POST = false: the caller has already folded post_scale into the scales it passes.
-template <int EPI_COLS, bool POST = true>
-__device__ __forceinline__ void store_cols(const GemmParams& p, const CUtensorMap* map_c, uint32_t stage, int lane, const float* acc,
-                                           const float* bscale_or_null, int64_t row, int col0, void* cbase) {
-  if (!p.out_f32) stage_wait(lane);
+// Bias, cast and store of one thread's EPI_COLS consecutive columns.  value(j) gives columns j .. j + 3 but for the bias,
+// bias points to this group's in shared memory.  Each case is a loop of its own without branches: with them in the loop
+// every 16 columns waited for their own loads, 2500 cycles a tile instead of 1600 (both with the store to the staging memory, which the MMAs share).
+template <int EPI_COLS, typename Value>
+__device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMap* map_c, uint32_t stage, int lane, int64_t row, int col0,
+                                           void* cbase, const __nv_bfloat16* bias, Value value) {
+  auto columns16 = [&](int j0, float* v, auto with_bias) {
 #pragma unroll
-  for (int j0 = 0; j0 < EPI_COLS; j0 += 16) {
-    float v[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      v[j] = acc[j0 + j];
-      if (bscale_or_null) v[j] *= bscale_or_null[j0 + j];
-      if (POST && p.post_scale != 1.f) v[j] = __fmul_rn(v[j], p.post_scale);
+    for (int j = 0; j < 16; j += 4) {
+      const float4 o = value(j0 + j);
+      v[j] = o.x;
+      v[j + 1] = o.y;
+      v[j + 2] = o.z;
+      v[j + 3] = o.w;
+      if (decltype(with_bias)::value) {
+        const uint2 b = *reinterpret_cast<const uint2*>(bias + j0 + j);
+        v[j] = __fadd_rn(v[j], __uint_as_float(b.x << 16));
+        v[j + 1] = __fadd_rn(v[j + 1], __uint_as_float(b.x & 0xffff0000u));
+        v[j + 2] = __fadd_rn(v[j + 2], __uint_as_float(b.y << 16));
+        v[j + 3] = __fadd_rn(v[j + 3], __uint_as_float(b.y & 0xffff0000u));
+      }
     }
-    if (p.bias) add_bias16(p.bias + col0 + j0, v);   // a uniform branch: no predicated-off loads and adds when there is no bias
-    if (p.out_f32) store16_f32(p, v, cbase, row, col0 + j0);
-    else stage16(stage + j0 / 64 * 4096, lane, j0 % 64 / 8, v);
-  }
-  if (!p.out_f32) stage_send<EPI_COLS / 64>(map_c, stage, lane, col0, (int)row - lane);
+  };
+  auto columns = [&](auto with_bias) {
+    if (p.out_f32) {
+#pragma unroll
+      for (int j0 = 0; j0 < EPI_COLS; j0 += 16) {
+        float v[16];
+        columns16(j0, v, with_bias);
+        store16_f32(p, v, cbase, row, col0 + j0);
+      }
+    } else {
+      stage_wait(lane);
+#pragma unroll
+      for (int j0 = 0; j0 < EPI_COLS; j0 += 16) {
+        float v[16];
+        columns16(j0, v, with_bias);
+        stage16(stage + j0 / 64 * 4096, lane, j0 % 64 / 8, v);
+      }
+      stage_send<EPI_COLS / 64>(map_c, stage, lane, col0, (int)row - lane);
+    }
+  };
+  if (p.bias) columns(std::true_type{});
+  else columns(std::false_type{});
 }
 
 // Scales, written by the kernel in front of this one in a chain: volatile, so that the compiler keeps the load behind
@@ -248,16 +286,21 @@ __device__ __forceinline__ float ld_scale(const float* ptr) {
 }
 
 template <int KIND, bool TWO, int BN>
-__global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND, BN>, 1)
+__global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND>, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   constexpr bool BLOCK = KIND != K_ROWCOL, SHIFTED = SHIFTED_OF<KIND>;
-  constexpr int EPI_WARPS = EPI_WARPS_OF<KIND, BN>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
+  constexpr int EPI_WARPS = EPI_WARPS_OF<KIND>, EPI_COLS = BN / (EPI_WARPS / 4), THREADS = 128 + 32 * EPI_WARPS;
   constexpr int STAGES = Cfg<TWO, BN>::STAGES, B_STAGE = Cfg<TWO, BN>::B_STAGE, OUT_STAGE = Cfg<TWO, BN>::OUT_STAGE;
   constexpr uint32_t STAGE_TX = Cfg<TWO, BN>::STAGE_TX;
   constexpr int BUFS = TMEM_COLS / BN;   // accumulators
   extern __shared__ uint8_t smem_raw[];
-  __shared__ SharedCtl<KIND, BN> ctl;
+  using Ctl = SharedCtl<KIND, BN>;
+  static_assert(offsetof(Ctl, bscale) % 16 == 0 && offsetof(Ctl, bias) % 8 == 0 && offsetof(Ctl, bstep) % 16 == 0 &&
+                    (KIND != K_BLOCK_FAST || (offsetof(Ctl, fbscale) % 16 == 0 && offsetof(Ctl, fbias) % 8 == 0)) &&
+                    offsetof(Ctl, tempty) == offsetof(Ctl, tfull) + BUFS * sizeof(uint64_t),
+                "vector reads, and the barriers that share a base register");
+  __shared__ Ctl ctl;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a = smem_base, smem_b = smem_base + STAGES * A_STAGE;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -348,7 +391,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       for (int t = I8L_UNIT; t < total_tiles && ok; t += I8L_N_UNITS) {
         const TileCoord tc = unit_tile(t);
         const int a_row = tc.m_blk * BM;
-        const int b_row = (p.b_batched ? (tc.m_blk / p.mpb) * p.N : 0) + tc.n_tile * BN + (TWO ? (int)rank * BM : 0);
+        const int b_row = (p.b_batched ? p.per_batch.div(tc.m_blk) * p.N : 0) + tc.n_tile * BN + (TWO ? (int)rank * BM : 0);
         for (int kb = 0; kb < KB; ++kb) {
           if (!(ok = mbar_wait<!BLOCK>(smem_u32(&ctl.empty[s]), ph ^ 1u, abort_flag, p.max_polls))) break;
           if (p.withhold && t == I8L_UNIT && kb == KB - 1) {
@@ -459,7 +502,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t u = 0;
       for (int t = I8L_UNIT; t < total_tiles; t += I8L_N_UNITS) {
         const TileCoord tc = unit_tile(t);
-        const int64_t bcol0 = (int64_t)(p.b_batched ? tc.m_blk / p.mpb : 0) * p.N + tc.n_tile * BN;
+        const int64_t bcol0 = (int64_t)(p.b_batched ? p.per_batch.div(tc.m_blk) : 0) * p.N + tc.n_tile * BN;
         const float* as_ptr = p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift);
         const int halves = chan || BN == NARROW ? 1 : 2;   // with per-channel B scales a factor is the A scale alone
         int e[2];                                   // factors are scaled by 2^e, the sums by 2^(149 - e)
@@ -551,6 +594,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               const int h = (chan || i < 128) ? 0 : 1, back = 149 - (h ? e[1] : e[0]);
               const float d = pow2f(back < 127 ? 0 : back - 127) * (h ? unit[1] : unit[0]);
               ctl.fbscale[buf][i] = chan && tc.n_tile * BN + i < p.N ? ld_scale(p.b_scale + bcol0 + i) * p.post_scale * d : d;
+              if (p.bias) ctl.fbias[buf][i] = tc.n_tile * BN + i < p.N ? p.bias[tc.n_tile * BN + i] : __float2bfloat16_rn(0.f);
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -685,19 +729,18 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const float2 fe = ctl.fend[unit & 1][wg];
           const float2 fe_mul = make_float2(fe.x, fe.x), fe_add = make_float2(fe.y, fe.y);
           const float4* bsc4 = reinterpret_cast<const float4*>(ctl.fbscale[unit & 1] + wg * EPI_COLS);
-          float2 out[EPI_COLS / 2];
-#pragma unroll
-          for (int j = 0; j < EPI_COLS / 4; ++j) {
-            const float4 bs = bsc4[j];
-            out[2 * j] = __fmul2_rn(__ffma2_rn(acc[2 * j], fe_mul, fe_add), make_float2(bs.x, bs.y));
-            out[2 * j + 1] = __fmul2_rn(__ffma2_rn(acc[2 * j + 1], fe_mul, fe_add), make_float2(bs.z, bs.w));
-          }
+          auto value = [&](int j) {
+            const float4 bs = bsc4[j / 4];
+            const float2 lo = __fmul2_rn(__ffma2_rn(acc[j / 2], fe_mul, fe_add), make_float2(bs.x, bs.y));
+            const float2 hi = __fmul2_rn(__ffma2_rn(acc[j / 2 + 1], fe_mul, fe_add), make_float2(bs.z, bs.w));
+            return make_float4(lo.x, lo.y, hi.x, hi.y);
+          };
           const int col0 = tc.n_tile * BN + wg * EPI_COLS;
           if (p.rs_rows && !p.out_f32 && !p.bias) {
             // Peer stores.  A lane owns one row, so a plain store instruction would send 32 separate 32-byte
             // pieces over NVLink; here the warp passes four rows at a time through shared memory (16-byte
             // slots, XOR-swizzled so that writers and readers are conflict-free) and every store instruction
-            // then covers four rows x 128 contiguous bytes.  Same values as store_cols.
+            // then covers four rows x 128 contiguous bytes.  Same values as store_tile.
             uint4* xp = reinterpret_cast<uint4*>(smem_raw + (out_stage() - smem_u32(smem_raw)));
             const int wr = lane & 3, rr = lane >> 3, rc = lane & 7;
             __nv_bfloat16* obase = static_cast<__nv_bfloat16*>(cbase) + (row - lane) * p.N + col0 + rc * 8;
@@ -705,7 +748,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int h = 0; h < EPI_COLS; h += 64) {
               uint32_t w[32];
 #pragma unroll
-              for (int j = 0; j < 32; ++j) w[j] = pack_bf16x2(out[h / 2 + j].x, out[h / 2 + j].y);
+              for (int j = 0; j < 32; j += 2) {
+                const float4 v = value(h + 2 * j);
+                w[j] = pack_bf16x2(v.x, v.y);
+                w[j + 1] = pack_bf16x2(v.z, v.w);
+              }
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 if ((lane >> 2) == j) {
@@ -720,7 +767,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               }
             }
           } else {
-            store_cols<EPI_COLS, false>(p, &map_c, out_stage(), lane, reinterpret_cast<const float*>(out), nullptr, row, col0, cbase);
+            store_tile<EPI_COLS>(p, &map_c, out_stage(), lane, row, col0, cbase, ctl.fbias[unit & 1] + wg * EPI_COLS, value);
           }
         }
         mbar_arrive(smem_u32(&ctl.ffree[unit & 1]));   // this tile's factors and column scales are no longer needed
@@ -729,17 +776,21 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else
     for (int t = I8L_UNIT; t < total_tiles; t += I8L_N_UNITS) {  // no early exit either (named barriers inside)
       const TileCoord tc = unit_tile(t);
-      const int batch = tc.m_blk / p.mpb;
+      const int batch = p.per_batch.div(tc.m_blk);
       const int64_t row = (int64_t)tc.m_blk * BM + tix;  // row in the folded [batch*M] space
       const int col0 = tc.n_tile * BN + wg * EPI_COLS;
       const bool active = col0 < p.N;
       const int64_t bcol0 = (int64_t)(p.b_batched ? batch : 0) * p.N + col0;  // first b_scale column index
       const bool chan = p.b_kind == I8L_BSCALE_CHANNEL && !p.dump;
-      if (chan) {  // K-invariant column scales of this group -> shared memory
+      if (chan || p.bias) {  // K-invariant column scales and bias of this group -> shared memory
         named_sync(1 + wg, 128);
-        if (tix < EPI_COLS) ctl.bscale[wg * EPI_COLS + tix] = active ? ld_scale(p.b_scale + bcol0 + tix) : 0.f;
+        if (tix < EPI_COLS) {
+          if (chan) ctl.bscale[wg * EPI_COLS + tix] = active ? ld_scale(p.b_scale + bcol0 + tix) : 0.f;
+          if (p.bias) ctl.bias[wg * EPI_COLS + tix] = active ? p.bias[col0 + tix] : __float2bfloat16_rn(0.f);
+        }
         named_sync(1 + wg, 128);
       }
+      const __nv_bfloat16* bias = ctl.bias + wg * EPI_COLS;
 
       if constexpr (SHIFTED) {
         // Before, with sixteen warps converting on two pipes, and now, 8192^3: row x channel 787 -> 607-620 us, column
@@ -826,13 +877,22 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
         if (active && __all_sync(0xffffffffu, !*abort_flag)) {
-          float out[EPI_COLS];
-#pragma unroll
-          for (int j = 0; j < EPI_COLS / 2; ++j) {
-            out[2 * j] = acc[j].x * FROM_SHIFTED;
-            out[2 * j + 1] = acc[j].y * FROM_SHIFTED;
-          }
-          store_cols<EPI_COLS>(p, &map_c, out_stage(), lane, out, !COLF && chan ? ctl.bscale + wg * EPI_COLS : nullptr, row, col0, p.c);
+          const float2 up = make_float2(FROM_SHIFTED, FROM_SHIFTED), post = make_float2(p.post_scale, p.post_scale);
+          auto store = [&](auto with_scale) {
+            store_tile<EPI_COLS>(p, &map_c, out_stage(), lane, row, col0, p.c, bias, [&](int j) {
+              float2 lo = __fmul2_rn(acc[j / 2], up), hi = __fmul2_rn(acc[j / 2 + 1], up);
+              if (decltype(with_scale)::value) {
+                const float4 bs = *reinterpret_cast<const float4*>(ctl.bscale + wg * EPI_COLS + j);
+                lo = __fmul2_rn(lo, make_float2(bs.x, bs.y));
+                hi = __fmul2_rn(hi, make_float2(bs.z, bs.w));
+              }
+              lo = __fmul2_rn(lo, post);
+              hi = __fmul2_rn(hi, post);
+              return make_float4(lo.x, lo.y, hi.x, hi.y);
+            });
+          };
+          if (!COLF && chan) store(std::true_type{});
+          else store(std::false_type{});
         }
       } else {
         // ---- generic paths: reference operation order, per-column / per-step scales, dumps, row x column
@@ -853,15 +913,41 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               named_sync(1 + wg, 128);
             }
           }
-          float sar = 0.f;
-          if (!BLOCK && !p.dump) {
-            sar = ld_scale(p.a_scale + row);
-            if (!p.out_f32) stage_wait(lane);
-          }
+          const float sar = !BLOCK && !p.dump ? ld_scale(p.a_scale + row) : 0.f;
           ok = ok && __all_sync(0xffffffffu, mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls));   // per warp: what follows synchronises it
           tc_fence_after();
           const bool live = ok && active;
           const uint32_t taddr = tmem_base + lane_addr + ab * BN + wg * EPI_COLS;
+          if (!BLOCK && !p.dump) {
+            // row x column: the whole share of the tile into registers, the buffer back, then scale and store
+            uint32_t r[EPI_COLS];
+            if (live) {
+#pragma unroll
+              for (int c = 0; c < EPI_COLS; c += 16) tc_ld16(taddr + c, r + c);
+              tc_ld_wait();
+            }
+            release_accumulator();
+            if (live) {
+              const float2 sar2 = make_float2(sar, sar);
+              auto store = [&](auto in_two_steps) {
+                store_tile<EPI_COLS>(p, &map_c, out_stage(), lane, row, col0, p.c, bias, [&](int j) {
+                  const float4 bs = *reinterpret_cast<const float4*>(ctl.bscale + wg * EPI_COLS + j);
+                  const float2 lo = __fmul2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[j]), __int2float_rn((int)r[j + 1])), sar2), make_float2(bs.x, bs.y));
+                  const float2 hi = __fmul2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[j + 2]), __int2float_rn((int)r[j + 3])), sar2), make_float2(bs.z, bs.w));
+                  float4 v = make_float4(lo.x, lo.y, hi.x, hi.y);
+                  if (decltype(in_two_steps)::value) {
+                    // the reference stores the GEMM result in the output type before its 1/K pass: a bf16
+                    // rounding for bf16 outputs, none for fp32 ones
+                    if (!p.out_f32) v = make_float4(round_to_bf16(v.x), round_to_bf16(v.y), round_to_bf16(v.z), round_to_bf16(v.w));
+                    v = make_float4(__fmul_rn(v.x, p.post_scale), __fmul_rn(v.y, p.post_scale), __fmul_rn(v.z, p.post_scale), __fmul_rn(v.w, p.post_scale));
+                  }
+                  return v;
+                });
+              };
+              if (p.post_scale != 1.f || p.bias) store(std::true_type{});
+              else store(std::false_type{});
+            }
+          } else
 #pragma unroll
           for (int c = 0; c < EPI_COLS / 16; ++c) {
             uint32_t r[16];
@@ -893,48 +979,24 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                   acc[c * 16 + j] = __fadd_rn(acc[c * 16 + j], term);
                 }
               }
-            } else if (p.dump) {
+            } else {
               int32_t* o = static_cast<int32_t*>(p.c) + row * p.N + col0 + c * 16;
 #pragma unroll
               for (int j = 0; j < 16; j += 4)
                 *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-            } else {
-              // row x column epilogue straight from the accumulator chunk
-              const float4* bs4 = reinterpret_cast<const float4*>(ctl.bscale + wg * EPI_COLS + c * 16);
-              const float2 sar2 = make_float2(sar, sar);
-              float v[16];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float4 bs = bs4[j];
-                const float2 lo = __fmul2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[4 * j]), __int2float_rn((int)r[4 * j + 1])), sar2), make_float2(bs.x, bs.y));
-                const float2 hi = __fmul2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[4 * j + 2]), __int2float_rn((int)r[4 * j + 3])), sar2), make_float2(bs.z, bs.w));
-                v[4 * j] = lo.x;
-                v[4 * j + 1] = lo.y;
-                v[4 * j + 2] = hi.x;
-                v[4 * j + 3] = hi.y;
-              }
-              if (p.post_scale != 1.f || p.bias) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  // the reference stores the GEMM result in the output type before its 1/K pass: a bf16
-                  // rounding for bf16 outputs, none for fp32 ones
-                  if (!p.out_f32) v[j] = round_to_bf16(v[j]);
-                  v[j] = __fmul_rn(v[j], p.post_scale);
-                }
-                if (p.bias) add_bias16(p.bias + col0 + c * 16, v);
-              }
-              if (p.out_f32) store16_f32(p, v, p.c, row, col0 + c * 16);
-              else stage16(out_stage(), lane, 2 * c, v);
             }
           }
-          if (!BLOCK && live && !p.dump && !p.out_f32) stage_send<EPI_COLS / 64>(&map_c, out_stage(), lane, col0, (int)row - lane);
           if (++ab == BUFS) {
             ab = 0;
             aph ^= 1u;
           }
         }
         if constexpr (BLOCK) {
-          if (ok && active && !p.dump) store_cols<EPI_COLS>(p, &map_c, out_stage(), lane, acc, nullptr, row, col0, p.c);
+          if (ok && active && !p.dump)
+            store_tile<EPI_COLS>(p, &map_c, out_stage(), lane, row, col0, p.c, bias, [&](int j) {
+              return make_float4(__fmul_rn(acc[j], p.post_scale), __fmul_rn(acc[j + 1], p.post_scale),
+                                 __fmul_rn(acc[j + 2], p.post_scale), __fmul_rn(acc[j + 3], p.post_scale));
+            });
           if (p.b_kind == I8L_BSCALE_GROUP) named_sync(1 + wg, 128);   // bstep is free for the next tile (see the column factors above)
         }
       }
@@ -1109,7 +1171,7 @@ static int launch_kind(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   constexpr int SMEM_DYN = Cfg<TWO, BN>::SMEM_DYN;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  cfg.blockDim = dim3(128 + 32 * EPI_WARPS_OF<KIND, BN>, 1, 1);
+  cfg.blockDim = dim3(128 + 32 * EPI_WARPS_OF<KIND>, 1, 1);
   cfg.dynamicSmemBytes = SMEM_DYN;
   cfg.stream = st;
   if (TWO) {
@@ -1203,6 +1265,13 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
     const int64_t fit = (32ll << 20) / (128 * K);
     const int blocks = (int)(fit < 16 ? 16 : (fit > 32 ? 32 : fit));  // below 16 the B re-reads double (ncu: 17.6 vs 9.4 GB)
     p.raster = two ? blocks / 2 : blocks;
+  }
+  {
+    const int m_units = two ? p.m_blocks / 2 : p.m_blocks, last = m_units % p.raster;
+    p.per_group.set(p.raster * p.n_tiles);
+    p.full_group.set(p.raster);
+    p.last_group.set(last ? last : p.raster);
+    p.per_batch.set(p.mpb);
   }
   const int64_t tiles = (int64_t)(two ? p.m_blocks / 2 : p.m_blocks) * p.n_tiles;
   // One factor per (row or tile, K block) and 128 columns.  Divisors (fused backward, per-tile A scales only) take the
