@@ -265,6 +265,17 @@ I8L_API int i8l_linear_backward(const void* dy, const void* w, const int8_t* x_q
                    int flags, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
 
 /*
+ * The same with the bias gradient: db [N] = i8l_col_sum of dy, bf16, or NULL.
+ * i8l_col_sum: out[c] = sum over the rows of x [rows, cols], both bf16, rows and cols multiples of 128, x 16-byte aligned.
+ * Summed in fp32 and fp64 in an order that depends on the shape only, rounded once.  No counterpart in the reference.
+ */
+I8L_API int i8l_linear_backward_bias(const void* dy, const void* w, const int8_t* x_qt, const float* x_st, void* dx, void* dw,
+                   void* db,
+                   int64_t M, int64_t N, int64_t K, int gran, int qmode, int hadamard, float post_dx, float post_dw,
+                   int flags, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
+I8L_API int i8l_col_sum(const void* x, int64_t rows, int64_t cols, void* out, void* stream);
+
+/*
  * Non-blocking look at a status word (the `status` argument of the GEMMs) for hot loops.  i8l_status_open binds a
  * device int32 and a pinned host int32 (NULL on failure, see i8l_last_error; the handle lives as long as the
  * process).  i8l_status_poll returns I8L_ERR_TIMEOUT if the copy that an earlier poll started has completed and shows

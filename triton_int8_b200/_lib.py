@@ -38,6 +38,8 @@ SIGNATURES = {
     "i8l_sum_slots": [_P, _P, _I, _I64, _I64, _P],
     "i8l_quant_gemm": [_P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I, _I, _I, _I, _I, _F, _I, _P, _I64, _P, _P],
     "i8l_linear_backward": [_P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I, _I, _I, _F, _F, _I, _P, _I64, _P, _P],
+    "i8l_linear_backward_bias": [_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I, _I, _I, _F, _F, _I, _P, _I64, _P, _P],
+    "i8l_col_sum": [_P, _I64, _I64, _P, _P],
     "i8l_status_open": [_P, _P],
     "i8l_status_poll": [_P, _P],
     "i8l_status_reset": [_P],

@@ -22,6 +22,8 @@ int gemm_cta_budget();
 int sm_count();  // of the current device
 int32_t* mirror_of(const int32_t* status_word);   // see i8l_status_mirror; null without one
 
+// i8l_col_sum; in a chain it runs beside its neighbours.
+int col_sum(const void* x, int64_t rows, int64_t cols, void* out, cudaStream_t st);
 // Clears n floats; in a chain the next kernel waits for it before anything else.
 int clear(float* ptr, int64_t n, cudaStream_t st);
 // i8l_quant_col_t (rot = false) or i8l_quant_col_t_rot; zeroed: colmax is zero already.

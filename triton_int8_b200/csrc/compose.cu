@@ -80,16 +80,17 @@ extern "C" int i8l_quant_gemm(const void* a, const void* b, const void* bias, vo
   float* colmax = a_qt && a_gran == I8L_GRAN_ROW ? ws.take<float>(K) : nullptr;
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_quant_gemm: workspace of %lld bytes is too small", (long long)workspace_bytes);
   const LaunchChain chain(static_cast<cudaStream_t>(stream));
+  if (colmax) {   // ahead of the GEMM, while A is in L2
+    if (int e = quant_col_t(a, M, K, qmode, hadamard, a_qt, a_st, colmax, false, stream)) return e;
+  }
   if (a_qt && a_gran != I8L_GRAN_ROW) {   // both orientations of A from one call
     if (int e = i8l_quant_tile(a, batch, M, K, a_gran, qmode, hadamard, aq, as, a_qt, a_st, stream)) return e;
   } else {
     if (int e = quant(a, batch, M, K, a_gran, qmode, hadamard, aq, as, stream)) return e;
   }
   if (int e = quant(b, b_n, N, K, b_gran, qmode, hadamard, bq, bs, stream)) return e;
-  if (a_gran == I8L_GRAN_ROW) {
-    if (int e = i8l_gemm_rowcol(aq, bq, as, bs, b_batched, bias, post_scale, c, batch, M, N, K, flags, status, stream)) return e;
-    return a_qt ? quant_col_t(a, M, K, qmode, hadamard, a_qt, a_st, colmax, false, stream) : I8L_OK;
-  }
+  if (a_gran == I8L_GRAN_ROW)
+    return i8l_gemm_rowcol(aq, bq, as, bs, b_batched, bias, post_scale, c, batch, M, N, K, flags, status, stream);
   return i8l_gemm_block(aq, bq, as, bs, a_kind_of(a_gran), b_kind_of(b_gran), b_batched, bias, post_scale, c, batch, M, N, K,
                         flags, status, stream);
 }
@@ -98,6 +99,14 @@ extern "C" int i8l_linear_backward(const void* dy, const void* w, const int8_t* 
                                    int64_t M, int64_t N, int64_t K, int gran, int qmode, int hadamard, float post_dx,
                                    float post_dw, int flags, void* workspace, int64_t workspace_bytes, int32_t* status,
                                    void* stream) {
+  return i8l_linear_backward_bias(dy, w, x_qt, x_st, dx, dw, nullptr, M, N, K, gran, qmode, hadamard, post_dx, post_dw, flags,
+                                  workspace, workspace_bytes, status, stream);
+}
+
+extern "C" int i8l_linear_backward_bias(const void* dy, const void* w, const int8_t* x_qt, const float* x_st, void* dx, void* dw,
+                                        void* db, int64_t M, int64_t N, int64_t K, int gran, int qmode, int hadamard,
+                                        float post_dx, float post_dw, int flags, void* workspace, int64_t workspace_bytes,
+                                        int32_t* status, void* stream) {
   if (int e = check_extents(1, M, N, K)) return e;
   if (!workspace || (dw && (!x_qt || !x_st))) return fail(I8L_ERR_ARG, "i8l_linear_backward: bad pointers");
   if (gran == I8L_GRAN_TILE128X256) return fail(I8L_ERR_ARG, "i8l_linear_backward: unsupported gran=%d", gran);
@@ -127,6 +136,8 @@ extern "C" int i8l_linear_backward(const void* dy, const void* w, const int8_t* 
     if (int e = check_arch()) return e;
     if (int e = clear(colmax, K, static_cast<cudaStream_t>(stream))) return e;
   }
+  if (db)
+    if (int e = col_sum(dy, M, N, db, static_cast<cudaStream_t>(stream))) return e;
   if (whole_k) {
     if (dx)
       if (int e = i8l_quant_row(dy, M, N, qmode, hadamard, dyq, dys, stream)) return e;

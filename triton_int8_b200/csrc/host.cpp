@@ -32,7 +32,7 @@ using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 decltype(&i8l_quant_gemm) lib_quant_gemm = nullptr;
-decltype(&i8l_linear_backward) lib_linear_backward = nullptr;
+decltype(&i8l_linear_backward_bias) lib_linear_backward = nullptr;
 decltype(&i8l_status_peek) lib_status_peek = nullptr;
 PyObject* on_error = nullptr;       // (entry point, code, device index): raises
 PyObject* open_status = nullptr;    // (device index) -> (status word, poller), as integers
@@ -202,7 +202,7 @@ void backward_in_python(const Tensor& dy, const Tensor& weight, const Tensor& q,
 }
 
 void linear_backward(const Tensor& dy, const Tensor& weight, const Tensor& q, const Tensor& s, const Config& c, bool need_dx,
-                     bool need_dw, Tensor& dx, Tensor& dw) {
+                     bool need_dw, bool need_db, Tensor& dx, Tensor& dw, Tensor& db) {
   const int64_t M = dy.size(0), N = dy.size(1), K = weight.size(1);
   const int gran = c.whole_k ? I8L_GRAN_ROW : c.gran;
   bool ok = plain_thread() && plain(dy) && plain(weight) && weight.size(0) == N && weight.device() == dy.device();
@@ -211,20 +211,28 @@ void linear_backward(const Tensor& dy, const Tensor& weight, const Tensor& q, co
          s.scalar_type() == at::kFloat && q.is_contiguous() && s.is_contiguous() && q.sizes() == at::IntArrayRef({1, K, M}) &&
          s.numel() == scale_count(gran, 1, K, M);
   }
-  if (!ok) return backward_in_python(dy, weight, q, s, c, need_dx, need_dw, dx, dw);
+  // torch's sum where its graph is wanted (create_graph)
+  const bool own_sum = need_db && ok && !at::GradMode::is_enabled();
+  if (need_db && !own_sum) db = dy.sum(0);
+  if (!ok) {
+    if (need_dx || need_dw) backward_in_python(dy, weight, q, s, c, need_dx, need_dw, dx, dw);
+    return;
+  }
+  if (!need_dx && !need_dw && !own_sum) return;
   const int dev = dy.get_device();
   const c10::cuda::CUDAGuard guard(dev);
   Status& status = status_of(dev);
   if (need_dx) dx = at::empty({M, K}, dy.options());
   if (need_dw) dw = at::empty({N, K}, dy.options());
+  if (own_sum) db = at::empty({N}, dy.options());
   int64_t size = pad(4 * std::max(K, N));
   if (need_dx) size += pad(M * N) + pad(4 * scale_count(gran, 1, M, N)) + pad(4 * K) + (need_dw ? 0 : pad(K * N));
   if (need_dw) size += pad(N * M) + pad(4 * scale_count(gran, 1, N, M));
   const Tensor ws = bytes(size, dy);
-  check("i8l_linear_backward",
+  check("i8l_linear_backward_bias",
         lib_linear_backward(dy.data_ptr(), weight.data_ptr(), need_dw ? static_cast<const int8_t*>(q.data_ptr()) : nullptr,
                             need_dw ? static_cast<const float*>(s.data_ptr()) : nullptr, need_dx ? dx.data_ptr() : nullptr,
-                            need_dw ? dw.data_ptr() : nullptr, M, N, K, gran, c.whole_k ? I8L_QMODE_ROWRCP : c.qmode, c.hadamard,
+                            need_dw ? dw.data_ptr() : nullptr, own_sum ? db.data_ptr() : nullptr, M, N, K, gran, c.whole_k ? I8L_QMODE_ROWRCP : c.qmode, c.hadamard,
                             (float)c.post(N), (float)c.post(M), c.whole_k ? 0 : c.flags, ws.data_ptr(), size,
                             status.word.load(std::memory_order_relaxed), c10::cuda::getCurrentCUDAStream(dev).stream()),
         dev);
@@ -248,11 +256,9 @@ struct Int8LinearNode : torch::autograd::Function<Int8LinearNode> {
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const Tensor& dy = grads[0];
     const Tensor dy2 = dy.reshape({-1, dy.size(-1)}).contiguous();
-    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
     Tensor dx, dw, db;
-    if (need_dx || need_dw)
-      linear_backward(dy2, saved[0], saved.size() > 1 ? saved[1] : Tensor(), saved.size() > 1 ? saved[2] : Tensor(), c, need_dx, need_dw, dx, dw);
-    if (has_bias && ctx->needs_input_grad(2)) db = dy2.sum(0);
+    linear_backward(dy2, saved[0], saved.size() > 1 ? saved[1] : Tensor(), saved.size() > 1 ? saved[2] : Tensor(), c,
+                    ctx->needs_input_grad(0), ctx->needs_input_grad(1), has_bias && ctx->needs_input_grad(2), dx, dw, db);
     if (dx.defined()) dx = dx.view(ctx->saved_data["shape"].toIntVector());
     return {dx, dw, db, Tensor(), Tensor()};
   }
@@ -326,7 +332,7 @@ PyObject* py_quant_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// setup(address of i8l_quant_gemm, of i8l_linear_backward, of i8l_status_peek, on_error, open_status, py_backward)
+// setup(address of i8l_quant_gemm, of i8l_linear_backward_bias, of i8l_status_peek, on_error, open_status, py_backward)
 PyObject* py_setup(PyObject*, PyObject* args) {
   unsigned long long qg = 0, lb = 0, sp = 0;
   PyObject *err = nullptr, *open = nullptr, *bwd = nullptr;

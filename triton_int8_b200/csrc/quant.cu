@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace i8l {
 
@@ -453,6 +454,77 @@ col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
     for (int k = 1; k < 8; ++k) mm = fmaxf(mm, s_colred[k * 128 + tid]);
     atomicMax(reinterpret_cast<int*>(colmax + c_base + tid), __float_as_int(mm));
   }
+  chain_wait();
+}
+
+// ------------------------------------------------------------------------------------------------
+// Column sums of x [rows, cols] in bf16, the bias gradient.  A CTA of 256 threads sums a strip of 64 columns (a 128-byte
+// line per row) over its share of the rows, the CTAs of a cluster share a strip and add up through distributed shared
+// memory: one launch, no atomics, always the same order.  At most 128 values are added in a row in fp32, the rest in
+// fp64.  Bound by memory (L2, when its neighbours read the same tensor).  Against
+// torch's sum: [512, 1024] 8.9 -> 3.3 us, [4096, 4096] 15.7 -> 6.6, [32768, 8192] 98 -> 80 (6.7 TB/s), [32768, 256] 40 -> 11.5; the error
+// against float64 is the rounding to bf16 in both.
+// ------------------------------------------------------------------------------------------------
+constexpr int SUM_COLS = 64;
+__global__ void __launch_bounds__(256)
+col_sum_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, __nv_bfloat16* __restrict__ out, int first) {
+  __shared__ float s_part[32][SUM_COLS + 8];   // rows of 72 floats: 16-byte aligned, conflict-free in both directions
+  __shared__ double s_sum[SUM_COLS];
+  const int tid = threadIdx.x, c = tid & 7, r = tid >> 3;
+  const int64_t blocks = rows / 128, share = gridDim.y;
+  const int64_t begin = blocks * blockIdx.y / share * 128, end = blocks * (blockIdx.y + 1) / share * 128;
+  chain_start(first);
+  const uint4* src = reinterpret_cast<const uint4*>(x + (int64_t)blockIdx.x * SUM_COLS) + c;
+  double total[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) total[j] = 0.;
+  for (int64_t r0 = begin; r0 < end;) {
+    const int64_t stop = end - r0 > 4096 ? r0 + 4096 : end;   // 128 rows per thread
+    float sum[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum[j] = 0.f;
+#pragma unroll 2
+    for (; r0 < stop; r0 += 128) {
+      float v[4][8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) unpack8(__ldg(src + (r0 + 32 * i + r) * (cols / 8)), v[i]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[j] += (v[0][j] + v[1][j]) + (v[2][j] + v[3][j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) total[j] += (double)sum[j];
+  }
+  // the 32 threads of a column: fp32 is enough to hand a sum of fewer than 4096 rows on, more go in two parts
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    float* dst = &s_part[r][8 * c];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float hi = (float)total[j];
+      dst[j] = hi;
+      total[j] = isfinite(hi) ? total[j] - (double)hi : 0.;
+    }
+    __syncthreads();
+    if (tid < SUM_COLS) {
+      double t = part ? s_sum[tid] : 0.;
+#pragma unroll 8
+      for (int k = 0; k < 32; ++k) t += (double)s_part[k][tid];
+      s_sum[tid] = t;
+    }
+    __syncthreads();
+    if (end - begin <= 4096) break;   // the sums were fp32
+  }
+  if (share > 1) cluster_sync_all();
+  if (blockIdx.y == 0 && tid < SUM_COLS) {
+    double t = s_sum[tid];
+    for (uint32_t k = 1; k < share; ++k) {
+      double o;
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(o) : "r"(map_to_cta((uint32_t)__cvta_generic_to_shared(&s_sum[tid]), k)) : "memory");
+      t += o;
+    }
+    out[(int64_t)blockIdx.x * SUM_COLS + tid] = __float2bfloat16_rn((float)t);
+  }
+  if (share > 1) cluster_sync_all();   // the others' shared memory stays until it has been read
   chain_wait();
 }
 
@@ -1028,6 +1100,30 @@ static int launch_col_t(const void* x, int64_t rows, int64_t cols, bool rot, int
 }
 
 namespace i8l {
+int col_sum(const void* x, int64_t rows, int64_t cols, void* out, cudaStream_t st) {
+  if (int e = check_dims(1, rows, cols)) return e;
+  if (!x || !out) return fail(I8L_ERR_ARG, "null pointer");
+  if (!aligned16(x)) return fail(I8L_ERR_ALIGN, "x must be 16-byte aligned");
+  if (int e = check_arch()) return e;
+  // a strip of 64 columns on 1 to 8 CTAs, for two on each SM, but no fewer than 512 rows each
+  const int64_t strips = cols / SUM_COLS;
+  int share = 1;
+  while (share < 8 && strips * share < 2 * sm_count() && rows >= 1024 * share) share *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attrs[2];
+  cfg.gridDim = dim3((unsigned)strips, (unsigned)share, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = st;
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 1;
+  attrs[0].val.clusterDim.y = (unsigned)share;
+  attrs[0].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 1;
+  chain_attribute(cfg, attrs);
+  I8L_CUDA_OK(cudaLaunchKernelEx(&cfg, col_sum_kernel, static_cast<const __nv_bfloat16*>(x), rows, cols, static_cast<__nv_bfloat16*>(out), chain_first()));
+  return I8L_OK;
+}
 int clear(float* ptr, int64_t n, cudaStream_t st) {   // a kernel and not a memset, which would break the chain
   I8L_CUDA_OK(launch(clear_kernel, dim3((unsigned)((n + 1023) / 1024)), 1024, 0, st, ptr, n));
   chain_state.wait = 1;
@@ -1047,6 +1143,10 @@ int quant_col_t(const char* name, const void* x, int64_t rows, int64_t cols, int
   return fail(I8L_ERR_ARG, "%s: unsupported qmode=%d", name, qmode);
 }
 }  // namespace i8l
+
+extern "C" int i8l_col_sum(const void* x, int64_t rows, int64_t cols, void* out, void* stream) {
+  return col_sum(x, rows, cols, out, static_cast<cudaStream_t>(stream));
+}
 
 extern "C" int i8l_quant_col_t(const void* x, int64_t rows, int64_t cols, int qmode, int8_t* qt, float* scale_t,
                                float* colmax_scratch, void* stream) {

@@ -132,7 +132,7 @@ def host():
         except ImportError as e:
             raise ImportError(f"triton_int8_b200/_host.so is missing or does not fit this torch: build it with "
                               f"`python -m triton_int8_b200.build` ({e})") from e
-        mod.setup(L.address("i8l_quant_gemm"), L.address("i8l_linear_backward"), L.address("i8l_status_peek"), _on_error,
+        mod.setup(L.address("i8l_quant_gemm"), L.address("i8l_linear_backward_bias"), L.address("i8l_status_peek"), _on_error,
                   _open_status, _backward_in_python)
         _host = mod
     return _host
@@ -334,6 +334,15 @@ def linear_backward(dy, w, xt, gran, qmode, hadamard=0, post_dx=1.0, post_dw=1.0
           qmode, hadamard, float(post_dx), float(post_dw), flags, ws.data_ptr(), size, status.data_ptr(),
           tensors=(w, xqt, xst))
     return dx, dw
+
+
+def col_sum(x: torch.Tensor) -> torch.Tensor:
+    """x bf16 [R, C] -> bf16 [C], the sum over the rows."""
+    x = _check_bf16(x, "x")
+    R, C = x.shape
+    out = torch.empty((C,), dtype=torch.bfloat16, device=x.device)
+    _call("i8l_col_sum", x.device, x.data_ptr(), R, C, out.data_ptr())
+    return out
 
 
 def gemm_dump_i32(aq, bq, per_block=False, status=None):

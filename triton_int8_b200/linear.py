@@ -180,7 +180,9 @@ class Int8LinearFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
         need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         dx, dw = linear_backward(dy2, weight, tuple(saved) if saved else None, ctx.cfg, need_dx, need_dw)
-        db = dy2.sum(0).to(dy.dtype) if ctx.has_bias and ctx.needs_input_grad[2] else None
+        db = None
+        if ctx.has_bias and ctx.needs_input_grad[2]:   # torch's sum where its graph is wanted
+            db = dy2.sum(0).to(dy.dtype) if torch.is_grad_enabled() else K.col_sum(dy2)
         return (dx.view(ctx.x_shape) if dx is not None else None), dw, db, None, None
 
 
