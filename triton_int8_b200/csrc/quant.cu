@@ -259,10 +259,14 @@ quant_tile256_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t 
 // from ONE read, each with scales of its own.  One CTA of 128 threads per 128x128 tile; the tile is staged
 // in shared memory as bf16 and a thread owns a whole row, then a whole column, so that all seven butterfly
 // stages run in its registers as packed pairs: no shuffles, which together with 16-bit shared-memory reads
-// cost 4.2 load/store slots per element when four lanes shared a row and two a column (now 1.5).  Bound by
-// issue and latency at 12 warps per SM (150 registers; about 10 instructions per element and output) next to
-// HBM.  [32768, 8192]: both outputs 353 -> 300 us, q 194 -> 177, qt 284 -> 185; W^T of [28672, 8192] in its two
-// passes 404 -> 247.  A persistent form that copies the next tile meanwhile was slower (393 us with both outputs).
+// cost 4.2 load/store slots per element when four lanes shared a row and two a column.  The output rows leave the same
+// way as in the GEMMs, through shared memory in whole lines' halves (quant_store128).  No unit is near its limit over a
+// block's life, but each of its phases fills one (load/store, adds, conversions), with 12 warps per SM (150 registers;
+// about 10 instructions per element and output).  [32768, 8192], two lanes a column -> a column a thread -> staged
+// stores: both outputs 353 -> 294 -> 275 us, q 194 -> 171 -> 157, qt 284 -> 181 -> 166; W^T of [28672, 8192] in its two
+// passes 404 -> 241 -> 236.  Slower: a persistent form that copies the next tile meanwhile (393 us with both outputs),
+// fetching a later block's tile into L2 (315), two threads per row and column with half the registers and twice the warps
+// (316), blocks started apart from one another (304).
 // ------------------------------------------------------------------------------------------------
 constexpr int ROT_LD = 272;  // bytes per staged row: 256 + 16, conflict-free for 16-byte row reads and for column reads
 
@@ -324,27 +328,40 @@ __device__ __forceinline__ float max_without_nan(const uint32_t* h) {
   return hmax_of(hm);
 }
 
-// 128 rotated values -> 128 consecutive bytes (32-byte stores where the output pointer allows them).
-// FINITE: quant_piece_finite instead of the saturating conversions.
+// 128 rotated values per lane -> 128 bytes of row `lane` of the warp's rows, `pitch` bytes apart from `out` on; rows: how many
+// there are.  A lane owns a row, so a plain store instruction touches 32 lines, and the stores took a quarter of the
+// load/store unit's time.  The warp passes its rows through shared memory in halves (`stage`, 32 pieces of OUT_LD bytes), and an
+// instruction stores 64 bytes of eight rows.  FINITE: quant_piece_finite instead of the saturating conversions.
+constexpr int OUT_LD = 80;   // 64 + 16: conflict-free both ways
 template <int MODE, bool FINITE>
-__device__ __forceinline__ void quant_store128(const uint32_t* h, float s, int8_t* out, bool align32) {
+__device__ __forceinline__ void quant_stage64(const uint32_t* h, float s, uint32_t dst) {
 #pragma unroll
-  for (int i = 0; i < 64; i += 16) {
-    uint32_t w[8];
+  for (int i = 0; i < 32; i += 8) {
+    const uint2 a = FINITE ? quant_piece_finite<MODE>(make_uint4(h[i], h[i + 1], h[i + 2], h[i + 3]), s)
+                           : quant_piece<MODE>(make_uint4(h[i], h[i + 1], h[i + 2], h[i + 3]), s);
+    const uint2 b = FINITE ? quant_piece_finite<MODE>(make_uint4(h[i + 4], h[i + 5], h[i + 6], h[i + 7]), s)
+                           : quant_piece<MODE>(make_uint4(h[i + 4], h[i + 5], h[i + 6], h[i + 7]), s);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 2 * i), "r"(a.x), "r"(a.y), "r"(b.x), "r"(b.y) : "memory");
+  }
+}
+template <int MODE>
+__device__ __forceinline__ void quant_store128(const uint32_t* h, float s, bool finite, uint32_t stage, int lane, int8_t* out, int64_t pitch,
+                                               int rows) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint4 u = make_uint4(h[i + 4 * k], h[i + 4 * k + 1], h[i + 4 * k + 2], h[i + 4 * k + 3]);
-      const uint2 o = FINITE ? quant_piece_finite<MODE>(u, s) : quant_piece<MODE>(u, s);
-      w[2 * k] = o.x;
-      w[2 * k + 1] = o.y;
-    }
-    if (align32) {
-      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                   ::"l"(out + 2 * i), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+  for (int half = 0; half < 2; ++half) {
+    __syncwarp();   // what was staged before has been read
+    if (finite) quant_stage64<MODE, true>(h + 32 * half, s, stage + lane * OUT_LD);
+    else quant_stage64<MODE, false>(h + 32 * half, s, stage + lane * OUT_LD);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = 8 * i + (lane >> 2);
+      uint4 v;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                   : "r"(stage + row * OUT_LD + 16 * (lane & 3))
                    : "memory");
-    } else {
-      *reinterpret_cast<uint4*>(out + 2 * i) = make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4*>(out + 2 * i + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+      if (row < rows) *reinterpret_cast<uint4*>(out + row * pitch + 64 * half + 16 * (lane & 3)) = v;
     }
   }
 }
@@ -357,6 +374,7 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
                       float* __restrict__ scale, int8_t* __restrict__ qt, float* __restrict__ scale_t,
                       float* __restrict__ colmax, int first) {
   __shared__ __align__(16) uint8_t s_raw[128 * ROT_LD];
+  __shared__ __align__(16) uint8_t s_out[GRAN == GRAN_COLMAX_PASS ? 16 : 128 * OUT_LD];
   __shared__ float s_red[2][4];
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
@@ -412,10 +430,8 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
     else if (GRAN == I8L_GRAN_GROUP128) sc[(blockIdx.z * o_n + o_base + tid) * nkb + kb] = stored;
     else if (tid == 0) sc[(blockIdx.z * (o_n / 128) + o_base / 128) * nkb + kb] = stored;
     int8_t* out = ph == 0 ? q : qt;
-    const bool align32 = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;
-    int8_t* row = out + boff + (o_base + tid) * k_n + k_base;
-    if (finite) quant_store128<MODE, true>(h, s, row, align32);
-    else quant_store128<MODE, false>(h, s, row, align32);
+    quant_store128<MODE>(h, s, finite, (uint32_t)__cvta_generic_to_shared(s_out) + w * 32 * OUT_LD, l,
+                         out + boff + (o_base + 32 * w) * k_n + k_base, k_n, 32);
   }
   chain_wait();
 }
@@ -650,13 +666,14 @@ quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64
 
 // The same with the 128-point rotation.  A CTA takes as many whole rows as fit into 128 groups of 128 elements,
 // staged like the tiles above, and a thread owns a group: no shuffles, and each group is rotated once.  Bound by
-// issue next to HBM.  [11008, 4096] 69 -> 40 us, [28672, 8192] 183 -> 150, [8192, 256] 47 -> 9 against one CTA per
+// issue next to HBM.  [11008, 4096] 69 -> 33 us, [28672, 8192] 183 -> 142, [8192, 256] 47 -> 9 against one CTA per
 // row with a group in 16 lanes.
 template <int MODE>
 __global__ void __launch_bounds__(128, 3)
 quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int groups, int rows_per_cta, int8_t* __restrict__ q,
                      float* __restrict__ scale, int first) {
   __shared__ __align__(16) uint8_t s_raw[128 * ROT_LD];
+  __shared__ __align__(16) uint8_t s_out[128 * OUT_LD];
   __shared__ int s_max[128];
   const int tid = threadIdx.x, my_row = tid / groups;
   const int64_t row0 = (int64_t)blockIdx.x * rows_per_cta;
@@ -683,15 +700,19 @@ quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int grou
     atomicMax(&s_max[my_row], __float_as_int(m));   // |x| >= 0: the bit patterns order like integers
   }
   __syncthreads();
-  if (!live) return;
-  float s, stored;
-  make_scale<MODE>(__int_as_float(s_max[my_row]), s, stored);
-  if (tid == my_row * groups) scale[row0 + my_row] = stored;
-  int8_t* out = q + (row0 * groups + tid) * 128;
-  const bool align32 = (reinterpret_cast<uintptr_t>(q) & 31u) == 0;
-  if (finite) quant_store128<MODE, true>(h, s, out, align32);
-  else quant_store128<MODE, false>(h, s, out, align32);
-  chain_wait();   // the first group of a block is always live
+  const int w = tid >> 5, left = n - 32 * w;   // groups of this warp
+  if (left > 0) {
+    float s, stored;
+    make_scale<MODE>(__int_as_float(s_max[live ? my_row : 0]), s, stored);
+    if (live && tid == my_row * groups) scale[row0 + my_row] = stored;
+    if (!live) {
+#pragma unroll
+      for (int i = 0; i < 64; ++i) h[i] = 0;   // staged with the rest, not stored
+    }
+    quant_store128<MODE>(h, s, finite, (uint32_t)__cvta_generic_to_shared(s_out) + w * 32 * OUT_LD, tid & 31,
+                         q + (row0 * groups + 32 * w) * 128, 128, left);
+  }
+  chain_wait();
 }
 
 // Whole-row rotation of rows of G groups of 128 (G = 2..128).  A CTA takes 128/G whole rows.  Spans 1..64 run in
