@@ -22,6 +22,10 @@ int gemm_cta_budget();
 int sm_count();  // of the current device
 int32_t* mirror_of(const int32_t* status_word);   // see i8l_status_mirror; null without one
 
+// Both operands of a product, a [a_batch, a_rows, cols] (with its transpose if aqt) and b, in one launch: see quant.cu.
+int quant_pair(const void* a, int64_t a_batch, int64_t a_rows, int a_gran, int8_t* aq, float* as, int8_t* aqt, float* ast, const void* b,
+               int64_t b_batch, int64_t b_rows, int b_gran, int8_t* bq, float* bs, int64_t cols, int qmode, int hadamard,
+               cudaStream_t st);
 // i8l_col_sum; in a chain it runs beside its neighbours.
 int col_sum(const void* x, int64_t rows, int64_t cols, void* out, cudaStream_t st);
 // Clears n floats; in a chain the next kernel waits for it before anything else.

@@ -83,12 +83,19 @@ extern "C" int i8l_quant_gemm(const void* a, const void* b, const void* bias, vo
   if (colmax) {   // ahead of the GEMM, while A is in L2
     if (int e = quant_col_t(a, M, K, qmode, hadamard, a_qt, a_st, colmax, false, stream)) return e;
   }
-  if (a_qt && a_gran != I8L_GRAN_ROW) {   // both orientations of A from one call
+  const bool grouped_t = a_qt && a_gran == I8L_GRAN_GROUP128;   // needs launches of its own
+  const int paired = grouped_t ? 0
+                               : quant_pair(a, batch, M, a_gran, aq, as, colmax ? nullptr : a_qt, a_st, b, b_n, N, b_gran, bq, bs, K, qmode,
+                                            hadamard, static_cast<cudaStream_t>(stream));
+  if (paired < 0) return paired;
+  if (paired) {
+  } else if (a_qt && a_gran != I8L_GRAN_ROW) {   // both orientations of A from one call
     if (int e = i8l_quant_tile(a, batch, M, K, a_gran, qmode, hadamard, aq, as, a_qt, a_st, stream)) return e;
   } else {
     if (int e = quant(a, batch, M, K, a_gran, qmode, hadamard, aq, as, stream)) return e;
   }
-  if (int e = quant(b, b_n, N, K, b_gran, qmode, hadamard, bq, bs, stream)) return e;
+  if (!paired)
+    if (int e = quant(b, b_n, N, K, b_gran, qmode, hadamard, bq, bs, stream)) return e;
   if (a_gran == I8L_GRAN_ROW)
     return i8l_gemm_rowcol(aq, bq, as, bs, b_batched, bias, post_scale, c, batch, M, N, K, flags, status, stream);
   return i8l_gemm_block(aq, bq, as, bs, a_kind_of(a_gran), b_kind_of(b_gran), b_batched, bias, post_scale, c, batch, M, N, K,

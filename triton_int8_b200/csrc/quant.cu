@@ -56,18 +56,18 @@ constexpr float BF16_LARGEST = 3.3895314e38f;
 __device__ __forceinline__ float hmax_of(__nv_bfloat162 m) { return fmaxf(__low2float(m), __high2float(m)); }
 
 template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
-__global__ void __launch_bounds__(256, 4)
-quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
-                  int8_t* __restrict__ q, float* __restrict__ scale, int8_t* __restrict__ qt,
-                  float* __restrict__ scale_t, const float* __restrict__ colmax, int first) {
+__device__ __forceinline__ void
+quant_tile_body(const dim3 block, const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
+                int8_t* __restrict__ q, float* __restrict__ scale, int8_t* __restrict__ qt,
+                float* __restrict__ scale_t, const float* __restrict__ colmax, int first) {
   __shared__ float s_red[8];
   __shared__ float s_colred[(GRAN == I8L_GRAN_GROUP128 && OUT_T) ? 8 * 128 : 1];
   __shared__ float s_cols[(GRAN != I8L_GRAN_TILE128 && OUT_T) ? 128 : 1];
   __shared__ uint32_t s_t[OUT_T ? 128 * 32 : 1];
 
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, cc = l & 15, half = l >> 4;
-  const int64_t r_base = (int64_t)blockIdx.y * 128, c_base = (int64_t)blockIdx.x * 128;
-  const int64_t boff = (int64_t)blockIdx.z * rows * cols;
+  const int64_t r_base = (int64_t)block.y * 128, c_base = (int64_t)block.x * 128;
+  const int64_t boff = (int64_t)block.z * rows * cols;
   const __nv_bfloat16* xb = x + boff;
   chain_start(first);
 
@@ -104,8 +104,8 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
     make_scale<MODE>(m, s_tile, stored);
     if (tid == 0) {
       const int64_t nrb = rows / 128, ncb = cols / 128;
-      if (OUT_N) scale[((int64_t)blockIdx.z * nrb + blockIdx.y) * ncb + blockIdx.x] = stored;
-      if (OUT_T) scale_t[((int64_t)blockIdx.z * ncb + blockIdx.x) * nrb + blockIdx.y] = stored;
+      if (OUT_N) scale[((int64_t)block.z * nrb + block.y) * ncb + block.x] = stored;
+      if (OUT_T) scale_t[((int64_t)block.z * ncb + block.x) * nrb + block.y] = stored;
     }
   } else if (GRAN == I8L_GRAN_GROUP128 && OUT_N) {
 #pragma unroll
@@ -119,7 +119,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
         make_scale<MODE>(m, s_row[it][i], stored);
         if (cc == 0) {
           const int r = 16 * w + 8 * it + 4 * half + i;
-          scale[((int64_t)blockIdx.z * rows + r_base + r) * (cols / 128) + blockIdx.x] = stored;
+          scale[((int64_t)block.z * rows + r_base + r) * (cols / 128) + block.x] = stored;
         }
       }
   } else {  // column scales
@@ -155,8 +155,8 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
       make_scale<MODE>(m, s, stored);
       s_cols[tid] = s;
       if (GRAN == I8L_GRAN_GROUP128)
-        scale_t[((int64_t)blockIdx.z * cols + c_base + tid) * (rows / 128) + blockIdx.y] = stored;
-      else if (blockIdx.y == 0)
+        scale_t[((int64_t)block.z * cols + c_base + tid) * (rows / 128) + block.y] = stored;
+      else if (block.y == 0)
         scale_t[c_base + tid] = stored;
     }
     __syncthreads();
@@ -213,6 +213,13 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
     }
   }
   chain_wait();
+}
+template <int GRAN, int MODE, bool OUT_N, bool OUT_T>
+__global__ void __launch_bounds__(256, 4)
+quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
+                  int8_t* __restrict__ q, float* __restrict__ scale, int8_t* __restrict__ qt,
+                  float* __restrict__ scale_t, const float* __restrict__ colmax, int first) {
+  quant_tile_body<GRAN, MODE, OUT_N, OUT_T>(dim3(blockIdx.x, blockIdx.y, blockIdx.z), x, rows, cols, q, scale, qt, scale_t, colmax, first);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -616,12 +623,12 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __re
 // caches, and rows of 4096 elements do not leave half of a CTA idle.  Bound by HBM.  [11008, 4096] 39 -> 29 us,
 // [4096, 4096] 19.5 -> 15.4, [28672, 8192] 115.6 -> 109.4 (6.4 TB/s) against two sweeps by one CTA per row.
 template <int MODE, int T>
-__global__ void __launch_bounds__(256)
-quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
+__device__ __forceinline__ void
+quant_row_cached_body(unsigned block, const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
                         float* __restrict__ scale, int first) {
   __shared__ float s_red[8];
   const int tid = threadIdx.x, l = tid & 31, t = tid & (T - 1);
-  const int64_t row = (int64_t)blockIdx.x * (256 / T) + tid / T;
+  const int64_t row = (int64_t)block * (256 / T) + tid / T;
   const bool live = row < rows;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
   const int nchunks = live ? (int)(cols / 8) : 0;
@@ -662,6 +669,12 @@ quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64
   for (int i = 0; i < 8; ++i)
     if (i * T + t < nchunks) qr[i * T + t] = finite ? quant_piece_finite<MODE>(cache[i], s) : quant_piece<MODE>(cache[i], s);
   chain_wait();
+}
+template <int MODE, int T>
+__global__ void __launch_bounds__(256)
+quant_row_cached_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, int8_t* __restrict__ q,
+                        float* __restrict__ scale, int first) {
+  quant_row_cached_body<MODE, T>(blockIdx.x, x, rows, cols, q, scale, first);
 }
 
 // The same with the 128-point rotation.  A CTA takes as many whole rows as fit into 128 groups of 128 elements,
@@ -713,6 +726,37 @@ quant_row_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int grou
                          q + (row0 * groups + 32 * w) * 128, 128, left);
   }
   chain_wait();
+}
+
+// ------------------------------------------------------------------------------------------------
+// Two quantizers in one launch, for operands so small that the launch itself counts (quant_pair): blocks below `split` run the
+// first, the others the second.
+// ------------------------------------------------------------------------------------------------
+struct PairArgs {
+  const __nv_bfloat16* x;
+  int64_t batch, rows, cols;
+  int8_t *q, *qt;
+  float *scale, *scale_t;
+};
+template <int GRAN, int MODE, bool OUT_T> struct TileQuant {
+  static unsigned blocks(const PairArgs& a) { return (unsigned)(a.batch * (a.rows / 128) * (a.cols / 128)); }
+  static __device__ __forceinline__ void run(const PairArgs& a, unsigned id, int first) {
+    const unsigned nx = (unsigned)(a.cols / 128), ny = (unsigned)(a.rows / 128);
+    const dim3 block(id % nx, id / nx % ny, id / nx / ny);
+    quant_tile_body<GRAN, MODE, true, OUT_T>(block, a.x, a.rows, a.cols, a.q, a.scale, a.qt, a.scale_t, nullptr, first);
+  }
+};
+template <int MODE, int T> struct RowQuant {   // rows of at most 64 T elements
+  static unsigned blocks(const PairArgs& a) { return (unsigned)((a.batch * a.rows + 256 / T - 1) / (256 / T)); }
+  static __device__ __forceinline__ void run(const PairArgs& a, unsigned id, int first) {
+    quant_row_cached_body<MODE, T>(id, a.x, a.batch * a.rows, a.cols, a.q, a.scale, first);
+  }
+};
+template <typename A, typename B>
+__global__ void __launch_bounds__(256, 4)
+quant_pair_kernel(const PairArgs a, const PairArgs b, unsigned split, int first) {
+  if (blockIdx.x < split) A::run(a, blockIdx.x, first);
+  else B::run(b, blockIdx.x - split, first);
 }
 
 // Whole-row rotation of rows of G groups of 128 (G = 2..128).  A CTA takes 128/G whole rows.  Spans 1..64 run in
@@ -1010,6 +1054,55 @@ static int dispatch_tile(const void* x, int64_t batch, int64_t rows, int64_t col
 }  // namespace i8l
 
 using namespace i8l;
+
+namespace i8l {
+template <typename A, typename B>
+static int launch_pair(const PairArgs& a, const PairArgs& b, cudaStream_t st) {
+  const unsigned split = A::blocks(a);
+  const cudaError_t e = launch(quant_pair_kernel<A, B>, dim3(split + B::blocks(b)), 256, 0, st, a, b, split, chain_first());
+  return e == cudaSuccess ? 1 : fail(I8L_ERR_CUDA, "quant_pair: %s", cudaGetErrorString(e));
+}
+
+// Both operands of a product in one launch.  1: done, 0: not a pair that this takes, < 0: an error.  It pays where a call is
+// bound by its launches: M, N, K 128, 1024, 1024 forward 15.5 -> 13.0 us, 512, 1024, 1024 11.3 -> 9.4, 1024, 2048, 1024
+// 11.4 -> 10.3 a call; 1024, 1024, 2048 12.0 -> 11.8; 2048, 2048, 1024 12.7 -> 12.9; 1024, 1024, 3072 14.8 -> 15.2; 2048,
+// 1536, 2048 16.7 -> 17.3.  The line lies at 1.5 M elements.
+int quant_pair(const void* a, int64_t a_batch, int64_t a_rows, int a_gran, int8_t* aq, float* as, int8_t* aqt, float* ast, const void* b,
+               int64_t b_batch, int64_t b_rows, int b_gran, int8_t* bq, float* bs, int64_t cols, int qmode, int hadamard,
+               cudaStream_t st) {
+  constexpr int64_t MOST = 3ll << 19;
+  if (hadamard != I8L_HAD_NONE || cols > 4096 || a_batch * a_rows * cols > MOST || b_batch * b_rows * cols > MOST || !a || !b || !aligned16(a) || !aligned16(b) ||
+      !aligned16(aqt))
+    return 0;
+  if (int e = check_arch()) return e;
+  const PairArgs pa{static_cast<const __nv_bfloat16*>(a), a_batch, a_rows, cols, aq, aqt, as, ast};
+  const PairArgs pb{static_cast<const __nv_bfloat16*>(b), b_batch, b_rows, cols, bq, nullptr, bs, nullptr};
+  const bool t = aqt != nullptr;
+#define I8L_PAIR(...) return launch_pair<__VA_ARGS__>(pa, pb, st)
+#define I8L_TILE_ROW(G, Mo, TT)                                                               \
+  if (a_gran == G && b_gran == I8L_GRAN_ROW && qmode == Mo && t == TT) {                      \
+    if (cols <= 2048) I8L_PAIR(TileQuant<G, Mo, TT>, RowQuant<Mo, 32>);                \
+    I8L_PAIR(TileQuant<G, Mo, TT>, RowQuant<Mo, 64>);                                  \
+  }
+  I8L_TILE_ROW(I8L_GRAN_TILE128, I8L_QMODE_TRITON, false)
+  I8L_TILE_ROW(I8L_GRAN_TILE128, I8L_QMODE_TRITON, true)
+  I8L_TILE_ROW(I8L_GRAN_GROUP128, I8L_QMODE_RNE, false)
+  if (t) return 0;
+  if (a_gran == I8L_GRAN_ROW && b_gran == I8L_GRAN_ROW && qmode == I8L_QMODE_ROWRCP) {
+    if (cols <= 2048) I8L_PAIR(RowQuant<I8L_QMODE_ROWRCP, 32>, RowQuant<I8L_QMODE_ROWRCP, 32>);
+    I8L_PAIR(RowQuant<I8L_QMODE_ROWRCP, 64>, RowQuant<I8L_QMODE_ROWRCP, 64>);
+  }
+#define I8L_TILE_TILE(G, H, Mo) \
+  if (a_gran == G && b_gran == H && qmode == Mo) I8L_PAIR(TileQuant<G, Mo, false>, TileQuant<H, Mo, false>);
+  I8L_TILE_TILE(I8L_GRAN_TILE128, I8L_GRAN_TILE128, I8L_QMODE_TRITON)
+  I8L_TILE_TILE(I8L_GRAN_TILE128, I8L_GRAN_TILE128, I8L_QMODE_FUSED)
+  I8L_TILE_TILE(I8L_GRAN_TILE128, I8L_GRAN_GROUP128, I8L_QMODE_FUSED)
+#undef I8L_TILE_TILE
+#undef I8L_TILE_ROW
+#undef I8L_PAIR
+  return 0;
+}
+}  // namespace i8l
 
 extern "C" const char* i8l_last_error(void) { return g_err; }
 extern "C" int i8l_version(void) { return 100; }
