@@ -30,6 +30,8 @@ int quant_pair(const void* a, int64_t a_batch, int64_t a_rows, int a_gran, int8_
 int col_sum(const void* x, int64_t rows, int64_t cols, void* out, cudaStream_t st);
 // Clears n floats; in a chain the next kernel waits for it before anything else.
 int clear(float* ptr, int64_t n, cudaStream_t st);
+// Whether the next one keeps a column on chip, and needs no maxima in memory.
+bool col_t_in_one_pass(int64_t rows, bool rot);
 // i8l_quant_col_t (rot = false) or i8l_quant_col_t_rot; zeroed: colmax is zero already.
 int quant_col_t(const char* name, const void* x, int64_t rows, int64_t cols, int qmode, bool rot, int8_t* qt, float* scale_t,
                 float* colmax, bool zeroed, cudaStream_t st);

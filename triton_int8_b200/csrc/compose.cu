@@ -138,7 +138,7 @@ extern "C" int i8l_linear_backward_bias(const void* dy, const void* w, const int
   const LaunchChain chain(static_cast<cudaStream_t>(stream));
   // The column maxima of W start from zeros; cleared up front, where no other pass needs the scratch, the first maximum
   // pass does not have to wait for it.
-  const bool zeroed = dx && !whole_k;
+  const bool zeroed = dx && !whole_k && !col_t_in_one_pass(N, hadamard == I8L_HAD_128);
   if (zeroed) {
     if (int e = check_arch()) return e;
     if (int e = clear(colmax, K, static_cast<cudaStream_t>(stream))) return e;
