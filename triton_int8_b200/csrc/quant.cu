@@ -1368,7 +1368,8 @@ static int launch_col_t(const void* x, int64_t rows, int64_t cols, bool rot, int
 namespace i8l {
 bool col_t_in_one_pass(int64_t rows, bool rot) { return !rot && rows <= 8 * 4 * 128; }
 int col_sum(const void* x, int64_t rows, int64_t cols, void* out, cudaStream_t st) {
-  if (int e = check_dims(1, rows, cols)) return e;
+  if (rows <= 0 || cols <= 0 || rows % 128 || cols % 128 || cols / SUM_COLS > 0x7fffffffll)
+    return fail(I8L_ERR_SHAPE, "rows=%lld cols=%lld: positive multiples of 128", (long long)rows, (long long)cols);
   if (!x || !out) return fail(I8L_ERR_ARG, "null pointer");
   if (!aligned16(x)) return fail(I8L_ERR_ALIGN, "x must be 16-byte aligned");
   if (int e = check_arch()) return e;
