@@ -405,7 +405,7 @@ def main():
 
     from triton_int8_b200.linear import Int8Config
     cfg = Int8Config(hadamard=had)
-    launches_per_step = 8   # X, W, dY quantizers (one kernel each), W^T (column absmax + quantize), three GEMMs
+    launches_per_step = 9   # X, W, dY quantizers (one kernel each), W^T (clear, column absmax, quantize), three GEMMs
 
     def step(record=False):
         # forward
@@ -446,7 +446,7 @@ def main():
             gemm_events.append(e)
         return y, dx, dw
 
-    # The step (8 launches, plus the reduce-scatter when sharded) is captured once into a CUDA graph and the
+    # The step (9 launches, plus the reduce-scatter when sharded) is captured once into a CUDA graph and the
     # timed region replays it, at every GPU count alike: launches issued while nvidia-smi samples the clocks
     # wait on the driver (stalls of 40-180 ms inside single steps were seen), which a replay avoids, and 1 GPU
     # and 8 GPUs are timed in the same mode.  The same K steps are timed launch by launch right afterwards

@@ -151,3 +151,25 @@ def test_threads_with_streams_of_their_own():
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not bad
+
+
+def test_outputs_without_gradients_are_views_as_in_the_python_path():
+    """An in-place operation that would need gradients through the output is refused by both paths."""
+    lin = _layer({}).requires_grad_(False)
+    x = torch.randn(128, 256, device=DEV).to(torch.bfloat16)
+    p = torch.ones(384, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    for f in (lin, lambda t: _python(lin, t)):
+        y = f(x)
+        y.add_(1)
+        with pytest.raises(RuntimeError):
+            y.add_(p)
+        with torch.no_grad():
+            f(x).add_(1)
+
+
+def test_traced_module_records_the_python_function():
+    lin = _layer({})
+    x = torch.randn(128, 256, device=DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        graph = str(torch.jit.trace(lin, x, check_trace=False).graph)
+    assert "Int8LinearFn" in graph

@@ -77,7 +77,9 @@ struct LaunchChain {
     // while a stream is captured, the first kernel depends on whatever precedes it in full: the graph's edges into it
     // may come from other things than one kernel
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool plain = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    const bool unknown = cudaStreamIsCapturing(st, &cap) != cudaSuccess;
+    if (unknown) (void)cudaGetLastError();   // the legacy stream while another one is captured: the launches report it
+    const bool plain = unknown || cap != cudaStreamCaptureStatusNone;
     chain_state = ChainState{true, !plain, 1, 0};
   }
   ~LaunchChain() { chain_state = ChainState{}; }

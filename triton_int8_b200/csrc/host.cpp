@@ -294,8 +294,10 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const bool grad = at::GradMode::is_enabled();
     if (grad && (x.requires_grad() || weight.requires_grad() || (bias && bias->requires_grad())))
       y = Int8LinearNode::apply(x, weight, bias, c.code(), weight.requires_grad());
-    else
+    else {
+      const at::AutoGradMode off(false);   // as inside the node: a view made here is one made without gradients
       y = linear_forward(x, weight, bias ? &*bias : nullptr, c, nullptr);
+    }
   }
   return THPVariable_Wrap(y);
   END_HANDLE_TH_ERRORS
