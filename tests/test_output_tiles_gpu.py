@@ -79,3 +79,27 @@ def test_narrow_tiles_equal_wide_ones(kind, B, M, N, Kd):
     torch.cuda.synchronize()
     assert torch.equal(narrow, wide)
     K.check_status(DEV)
+
+
+@pytest.mark.parametrize("b_kind", ["tile", "group"])
+@pytest.mark.parametrize("B,M,N,Kd", [(1, 128, 128, 128), (2, 256, 640, 384), (1, 4992, 1664, 256)])   # grids of any other kind's narrow tiles, then of wide ones
+def test_divisors_per_row_of_a_take_wide_tiles_at_any_size(b_kind, B, M, N, Kd):
+    """Divisors with a scale per row and K block of A have no kernel of their own: the generic kind takes them, which has
+    wide tiles only.  Each K block costs three fp32 roundings (product of the scales, division, sum), the end one more."""
+    g = torch.Generator().manual_seed(M + N + Kd)
+    kb = Kd // 128
+    a = torch.randint(-127, 128, (B, M, Kd), generator=g, dtype=torch.int8)
+    b = torch.randint(-127, 128, (N, Kd), generator=g, dtype=torch.int8)
+    a_s = torch.rand(B, M, kb, generator=g) + 0.5
+    b_s = torch.rand(*{"tile": (N // 128, kb), "group": (N, kb)}[b_kind], generator=g) + 0.5
+    fb = (b_s.repeat_interleave(128, 0) if b_kind == "tile" else b_s).double().to(DEV)
+    ref, mag = torch.zeros(B, M, N, dtype=torch.double, device=DEV), torch.zeros(B, M, N, dtype=torch.double, device=DEV)
+    for k in range(kb):
+        cut = slice(k * 128, (k + 1) * 128)
+        term = a[:, :, cut].to(DEV).double() @ b[:, cut].to(DEV).double().t() / (a_s[:, :, k, None].to(DEV).double() * fb[:, k])
+        ref += term
+        mag += term.abs()
+    out = K.gemm_block(a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV), L.ASCALE_GROUP,
+                       {"tile": L.BSCALE_TILE, "group": L.BSCALE_GROUP}[b_kind], flags=L.GEMM_DIVIDE | L.GEMM_OUT_F32)
+    K.check_status(DEV)
+    assert ((out.double() - ref).abs() <= (3 * kb + 1) * 2.0 ** -24 * mag).all()

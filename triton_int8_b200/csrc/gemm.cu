@@ -88,7 +88,7 @@ struct GemmParams {
   int32_t* mirror;   // pinned host memory that follows the status word (i8l_status_mirror), or null
   int m_blocks;  // batch*M/128
   int mpb;       // M/128 (m-blocks per batch)
-  int n_tiles;   // ceil(N/256)
+  int n_tiles;   // ceil(N / columns of a tile)
   int M, N, KB;  // KB = K/128
   int a_kind, b_kind, b_batched;
   int exact, divide, out_f32, dump;  // dump: 0 none, 1 whole-K int32, 2 per-K-block int32
@@ -1227,13 +1227,21 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   if (!a_q || !b_q || !p.c) return fail(I8L_ERR_ARG, "null pointer");
   if (!aligned16(a_q) || !aligned16(b_q) || !aligned16(p.c)) return fail(I8L_ERR_ALIGN, "a_q, b_q, c must be 16-byte aligned");
   if (int e = check_arch()) return e;
+  // One factor per (row or tile, K block) and 128 columns.  Divisors (fused backward, per-tile A scales only) take the
+  // exact conversion of the row kind: the fast kind's running shift rounds to about 7e-6, the fused variants are held
+  // to 1e-6.
+  const bool a_group = p.a_kind == I8L_ASCALE_GROUP, b_group = p.b_kind == I8L_BSCALE_GROUP;
+  const bool factors = block && !p.exact && !p.dump;
+  const bool scalar_factor = factors && !b_group && (!p.divide || !a_group);
+  const bool column_factor = factors && !a_group && b_group;
+  const bool outer_factor = factors && !p.divide && a_group && b_group;
+  const bool generic = block && !scalar_factor && !column_factor && !outer_factor;   // this kind has wide tiles only
+  const int64_t m_blocks = batch * M / 128, wide_tiles = (N + WIDE - 1) / WIDE;
+  const int percent = !block ? 80 : outer_factor ? 67 : 62;
+  const bool narrow = !generic && narrow_tiles(m_blocks * wide_tiles, m_blocks * (N / NARROW), gemm_cta_budget(), percent);
   // CTA pairs (cta_group::2) need two 128-row blocks of the same batch per tile.  They pay off for the
   // whole-K accumulation (half the B traffic per SM: +2.5 % sustained at the power cap); the per-K-block
   // hand-off of the block-scaled kinds is slower across two CTAs (990 vs 1510 TOP/s), so those stay 1-CTA.
-  const bool exact_path = block && (p.exact || p.dump);   // the generic kind has wide tiles only
-  const int64_t m_blocks = batch * M / 128, wide_tiles = (N + WIDE - 1) / WIDE;
-  const int percent = !block ? 80 : (p.a_kind == I8L_ASCALE_GROUP && p.b_kind == I8L_BSCALE_GROUP ? 67 : 62);
-  const bool narrow = !exact_path && narrow_tiles(m_blocks * wide_tiles, m_blocks * (N / NARROW), gemm_cta_budget(), percent);
   const bool two = !block && !narrow && (M % 256 == 0);
   const int BN = narrow ? NARROW : WIDE;
   (void)chain_first();   // GEMMs always wait
@@ -1274,22 +1282,16 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
     p.per_batch.set(p.mpb);
   }
   const int64_t tiles = (int64_t)(two ? p.m_blocks / 2 : p.m_blocks) * p.n_tiles;
-  // One factor per (row or tile, K block) and 128 columns.  Divisors (fused backward, per-tile A scales only) take the
-  // exact conversion of the row kind: the fast kind's running shift rounds to about 7e-6, the fused variants are held
-  // to 1e-6.
-  const bool scalar_factor = block && !exact_path && p.b_kind != I8L_BSCALE_GROUP && (!p.divide || p.a_kind == I8L_ASCALE_TILE);
-  const bool column_factor = block && !exact_path && p.a_kind == I8L_ASCALE_TILE && p.b_kind == I8L_BSCALE_GROUP;
-  const bool outer_factor = block && !exact_path && !p.divide && p.a_kind == I8L_ASCALE_GROUP && p.b_kind == I8L_BSCALE_GROUP;
 #define I8L_KIND(K) \
   (narrow ? launch_kind<K, false, NARROW>(ma, mb, mc, p, tiles, st) : launch_kind<K, false, WIDE>(ma, mb, mc, p, tiles, st))
   if (!block) return two ? launch_kind<K_ROWCOL, true, WIDE>(ma, mb, mc, p, tiles, st) : I8L_KIND(K_ROWCOL);
-  if (scalar_factor && p.a_kind == I8L_ASCALE_TILE && !p.divide) return I8L_KIND(K_BLOCK_FAST);
+  if (generic) return launch_kind<K_BLOCK_GEN, false, WIDE>(ma, mb, mc, p, tiles, st);
+  if (scalar_factor && !a_group && !p.divide) return I8L_KIND(K_BLOCK_FAST);
   if (scalar_factor && p.divide) return I8L_KIND(K_BLOCK_TILEDIV);
   if (scalar_factor) return I8L_KIND(K_BLOCK_ROWFAC);
   if (outer_factor) return I8L_KIND(K_BLOCK_OUTER);
-  if (column_factor) return I8L_KIND(K_BLOCK_COLFAC);
+  return I8L_KIND(K_BLOCK_COLFAC);
 #undef I8L_KIND
-  return launch_kind<K_BLOCK_GEN, false, WIDE>(ma, mb, mc, p, tiles, st);
 }
 
 }  // namespace i8l
