@@ -1,6 +1,6 @@
 """The kernels of one composed call overlap on the device (programmatic serialization).  Many calls in a row, each on
 other inputs and all in the same recycled memory, equal the separate steps, which are launched one after the other, bit
-for bit; so does a replayed graph."""
+for bit; so does a replayed graph, and so do calls whose operands the kernels right in front of them write."""
 import pytest
 import torch
 
@@ -80,3 +80,43 @@ def test_chain_in_a_graph_equals_separate_steps():
         torch.cuda.synchronize()
         for got, want in zip(out, ref):
             assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("cfg", [dict(), dict(hadamard=128), dict(scaling="row128", round="rne"), dict(scaling="double_channel"),
+                                 dict(scaling="double_channel", hadamard=-1)], ids=str)
+@pytest.mark.parametrize("M", [128, 4096])
+def test_operands_written_by_the_kernel_in_front(cfg, M):
+    """An elementwise kernel writes the input, the weight or the output gradient right before the call, in place over the
+    previous call's values, and one layer's output is the next one's input: the results are those of synchronised calls."""
+    from triton_int8_b200.linear import Int8Linear
+    torch.manual_seed(M)
+    r = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16)
+    lins = [Int8Linear(a, b, device=DEV, config=Int8Config(**cfg)) for a, b in ((1024, 512), (512, 2048))]
+    xs, dys, ws = [r(M, 1024) for _ in range(3)], [r(M, 2048) for _ in range(3)], [r(2048, 512) * 0.02 for _ in range(3)]
+    x, dy = torch.zeros_like(xs[0]).requires_grad_(True), torch.zeros_like(dys[0])
+
+    def step(k, sync):
+        wait = torch.cuda.synchronize if sync else lambda: None
+        with torch.no_grad():
+            torch.mul(ws[k], 1, out=lins[1].weight)
+            torch.mul(xs[k], 1, out=x)
+        wait()
+        h = lins[0](x)
+        wait()
+        y = lins[1](h)
+        wait()
+        torch.mul(dys[k], 1, out=dy)
+        wait()
+        grads = torch.autograd.grad(y, [x, *lins[0].parameters(), *lins[1].parameters()], dy)
+        wait()
+        return [y.detach(), *grads]
+
+    refs = [step(k, True) for k in range(3)]
+    outs = []
+    for k in range(24):
+        outs.append(step(k % 3, False))
+        if len(outs) == 6:
+            torch.cuda.synchronize()
+            for j, out in enumerate(outs):
+                assert all(torch.equal(got, ref) for got, ref in zip(out, refs[(k - 5 + j) % 3])), f"call {k - 5 + j}"
+            outs = []

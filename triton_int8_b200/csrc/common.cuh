@@ -65,6 +65,20 @@ __device__ __forceinline__ void chain_start(int first) {
   chain_trigger();
 }
 
+// How the kernels of a chain read tensors and scales.  A kernel ahead in the stream may write that memory while this grid is
+// resident already, so it is no read-only memory in PTX's sense (ld.global.nc, __ldg), whose loads may move ahead of the wait; an
+// ordinary load is ordered by it.  volatile as the wait is, so that the compiler keeps the order too.
+__device__ __forceinline__ uint4 chain_load(const uint4* ptr) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(ptr));
+  return v;
+}
+__device__ __forceinline__ float chain_load(const float* ptr) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(ptr));
+  return v;
+}
+
 // This host thread's chain.
 struct ChainState {
   bool active, attribute;   // a chain is being launched; its next kernel may start ahead of its predecessor's end

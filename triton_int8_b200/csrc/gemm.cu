@@ -277,14 +277,6 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
   else columns(std::false_type{});
 }
 
-// Scales, written by the kernel in front of this one in a chain: volatile, so that the compiler keeps the load behind
-// chain_wait (it may move a __ldg ahead of it).  Ordinary loads: row x column factors, 4096^3, 134 -> 142 us.
-__device__ __forceinline__ float ld_scale(const float* ptr) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(ptr));
-  return v;
-}
-
 template <int KIND, bool TWO, int BN>
 __global__ void __launch_bounds__(128 + 32 * EPI_WARPS_OF<KIND>, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -516,9 +508,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             break;
           }
           auto factor = [&](int h, int d) {
-            const float a = ld_scale(as_ptr + (d >> p.a_kshift));
+            const float a = chain_load(as_ptr + (d >> p.a_kshift));
             if (chan || tc.n_tile * BN + h * 128 >= p.N) return a;   // no second half: a number that does no harm
-            return a * (ld_scale(p.b_scale + ((bcol0 >> 7) + h) * KB + d) * p.post_scale);
+            return a * (chain_load(p.b_scale + ((bcol0 >> 7) + h) * KB + d) * p.post_scale);
           };
           if (k0 == 0) {
             float m[2] = {0.f, 0.f};
@@ -593,7 +585,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int i = lane; i < BN; i += 32) {
               const int h = (chan || i < 128) ? 0 : 1, back = 149 - (h ? e[1] : e[0]);
               const float d = pow2f(back < 127 ? 0 : back - 127) * (h ? unit[1] : unit[0]);
-              ctl.fbscale[buf][i] = chan && tc.n_tile * BN + i < p.N ? ld_scale(p.b_scale + bcol0 + i) * p.post_scale * d : d;
+              ctl.fbscale[buf][i] = chan && tc.n_tile * BN + i < p.N ? chain_load(p.b_scale + bcol0 + i) * p.post_scale * d : d;
               if (p.bias) ctl.fbias[buf][i] = tc.n_tile * BN + i < p.N ? p.bias[tc.n_tile * BN + i] : __float2bfloat16_rn(0.f);
             }
 #pragma unroll
@@ -785,7 +777,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (chan || p.bias) {  // K-invariant column scales and bias of this group -> shared memory
         named_sync(1 + wg, 128);
         if (tix < EPI_COLS) {
-          if (chan) ctl.bscale[wg * EPI_COLS + tix] = active ? ld_scale(p.b_scale + bcol0 + tix) : 0.f;
+          if (chan) ctl.bscale[wg * EPI_COLS + tix] = active ? chain_load(p.b_scale + bcol0 + tix) : 0.f;
           if (p.bias) ctl.bias[wg * EPI_COLS + tix] = active ? p.bias[col0 + tix] : __float2bfloat16_rn(0.f);
         }
         named_sync(1 + wg, 128);
@@ -811,9 +803,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // column kind).  4096^3: row x channel 97.5 -> 92.3 us, row x tile 96.2 -> 88.8, column 129.6 -> 114.1, divisors 93.5 -> 90.7.
         float a_next, b_next = 1.f;
         auto load_scales = [&](int d) {
-          a_next = ld_scale(as_ptr + d);
-          if (COLF) b_next = publish ? ld_scale(bc_ptr + d) : 1.f;
-          else if (!chan && active) b_next = ld_scale(bt_ptr + d);
+          a_next = chain_load(as_ptr + d);
+          if (COLF) b_next = publish ? chain_load(bc_ptr + d) : 1.f;
+          else if (!chan && active) b_next = chain_load(bt_ptr + d);
         };
         asm volatile("" : "+l"(bc_ptr));   // kept in registers: recomputed in every K block otherwise (column kind 877 -> 851 us)
         float2 acc[EPI_COLS / 2];
@@ -905,15 +897,15 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int d = 0; d < ndrain; ++d) {
           float sa = 1.f, sb = 1.f;
           if (BLOCK && !p.dump) {
-            sa = p.a_kind == I8L_ASCALE_GROUP ? ld_scale(p.a_scale + row * KB + d)
-                                              : ld_scale(p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift) + (d >> p.a_kshift));
-            if (p.b_kind == I8L_BSCALE_TILE && active) sb = ld_scale(p.b_scale + (bcol0 >> 7) * KB + d);
+            sa = p.a_kind == I8L_ASCALE_GROUP ? chain_load(p.a_scale + row * KB + d)
+                                              : chain_load(p.a_scale + (int64_t)tc.m_blk * (KB >> p.a_kshift) + (d >> p.a_kshift));
+            if (p.b_kind == I8L_BSCALE_TILE && active) sb = chain_load(p.b_scale + (bcol0 >> 7) * KB + d);
             if (p.b_kind == I8L_BSCALE_GROUP) {
-              if (tix < EPI_COLS) ctl.bstep[d & 1][wg * EPI_COLS + tix] = active ? ld_scale(p.b_scale + (bcol0 + tix) * KB + d) : 0.f;
+              if (tix < EPI_COLS) ctl.bstep[d & 1][wg * EPI_COLS + tix] = active ? chain_load(p.b_scale + (bcol0 + tix) * KB + d) : 0.f;
               named_sync(1 + wg, 128);
             }
           }
-          const float sar = !BLOCK && !p.dump ? ld_scale(p.a_scale + row) : 0.f;
+          const float sar = !BLOCK && !p.dump ? chain_load(p.a_scale + row) : 0.f;
           ok = ok && __all_sync(0xffffffffu, mbar_wait<!BLOCK>(smem_u32(&ctl.tfull[ab]), aph, abort_flag, p.max_polls));   // per warp: what follows synchronises it
           tc_fence_after();
           const bool live = ok && active;

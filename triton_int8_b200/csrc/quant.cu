@@ -78,7 +78,7 @@ quant_tile_body(const dim3 block, const __nv_bfloat16* __restrict__ x, int64_t r
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = 16 * w + 8 * it + 4 * half + i;
-      raw[it][i] = __ldg(reinterpret_cast<const uint4*>(xb + (r_base + r) * cols + c_base + 8 * cc));
+      raw[it][i] = chain_load(reinterpret_cast<const uint4*>(xb + (r_base + r) * cols + c_base + 8 * cc));
     }
 
   // ---- scales
@@ -149,7 +149,7 @@ quant_tile_body(const dim3 block, const __nv_bfloat16* __restrict__ x, int64_t r
         for (int k = 1; k < 8; ++k) m = fmaxf(m, s_colred[k * 128 + tid]);
       } else {
         chain_wait();
-        m = __ldcg(colmax + c_base + tid);
+        m = chain_load(colmax + c_base + tid);
       }
       float s, stored;
       make_scale<MODE>(m, s, stored);
@@ -240,7 +240,7 @@ quant_tile256_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t 
   __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    raw[i] = __ldg(reinterpret_cast<const uint4*>(x + boff + (r_base + 16 * w + i) * cols + c_base + 8 * l));
+    raw[i] = chain_load(reinterpret_cast<const uint4*>(x + boff + (r_base + 16 * w + i) * cols + c_base + 8 * l));
     m2 = absmax8(raw[i], m2);
   }
   float m = hmax_of(m2);
@@ -427,7 +427,7 @@ quant_tile_rot_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t
     }
     if (GRAN == GRAN_COLFULL) {
       chain_wait();
-      m = __ldcg(colmax + c_base + tid);
+      m = chain_load(colmax + c_base + tid);
     }
     make_scale<MODE>(m, s, stored);
     const int64_t o_base = ph == 0 ? r_base : c_base, k_base = ph == 0 ? c_base : r_base;  // output row, contraction axis
@@ -459,7 +459,7 @@ col_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t col
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = 16 * w + 8 * it + 4 * half + i;
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + (r_base + r) * cols + c_base + 8 * cc));
+      const uint4 u = chain_load(reinterpret_cast<const uint4*>(x + (r_base + r) * cols + c_base + 8 * cc));
       float v[8];
       unpack8(u, v);
 #pragma unroll
@@ -524,7 +524,7 @@ quant_col_strip_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_
 #pragma unroll
   for (int b = 0; b < BLOCKS; ++b)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) raw[b][i] = b < mine ? __ldg(src + (b * 128 + i) * (cols / 8)) : make_uint4(0, 0, 0, 0);
+    for (int i = 0; i < 4; ++i) raw[b][i] = b < mine ? chain_load(src + (b * 128 + i) * (cols / 8)) : make_uint4(0, 0, 0, 0);
   // column maxima, with and without NaNs
   __nv_bfloat162 any = __floats2bfloat162_rn(0.f, 0.f), m[4];
 #pragma unroll
@@ -633,7 +633,7 @@ col_sum_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols, 
     for (; r0 < stop; r0 += 128) {
       float v[4][8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) unpack8(__ldg(src + (r0 + 32 * i + r) * (cols / 8)), v[i]);
+      for (int i = 0; i < 4; ++i) unpack8(chain_load(src + (r0 + 32 * i + r) * (cols / 8)), v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) sum[j] += (v[0][j] + v[1][j]) + (v[2][j] + v[3][j]);
     }
@@ -693,7 +693,7 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __re
   for (int base = 0; base < nchunks; base += 256) {
     const int ch = base + tid;
     float v[8];
-    if (ch < nchunks) unpack8(__ldg(xr + ch), v);
+    if (ch < nchunks) unpack8(chain_load(xr + ch), v);
     else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = 0.f;
@@ -721,7 +721,7 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8_t* __re
   for (int base = 0; base < nchunks; base += 256) {
     const int ch = base + tid;
     float v[8];
-    if (ch < nchunks) unpack8(__ldg(xr + ch), v);
+    if (ch < nchunks) unpack8(chain_load(xr + ch), v);
     else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = 0.f;
@@ -758,7 +758,7 @@ quant_row_cached_body(unsigned block, const __nv_bfloat16* __restrict__ x, int64
   chain_start(first);
   uint4 cache[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) cache[i] = i * T + t < nchunks ? __ldg(xr + i * T + t) : make_uint4(0, 0, 0, 0);
+  for (int i = 0; i < 8; ++i) cache[i] = i * T + t < nchunks ? chain_load(xr + i * T + t) : make_uint4(0, 0, 0, 0);
   __nv_bfloat162 hm = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -1043,7 +1043,7 @@ quant_row_hadfull_kernel(const __nv_bfloat16* __restrict__ x, int64_t cols, int8
   for (int base = 0; base < nchunks; base += 256) {
     const int ch = base + tid;
     float v[8];
-    if (ch < nchunks) unpack8(__ldg(xr + ch), v);
+    if (ch < nchunks) unpack8(chain_load(xr + ch), v);
     else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = 0.f;
