@@ -74,6 +74,24 @@ def test_product_calls_validate_before_any_launch(lib):
     assert backward(gran=5, ws_bytes=1 << 20) == -6 and backward(x_qt=None, ws_bytes=1 << 20) == -6
 
 
+@pytest.mark.parametrize("off", [1, 4, 8])
+def test_product_calls_refuse_a_workspace_off_its_alignment(lib, off):
+    """... before any launch, whichever kernels would write to it: small operands share a launch, long columns have their
+    maxima cleared first, the bias gradient comes first.  No device here: what passes the checks ends in another error."""
+    buf = ctypes.create_string_buffer(1 << 12)
+    p = ctypes.addressof(buf); p += (256 - p % 256) % 256
+    for gran, b_gran, qmode in ((0, 2, 0), (1, 2, 1), (2, 2, 3), (0, 0, 0), (5, 2, 0)):
+        for M in (128, 65536):
+            for a_qt in (None, p) if b_gran == 2 and gran != 5 else (None,):
+                assert lib.i8l_quant_gemm(p, p, None, p, a_qt, a_qt, 1, M, 256, 256, 0, gran, b_gran, qmode, 0, 1.0, 0, p + off,
+                                          1 << 40, None, None) == -2
+    for gran, qmode in ((0, 0), (1, 1), (2, 3)):
+        for N in (128, 8192):
+            for dx, dw, db in ((p, p, p), (p, None, None), (None, p, None), (p, p, None)):
+                assert lib.i8l_linear_backward_bias(p, p, p, p, dx, dw, db, 128, N, 128, gran, qmode, 0, 1.0, 1.0, 0, p + off,
+                                                    1 << 40, None, None) == -2
+
+
 @pytest.mark.parametrize("batch,M,N", [(65535, 128, 128), (70000, 128, 128), (131071, 128, 256), ((1 << 24) - 1, 128, 128)])
 def test_product_call_takes_the_batches_of_its_steps(lib, batch, M, N):
     """Per-row scales have no limit on the batch of their own: the quantizer and the GEMM take batch * M below 2^31.  The

@@ -79,6 +79,7 @@ extern "C" int i8l_quant_gemm(const void* a, const void* b, const void* bias, vo
   float* bs = ws.take<float>(scale_count(b_gran, b_n, N, K));
   float* colmax = a_qt && a_gran == I8L_GRAN_ROW ? ws.take<float>(K) : nullptr;
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_quant_gemm: workspace of %lld bytes is too small", (long long)workspace_bytes);
+  if (!aligned16(workspace)) return fail(I8L_ERR_ALIGN, "i8l_quant_gemm: the workspace must be aligned");   // every piece then is
   const LaunchChain chain(static_cast<cudaStream_t>(stream));
   if (colmax) {   // ahead of the GEMM, while A is in L2
     if (int e = quant_col_t(a, M, K, qmode, hadamard, a_qt, a_st, colmax, false, stream)) return e;
@@ -135,6 +136,7 @@ extern "C" int i8l_linear_backward_bias(const void* dy, const void* w, const int
   }
   float* colmax = ws.take<float>(K > N ? K : N);
   if (ws.short_of_space) return fail(I8L_ERR_ARG, "i8l_linear_backward: workspace of %lld bytes is too small", (long long)workspace_bytes);
+  if ((dx || dw) && !aligned16(workspace)) return fail(I8L_ERR_ALIGN, "i8l_linear_backward: the workspace must be aligned");
   const LaunchChain chain(static_cast<cudaStream_t>(stream));
   // The column maxima of W start from zeros; cleared up front, where no other pass needs the scratch, the first maximum
   // pass does not have to wait for it.
