@@ -120,3 +120,30 @@ def test_operands_written_by_the_kernel_in_front(cfg, M):
             for j, out in enumerate(outs):
                 assert all(torch.equal(got, ref) for got, ref in zip(out, refs[(k - 5 + j) % 3])), f"call {k - 5 + j}"
             outs = []
+
+
+def test_a_cta_limit_keeps_sms_free_inside_a_call():
+    """Under a limit the backward call's second GEMM does not sit on the free SMs while the first one runs: short kernels on
+    another stream, one after the other, are done long before the first GEMM, half of the call's time."""
+    from triton_int8_b200 import kernels as K
+    x, w, dy, _ = _inputs((16384, 8192, 16384), 1)[0]
+    saved = LN.linear_forward(x, w, None)[1]
+    side = torch.cuda.Stream()
+    ev = lambda: torch.cuda.Event(enable_timing=True)
+    share = []
+    for _ in range(3):
+        start, others, end = ev(), ev(), ev()
+        torch.cuda.synchronize()
+        start.record()
+        side.wait_event(start)
+        with K.cta_limit(140):
+            LN.linear_backward(dy, w, saved)
+        end.record()
+        with torch.cuda.stream(side):
+            for _ in range(20):
+                torch.cuda._sleep(50_000)   # 25 to 40 us each
+            others.record()
+        torch.cuda.synchronize()
+        share.append(start.elapsed_time(others) / start.elapsed_time(end))
+    K.check_status(DEV)
+    assert min(share) < 0.4, share

@@ -55,7 +55,7 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 //   Quantizers behind it read the caller's inputs and write memory that no kernel of the chain reads or writes before them.
 //   They trigger first thing and wait at their end, so that "predecessor completed" covers the whole chain.
 //   Passes that need a predecessor's result (scales from a column maximum) and GEMMs wait behind their set-up, and a GEMM
-//   triggers only another GEMM, the rest starts when its blocks have ended; a kernel
+//   triggers only another GEMM, and none under a limit on its CTAs; the rest starts when its blocks have ended.  A kernel
 //   that clears memory for a later pass and the one behind it wait like a first one.
 // Outside a chain both instructions do nothing.
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

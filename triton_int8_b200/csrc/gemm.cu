@@ -1237,7 +1237,8 @@ static int launch_gemm(bool block, const int8_t* a_q, const int8_t* b_q, GemmPar
   const bool two = !block && !narrow && (M % 256 == 0);
   const int BN = narrow ? NARROW : WIDE;
   (void)chain_first();   // GEMMs always wait
-  p.early = chain_state.gemm_next;
+  // Not under a limit on the CTAs: those of the next GEMM would wait on the very SMs that the limit keeps free.
+  p.early = chain_state.gemm_next && gemm_cta_budget() == sm_count();
   chain_state.gemm_next = 0;
   CUtensorMap ma, mb, mc;
   if (int e = make_map(&ma, a_q, batch * M, K, BM)) return e;
