@@ -173,3 +173,30 @@ def test_traced_module_records_the_python_function():
     with torch.no_grad():
         graph = str(torch.jit.trace(lin, x, check_trace=False).graph)
     assert "Int8LinearFn" in graph
+
+
+@pytest.mark.parametrize("path", ["native", "python"])
+@pytest.mark.parametrize("off", [0, 1, 4])
+def test_bias_gradient_alone_takes_any_contiguous_gradient(path, off):
+    """With only the bias trainable no kernel but the sum reads the gradient: one that starts off a 16-byte boundary (a
+    slice of a larger buffer) is taken.  One rounding to bf16, behind at most 256 fp32 sums."""
+    lin = _layer({})
+    lin.weight.requires_grad_(False)
+    x = torch.randn(256, 256, device=DEV).to(torch.bfloat16)
+    dy = torch.randn(off + 256 * 384, device=DEV).to(torch.bfloat16)[off:].view(256, 384)
+    y = lin(x) if path == "native" else _python(lin, x)
+    y.backward(dy)
+    ref = dy.double().sum(0)
+    bound = ref.abs() * 2.0 ** -8 + dy.double().abs().sum(0) * 2.0 ** -24 * 256
+    assert ((lin.bias.grad.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("cfg,path", [({}, "native"), (dict(scaling="double_channel", hadamard=-1), "python")])
+def test_bias_gradient_alone_of_a_batch_of_gradients(cfg, path):
+    lin = _layer(cfg)
+    lin.weight.requires_grad_(False)
+    x = torch.randn(256, 256, device=DEV).to(torch.bfloat16)
+    dys = torch.randn(3, 256, 384, device=DEV).to(torch.bfloat16)
+    y = lin(x) if path == "native" else _python(lin, x)
+    db, = torch.autograd.grad(y, lin.bias, dys, is_grads_batched=True)
+    assert torch.equal(db, dys.sum(1))

@@ -211,8 +211,8 @@ void linear_backward(const Tensor& dy, const Tensor& weight, const Tensor& q, co
          s.scalar_type() == at::kFloat && q.is_contiguous() && s.is_contiguous() && q.sizes() == at::IntArrayRef({1, K, M}) &&
          s.numel() == scale_count(gran, 1, K, M);
   }
-  // torch's sum where its graph is wanted (create_graph)
-  const bool own_sum = need_db && ok && !at::GradMode::is_enabled();
+  // torch's sum where its graph is wanted (create_graph), and where the kernel's 16-byte loads do not fit
+  const bool own_sum = need_db && ok && !at::GradMode::is_enabled() && reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0;
   if (need_db && !own_sum) db = dy.sum(0);
   if (!ok) {
     if (need_dx || need_dw) backward_in_python(dy, weight, q, s, c, need_dx, need_dw, dx, dw);

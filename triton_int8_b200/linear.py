@@ -181,8 +181,10 @@ class Int8LinearFn(torch.autograd.Function):
         need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         dx, dw = linear_backward(dy2, weight, tuple(saved) if saved else None, ctx.cfg, need_dx, need_dw)
         db = None
-        if ctx.has_bias and ctx.needs_input_grad[2]:   # torch's sum where its graph is wanted
-            db = dy2.sum(0).to(dy.dtype) if torch.is_grad_enabled() else K.col_sum(dy2)
+        if ctx.has_bias and ctx.needs_input_grad[2]:
+            # torch's sum where its graph is wanted, under a transform, and where the kernel's 16-byte loads do not fit
+            own = not torch.is_grad_enabled() and torch._C._has_storage(dy2) and dy2.data_ptr() % 16 == 0
+            db = K.col_sum(dy2) if own else dy2.sum(0).to(dy.dtype)
         return (dx.view(ctx.x_shape) if dx is not None else None), dw, db, None, None
 
 
