@@ -200,3 +200,41 @@ def test_bias_gradient_alone_of_a_batch_of_gradients(cfg, path):
     y = lin(x) if path == "native" else _python(lin, x)
     db, = torch.autograd.grad(y, lin.bias, dys, is_grads_batched=True)
     assert torch.equal(db, dys.sum(1))
+
+
+FIRST_USE = """
+import threading
+import torch
+from triton_int8_b200 import _lib as L, kernels as K
+from triton_int8_b200.linear import Int8Linear
+lin = Int8Linear(256, 384, device="cuda").requires_grad_(False)
+x = torch.randn(128, 256, device="cuda").to(torch.bfloat16)
+torch.cuda.synchronize()
+start = threading.Barrier(8)
+ts = [threading.Thread(target=lambda: (start.wait(), lin(x))) for _ in range(8)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+torch.cuda.synchronize()
+lib = L.load()
+lib.i8l_test_set_wait_limit(256, 1)
+lin(x)
+torch.cuda.synchronize()
+lib.i8l_test_set_wait_limit(0, 0)
+try:
+    lin(x)
+except L.I8LError as e:
+    assert e.code == L.TIMEOUT
+else:
+    raise SystemExit("not reported")
+lin(x)
+K.check_status("cuda")
+"""
+
+
+def test_a_timeout_is_reported_once_after_a_first_use_by_several_threads():
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_USE], cwd=root, capture_output=True, text=True, timeout=240)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -63,7 +63,7 @@ class WithoutGil {
 
 struct Status {
   std::atomic<int32_t*> word{nullptr};
-  void* poller = nullptr;
+  std::atomic<void*> poller{nullptr};
 };
 constexpr int MAX_DEVICES = 64;
 std::array<Status, MAX_DEVICES> statuses;
@@ -78,7 +78,7 @@ Status& status_of(int dev) {
     const int ok = PyArg_ParseTuple(r, "KK", &word, &poller);
     Py_DECREF(r);
     if (!ok) throw_python_error();
-    s.poller = reinterpret_cast<void*>(poller);
+    s.poller.store(reinterpret_cast<void*>(poller), std::memory_order_relaxed);   // the same pair for every thread that comes here
     s.word.store(reinterpret_cast<int32_t*>(word), std::memory_order_release);
   }
   return s;
@@ -290,7 +290,7 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   {
     const WithoutGil no_gil;
     const int dev = x.get_device();
-    check("i8l_status_peek", lib_status_peek(status_of(dev).poller), dev);   // an earlier GEMM gave up a wait
+    check("i8l_status_peek", lib_status_peek(status_of(dev).poller.load(std::memory_order_relaxed)), dev);   // an earlier GEMM gave up a wait
     const bool grad = at::GradMode::is_enabled();
     if (grad && (x.requires_grad() || weight.requires_grad() || (bias && bias->requires_grad())))
       y = Int8LinearNode::apply(x, weight, bias, c.code(), weight.requires_grad());

@@ -2,6 +2,8 @@
 current CUDA stream.  These are the building blocks of the fwd_32 / bwd_33 variants."""
 from __future__ import annotations
 
+import threading
+
 import torch
 
 from . import _lib as L
@@ -36,6 +38,7 @@ def _call(name: str, dev: torch.device, *args, tensors=()) -> None:
 # from here.  check_status() reads it (synchronously); poll_status() is the cheap form for a training
 # loop: it looks at a copy started by the previous poll and starts the next one, never blocking.
 _STATUS: dict = {}
+_STATUS_LOCK = threading.Lock()   # one word per device, also when several threads come first
 
 
 class _StatusWord:
@@ -57,7 +60,10 @@ def _status_of(dev: torch.device) -> "_StatusWord":
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     st = _STATUS.get(key)
     if st is None:
-        st = _STATUS[key] = _StatusWord(torch.device("cuda", key))
+        with _STATUS_LOCK:
+            st = _STATUS.get(key)
+            if st is None:
+                st = _STATUS[key] = _StatusWord(torch.device("cuda", key))
     return st
 
 
