@@ -128,6 +128,49 @@ def test_a_gemm_that_gave_up_is_reported_by_the_next_forward():
     assert torch.equal(y, _python(lin, x))
 
 
+def _give_up(lin, x):
+    lib = L.load()
+    assert lib.i8l_test_set_wait_limit(256, 1) == 0
+    try:
+        lin(x)
+        torch.cuda.synchronize()
+    finally:
+        assert lib.i8l_test_set_wait_limit(0, 0) == 0
+
+
+def test_a_cleared_status_word_is_not_reported():
+    lin = _layer({})
+    x = torch.randn(128, 256, device=DEV).to(torch.bfloat16)
+    y = lin(x)
+    _give_up(lin, x)
+    word = K.device_status(x.device)
+    assert word.item() == L.TIMEOUT
+    word.zero_()
+    assert torch.equal(lin(x), y)
+    _give_up(lin, x)
+    with pytest.raises(L.I8LError):   # the next one is
+        lin(x)
+    K.check_status(DEV)
+
+
+def test_a_timeout_waits_until_a_capture_is_over():
+    lin = _layer({}).requires_grad_(False)
+    x = torch.randn(128, 256, device=DEV).to(torch.bfloat16)
+    ref = lin(x)
+    _give_up(lin, x)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = lin(x)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, ref)
+    with pytest.raises(L.I8LError) as e:
+        lin(x)
+    assert e.value.code == L.TIMEOUT
+    assert torch.equal(lin(x), ref)
+    K.check_status(DEV)
+
+
 def test_threads_with_streams_of_their_own():
     lin = _layer(dict(hadamard=128))
     xs = [torch.randn(256, 256, device=DEV).to(torch.bfloat16) for _ in range(4)]

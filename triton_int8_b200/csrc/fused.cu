@@ -348,7 +348,10 @@ fused_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   __syncthreads();
   if (threadIdx.x == 0 && ctl.abort_flag && p.status) {
     atomicExch(p.status, I8L_ERR_TIMEOUT);
-    if (p.mirror) *static_cast<volatile int32_t*>(p.mirror) = I8L_ERR_TIMEOUT;
+    if (p.mirror) {
+      __threadfence_system();   // who sees the mirror finds the word set
+      *static_cast<volatile int32_t*>(p.mirror) = I8L_ERR_TIMEOUT;
+    }
   }
   if (warp == 1) {
     tc_fence_after();

@@ -1003,7 +1003,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (TWO) cluster_sync_all();  // no remote arrival or tensor-memory write of the pair is still pending
   if (threadIdx.x == 0 && ctl.abort_flag && p.status) {
     atomicExch(p.status, I8L_ERR_TIMEOUT);
-    if (p.mirror) *static_cast<volatile int32_t*>(p.mirror) = I8L_ERR_TIMEOUT;
+    if (p.mirror) {
+      __threadfence_system();   // who sees the mirror finds the word set
+      *static_cast<volatile int32_t*>(p.mirror) = I8L_ERR_TIMEOUT;
+    }
   }
   if (warp == 1) {
     tc_fence_after();

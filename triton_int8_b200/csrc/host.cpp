@@ -35,6 +35,7 @@ decltype(&i8l_quant_gemm) lib_quant_gemm = nullptr;
 decltype(&i8l_linear_backward_bias) lib_linear_backward = nullptr;
 decltype(&i8l_status_peek) lib_status_peek = nullptr;
 PyObject* on_error = nullptr;       // (entry point, code, device index): raises
+PyObject* on_timeout = nullptr;     // (device index): raises, or returns where there is nothing to report now
 PyObject* open_status = nullptr;    // (device index) -> (status word, poller), as integers
 PyObject* py_backward = nullptr;    // the Python path of the backward pass
 
@@ -91,6 +92,14 @@ void check(const char* name, int rc, int dev) {
   Py_XDECREF(r);
   if (!PyErr_Occurred()) PyErr_Format(PyExc_RuntimeError, "%s failed with code %d", name, rc);
   throw_python_error();
+}
+
+void report_timeout(int dev) {   // an earlier GEMM gave up a wait
+  if (lib_status_peek(status_of(dev).poller.load(std::memory_order_relaxed)) == I8L_OK) return;
+  const WithGil gil;
+  PyObject* r = PyObject_CallFunction(on_timeout, "i", dev);
+  if (!r) throw_python_error();
+  Py_DECREF(r);
 }
 
 // A dense bf16 CUDA tensor with its own memory and nothing that a dispatcher would have to see.
@@ -289,8 +298,7 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Tensor y;
   {
     const WithoutGil no_gil;
-    const int dev = x.get_device();
-    check("i8l_status_peek", lib_status_peek(status_of(dev).poller.load(std::memory_order_relaxed)), dev);   // an earlier GEMM gave up a wait
+    report_timeout(x.get_device());
     const bool grad = at::GradMode::is_enabled();
     if (grad && (x.requires_grad() || weight.requires_grad() || (bias && bias->requires_grad())))
       y = Int8LinearNode::apply(x, weight, bias, c.code(), weight.requires_grad());
@@ -334,18 +342,20 @@ PyObject* py_quant_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// setup(address of i8l_quant_gemm, of i8l_linear_backward_bias, of i8l_status_peek, on_error, open_status, py_backward)
+// setup(address of i8l_quant_gemm, of i8l_linear_backward_bias, of i8l_status_peek, on_error, on_timeout, open_status, py_backward)
 PyObject* py_setup(PyObject*, PyObject* args) {
   unsigned long long qg = 0, lb = 0, sp = 0;
-  PyObject *err = nullptr, *open = nullptr, *bwd = nullptr;
-  if (!PyArg_ParseTuple(args, "KKKOOO", &qg, &lb, &sp, &err, &open, &bwd)) return nullptr;
+  PyObject *err = nullptr, *timeout = nullptr, *open = nullptr, *bwd = nullptr;
+  if (!PyArg_ParseTuple(args, "KKKOOOO", &qg, &lb, &sp, &err, &timeout, &open, &bwd)) return nullptr;
   lib_quant_gemm = reinterpret_cast<decltype(lib_quant_gemm)>(qg);
   lib_linear_backward = reinterpret_cast<decltype(lib_linear_backward)>(lb);
   lib_status_peek = reinterpret_cast<decltype(lib_status_peek)>(sp);
   Py_INCREF(err);
+  Py_INCREF(timeout);
   Py_INCREF(open);
   Py_INCREF(bwd);
   on_error = err;
+  on_timeout = timeout;
   open_status = open;
   py_backward = bwd;
   Py_RETURN_NONE;

@@ -111,10 +111,19 @@ _host = None
 
 
 def _on_error(name: str, code: int, index: int) -> None:
-    dev = torch.device("cuda", index)
-    if name == "i8l_status_peek":
-        _raise_if_set(_status_of(dev), code)
     raise L.I8LError(code, L.load().i8l_last_error().decode())
+
+
+def _on_timeout(index: int) -> None:
+    """The mirror of a status word is set.  Nothing happens while the stream is being captured, as in poll_status: a later call
+    reports it.  A word that its owner has cleared since is not reported."""
+    st = _status_of(torch.device("cuda", index))
+    with torch.cuda.device(st.dev):
+        if torch.cuda.is_current_stream_capturing():
+            return
+    code = int(st.word.item())
+    _raise_if_set(st, code)
+    L.call("i8l_status_reset", st.poller)
 
 
 def _open_status(index: int):
@@ -139,7 +148,7 @@ def host():
             raise ImportError(f"triton_int8_b200/_host.so is missing or does not fit this torch: build it with "
                               f"`python -m triton_int8_b200.build` ({e})") from e
         mod.setup(L.address("i8l_quant_gemm"), L.address("i8l_linear_backward_bias"), L.address("i8l_status_peek"), _on_error,
-                  _open_status, _backward_in_python)
+                  _on_timeout, _open_status, _backward_in_python)
         _host = mod
     return _host
 
