@@ -42,8 +42,20 @@ def needs_build() -> bool:
     return _stale(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS)
 
 
+def host_abi() -> str:
+    """What _host.so is built against: a module for another torch or Python may load all the same and then misread their
+    objects."""
+    import sysconfig
+
+    import torch
+    return f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+
+
 def needs_host_build() -> bool:
-    return _stale(HOST_PATH, [HOST_SOURCE, ABI_HEADER])
+    if _stale(HOST_PATH, [HOST_SOURCE, ABI_HEADER]):
+        return True
+    with open(HOST_PATH, "rb") as f:
+        return host_abi().encode() + b"\0" not in f.read()
 
 
 def _host_command() -> list:
@@ -55,7 +67,7 @@ def _host_command() -> list:
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), cuda,
                sysconfig.get_paths()["include"]]
     return [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in include),
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DI8L_HOST_ABI="{host_abi()}"', *(f"-isystem{i}" for i in include),
             "-o", HOST_PATH, HOST_SOURCE, f"-L{os.path.join(root, 'lib')}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
             "-lc10_cuda"]
 

@@ -370,4 +370,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "abi", I8L_HOST_ABI)) Py_CLEAR(m);   // see host_abi in build.py
+  return m;
+}

@@ -144,6 +144,9 @@ def host():
         L.load()
         try:
             from . import _host as mod
+            from .build import host_abi
+            if mod.abi != host_abi():
+                raise ImportError(f"built for {mod.abi}, this is {host_abi()}")
         except ImportError as e:
             raise ImportError(f"triton_int8_b200/_host.so is missing or does not fit this torch: build it with "
                               f"`python -m triton_int8_b200.build` ({e})") from e
