@@ -93,7 +93,8 @@ I8L_API int i8l_quant_row(const void* x, int64_t rows, int64_t cols, int qmode, 
 /*
  * Quantise the transpose of x (bf16 [rows, cols]) with one scale per column of x: the operand is
  * x^T [cols, rows], contraction axis = rows.  qt int8 [cols, rows], scale_t fp32 [cols].
- * colmax_scratch: fp32 [cols] device scratch, overwritten.  hadamard: NONE only.
+ * colmax_scratch: fp32 [cols] device scratch, overwritten where rows > 4096 (shorter columns are kept on chip; it must not be
+ * NULL all the same).  hadamard: NONE only.
  * No counterpart function in the reference: it is triton_per_token_quant applied to W^T, which a
  * linear layer's dX = dY W needs (the reference would transpose on the host first).
  */
@@ -121,9 +122,10 @@ I8L_API int i8l_quant_col_t_rot(const void* x, int64_t rows, int64_t cols, int q
  *   - The first call on each device resolves the array's device address (a synchronous runtime
  *     query made with that device current); make that first call before any stream capture.
  *   - Nothing is allocated or freed, by this function or by anything it calls.
- *   - All calls on a device share the one array; it is re-zeroed on the given stream at the start
- *     of every call, so back-to-back calls on one stream are safe, but two calls whose kernels
- *     may overlap on the GPU (different streams) race on it and give wrong scales.
+ *   - All calls on a device with rows > 4096 share the one array; it is re-zeroed on the given stream at
+ *     the start of each, so back-to-back calls on one stream are safe, but two of them whose kernels
+ *     may overlap on the GPU (different streams) race on it and give wrong scales.  Calls with
+ *     rows <= 4096 do not touch it; the limit on cols holds for them too.
  */
 #define I8L_STATIC_SCRATCH_MAX_COLS 65536
 I8L_API int i8l_quant_col_t_static(const void* x, int64_t rows, int64_t cols, int qmode, int8_t* qt,
