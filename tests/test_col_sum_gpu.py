@@ -20,7 +20,9 @@ def test_col_sum(rows, cols):
     x[3, 77] = float("inf")
     x[4, 78] = float("nan")
     got, ref = K.col_sum(x), x.double().sum(0)
-    assert torch.equal(got, K.col_sum(x)) or got.isnan().any()
+    for _ in range(3):   # the order depends on the shape only
+        torch.cuda._sleep(10_000)
+        assert torch.equal(got.view(torch.int16), K.col_sum(x).view(torch.int16))
     fin = ref.isfinite()
     assert torch.equal(got.double()[~fin].isnan(), ref[~fin].isnan()) and got[77] == float("inf")
     # one rounding to bf16, behind fp32 sums of at most 128 values and their 3 levels

@@ -63,6 +63,38 @@ def test_calls_in_a_row_equal_separate_steps(shape, scaling, rnd, had):
             assert torch.equal(got, ref), f"call {k}: {name}"
 
 
+@pytest.mark.parametrize("scaling,rnd,had", [("tile128", "half_up", 0), ("tile128", "half_up", 128), ("row128", "rne", 0),
+                                             ("double_channel", "half_up", 0)])
+@pytest.mark.parametrize("shape", [(256, 4352, 256), (4224, 4352, 256), (1920, 640, 1408)])   # N, then M too, above 4096: maxima in memory
+def test_training_steps_in_a_row_equal_separate_steps(shape, scaling, rnd, had):
+    """With the bias gradient in the chain (from 1024 rows on several CTAs share its columns) and column maxima that are
+    cleared in it."""
+    from triton_int8_b200 import kernels as K
+    from triton_int8_b200.linear import Int8Linear
+    cfg = Int8Config(scaling=scaling, round=rnd, hadamard=had)
+    M, N, Kd = shape
+    ins = _inputs(shape, 3)
+    lin = Int8Linear(Kd, N, device=DEV, config=cfg)
+    refs = []
+    for x, w, dy, bias in ins:
+        refs.append([t.clone() for t in (*_separate(x, w, dy, bias, cfg), K.col_sum(dy))])
+        torch.cuda.synchronize()
+
+    def step(x, w, dy, bias):
+        with torch.no_grad():
+            lin.weight.copy_(w)
+            lin.bias.copy_(bias)
+        x = x.detach().requires_grad_(True)
+        y = lin(x)
+        return [y.detach(), *torch.autograd.grad(y, (x, lin.weight, lin.bias), dy)]
+
+    outs = [step(*ins[k % 3]) for k in range(12)]   # nothing waits in between
+    torch.cuda.synchronize()
+    for k, out in enumerate(outs):
+        for name, got, ref in zip(("y", "dx", "dw", "db"), out, refs[k % 3]):
+            assert torch.equal(got, ref), f"call {k}: {name}"
+
+
 def test_chain_in_a_graph_equals_separate_steps():
     cfg = Int8Config(hadamard=128)
     ins = _inputs((1920, 640, 1408), 3)
