@@ -1189,7 +1189,8 @@ static int launch_pair(const PairArgs& a, const PairArgs& b, cudaStream_t st) {
 // Both operands of a product in one launch.  1: done, 0: not a pair that this takes, < 0: an error.  It pays where a call is
 // bound by its launches: M, N, K 128, 1024, 1024 forward 15.5 -> 13.0 us, 512, 1024, 1024 11.3 -> 9.4, 1024, 2048, 1024
 // 11.4 -> 10.3 a call; 1024, 1024, 2048 12.0 -> 11.8; 2048, 2048, 1024 12.7 -> 12.9; 1024, 1024, 3072 14.8 -> 15.2; 2048,
-// 1536, 2048 16.7 -> 17.3.  The line lies at 1.5 M elements.
+// 1536, 2048 16.7 -> 17.3.  The line lies at 1.5 M elements of either operand, which is on the safe side: of these shapes it leaves
+// the two launches to 1024, 2048, 1024 too.  A line on the sum of both has not been measured at few tokens and wide weights.
 int quant_pair(const void* a, int64_t a_batch, int64_t a_rows, int a_gran, int8_t* aq, float* as, int8_t* aqt, float* ast, const void* b,
                int64_t b_batch, int64_t b_rows, int b_gran, int8_t* bq, float* bs, int64_t cols, int qmode, int hadamard,
                cudaStream_t st) {
